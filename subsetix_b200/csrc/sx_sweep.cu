@@ -11,12 +11,12 @@
 // in_k(x)), where f is the expression as a boolean function.  MODE_TABLE
 // computes exactly that from a truth table of f.
 //
-// MODE_UNION merges widened intervals ([b - w, e + w)) from k row-shifted
+// Union mode merges widened intervals ([b - w, e + w)) from k row-shifted
 // views of one set.  A run continues while the next begin is <= the running
 // end.  This is the merge of subsetix_cupy/kernels.py:292-381 after the
 // (row, begin) sort of morphology.py:21-107, which dilation uses
-// (morphology.py:211-248).  It needs non-empty intervals with strictly
-// increasing begins and ends inside each row.
+// (morphology.py:211-248).  It needs non-empty intervals with non-decreasing
+// begins and ends inside each row (sx_union_kernel).
 //
 // Layout of the work.  One lane owns one row of the aligned row list, and a
 // warp owns a tile of 32 consecutive rows.  A lane sweeps its row as a k-way
@@ -49,8 +49,6 @@
 
 #define SX_SWEEP_WARPS 8
 #define SX_GROUP 32
-
-enum { MODE_TABLE = 0, MODE_UNION = 1 };
 
 // Look-back state in the workspace: counters[4] | tile status[tiles] |
 // group status[groups] | group sum[groups] | group count[groups].
@@ -221,97 +219,7 @@ __device__ __forceinline__ int sx_sweep_table(const SxBoolArgs& A, const int* s,
 // by `widen` ([b - w, e + w)), or coarsened by `scale` ([floor(b/r), ceil(e/r))).
 __device__ __forceinline__ int sx_floordiv(int a, int r) { return a >= 0 ? a / r : -((-a + r - 1) / r); }
 
-__device__ __forceinline__ int sx_tb(const SxLeafDev& L, int i)
-{
-    const int b = __ldg(L.begin + i);
-    return L.scale > 1 ? sx_floordiv(b, L.scale) : b - L.widen;
-}
-
-__device__ __forceinline__ int sx_te(const SxLeafDev& L, int i)
-{
-    const int e = __ldg(L.end + i);
-    return L.scale > 1 ? -sx_floordiv(-e, L.scale) : e + L.widen;
-}
-
-// One row, K views of interval sets (row-shifted, widened or coarsened):
-// their union with the reference's merge semantics (touching runs join).
-// Begins and ends of a view must each be non-decreasing; every event at a
-// coordinate is applied before the run state is examined.
-template <int K, bool WRITE>
-__device__ __forceinline__ int sx_sweep_union(const SxBoolArgs& A, const int* s, const int* cnt, int* out_b, int* out_e,
-                                              long long pos, bool& bad, bool& over)
-{
-    int qb[K], qe[K], hb[K], he[K];
-    int rem = 0;
-#pragma unroll
-    for (int l = 0; l < K; ++l) {
-        qb[l] = 0;
-        qe[l] = 0;
-        hb[l] = cnt[l] > 0 ? sx_tb(A.leaf[l], s[l]) : INT_MAX;
-        he[l] = cnt[l] > 0 ? sx_te(A.leaf[l], s[l]) : INT_MAX;
-        rem += 2 * cnt[l];
-    }
-    int active = 0;
-    int run_start = 0;
-    int n = 0;
-    while (rem > 0) {
-        int c = INT_MAX;
-#pragma unroll
-        for (int l = 0; l < K; ++l) {
-            if (qb[l] < cnt[l]) c = min(c, hb[l]);
-            if (qe[l] < cnt[l]) c = min(c, he[l]);
-        }
-        const bool was = active > 0;
-#pragma unroll
-        for (int l = 0; l < K; ++l) {
-            // ends before begins: an element whose begin has not been taken at
-            // an earlier coordinate is empty (or reversed) and breaks the contract
-            while (qe[l] < cnt[l] && he[l] == c) {
-                --active;
-                --rem;
-                if (qe[l] >= qb[l]) bad = true;
-                const int qn = ++qe[l];
-                if (qn < cnt[l]) {
-                    const int v = sx_te(A.leaf[l], s[l] + qn);
-                    if (v < c) bad = true;
-                    he[l] = v;
-                }
-            }
-            while (qb[l] < cnt[l] && hb[l] == c) {
-                ++active;
-                --rem;
-                const int qn = ++qb[l];
-                if (qn < cnt[l]) {
-                    const int v = sx_tb(A.leaf[l], s[l] + qn);
-                    if (v < c) bad = true;
-                    hb[l] = v;
-                }
-            }
-        }
-        const bool now = active > 0;
-        if (now != was) {
-            if (now) {
-                run_start = c;
-            } else {
-                if (WRITE) {
-                    const long long o = pos + n;
-                    if (o < A.capacity) {
-                        out_b[o] = run_start;
-                        out_e[o] = c;
-                    } else {
-                        over = true;
-                    }
-                }
-                ++n;
-            }
-        }
-        if (active < 0) bad = true;
-        if (c == INT_MAX) break;
-    }
-    return n;
-}
-
-template <int K, int MODE>
+template <int K>
 __global__ void __launch_bounds__(32 * SX_SWEEP_WARPS) sx_sweep_kernel(SxBoolArgs A, SxSweepState st, int tiles)
 {
     const int lane = threadIdx.x & 31;
@@ -328,16 +236,13 @@ __global__ void __launch_bounds__(32 * SX_SWEEP_WARPS) sx_sweep_kernel(SxBoolArg
 #pragma unroll
     for (int l = 0; l < K; ++l) {
         const int a = active ? A.leaf[l].off[row] : 0;
-        const int b = active ? (A.leaf[l].off_end ? A.leaf[l].off_end[row] : A.leaf[l].off[row + 1]) : 0;
+        const int b = active ? A.leaf[l].off[row + 1] : 0;
         s[l] = a;
-        lim[l] = MODE == MODE_TABLE ? 2 * (b - a) : (b - a);
+        lim[l] = 2 * (b - a);
     }
     bool bad = false, over = false;
     int count = 0;
-    if (active) {
-        count = MODE == MODE_TABLE ? sx_sweep_table<K, false>(A, s, lim, nullptr, nullptr, 0, bad, over)
-                                   : sx_sweep_union<K, false>(A, s, lim, nullptr, nullptr, 0, bad, over);
-    }
+    if (active) count = sx_sweep_table<K, false>(A, s, lim, nullptr, nullptr, 0, bad, over);
     int incl = count;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -351,10 +256,7 @@ __global__ void __launch_bounds__(32 * SX_SWEEP_WARPS) sx_sweep_kernel(SxBoolArg
         const long long pos = (long long)base + incl - count;
         if (count > 0) {
             bool bad2 = false;
-            if (MODE == MODE_TABLE)
-                sx_sweep_table<K, true>(A, s, lim, A.out_begin, A.out_end, pos, bad2, over);
-            else
-                sx_sweep_union<K, true>(A, s, lim, A.out_begin, A.out_end, pos, bad2, over);
+            sx_sweep_table<K, true>(A, s, lim, A.out_begin, A.out_end, pos, bad2, over);
         }
         A.out_off[row + 1] = base + incl;
         if (row == 0) A.out_off[0] = 0;
@@ -2676,6 +2578,285 @@ __global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepSt
     sxs_report(A, tile, tiles, base, total, flags);
 }
 
+// ---------------------------------------------------------------------------
+// Union sweep: sx_union_kernel<K> (SX_MODE_UNION: dilation, restriction,
+// compaction).
+//
+// K row-shifted views of interval sets, each interval widened or coarsened,
+// merged per output row with the reference's rule (a run continues while the
+// next begin is <= the running end).  Begins and ends of a view must each be
+// non-decreasing in a row and transformed intervals non-empty; anything else
+// raises SXF_CONTRACT.
+//
+// A warp owns a tile of 32 / LPR output rows and LPR lanes sweep each row
+// (LPR a power of two up to 32).  What bounds such a sweep is the serial walk
+// along a row, not bytes, so a row is cut into LPR pieces as soon as whole
+// rows do not fill the chip (sx_union_shape): piece i takes the intervals
+// whose begin lies in [p_i, p_{i+1}), the pivots being begins of the row's
+// longest view, starts in every view at the first begin not below p_i (a
+// binary search) and knows the run it continues from the end just before that
+// position (ends do not decrease).  Walking intervals instead of boundaries
+// halves the steps.  A run's end is written by the piece that opens the next
+// run, the last one by the row's last piece, so pieces need only the rank of
+// their first start, from one warp scan and the look-back.
+//
+// All views of one set read the same arrays, and the rows under a tile are
+// contiguous in them, so the tile's intervals are staged once in shared
+// memory (two bulk copies) however many views there are.  Tiles above the
+// slice, and leaves with different arrays or transforms, run the same code on
+// global memory.  Every interval is swept twice (count, then write): keeping
+// provisional runs would take K times the staged size.
+//
+// Measured figures and the choice of LPR: sx_union_shape.
+// ---------------------------------------------------------------------------
+#define SXU_WARPS 4
+#define SXU_HDR_WORDS 4
+
+__host__ __device__ inline int sxu_slice_words(int cap) { return SXU_HDR_WORDS + 2 * ((cap + 11) & ~3); }
+
+__device__ __forceinline__ int sxu_tb(int b, int widen, int scale)
+{
+    if (scale <= 1) return b - widen;
+    return (scale & (scale - 1)) == 0 ? b >> (31 - __clz(scale)) : sx_floordiv(b, scale);
+}
+
+__device__ __forceinline__ int sxu_te(int e, int widen, int scale)
+{
+    if (scale <= 1) return e + widen;
+    return (scale & (scale - 1)) == 0 ? -((-e) >> (31 - __clz(scale))) : -sx_floordiv(-e, scale);
+}
+
+// Begin and end of element i of view l: staged and transformed (SM), or from global memory.
+template <bool SM>
+__device__ __forceinline__ int sxu_b(const SxBoolArgs& A, const int* SB, int l, int i)
+{
+    return SM ? SB[i] : sxu_tb(__ldg(A.leaf[l].begin + i), A.leaf[l].widen, A.leaf[l].scale);
+}
+
+template <bool SM>
+__device__ __forceinline__ int sxu_e(const SxBoolArgs& A, const int* SE, int l, int i)
+{
+    return SM ? SE[i] : sxu_te(__ldg(A.leaf[l].end + i), A.leaf[l].widen, A.leaf[l].scale);
+}
+
+// One piece: elements [p0, ...) of every view with begins below khi.  Returns
+// the runs that start in it; pos comes back at the first elements not taken,
+// ce as the running end and open as whether the row has a run so far.  With
+// WRITE the starts go to ranks rank, rank + 1, ...
+template <int K, bool SM, bool WRITE>
+__device__ __forceinline__ int sxu_sweep(const SxBoolArgs& A, const int* SB, const int* SE, const int (&p0)[K],
+                                         const int (&lo)[K], const int (&hi)[K], int khi, long long rank, int (&pos)[K],
+                                         int& ce, bool& open, bool& bad)
+{
+    int h[K], el[K];
+    open = false;
+    ce = INT_MIN;
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        pos[l] = p0[l];
+        h[l] = pos[l] < hi[l] ? sxu_b<SM>(A, SB, l, pos[l]) : INT_MAX;
+        el[l] = INT_MIN;
+        if (pos[l] > lo[l]) {
+            el[l] = sxu_e<SM>(A, SE, l, pos[l] - 1);
+            ce = max(ce, el[l]);
+            open = true;
+        }
+    }
+    int n = 0;
+    while (true) {
+        int c = h[0];
+#pragma unroll
+        for (int l = 1; l < K; ++l) c = min(c, h[l]);
+        if (c >= khi) break;
+        if (!open || c > ce) {
+            if (WRITE) {
+                const long long o = rank + n;
+                if (o < A.capacity) {
+                    A.out_begin[o] = c;
+                    if (open) A.out_end[o - 1] = ce;
+                }
+            }
+            ++n;
+            open = true;
+        }
+#pragma unroll
+        for (int l = 0; l < K; ++l) {
+            if (h[l] == c) {
+                const int e = sxu_e<SM>(A, SE, l, pos[l]);
+                if (e <= c || e < el[l]) bad = true;
+                el[l] = e;
+                ce = max(ce, e);
+                const int q = ++pos[l];
+                h[l] = q < hi[l] ? sxu_b<SM>(A, SB, l, q) : INT_MAX;
+                if (h[l] < c) bad = true;
+            }
+        }
+    }
+    return n;
+}
+
+// First element of view l in [lo, hi) whose begin is not below v.
+template <bool SM>
+__device__ __forceinline__ int sxu_lower(const SxBoolArgs& A, const int* SB, int l, int lo, int hi, int v)
+{
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if (sxu_b<SM>(A, SB, l, mid) < v) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// Pivots and start positions of a lane's piece.
+template <int K, bool SM>
+__device__ __forceinline__ void sxu_start(const SxBoolArgs& A, const int* SB, const int (&lo)[K], const int (&hi)[K],
+                                          int piece, int lg, int (&p0)[K], int& khi)
+{
+    khi = INT_MAX;
+#pragma unroll
+    for (int l = 0; l < K; ++l) p0[l] = lo[l];
+    if (lg == 0) return;
+    int m = 0, big_lo = 0, big = 0;
+#pragma unroll
+    for (int l = 0; l < K; ++l)
+        if (hi[l] - lo[l] > m) {
+            m = hi[l] - lo[l];
+            big_lo = lo[l];
+            big = l;
+        }
+    if (m == 0) return;
+    if (piece + 1 < (1 << lg)) khi = sxu_b<SM>(A, SB, big, big_lo + (int)(((long long)(piece + 1) * m) >> lg));
+    if (piece > 0) {
+        const int klo = sxu_b<SM>(A, SB, big, big_lo + (int)(((long long)piece * m) >> lg));
+#pragma unroll
+        for (int l = 0; l < K; ++l) p0[l] = sxu_lower<SM>(A, SB, l, lo[l], hi[l], klo);
+    }
+}
+
+template <int K>
+__global__ void __launch_bounds__(32 * SXU_WARPS) sx_union_kernel(SxBoolArgs A, SxSweepState st, int tiles, int lg,
+                                                                  int cap, int shared)
+{
+    extern __shared__ __align__(16) int sxu_smem[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (blockIdx.x * SXU_WARPS + wid >= tiles) return;  // exactly `tiles` warps take tickets
+    int* const slice = sxu_smem + wid * sxu_slice_words(cap);
+    unsigned long long* bar = (unsigned long long*)slice;
+    int* const raw = slice + SXU_HDR_WORDS;
+
+    int tile = 0;
+    if (lane == 0) {
+        tile = (int)atomicAdd(&st.counters[0], 1u);
+        sxs_bar_init(bar);
+    }
+    tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
+    const int TR = 32 >> lg;
+    const int r0 = tile * TR;
+    const int row = lane >> lg, piece = lane & ((1 << lg) - 1);
+    const int y = r0 + row;
+    const bool act = y < A.rows;
+    bool bad = false;
+    int lo[K], hi[K];
+    int gs = INT_MAX, ge = INT_MIN;
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        const int a = act ? A.leaf[l].off[y] : 0;
+        const int b = act ? (A.leaf[l].off_end ? A.leaf[l].off_end[y] : A.leaf[l].off[y + 1]) : 0;
+        if (b < a) bad = true;  // row ranges must not run backwards
+        lo[l] = a;
+        hi[l] = b > a ? b : a;
+        if (b > a) {
+            gs = min(gs, a);
+            ge = max(ge, b);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        gs = min(gs, __shfl_xor_sync(0xFFFFFFFFu, gs, o));
+        ge = max(ge, __shfl_xor_sync(0xFFFFFFFFu, ge, o));
+    }
+    const int ns = gs < ge ? ge - gs : 0;
+    bool staged = shared && ns > 0 && ns <= cap;
+    unsigned flags = 0u;
+    const int *SB = raw, *SE = raw;
+    if (staged) {
+        const int* gb = A.leaf[0].begin + gs;
+        const int* gq = A.leaf[0].end + gs;
+        const uintptr_t b0 = (uintptr_t)gb & ~(uintptr_t)15, e0 = (uintptr_t)gq & ~(uintptr_t)15;
+        const unsigned nb = (unsigned)((((uintptr_t)(gb + ns) + 15) & ~(uintptr_t)15) - b0);
+        const unsigned ne = (unsigned)((((uintptr_t)(gq + ns) + 15) & ~(uintptr_t)15) - e0);
+        int* const second = raw + ((ns + 11) & ~3);  // at most ns + 6 copied words
+        SB = raw + (((uintptr_t)gb & 15) >> 2);
+        SE = second + (((uintptr_t)gq & 15) >> 2);
+        if (lane == 0) {
+            sxs_bar_expect(bar, nb + ne);
+            sxs_bulk_copy(raw, (const void*)b0, nb, bar);
+            sxs_bulk_copy(second, (const void*)e0, ne, bar);
+        }
+        __syncwarp();
+        if (!__all_sync(0xFFFFFFFFu, sxs_bar_wait(bar))) {
+            flags |= SXF_TIMEOUT;
+            staged = false;
+        }
+    }
+    if (staged) {
+        const int widen = A.leaf[0].widen, scale = A.leaf[0].scale;
+        if (widen != 0 || scale > 1) {
+            int *wb = (int*)SB, *we = (int*)SE;
+            for (int j = lane; j < ns; j += 32) {
+                wb[j] = sxu_tb(wb[j], widen, scale);
+                we[j] = sxu_te(we[j], widen, scale);
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int l = 0; l < K; ++l) {
+            const bool some = lo[l] < hi[l];
+            lo[l] = some ? lo[l] - gs : 0;
+            hi[l] = some ? hi[l] - gs : 0;
+        }
+    }
+    int p0[K], pos[K], khi, ce, n;
+    bool open;
+    if (staged) {
+        sxu_start<K, true>(A, SB, lo, hi, piece, lg, p0, khi);
+        n = sxu_sweep<K, true, false>(A, SB, SE, p0, lo, hi, khi, 0, pos, ce, open, bad);
+    } else {
+        sxu_start<K, false>(A, SB, lo, hi, piece, lg, p0, khi);
+        n = sxu_sweep<K, false, false>(A, SB, SE, p0, lo, hi, khi, 0, pos, ce, open, bad);
+    }
+    // consecutive pieces of a row meet, and the last one ends with the row: with
+    // the checks inside the pieces that makes every view's row non-decreasing
+    const bool last = piece == (1 << lg) - 1;
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        const int nxt = __shfl_down_sync(0xFFFFFFFFu, p0[l], 1);
+        if (pos[l] != (last ? hi[l] : nxt)) bad = true;
+    }
+    if (__any_sync(0xFFFFFFFFu, bad)) {
+        flags |= SXF_CONTRACT;
+        n = 0;  // pieces may overlap on such input: the tile writes nothing
+    }
+    const bool write = !(flags & SXF_CONTRACT);
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    const int base = sxs_lookback(A, st, tile, total, flags);
+    if (write) {
+        const long long rank = (long long)base + incl - n;
+        if (staged) sxu_sweep<K, true, true>(A, SB, SE, p0, lo, hi, khi, rank, pos, ce, open, bad);
+        else sxu_sweep<K, false, true>(A, SB, SE, p0, lo, hi, khi, rank, pos, ce, open, bad);
+        const long long end_at = (long long)base + incl - 1;  // the row's last run
+        if (last && open && end_at < A.capacity) A.out_end[end_at] = ce;
+    }
+    if (act && last) A.out_off[y + 1] = base + incl;
+    if (tile == 0 && lane == 0) A.out_off[0] = 0;
+    sxs_report(A, tile, tiles, base, total, flags);
+}
+
 size_t sx_sweep_state_bytes(long long tiles)
 {
     const long long groups = (tiles + SX_GROUP - 1) / SX_GROUP;
@@ -2702,7 +2883,7 @@ static SxSweepState sx_sweep_state(void* ws, long long tiles)
     return st;
 }
 
-template <int K, int MODE>
+template <int K>
 static cudaError_t sx_sweep_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, cudaStream_t stream)
 {
     // Residency cap through unused dynamic shared memory.  Fewer resident
@@ -2714,14 +2895,14 @@ static cudaError_t sx_sweep_launch_k(const SxBoolArgs& A, const SxSweepState& st
         if (pad < 0) pad = 0;
         static int configured = 0;
         if (pad > configured) {
-            cudaError_t err = cudaFuncSetAttribute(sx_sweep_kernel<K, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaError_t err = cudaFuncSetAttribute(sx_sweep_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    pad);
             if (err != cudaSuccess) return err;
             configured = pad;
         }
     }
     const int blocks = (tiles + SX_SWEEP_WARPS - 1) / SX_SWEEP_WARPS;
-    sx_sweep_kernel<K, MODE><<<blocks, 32 * SX_SWEEP_WARPS, pad, stream>>>(A, st, tiles);
+    sx_sweep_kernel<K><<<blocks, 32 * SX_SWEEP_WARPS, pad, stream>>>(A, st, tiles);
     return cudaGetLastError();
 }
 
@@ -2845,6 +3026,47 @@ static cudaError_t sx_rlane16_launch_k(const SxBoolArgs& A, const SxSweepState& 
     return sx_rlane16_launch_kl<K, 1>(A, st, tiles, cap_words, warps, stream);
 }
 
+// Union sweep shape: log2 of the lanes per row.  More lanes while whole rows
+// give fewer than about 700 lanes per SM and a piece keeps two intervals of a
+// view.  Measured per launch (B200, 1, 2, 4, 8, 16, 32 lanes per row): 3 views
+// of 32,768 rows with 34 intervals 26 (2 lanes), 21.9, 28.3, 40.8, 67 us, one
+// lane per row over global memory 257 us; 7 views of 3001 such rows 66, 41,
+// 27, 20, 17.7, 18.8 us against 630 us; 2 sub-rows of 8192 rows with 4
+// intervals 8.8, 7.7, 7.6, 8.2, 10, 13 us against 35 us.
+static int sx_union_shape(const SxBoolArgs& A, size_t workspace_bytes)
+{
+    const long long per_row = A.capacity / ((long long)A.k * A.rows);  // intervals of one view in a row
+    int lg = 0;
+    while (lg < 5 && ((long long)A.rows << lg) < 148 * 700 && (per_row >> (lg + 1)) >= 2) ++lg;
+    while (lg > 0 && sx_sweep_state_bytes((((long long)A.rows << lg) + 31) / 32) > workspace_bytes) --lg;
+    return lg;
+}
+
+template <int K>
+static cudaError_t sx_union_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int lg,
+                                     cudaStream_t stream)
+{
+    int shared = 1;
+    for (int l = 1; l < K; ++l)
+        shared = shared && A.leaf[l].begin == A.leaf[0].begin && A.leaf[l].end == A.leaf[0].end &&
+                 A.leaf[l].widen == A.leaf[0].widen && A.leaf[l].scale == A.leaf[0].scale;
+    // staged intervals per tile: 1.5 times the mean of the source rows under it
+    const long long tr = 32 >> lg;
+    const long long src_rows = A.leaf[0].scale > 1 ? tr * K : tr + K - 1;
+    long long cap = (3 * (A.capacity / K + 1) / A.rows + 1) * src_rows / 2 + 32;
+    if (cap > 6000) cap = 6000;
+    static int configured = 0;  // largest dynamic shared memory set for this instantiation
+    const int bytes = SXU_WARPS * sxu_slice_words((int)cap) * (int)sizeof(int);
+    if (bytes > configured) {
+        cudaError_t err = cudaFuncSetAttribute(sx_union_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (err != cudaSuccess) return err;
+        configured = bytes;
+    }
+    const int blocks = (tiles + SXU_WARPS - 1) / SXU_WARPS;
+    sx_union_kernel<K><<<blocks, 32 * SXU_WARPS, bytes, stream>>>(A, st, tiles, lg, (int)cap, shared);
+    return cudaGetLastError();
+}
+
 // Segmented sweep shape: `keys` boundaries per tile (0: 1.25x the average
 // plus slack), stored twice (lists and output area), at most 200 KiB per
 // block; `warps` per block (0: about 48 boundaries per thread).
@@ -2892,7 +3114,11 @@ cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspac
     // The segmented sweep takes tiles of 16 rows when the workspace holds
     // their look-back state (smaller tiles keep more blocks resident), else 32.
     const bool seg = !union_mode && (A.tune_kernel == 0 || A.tune_kernel >= 4);
-    int tr = 32;
+    int tr = 32, lg = 0;
+    if (union_mode) {
+        lg = sx_union_shape(A, workspace_bytes);
+        tr = 32 >> lg;
+    }
     if (seg) {
         tr = A.tune_tile_rows > 0 ? A.tune_tile_rows : (A.tune_kernel == 4 ? 32 : 8);
         if (A.tune_kernel == 6 && tr > 8) tr = 8;  // 16-bit keys hold 3 row bits
@@ -2908,15 +3134,15 @@ cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspac
     const int t = (int)tiles;
     if (union_mode) {
         switch (A.k) {
-            case 1: return sx_sweep_launch_k<1, MODE_UNION>(A, st, t, stream);
-            case 2: return sx_sweep_launch_k<2, MODE_UNION>(A, st, t, stream);
-            case 3: return sx_sweep_launch_k<3, MODE_UNION>(A, st, t, stream);
-            case 4: return sx_sweep_launch_k<4, MODE_UNION>(A, st, t, stream);
-            case 5: return sx_sweep_launch_k<5, MODE_UNION>(A, st, t, stream);
-            case 6: return sx_sweep_launch_k<6, MODE_UNION>(A, st, t, stream);
-            case 7: return sx_sweep_launch_k<7, MODE_UNION>(A, st, t, stream);
-            case 8: return sx_sweep_launch_k<8, MODE_UNION>(A, st, t, stream);
-            case 9: return sx_sweep_launch_k<9, MODE_UNION>(A, st, t, stream);
+            case 1: return sx_union_launch_k<1>(A, st, t, lg, stream);
+            case 2: return sx_union_launch_k<2>(A, st, t, lg, stream);
+            case 3: return sx_union_launch_k<3>(A, st, t, lg, stream);
+            case 4: return sx_union_launch_k<4>(A, st, t, lg, stream);
+            case 5: return sx_union_launch_k<5>(A, st, t, lg, stream);
+            case 6: return sx_union_launch_k<6>(A, st, t, lg, stream);
+            case 7: return sx_union_launch_k<7>(A, st, t, lg, stream);
+            case 8: return sx_union_launch_k<8>(A, st, t, lg, stream);
+            case 9: return sx_union_launch_k<9>(A, st, t, lg, stream);
             default: return cudaErrorInvalidValue;
         }
     }
@@ -3035,14 +3261,14 @@ cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspac
     if (B.tune_kernel == 1) {
         const SxBoolArgs& A = B;
         switch (A.k) {
-            case 1: return sx_sweep_launch_k<1, MODE_TABLE>(A, st, t, stream);
-            case 2: return sx_sweep_launch_k<2, MODE_TABLE>(A, st, t, stream);
-            case 3: return sx_sweep_launch_k<3, MODE_TABLE>(A, st, t, stream);
-            case 4: return sx_sweep_launch_k<4, MODE_TABLE>(A, st, t, stream);
-            case 5: return sx_sweep_launch_k<5, MODE_TABLE>(A, st, t, stream);
-            case 6: return sx_sweep_launch_k<6, MODE_TABLE>(A, st, t, stream);
-            case 7: return sx_sweep_launch_k<7, MODE_TABLE>(A, st, t, stream);
-            case 8: return sx_sweep_launch_k<8, MODE_TABLE>(A, st, t, stream);
+            case 1: return sx_sweep_launch_k<1>(A, st, t, stream);
+            case 2: return sx_sweep_launch_k<2>(A, st, t, stream);
+            case 3: return sx_sweep_launch_k<3>(A, st, t, stream);
+            case 4: return sx_sweep_launch_k<4>(A, st, t, stream);
+            case 5: return sx_sweep_launch_k<5>(A, st, t, stream);
+            case 6: return sx_sweep_launch_k<6>(A, st, t, stream);
+            case 7: return sx_sweep_launch_k<7>(A, st, t, stream);
+            case 8: return sx_sweep_launch_k<8>(A, st, t, stream);
             default: return cudaErrorInvalidValue;
         }
     }
