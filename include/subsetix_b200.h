@@ -436,6 +436,44 @@ int sx_upwind_adjoint_chunked(int dtype, const int32_t* row_offsets, const int32
                               double dt, double dx, double dy, double* grad_velocity, void* scratch,
                               size_t scratch_bytes, void* stream);
 
+/* Flat form of sx_upwind and its adjoint, for geometry whose rows are sorted
+ * and disjoint (as for sx_upwind_chunked) and whose cells all lie in the
+ * domain; same values.  The plan holds, per group of four consecutive values,
+ * where the neighbours sit (sx_flat.cu describes the arrays):
+ *   below, above   int32 per group, ceil(cells / 4) entries each
+ *   flags          uint16 per group
+ *   side           8 * n ints, 16-byte aligned: the irregular groups' indices
+ * sx_upwind_flat_plan fills them for cell_offsets that are the prefix sum of
+ * the interval lengths (cells = cell_offsets[n]) and writes span[2] (device) =
+ * {smallest begin, largest end}: the plan serves steps whose width covers
+ * them (0 <= span[0], span[1] <= width); rows must lie in [0, height).
+ * sx_upwind_flat_bands: cells band_cell[q] .. band_cell[q + 1] - 1 take band
+ * q's row of the band table (sx_upwind_band_table); band_cell[0] = 0.
+ * sx_upwind_flat_adjoint: as sx_upwind_adjoint; with accumulate the velocity
+ * gradient is added to grad_velocity.  scratch:
+ * sx_upwind_flat_adjoint_scratch_bytes(cells) bytes, zero before its first use,
+ * not shared by calls that may overlap. */
+typedef struct sx_flat_plan {
+    const int32_t* below;
+    const int32_t* above;
+    const uint16_t* flags;
+    const int32_t* side;
+    int64_t n;
+    int64_t cells;
+} sx_flat_plan;
+int sx_upwind_flat_plan(const int32_t* rows, const int32_t* row_offsets, int32_t row_count, const int32_t* begin,
+                        const int32_t* end, const int32_t* cell_offsets, int64_t n, int64_t cells,
+                        const int32_t* lookup, int32_t height, int32_t* below, int32_t* above, uint16_t* flags,
+                        int32_t* side, int32_t* span, void* stream);
+int sx_upwind_flat(int dtype, const sx_flat_plan* plan, const void* values, void* out, double a, double b, double dt,
+                   double dx, double dy, void* stream);
+int sx_upwind_flat_bands(int dtype, const sx_flat_plan* plan, const void* values, void* out, double a, double b,
+                         const int32_t* band_cell, const void* band_table, int32_t nbands, void* stream);
+size_t sx_upwind_flat_adjoint_scratch_bytes(int64_t cells);
+int sx_upwind_flat_adjoint(int dtype, const sx_flat_plan* plan, const void* grad_out, const void* values,
+                           void* grad_in, double a, double b, double dt, double dx, double dy, double* grad_velocity,
+                           int accumulate, void* scratch, size_t scratch_bytes, void* stream);
+
 /* Threshold run-length encoding of a full width x height float32 grid
  * (subsetix_amr2/regrid.py:20-124 K11/K12, and regrid.py:172-223 K14 when
  * gradient = 1): a run is a stretch of value >= threshold, where value is

@@ -462,6 +462,50 @@ def upwind_chunked(offsets, begin, end, cell_offs, chunk_info, chunks: int, look
                                      stream_handle(device)), "sx_upwind_chunked")
 
 
+class FlatPlan:
+    """Plan of sx_upwind_flat for sorted, disjoint rows and packed values, with the columns it spans (one read-back)."""
+
+    __slots__ = ("cells", "lo", "hi", "_keep", "_struct", "_ref")
+
+    def __init__(self, rows, offsets, begin, end, cell_offs, cells: int, lookup, height: int, device):
+        lib = _lib.load()
+        n, cells = int(begin.numel()), int(cells)
+        groups = (cells + 3) // 4
+        below, above = empty_i32(groups, device), empty_i32(groups, device)
+        flags = torch.empty(groups, dtype=torch.int16, device=device)
+        side = empty_i32(8 * n, device)
+        span = empty_i32(2, device)
+        _lib.check(lib.sx_upwind_flat_plan(ptr(rows), ptr(offsets), int(rows.numel()), ptr(begin), ptr(end),
+                                           ptr(cell_offs), n, cells, ptr(lookup), int(height), ptr(below), ptr(above),
+                                           ptr(flags), ptr(side), ptr(span), stream_handle(device)),
+                   "sx_upwind_flat_plan")
+        self.cells = cells
+        self.lo, self.hi = span.tolist()
+        self._keep = (below, above, flags, side)
+        self._struct = _lib.SxFlatPlan(ptr(below), ptr(above), ptr(flags), ptr(side), n, cells)
+        self._ref = ctypes.byref(self._struct)
+
+    def covers(self, width: int) -> bool:
+        """Whether every cell lies in columns [0, width)."""
+        return self.cells > 0 and self.lo >= 0 and self.hi <= int(width)
+
+    def step(self, values, out, a, b, dt, dx, dy, device) -> None:
+        _lib.check(_lib.load().sx_upwind_flat(_dtype_code(values), self._ref, ptr(values), ptr(out), float(a), float(b),
+                                              float(dt), float(dx), float(dy), stream_handle(device)), "sx_upwind_flat")
+
+    def step_bands(self, values, out, a, b, band_cell, band_table, bands: int, device) -> None:
+        _lib.check(_lib.load().sx_upwind_flat_bands(_dtype_code(values), self._ref, ptr(values), ptr(out), float(a),
+                                                    float(b), ptr(band_cell), ptr(band_table), int(bands),
+                                                    stream_handle(device)), "sx_upwind_flat_bands")
+
+    def adjoint(self, w, u, out, a, b, dt, dx, dy, grad, scratch, device) -> None:
+        """``out`` = the transposed step of ``w``; the velocity gradient is added to ``grad``."""
+        _lib.check(_lib.load().sx_upwind_flat_adjoint(_dtype_code(w), self._ref, ptr(w), ptr(u), ptr(out), float(a),
+                                                      float(b), float(dt), float(dx), float(dy), ptr(grad), 1,
+                                                      ptr(scratch), int(scratch.numel()), stream_handle(device)),
+                   "sx_upwind_flat_adjoint")
+
+
 def threshold_rle(values, width: int, height: int, threshold: float, gradient: bool, device):
     """Runs of value >= threshold per row of a full grid.  Returns ``(begin, end, offsets)`` (synchronising)."""
     lib = _lib.load()

@@ -49,6 +49,11 @@ class SxRowList(ctypes.Structure):
                 ("skip_empty", ctypes.c_int32), ("div", ctypes.c_int32), ("phase", ctypes.c_int32)]
 
 
+class SxFlatPlan(ctypes.Structure):
+    _fields_ = [("below", c_vp), ("above", c_vp), ("flags", c_vp), ("side", c_vp), ("n", ctypes.c_int64),
+                ("cells", ctypes.c_int64)]
+
+
 # name -> (restype, argtypes)
 _SIGNATURES = {
     "sx_abi_version": (ctypes.c_int, []),
@@ -124,6 +129,16 @@ _SIGNATURES = {
                                                  c_vp, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_double,
                                                  ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                                  c_vp, c_vp, ctypes.c_size_t, c_vp]),
+    "sx_upwind_flat_plan": (ctypes.c_int, [c_vp, c_vp, ctypes.c_int32, c_vp, c_vp, c_vp, ctypes.c_int64, ctypes.c_int64,
+                                           c_vp, ctypes.c_int32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "sx_upwind_flat": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(SxFlatPlan), c_vp, c_vp, ctypes.c_double,
+                                      ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double, c_vp]),
+    "sx_upwind_flat_bands": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(SxFlatPlan), c_vp, c_vp, ctypes.c_double,
+                                            ctypes.c_double, c_vp, c_vp, ctypes.c_int32, c_vp]),
+    "sx_upwind_flat_adjoint_scratch_bytes": (ctypes.c_size_t, [ctypes.c_int64]),
+    "sx_upwind_flat_adjoint": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(SxFlatPlan), c_vp, c_vp, c_vp,
+                                              ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,
+                                              ctypes.c_double, c_vp, ctypes.c_int, c_vp, ctypes.c_size_t, c_vp]),
     "sx_threshold_rle": (ctypes.c_int, [c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_float, ctypes.c_int, c_vp,
                                         c_vp, c_vp, c_vp, c_vp]),
     "sx_gradient_magnitude": (ctypes.c_int, [c_vp, ctypes.c_int32, ctypes.c_int32, c_vp, c_vp]),

@@ -60,18 +60,56 @@ class Level:
         if bad:
             raise ValueError("interval_set rows exceed provided height")
         self.direct = not (_core.check_rows(self.begin, self.end, self.off, device) & _ROWS_UNSAFE)
-        self.chunk_off, self.chunks = (_core.upwind_plan(self.rows, self.off, self.begin, self.end, self.cell_off,
-                                                         self.lookup, self.height, device) if self.direct else (None, 0))
-        self.table = (_core.upwind_table(self.begin, self.end, self.cell_off, self.chunk_off, self.chunks, self.cells,
-                                         device) if self.direct else None)
         self.device = device
+        self._chunk_off, self._chunks, self._table = None, 0, None
+        self._chunked = False
+        self.flat = (_core.FlatPlan(self.rows, self.off, self.begin, self.end, self.cell_off, self.cells, self.lookup,
+                                    self.height, device) if self.direct else None)
+        if self.flat is not None and not self.flat.covers(self.width):
+            self.flat = None  # cells outside the domain: the chunk plan's kernels test every column
+            self._chunk_plan()  # built here, so that steps can be captured
         lib = _lib.load()
         nbytes = max(int(lib.sx_upwind_adjoint_scratch_bytes(self.cells)),
-                     int(lib.sx_upwind_adjoint_chunked_scratch_bytes(self.chunks)))
+                     int(lib.sx_upwind_adjoint_chunked_scratch_bytes((1 << 31) - 1)))
         self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        # the flat adjoint's block counter must start at zero (every launch leaves it so)
+        self.flat_scratch = torch.zeros(int(lib.sx_upwind_flat_adjoint_scratch_bytes(self.cells)), dtype=torch.uint8,
+                                        device=device)
+
+    def _chunk_plan(self) -> None:
+        if not self._chunked and self.direct:
+            self._chunk_off, self._chunks = _core.upwind_plan(self.rows, self.off, self.begin, self.end, self.cell_off,
+                                                              self.lookup, self.height, self.device)
+            self._table = _core.upwind_table(self.begin, self.end, self.cell_off, self._chunk_off, self._chunks,
+                                             self.cells, self.device)
+        self._chunked = True
+
+    @property
+    def chunk_off(self) -> Optional[torch.Tensor]:
+        """Chunk plan (built on first use; None when the rows are not sorted and disjoint)."""
+        self._chunk_plan()
+        return self._chunk_off
+
+    @property
+    def chunks(self) -> int:
+        self._chunk_plan()
+        return self._chunks
+
+    @property
+    def table(self) -> Optional[torch.Tensor]:
+        """Neighbour table of the chunk plan; None makes the chunked kernels search the neighbour rows."""
+        self._chunk_plan()
+        return self._table
+
+    @table.setter
+    def table(self, value: Optional[torch.Tensor]) -> None:
+        self._chunk_plan()
+        self._table = value
 
     def step(self, u: torch.Tensor, out: torch.Tensor, a: float, b: float, dt: float) -> torch.Tensor:
-        if self.chunk_off is not None:
+        if self.flat is not None:
+            self.flat.step(u, out, a, b, dt, self.dx, self.dy, self.device)
+        elif self.chunk_off is not None:
             _core.upwind_chunked(self.off, self.begin, self.end, self.cell_off, self.chunk_off, self.chunks,
                                  self.lookup, u, out, self.width, self.height, a, b, dt, self.dx, self.dy, self.device,
                                  table=self.table)
@@ -85,6 +123,9 @@ class Level:
         """dL/du for one step, and dL/d(a, b) added into ``grad_ab`` (float64 device pair)."""
         lib = _lib.load()
         ubar = torch.empty_like(w)
+        if self.flat is not None:
+            self.flat.adjoint(w, u, ubar, a, b, dt, self.dx, self.dy, grad_ab, self.flat_scratch, self.device)
+            return ubar
         g = torch.empty(2, dtype=torch.float64, device=self.device)
         code = _lib.SX_F64 if w.dtype == torch.float64 else _lib.SX_F32
         if self.chunk_off is not None:

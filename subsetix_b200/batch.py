@@ -8,7 +8,7 @@ operation for every set at once.  The upwind step reads rows ``y - 1`` and
 ``y + 1``, which are empty between bands, so the zero-exterior update of each
 set is unchanged as long as every set lies inside its own domain
 ``[0, width_i) x [0, height_i)``; each band carries its own spacing and time
-step (``sx_upwind_chunked_bands``), so set ``i`` gets exactly the values of
+step (``sx_upwind_flat_bands``), so set ``i`` gets exactly the values of
 its own ``step_upwind_interval`` call with ``dx = dy = 1 / side_i``.
 
 :class:`BatchStep` runs the union and intersection of two batches and one
@@ -16,7 +16,7 @@ upwind step of the first batch's field as three launches on fixed buffers
 with no host synchronisation, so the whole step can be captured in one CUDA
 graph and replayed; the three launches stay separate kernels because the two
 sweeps write data-dependent output sizes through a look-back over their own
-tiles, while the stencil walks a fixed chunk plan of different geometry.
+tiles, while the stencil walks a fixed plan of different geometry.
 
 This is the batching the reference lacks: there every set is one Python
 call with its own launches and host synchronisations.
@@ -42,16 +42,21 @@ _ROWS_UNSAFE = _lib.ROWS_UNSORTED_BEGIN | _lib.ROWS_OVERLAP | _lib.ROWS_EMPTY
 
 @dataclass
 class _StencilPlan:
-    """Per-batch data of the banded stencil, built once: cell offsets, row lookup, chunk plan, row bands."""
+    """Per-batch data of the banded stencil, built once: cell offsets, row lookup and the flat plan.
+
+    ``band_cell`` (first value of each band) is None when some row lies in no
+    band; such batches, and steps whose width does not cover every cell, take
+    the chunk plan (:meth:`SetBatch.chunk_plan`), which leaves rows without a
+    band unwritten and tests every column against the width.
+    """
 
     cell_off: torch.Tensor
     cells: int
     lookup: torch.Tensor
     height: int
-    chunk_off: Optional[torch.Tensor]
-    chunks: int
-    row_band: torch.Tensor
-    table: Optional[torch.Tensor] = None
+    direct: bool
+    flat: Optional[_core.FlatPlan]
+    band_cell: Optional[torch.Tensor]
 
 
 @dataclass
@@ -66,6 +71,7 @@ class SetBatch:
     bases: List[int]
     heights: List[int]
     _plan: Optional[_StencilPlan] = field(default=None, repr=False, compare=False)
+    _chunks: Optional[tuple] = field(default=None, repr=False, compare=False)
     _tables: dict = field(default_factory=dict, repr=False, compare=False)
 
     @classmethod
@@ -118,7 +124,7 @@ class SetBatch:
 
     # -- the stencil's fixed data ---------------------------------------------------------------------------------
     def stencil_plan(self) -> _StencilPlan:
-        """Cell offsets, row lookup, chunk plan and row bands of the combined set (built on first use)."""
+        """Cell offsets, row lookup and flat plan of the combined set (built on first use)."""
         if self._plan is None:
             s = self.combined
             dev = _t(s.row_offsets).device
@@ -129,13 +135,33 @@ class SetBatch:
             if bad:
                 raise ValueError("batch rows outside the band layout")
             direct = not (_core.check_rows(b, e, off, dev) & _ROWS_UNSAFE)
-            chunk_off, chunks = (_core.upwind_plan(rows, off, b, e, cell_off, lookup, H, dev) if direct else (None, 0))
-            table = _core.upwind_table(b, e, cell_off, chunk_off, chunks, cells, dev) if direct else None
-            band = torch.full((H,), -1, dtype=I32, device=dev)
+            flat, band_cell = None, None
+            if direct and self.bases:
+                flat = _core.FlatPlan(rows, off, b, e, cell_off, cells, lookup, H, dev)
+                # first value of the rows from each band's base on, and of the rows after its last one
+                edges = torch.tensor(self.bases + [x + h for x, h in zip(self.bases, self.heights)], dtype=I32,
+                                     device=dev)
+                at = cell_off[off[torch.searchsorted(rows, edges).long()].long()]
+                first, last = at[:len(self.bases)], at[len(self.bases):]
+                ends = torch.cat([first[1:], cell_off[-1:]])
+                if bool((first[0] == 0) & torch.equal(last, ends)):
+                    band_cell = torch.cat([first, cell_off[-1:]]).contiguous()
+            self._plan = _StencilPlan(cell_off, cells, lookup, H, direct, flat, band_cell)
+        return self._plan
+
+    def chunk_plan(self) -> tuple:
+        """``(chunk info, chunks, neighbour table, row bands)`` of the chunked stencil (built on first use)."""
+        if self._chunks is None:
+            plan, s = self.stencil_plan(), self.combined
+            b, e, off, rows = _t(s.begin), _t(s.end), _t(s.row_offsets), _t(s.rows)
+            dev = off.device
+            info, chunks = _core.upwind_plan(rows, off, b, e, plan.cell_off, plan.lookup, plan.height, dev)
+            table = _core.upwind_table(b, e, plan.cell_off, info, chunks, plan.cells, dev)
+            band = torch.full((plan.height,), -1, dtype=I32, device=dev)
             for i, (base, h) in enumerate(zip(self.bases, self.heights)):
                 band[base:base + h] = i
-            self._plan = _StencilPlan(cell_off, cells, lookup, H, chunk_off, chunks, band, table)
-        return self._plan
+            self._chunks = (info, chunks, table, band)
+        return self._chunks
 
     def band_table(self, dtype: torch.dtype, spacing: Sequence[Tuple[float, float, float]]) -> torch.Tensor:
         """Device table of per-band (dx, dy, dt) in the kernel's form for ``dtype`` (cached per spacing)."""
@@ -187,7 +213,7 @@ def batched_upwind(batch: SetBatch, values: torch.Tensor, *, width, a: float, b:
     if int(vals.numel()) != plan.cells:
         raise ValueError(f"the batch has {plan.cells} cells, got {int(vals.numel())} values")
     res = torch.empty_like(vals) if out is None else _t(out)
-    if plan.chunk_off is None:
+    if not plan.direct:
         if len(set(zip(dts, dxs, dys))) != 1:
             raise ValueError("per-set spacing needs sorted, disjoint, non-empty intervals in every row")
         field = IntervalField(interval_set=batch.combined, values=vals, interval_cell_offsets=plan.cell_off)
@@ -200,15 +226,19 @@ def batched_upwind(batch: SetBatch, values: torch.Tensor, *, width, a: float, b:
 
 def _upwind_bands(batch: SetBatch, plan: _StencilPlan, table: torch.Tensor, vals: torch.Tensor, out: torch.Tensor,
                   width: int, a: float, b: float) -> None:
+    dev = vals.device
+    if plan.band_cell is not None and plan.flat.covers(width):
+        plan.flat.step_bands(vals, out, a, b, plan.band_cell, table, len(batch.bases), dev)
+        return
     s = batch.combined
+    info, chunks, nbr, row_band = batch.chunk_plan()
     lib = _lib.load()
     code = _lib.SX_F64 if vals.dtype == torch.float64 else _lib.SX_F32
     _lib.check(lib.sx_upwind_chunked_bands(code, ptr(_t(s.row_offsets)), ptr(_t(s.begin)), ptr(_t(s.end)),
-                                           ptr(plan.cell_off), ptr(plan.chunk_off), int(plan.chunks),
-                                           ptr(plan.lookup), ptr(plan.table), ptr(vals), ptr(out), int(width),
-                                           int(plan.height),
-                                           float(a), float(b), ptr(plan.row_band), ptr(table), len(batch.bases),
-                                           stream_handle(vals.device)), "sx_upwind_chunked_bands")
+                                           ptr(plan.cell_off), ptr(info), int(chunks), ptr(plan.lookup), ptr(nbr),
+                                           ptr(vals), ptr(out), int(width), int(plan.height), float(a), float(b),
+                                           ptr(row_band), ptr(table), len(batch.bases), stream_handle(dev)),
+               "sx_upwind_chunked_bands")
 
 
 class BatchStep:
@@ -235,8 +265,10 @@ class BatchStep:
         self.width = int(max(_per_set(width, n, "width")))
         self.values = _t(values)
         self.plan = A.stencil_plan()
-        if self.plan.chunk_off is None:
+        if not self.plan.direct:
             raise ValueError("BatchStep needs sorted, disjoint, non-empty intervals in every row")
+        if self.plan.band_cell is None or not self.plan.flat.covers(self.width):
+            A.chunk_plan()  # built here, so that the step can be captured
         self.table = A.band_table(self.values.dtype, list(zip(_per_set(dx, n, "dx"), _per_set(dy, n, "dy"),
                                                                _per_set(dt, n, "dt"))))
         self.out = torch.empty_like(self.values)

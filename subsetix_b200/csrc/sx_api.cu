@@ -617,6 +617,95 @@ int sx_upwind_f64(const int32_t* rows, const int32_t* row_offsets, int32_t row_c
                      width, height, a, b, dt, dx, dy, direct, stream);
 }
 
+// Device view of a plan, or an error code after checking it.
+static int flat_plan(const sx_flat_plan* plan, const char* what, SxFlatPlan* P)
+{
+    if (!plan || plan->n < 0 || plan->n > INT32_MAX || plan->cells < 0 || plan->cells > INT32_MAX)
+        return fail(SX_ERR_INVALID, "%s: bad plan", what);
+    if (plan->cells > 0 && (!plan->below || !plan->above || !plan->flags || !plan->side))
+        return fail(SX_ERR_INVALID, "%s: null plan array", what);
+    if (((uintptr_t)plan->side & 15u) != 0) return fail(SX_ERR_INVALID, "%s: side must be 16-byte aligned", what);
+    P->dn = plan->below;
+    P->up = plan->above;
+    P->bits = plan->flags;
+    P->side_dn = (const int4*)plan->side;
+    P->side_up = P->side_dn + plan->n;
+    P->cells = plan->cells;
+    return SX_OK;
+}
+
+int sx_upwind_flat_plan(const int32_t* rows, const int32_t* row_offsets, int32_t row_count, const int32_t* begin,
+                        const int32_t* end, const int32_t* cell_offsets, int64_t n, int64_t cells,
+                        const int32_t* lookup, int32_t height, int32_t* below, int32_t* above, uint16_t* flags,
+                        int32_t* side, int32_t* span, void* stream)
+{
+    if (row_count < 0 || n < 0 || n > INT32_MAX || cells < 0 || cells > INT32_MAX || height <= 0)
+        return fail(SX_ERR_INVALID, "sx_upwind_flat_plan: bad size");
+    if (!span) return fail(SX_ERR_INVALID, "sx_upwind_flat_plan: null span");
+    if (cells > 0 && (!rows || !row_offsets || !begin || !end || !cell_offsets || !lookup || !below || !above ||
+                      !flags || !side || n == 0 || row_count == 0))
+        return fail(SX_ERR_INVALID, "sx_upwind_flat_plan: null argument");
+    if (((uintptr_t)side & 15u) != 0) return fail(SX_ERR_INVALID, "sx_upwind_flat_plan: side must be 16-byte aligned");
+    cudaError_t err = sx_flat_plan_launch(rows, row_offsets, row_count, begin, end, cell_offsets, (int)n, cells,
+                                          lookup, height, below, above, flags, side, span, (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_upwind_flat_plan");
+    return SX_OK;
+}
+
+int sx_upwind_flat(int dtype, const sx_flat_plan* plan, const void* values, void* out, double a, double b, double dt,
+                   double dx, double dy, void* stream)
+{
+    SxFlatPlan P;
+    if (dtype != SX_F32 && dtype != SX_F64) return fail(SX_ERR_INVALID, "sx_upwind_flat: dtype %d", dtype);
+    if (int rc = flat_plan(plan, "sx_upwind_flat", &P)) return rc;
+    if (P.cells > 0 && (!values || !out)) return fail(SX_ERR_INVALID, "sx_upwind_flat: null argument");
+    if (P.cells > 0 && values == out) return fail(SX_ERR_INVALID, "sx_upwind_flat: out must not alias values");
+    cudaError_t err = sx_flat_step_launch(P, dtype == SX_F64, values, out, a, b, dt, dx, dy, (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_upwind_flat");
+    return SX_OK;
+}
+
+int sx_upwind_flat_bands(int dtype, const sx_flat_plan* plan, const void* values, void* out, double a, double b,
+                         const int32_t* band_cell, const void* band_table, int32_t nbands, void* stream)
+{
+    SxFlatPlan P;
+    if (dtype != SX_F32 && dtype != SX_F64) return fail(SX_ERR_INVALID, "sx_upwind_flat_bands: dtype %d", dtype);
+    if (int rc = flat_plan(plan, "sx_upwind_flat_bands", &P)) return rc;
+    if (nbands < 0) return fail(SX_ERR_INVALID, "sx_upwind_flat_bands: negative band count");
+    if (P.cells > 0 && (!values || !out || !band_cell || !band_table || nbands == 0))
+        return fail(SX_ERR_INVALID, "sx_upwind_flat_bands: null argument");
+    if (P.cells > 0 && values == out) return fail(SX_ERR_INVALID, "sx_upwind_flat_bands: out must not alias values");
+    cudaError_t err = sx_flat_step_bands_launch(P, dtype == SX_F64, values, out, a, b, band_cell, band_table, nbands,
+                                                (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_upwind_flat_bands");
+    return SX_OK;
+}
+
+size_t sx_upwind_flat_adjoint_scratch_bytes(int64_t cells)
+{
+    return 16 + (size_t)sx_flat_adjoint_parts(cells) * 2 * sizeof(double);
+}
+
+int sx_upwind_flat_adjoint(int dtype, const sx_flat_plan* plan, const void* grad_out, const void* values,
+                           void* grad_in, double a, double b, double dt, double dx, double dy, double* grad_velocity,
+                           int accumulate, void* scratch, size_t scratch_bytes, void* stream)
+{
+    SxFlatPlan P;
+    if (dtype != SX_F32 && dtype != SX_F64) return fail(SX_ERR_INVALID, "sx_upwind_flat_adjoint: dtype %d", dtype);
+    if (int rc = flat_plan(plan, "sx_upwind_flat_adjoint", &P)) return rc;
+    if (!grad_velocity || (P.cells > 0 && (!grad_out || !values || !grad_in)))
+        return fail(SX_ERR_INVALID, "sx_upwind_flat_adjoint: null argument");
+    if (P.cells > 0 && (grad_in == grad_out || grad_in == values))
+        return fail(SX_ERR_INVALID, "sx_upwind_flat_adjoint: grad_in must not alias its inputs");
+    if (!scratch || ((uintptr_t)scratch & 15u) != 0 || scratch_bytes < sx_upwind_flat_adjoint_scratch_bytes(P.cells))
+        return fail(SX_ERR_WORKSPACE, "sx_upwind_flat_adjoint: scratch needs %zu bytes, 16-byte aligned",
+                    sx_upwind_flat_adjoint_scratch_bytes(P.cells));
+    cudaError_t err = sx_flat_adjoint_launch(P, dtype == SX_F64, grad_out, values, grad_in, a, b, dt, dx, dy, scratch,
+                                             grad_velocity, accumulate, (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_upwind_flat_adjoint");
+    return SX_OK;
+}
+
 size_t sx_upwind_adjoint_scratch_bytes(int64_t cells)
 {
     return (size_t)sx_upwind_adjoint_parts(cells) * 2 * sizeof(double);

@@ -7,6 +7,7 @@
 // * A block-wide exclusive scan.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -186,3 +187,49 @@ __device__ __forceinline__ float sx_grad_norm(float gx, float gy)
     return __fsqrt_rn(__fmaf_rn(gx, gx, __fmul_rn(gy, gy)));
 }
 
+// ---------------------------------------------------------------------------
+// Arithmetic helpers without contraction (float and double)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float sx_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sx_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float sx_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float sx_div(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ float sx_sqrt(float a) { return __fsqrt_rn(a); }
+__device__ __forceinline__ double sx_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sx_sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double sx_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double sx_div(double a, double b) { return __ddiv_rn(a, b); }
+
+// x / d, or x * d when the launcher passed the reciprocal of a power-of-two
+// spacing instead (pow2 != 0): dividing by 2^k and multiplying by 2^-k have
+// the same exact real result, so the rounded results are identical.
+template <typename T>
+__device__ __forceinline__ T sx_over(T x, T d, int pow2)
+{
+    return pow2 ? sx_mul(x, d) : sx_div(x, d);
+}
+
+// Spacings that are powers of two (in the kernel's precision) become their
+// exact reciprocals.
+template <typename T>
+inline int sx_pow2_pair(T& dx, T& dy)
+{
+    int ex, ey;
+    if (!(frexp((double)dx, &ex) == 0.5 && frexp((double)dy, &ey) == 0.5)) return 0;
+    const T ix = (T)1 / dx, iy = (T)1 / dy;
+    if (!std::isfinite((double)ix) || !std::isfinite((double)iy)) return 0;  // reciprocal out of range
+    dx = ix;
+    dy = iy;
+    return 1;
+}
+
+// Row ordinal of interval i: the last p with off[p] <= i and off[p+1] > i.
+__device__ __forceinline__ int sx_row_of(const int* __restrict__ off, int rows, int i)
+{
+    int lo = 0, hi = rows - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (off[mid] <= i) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}

@@ -164,6 +164,26 @@ cudaError_t sx_upwind_adjoint_chunk_launch(const int* off, const int* b, const i
                                            const void* w, const void* u, void* ubar, int width, int height, double a,
                                            double bb, double dt, double dx, double dy, int dbl, double* partial,
                                            double* grads, cudaStream_t stream);
+// Flat stencil (sx_flat.cu)
+struct SxFlatPlan {
+    const int* dn;
+    const int* up;
+    const unsigned short* bits;
+    const int4* side_dn;
+    const int4* side_up;
+    long long cells;
+};
+int sx_flat_adjoint_parts(long long cells);
+cudaError_t sx_flat_plan_launch(const int* rows, const int* off, int row_count, const int* b, const int* e,
+                                const int* coff, int n, long long cells, const int* lookup, int height, int* dn,
+                                int* up, unsigned short* bits, void* side, int* span, cudaStream_t stream);
+cudaError_t sx_flat_step_launch(const SxFlatPlan& P, int dbl, const void* v, void* out, double a, double bb, double dt,
+                                double dx, double dy, cudaStream_t stream);
+cudaError_t sx_flat_step_bands_launch(const SxFlatPlan& P, int dbl, const void* v, void* out, double a, double bb,
+                                      const int* band_cell, const void* band_table, int nbands, cudaStream_t stream);
+cudaError_t sx_flat_adjoint_launch(const SxFlatPlan& P, int dbl, const void* w, const void* u, void* ubar, double a,
+                                   double bb, double dt, double dx, double dy, void* scratch, double* grads,
+                                   int accumulate, cudaStream_t stream);
 // Level coupling by index tables (sx_coupling.cu)
 cudaError_t sx_index_copy_launch(int dtype, long long n, const int* dst_idx, const int* src_idx, const void* src,
                                  void* dst, cudaStream_t stream);

@@ -2,11 +2,12 @@
 
 Arguments, checks and results follow ``subsetix_cupy/interval_stencil.py``
 of the reference.  On geometry whose rows are sorted and disjoint (the
-usual case, checked once per set) the chunked kernel ``sx_upwind_chunked``
-runs: warps take chunks of 128 cells of one interval in four coalesced
-sub-rounds, exchange left/right neighbours by shuffles and find the cells
-above and below through a per-cell neighbour table built with the plan.  Other geometry takes ``sx_upwind``, which assigns 256 consecutive
-cells to each block and searches every neighbour.  Both give the same
+usual case, checked once per set) and whose cells lie in the domain the flat
+kernel ``sx_upwind_flat`` runs: a thread updates four consecutive values and a
+plan built once per set says where their neighbours sit.  Cells outside the
+domain take the chunked kernel ``sx_upwind_chunked`` (warps take 128-cell
+chunks of one interval, with a per-cell neighbour table), other geometry
+``sx_upwind``, which searches every neighbour.  All three give the same
 values.  Float32 is the
 reference's arithmetic.  Float64 values run the same formula in double
 precision (an addition of this package).
@@ -34,24 +35,35 @@ class _Geometry:
     lookup (and its synchronising range check) once.
     """
 
-    __slots__ = ("height", "lookup", "direct", "chunk_off", "chunks", "cell_off", "table", "_seen")
+    __slots__ = ("height", "lookup", "direct", "cells", "cell_off", "flat", "_chunk", "_seen")
 
-    def __init__(self, height: int, lookup: torch.Tensor, direct: bool, chunk_off=None, chunks: int = 0,
-                 cell_off=None, table=None):
+    def __init__(self, height: int, lookup: torch.Tensor, direct: bool, cells: int = 0, cell_off=None, flat=None):
         self.height = height
         self.lookup = lookup
         self.direct = direct
-        self.chunk_off = chunk_off
-        self.chunks = chunks
+        self.cells = cells
         self.cell_off = cell_off
-        self.table = table
+        self.flat = flat
+        self._chunk = None
         self._seen = None
+
+    @property
+    def has_chunk_plan(self) -> bool:
+        return self._chunk is not None
+
+    def chunk_plan(self, rows, off, b, e, device):
+        """``(chunk info, chunks, neighbour table)`` of the chunked kernel, built on first use."""
+        if self._chunk is None:
+            info, chunks = _core.upwind_plan(rows, off, b, e, self.cell_off, self.lookup, self.height, device)
+            table = _core.upwind_table(b, e, self.cell_off, info, chunks, self.cells, device)
+            self._chunk = (info, chunks, table)
+        return self._chunk
 
     def canonical(self, cell_off: torch.Tensor) -> bool:
         """Whether ``cell_off`` is the prefix sum of the interval lengths.
 
-        The chunk plan holds value indices taken from that prefix sum, so the
-        chunked kernel serves only fields laid out that way.  The answer for
+        The plans hold value indices taken from that prefix sum, so the flat
+        and chunked kernels serve only fields laid out that way.  The answer for
         one offsets tensor is kept until the tensor is modified in place.
         """
         seen = self._seen
@@ -78,13 +90,12 @@ def _geometry(interval_set, height: int) -> _Geometry:
         raise ValueError("interval_set rows exceed provided height")
     flags = _core.check_rows(_t(interval_set.begin), _t(interval_set.end), _t(interval_set.row_offsets), device)
     direct = not (flags & (_lib.ROWS_UNSORTED_BEGIN | _lib.ROWS_OVERLAP | _lib.ROWS_EMPTY))
-    chunk_off, chunks, coff, table = (None, 0, None, None)
+    coff, cells, flat = None, 0, None
     if direct:
-        b, e = _t(interval_set.begin), _t(interval_set.end)
+        b, e, off = _t(interval_set.begin), _t(interval_set.end), _t(interval_set.row_offsets)
         coff, cells = _core.cell_offsets(b, e, device)
-        chunk_off, chunks = _core.upwind_plan(rows, _t(interval_set.row_offsets), b, e, coff, lookup, height, device)
-        table = _core.upwind_table(b, e, coff, chunk_off, chunks, cells, device)
-    geo = _Geometry(height, lookup, direct, chunk_off, chunks, coff, table)
+        flat = _core.FlatPlan(rows, off, b, e, coff, cells, lookup, height, device)
+    geo = _Geometry(height, lookup, direct, cells, coff, flat)
     try:
         object.__setattr__(interval_set, "_sx_stencil", geo)
     except Exception:  # pragma: no cover - sets that refuse attributes
@@ -137,11 +148,15 @@ def step_upwind_interval(field: IntervalField, *, width: int, height: int, a: fl
         if bool(((rid < 0) | (rid >= height)).any()) or int(geo.lookup[rid.long()].min().item()) < 0:
             raise ValueError("interval_set rows exceed provided height")
     vals = vals.contiguous()
-    if (geo.chunk_off is not None and rid is None and out_t.data_ptr() != vals.data_ptr()
-            and geo.canonical(cell_off)):
-        # fixed geometry with sorted, disjoint rows and packed values: the chunked kernel (same results)
-        _core.upwind_chunked(_t(s.row_offsets), begin, _t(s.end), cell_off, geo.chunk_off, geo.chunks, geo.lookup, vals,
-                             out_t, width, height, a, b, dt, dx, dy, device, table=geo.table)
+    plan = (geo.flat is not None and rid is None and out_t.data_ptr() != vals.data_ptr() and geo.canonical(cell_off)
+            and int(vals.numel()) >= geo.cells)
+    # fixed geometry with sorted, disjoint rows and packed values takes a plan (same results as the generic kernel)
+    if plan and geo.flat.covers(width):
+        geo.flat.step(vals, out_t, a, b, dt, dx, dy, device)
+    elif plan and (geo.has_chunk_plan or not torch.cuda.is_current_stream_capturing()):
+        info, chunks, table = geo.chunk_plan(_t(s.rows), _t(s.row_offsets), begin, _t(s.end), device)
+        _core.upwind_chunked(_t(s.row_offsets), begin, _t(s.end), cell_off, info, chunks, geo.lookup, vals, out_t,
+                             width, height, a, b, dt, dx, dy, device, table=table)
     else:
         _core.upwind(_t(s.rows), _t(s.row_offsets), begin, _t(s.end), cell_off, int(vals.numel()), geo.lookup, vals,
                      out_t, width, height, a, b, dt, dx, dy, geo.direct and rid is None, device, row_ids=rid)
