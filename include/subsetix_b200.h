@@ -537,6 +537,12 @@ int sx_cell_quads(int dtype, const int32_t* row_offsets, const int32_t* rows, in
  *   sx_index_block_mean_adj  the transpose: in_bar[in_idx[j*group+m]] +=
  *                            out_bar[out_idx[j]] * norm, then out_bar[out_idx[j]]
  *                            = 0; in_idx entries must be distinct;
+ *   sx_run_block_mean{,_adj} the same on runs of consecutive coarse cells (the
+ *                            children of consecutive cells are consecutive in
+ *                            each of the `ratio` sub-rows).  plan: `stride`
+ *                            ints per run (a multiple of 4, >= 2 + ratio):
+ *                            first coarse value, cells (1 to 64), first child
+ *                            of each sub-row;
  *   sx_index_segment_add     dst[dst_idx[s]] += sum over t in [seg_off[s],
  *                            seg_off[s+1]) of src[src_idx[t]], in order, and
  *                            src[src_idx[t]] = 0 when zero_src: the transpose
@@ -550,6 +556,10 @@ int sx_index_block_mean(int dtype, int64_t n, int32_t group, double norm, const 
                         const int32_t* in_idx, const void* in, void* out, void* stream);
 int sx_index_block_mean_adj(int dtype, int64_t n, int32_t group, double norm, const int32_t* out_idx,
                             const int32_t* in_idx, void* out_bar, void* in_bar, void* stream);
+int sx_run_block_mean(int dtype, int64_t runs, int32_t ratio, int32_t stride, double norm, const int32_t* plan,
+                      const void* fine, void* coarse, void* stream);
+int sx_run_block_mean_adj(int dtype, int64_t runs, int32_t ratio, int32_t stride, double norm, const int32_t* plan,
+                          void* coarse_bar, void* fine_bar, void* stream);
 int sx_index_segment_add(int dtype, int64_t nseg, const int32_t* seg_off, const int32_t* src_idx,
                          const int32_t* dst_idx, void* src, void* dst, int zero_src, void* stream);
 

@@ -160,6 +160,10 @@ _SIGNATURES = {
                                            c_vp, c_vp, c_vp]),
     "sx_index_block_mean_adj": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, ctypes.c_int32, ctypes.c_double, c_vp,
                                                c_vp, c_vp, c_vp, c_vp]),
+    "sx_run_block_mean": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_double,
+                                         c_vp, c_vp, c_vp, c_vp]),
+    "sx_run_block_mean_adj": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32,
+                                             ctypes.c_double, c_vp, c_vp, c_vp, c_vp]),
     "sx_index_segment_add": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_int,
                                             c_vp]),
     "sx_upwind_full": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,

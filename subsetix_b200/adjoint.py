@@ -15,10 +15,10 @@ states per level instead of ``steps``.
 takes its coarse parents' values (injection), every level is advanced on its
 cells plus that ring, and after the step the coarse cells under a finer level
 take the mean of their children (restriction, finest level first).  Each
-coupling is a gather or a block mean over index tables built once for the
-fixed geometry (``sx_index_copy``, ``sx_index_block_mean``); the backward
-pass applies their transposes (``sx_index_segment_add``,
-``sx_index_block_mean_adj``) around the adjoint upwind kernel, in reverse
+coupling is a gather over an index table or a block mean over runs of cells,
+built once for the fixed geometry (``sx_index_copy``, ``sx_run_block_mean``);
+the backward pass applies their transposes (``sx_index_segment_add``,
+``sx_run_block_mean_adj``) around the adjoint upwind kernel, in reverse
 order.
 
 There is no counterpart in the reference, which has no derivatives.
@@ -325,8 +325,25 @@ class Hierarchy:
             child = _positions(s, s_off, chy, chx)
             if bool((cpos < 0).any()) or bool((child < 0).any()):
                 raise ValueError(f"level {k}: a coarse cell under it does not have all its children in it")
-            child = inner[child.to(torch.int64)]
-            self.cover.append((cpos.contiguous(), child.contiguous()))
+            self.cover.append(self._cover_runs(covered, prev, lvl, r))
+
+    @staticmethod
+    def _cover_runs(covered: IntervalSet, prev: Level, lvl: Level, r: int) -> tuple:
+        """Plan of sx_run_block_mean: ``(runs, ints per run, plan)``, runs of up to 64 cells of one covered interval."""
+        b, e = _t(covered.begin).to(torch.int64), _t(covered.end).to(torch.int64)
+        y = _t(covered.interval_rows()).to(torch.int64)
+        per = (e - b + 63) // 64
+        which = torch.repeat_interleave(torch.arange(b.numel(), device=b.device), per)
+        nth = torch.arange(which.numel(), device=b.device) - (torch.cumsum(per, 0) - per)[which]
+        x, row = b[which] + 64 * nth, y[which]
+        stride = (2 + r + 3) // 4 * 4
+        plan = torch.zeros((which.numel(), stride), dtype=torch.int32, device=b.device)
+        plan[:, 0] = _positions(prev.interval_set, prev.cell_off, row.to(torch.int32), x.to(torch.int32))
+        plan[:, 1] = torch.clamp(e[which] - x, max=64)
+        for dy in range(r):
+            plan[:, 2 + dy] = _positions(lvl.interval_set, lvl.cell_off, (row * r + dy).to(torch.int32),
+                                         (x * r).to(torch.int32))
+        return int(plan.shape[0]), stride, plan
 
     # -- the coupled step and its transpose ------------------------------------------------------------------------
     def _fill_ghosts(self, u: List[torch.Tensor]) -> None:
@@ -338,12 +355,11 @@ class Hierarchy:
 
     def _restrict(self, u: List[torch.Tensor]) -> None:
         lib = _lib.load()
-        r2 = self.ratio * self.ratio
+        r = self.ratio
         for k in range(len(self.levels) - 1, 0, -1):
-            cpos, child = self.cover[k]
-            _lib.check(lib.sx_index_block_mean(_code(u[k]), int(cpos.numel()), r2, 1.0 / r2, ptr(cpos), ptr(child),
-                                               ptr(u[k]), ptr(u[k - 1]), stream_handle(u[k].device)),
-                       "sx_index_block_mean")
+            runs, stride, plan = self.cover[k]
+            _lib.check(lib.sx_run_block_mean(_code(u[k]), runs, r, stride, 1.0 / (r * r), ptr(plan), ptr(u[k]),
+                                             ptr(u[k - 1]), stream_handle(u[k].device)), "sx_run_block_mean")
 
     def step(self, u: List[torch.Tensor], a: float, b: float, dt: float) -> Tuple[List[torch.Tensor], List[torch.Tensor]]:
         """One coupled step of the extended-level fields ``u``; returns (new fields, upwind inputs)."""
@@ -356,12 +372,11 @@ class Hierarchy:
                      grad_ab: torch.Tensor) -> List[torch.Tensor]:
         """Transpose of :meth:`step` applied to ``w`` (modified); ``inputs`` are that step's upwind inputs."""
         lib = _lib.load()
-        r2 = self.ratio * self.ratio
+        r = self.ratio
         for k in range(1, len(self.levels)):
-            cpos, child = self.cover[k]
-            _lib.check(lib.sx_index_block_mean_adj(_code(w[k]), int(cpos.numel()), r2, 1.0 / r2, ptr(cpos),
-                                                   ptr(child), ptr(w[k - 1]), ptr(w[k]), stream_handle(w[k].device)),
-                       "sx_index_block_mean_adj")
+            runs, stride, plan = self.cover[k]
+            _lib.check(lib.sx_run_block_mean_adj(_code(w[k]), runs, r, stride, 1.0 / (r * r), ptr(plan), ptr(w[k - 1]),
+                                                 ptr(w[k]), stream_handle(w[k].device)), "sx_run_block_mean_adj")
         w = [lvl.adjoint(x, u, a, b, dt, grad_ab) for lvl, x, u in zip(self.levels, w, inputs)]
         for k in range(len(self.levels) - 1, 0, -1):
             _, _, seg_off, src, dst = self.ghost[k]

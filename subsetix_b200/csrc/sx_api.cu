@@ -904,6 +904,34 @@ int sx_index_block_mean_adj(int dtype, int64_t n, int32_t group, double norm, co
     return err == cudaSuccess ? SX_OK : cuda_fail(err, "sx_index_block_mean_adj");
 }
 
+static int run_check(const char* what, int dtype, int64_t runs, int32_t ratio, int32_t stride, const int32_t* plan,
+                     const void* fine, const void* coarse)
+{
+    if (int rc = coupling_check(what, dtype, runs)) return rc;
+    if (runs > INT32_MAX / 32 || ratio < 1 || stride < 2 + ratio || (stride & 3) != 0)
+        return fail(SX_ERR_INVALID, "%s: bad runs, ratio or stride", what);
+    if (runs > 0 && (!plan || !fine || !coarse)) return fail(SX_ERR_INVALID, "%s: null argument", what);
+    return SX_OK;
+}
+
+int sx_run_block_mean(int dtype, int64_t runs, int32_t ratio, int32_t stride, double norm, const int32_t* plan,
+                      const void* fine, void* coarse, void* stream)
+{
+    if (int rc = run_check("sx_run_block_mean", dtype, runs, ratio, stride, plan, fine, coarse)) return rc;
+    cudaError_t err = sx_run_block_mean_launch(dtype, 0, runs, ratio, stride, norm, plan, coarse, (void*)fine,
+                                               (cudaStream_t)stream);
+    return err == cudaSuccess ? SX_OK : cuda_fail(err, "sx_run_block_mean");
+}
+
+int sx_run_block_mean_adj(int dtype, int64_t runs, int32_t ratio, int32_t stride, double norm, const int32_t* plan,
+                          void* coarse_bar, void* fine_bar, void* stream)
+{
+    if (int rc = run_check("sx_run_block_mean_adj", dtype, runs, ratio, stride, plan, fine_bar, coarse_bar)) return rc;
+    cudaError_t err = sx_run_block_mean_launch(dtype, 1, runs, ratio, stride, norm, plan, coarse_bar, fine_bar,
+                                               (cudaStream_t)stream);
+    return err == cudaSuccess ? SX_OK : cuda_fail(err, "sx_run_block_mean_adj");
+}
+
 int sx_index_segment_add(int dtype, int64_t nseg, const int32_t* seg_off, const int32_t* src_idx,
                          const int32_t* dst_idx, void* src, void* dst, int zero_src, void* stream)
 {
