@@ -483,6 +483,15 @@ int sx_upwind_flat_adjoint(int dtype, const sx_flat_plan* plan, const void* grad
  * (exclusive scan of counts), out_begin/out_end written. */
 int sx_threshold_rle(const float* values, int32_t width, int32_t height, float threshold, int gradient, int32_t* counts,
                      const int32_t* offsets, int32_t* out_begin, int32_t* out_end, void* stream);
+/* The same in one pass over the values: sx_threshold_mask writes one bit per
+ * cell, mask[height][ceil(width / 32)], offsets[height + 1] (exclusive scan of
+ * the rows' run counts) and result = {runs, flags}; sx_mask_runs then stores
+ * the runs.  workspace: sx_threshold_mask_workspace_bytes(height). */
+size_t sx_threshold_mask_workspace_bytes(int32_t height);
+int sx_threshold_mask(const float* values, int32_t width, int32_t height, float threshold, int gradient, uint32_t* mask,
+                      int32_t* offsets, int32_t* result, void* workspace, size_t workspace_bytes, void* stream);
+int sx_mask_runs(const uint32_t* mask, int32_t width, int32_t height, const int32_t* offsets, int32_t* out_begin,
+                 int32_t* out_end, void* stream);
 /* Gradient magnitude of a full grid, same formula (regrid.py:172-274, K14). */
 int sx_gradient_magnitude(const float* values, int32_t width, int32_t height, float* out, void* stream);
 int sx_gradient_threshold_rle(const float* values, int32_t width, int32_t height, float threshold, int32_t* counts,

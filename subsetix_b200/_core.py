@@ -509,16 +509,21 @@ class FlatPlan:
 def threshold_rle(values, width: int, height: int, threshold: float, gradient: bool, device):
     """Runs of value >= threshold per row of a full grid.  Returns ``(begin, end, offsets)`` (synchronising)."""
     lib = _lib.load()
-    counts = empty_i32(height, device)
+    width, height = int(width), int(height)
+    mask = empty_i32(height * ((width + 31) // 32), device)
+    off = empty_i32(height + 1, device)
+    result = empty_i32(2, device)
     s = stream_handle(device)
-    _lib.check(lib.sx_threshold_rle(ptr(values), int(width), int(height), float(threshold), 1 if gradient else 0,
-                                    ptr(counts), None, None, None, s), "sx_threshold_rle(count)")
-    off, total = scan(counts, device)
+    wsp, wsn = workspace(device, lib.sx_threshold_mask_workspace_bytes(height))
+    _lib.check(lib.sx_threshold_mask(ptr(values), width, height, float(threshold), 1 if gradient else 0, ptr(mask),
+                                     ptr(off), ptr(result), wsp, wsn, s), "sx_threshold_mask")
+    total, flags = read_pair(result)
+    if flags & _lib.FLAG_TIMEOUT:
+        raise _lib.SubsetixError("sx_threshold_mask: look-back wait timed out")
     ob = empty_i32(total, device)
     oe = empty_i32(total, device)
     if total:
-        _lib.check(lib.sx_threshold_rle(ptr(values), int(width), int(height), float(threshold), 1 if gradient else 0,
-                                        None, ptr(off), ptr(ob), ptr(oe), s), "sx_threshold_rle(write)")
+        _lib.check(lib.sx_mask_runs(ptr(mask), width, height, ptr(off), ptr(ob), ptr(oe), s), "sx_mask_runs")
     return ob, oe, off
 
 

@@ -790,6 +790,33 @@ int sx_threshold_rle(const float* values, int32_t width, int32_t height, float t
     return SX_OK;
 }
 
+size_t sx_threshold_mask_workspace_bytes(int32_t height) { return scan_state_bytes(sx_mask_tiles(height < 1 ? 1 : height)); }
+
+int sx_threshold_mask(const float* values, int32_t width, int32_t height, float threshold, int gradient, uint32_t* mask,
+                      int32_t* offsets, int32_t* result, void* workspace, size_t workspace_bytes, void* stream)
+{
+    if (width <= 0 || height <= 0) return fail(SX_ERR_INVALID, "sx_threshold_mask: width and height must be positive");
+    if ((long long)width * height > INT32_MAX) return fail(SX_ERR_INVALID, "sx_threshold_mask: grid too large");
+    if (!values || !mask || !offsets || !result) return fail(SX_ERR_INVALID, "sx_threshold_mask: null argument");
+    const size_t need = sx_threshold_mask_workspace_bytes(height);
+    if (!workspace || workspace_bytes < need)
+        return fail(SX_ERR_WORKSPACE, "sx_threshold_mask: workspace needs %zu bytes, got %zu", need, workspace_bytes);
+    cudaError_t err = sx_mask_launch(values, width, height, threshold, gradient ? 1 : 0, mask, offsets, result,
+                                     scan_state(workspace, sx_mask_tiles(height)), (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_threshold_mask");
+    return SX_OK;
+}
+
+int sx_mask_runs(const uint32_t* mask, int32_t width, int32_t height, const int32_t* offsets, int32_t* out_begin,
+                 int32_t* out_end, void* stream)
+{
+    if (width <= 0 || height <= 0) return fail(SX_ERR_INVALID, "sx_mask_runs: width and height must be positive");
+    if (!mask || !offsets || !out_begin || !out_end) return fail(SX_ERR_INVALID, "sx_mask_runs: null argument");
+    cudaError_t err = sx_mask_runs_launch(mask, width, height, offsets, out_begin, out_end, (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_mask_runs");
+    return SX_OK;
+}
+
 int sx_gradient_magnitude(const float* values, int32_t width, int32_t height, float* out, void* stream)
 {
     if (width <= 0 || height <= 0) return fail(SX_ERR_INVALID, "sx_gradient_magnitude: width and height must be positive");

@@ -1455,38 +1455,6 @@ cudaError_t sx_gather_i32_launch(const int* idx, int count, const int* src, int*
 
 // Gradient magnitude of a full width x height grid into a float32 array
 // (regrid.py:172-274); the same per-cell formula as the fused RLE.
-__global__ void sx_gradient_kernel(const float* __restrict__ d, int width, int height, float* __restrict__ out)
-{
-    const long long cells = (long long)width * height;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < cells;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(idx / width), x = (int)(idx - (long long)y * width);
-        const float c = d[idx];
-        float gx = 0.0f, gy = 0.0f;
-        if (width > 1) {
-            if (x == 0) gx = __fsub_rn(d[idx + 1], c);
-            else if (x == width - 1) gx = __fsub_rn(c, d[idx - 1]);
-            else gx = __fmul_rn(__fsub_rn(d[idx + 1], d[idx - 1]), 0.5f);
-        }
-        if (height > 1) {
-            if (y == 0) gy = __fsub_rn(d[idx + width], c);
-            else if (y == height - 1) gy = __fsub_rn(c, d[idx - width]);
-            else gy = __fmul_rn(__fsub_rn(d[idx + width], d[idx - width]), 0.5f);
-        }
-        out[idx] = sx_grad_norm(gx, gy);
-    }
-}
-
-cudaError_t sx_gradient_launch(const float* d, int width, int height, float* out, cudaStream_t stream)
-{
-    const long long cells = (long long)width * height;
-    if (cells <= 0) return cudaSuccess;
-    long long g = (cells + 255) / 256;
-    if (g > 148 * 32) g = 148 * 32;
-    sx_gradient_kernel<<<(int)g, 256, 0, stream>>>(d, width, height, out);
-    return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------

@@ -116,6 +116,11 @@ cudaError_t sx_upwind_launch(const int* rows, const int* rid, const int* off, in
                              cudaStream_t stream);
 cudaError_t sx_threshold_launch(const float* d, int width, int height, float thr, int grad, int* counts,
                                 const int* offsets, int* ob, int* oe, cudaStream_t stream);
+int sx_mask_tiles(int H);
+cudaError_t sx_mask_launch(const float* d, int W, int H, float thr, int grad, unsigned* mask, int* offsets, int* result,
+                           const SxScanState& st, cudaStream_t stream);
+cudaError_t sx_mask_runs_launch(const unsigned* mask, int W, int H, const int* offsets, int* ob, int* oe,
+                                cudaStream_t stream);
 cudaError_t sx_mass_launch(const void* v, long long n, int dbl, double scale, double* part, int parts, double* out,
                            cudaStream_t stream);
 cudaError_t sx_locate_cells_launch(const int* rows, const int* off, const int* b, const int* e, int row_count,

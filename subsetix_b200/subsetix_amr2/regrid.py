@@ -1,11 +1,10 @@
 """Refinement tagging and grading (drop-in for ``subsetix_amr2.regrid``).
 
 Follows ``subsetix_amr2/regrid.py`` of the reference.  The gradient and the
-threshold run-length encoding are fused into one kernel
-(``sx_threshold_rle`` with ``gradient = 1``): one warp per row, where each
-lane computes the gradient magnitude of its cell, and a ballot plus popc
-turn the predicate into run starts and ends.  The gradient field itself is
-only materialised when asked for (:func:`gradient_magnitude_interval_field`).
+threshold run-length encoding are fused: one pass over the field
+(``sx_threshold_mask``) leaves one bit per cell and the rows' run offsets, and
+``sx_mask_runs`` stores the runs.  The gradient field itself is only
+materialised when asked for (:func:`gradient_magnitude_interval_field`).
 """
 
 from __future__ import annotations
