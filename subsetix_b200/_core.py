@@ -239,6 +239,33 @@ def merge_rows(begin: torch.Tensor, end: torch.Tensor, offsets: torch.Tensor, de
     return ob, oe, off
 
 
+def box_sweep(begin, end, offsets, rows, device, *, dense: bool, y_base: int, out_rows: int, x_lo: int, x_hi: int,
+              halo_y: int, w_center: int, w_other: int, erode: bool = False, compact: bool = False):
+    """sx_box_sweep and its read-back: ``(begin, end, offsets, row ids or None, total, flags)``.
+
+    begin and end are capacity buffers; with ``compact`` offsets and row ids
+    are cut to the kept rows.
+    """
+    lib = _lib.load()
+    n, out_rows = int(begin.numel()), int(out_rows)
+    views = 2 * int(halo_y) + 1
+    cap = views * n + (views + 1) * out_rows if erode else max(1, views * n)
+    box = _lib.SxBox(ptr(begin), ptr(end), ptr(offsets), None if dense else ptr(rows), n, int(offsets.numel()) - 1,
+                     1 if dense else 0, 0, int(y_base), out_rows, int(x_lo), int(x_hi), int(halo_y), int(w_center),
+                     int(w_other), 1 if erode else 0)
+    ob, oe = empty_i32(cap, device), empty_i32(cap, device)
+    off = empty_i32(out_rows + 1, device)
+    ids = empty_i32(out_rows, device) if compact else None
+    result = empty_i32(3, device)
+    wsp, wsn = workspace(device, lib.sx_bool_workspace_bytes(out_rows))
+    _lib.check(lib.sx_box_sweep(ctypes.byref(box), ptr(ob), ptr(oe), ptr(off), ptr(ids), cap, ptr(result), wsp, wsn,
+                                stream_handle(device)), "sx_box_sweep")
+    total, flags, kept = result.tolist()
+    if compact:
+        off, ids = off[:kept + 1], ids[:kept]
+    return ob, oe, off, ids, total, flags
+
+
 def align_rows(lists: Sequence[tuple], row_min: int, row_max: int, device, want_offsets: Sequence[bool],
                want_ends: Optional[Sequence[bool]] = None):
     """Sorted union of ``floor((rows + shift) / div)`` over the lists, plus aligned offsets.

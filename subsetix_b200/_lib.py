@@ -49,6 +49,12 @@ class SxRowList(ctypes.Structure):
                 ("skip_empty", ctypes.c_int32), ("div", ctypes.c_int32), ("phase", ctypes.c_int32)]
 
 
+class SxBox(ctypes.Structure):
+    _fields_ = [("begin", c_vp), ("end", c_vp), ("row_offsets", c_vp), ("rows", c_vp), ("n", ctypes.c_int64)] + [
+        (name, ctypes.c_int32) for name in ("row_count", "dense", "row0", "y_base", "out_rows", "x_lo", "x_hi", "halo_y",
+                                            "w_center", "w_other", "erode")]
+
+
 class SxFlatPlan(ctypes.Structure):
     _fields_ = [("below", c_vp), ("above", c_vp), ("flags", c_vp), ("side", c_vp), ("n", ctypes.c_int64),
                 ("cells", ctypes.c_int64)]
@@ -129,6 +135,8 @@ _SIGNATURES = {
                                                  c_vp, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_double,
                                                  ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                                  c_vp, c_vp, ctypes.c_size_t, c_vp]),
+    "sx_box_sweep": (ctypes.c_int, [ctypes.POINTER(SxBox), c_vp, c_vp, c_vp, c_vp, ctypes.c_int64, c_vp, c_vp,
+                                    ctypes.c_size_t, c_vp]),
     "sx_upwind_flat_plan": (ctypes.c_int, [c_vp, c_vp, ctypes.c_int32, c_vp, c_vp, c_vp, ctypes.c_int64, ctypes.c_int64,
                                            c_vp, ctypes.c_int32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "sx_upwind_flat": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(SxFlatPlan), c_vp, c_vp, ctypes.c_double,

@@ -196,6 +196,58 @@ int sx_scan_i32(const int32_t* in, int64_t n, int32_t* out, int32_t* result, voi
     return SX_OK;
 }
 
+int sx_box_sweep(const sx_box* box, int32_t* out_begin, int32_t* out_end, int32_t* out_offsets, int32_t* out_row_ids,
+                 int64_t capacity, int32_t* result, void* workspace, size_t workspace_bytes, void* stream)
+{
+    if (!box || !out_offsets || !result) return fail(SX_ERR_INVALID, "sx_box_sweep: null argument");
+    if (box->n < 0 || box->n > INT32_MAX || box->row_count < 0 || box->out_rows < 0 || capacity < 0)
+        return fail(SX_ERR_INVALID, "sx_box_sweep: negative size");
+    if (box->out_rows >= (1 << 26)) return fail(SX_ERR_INVALID, "sx_box_sweep: at most 2^26 - 1 output rows");
+    if (box->halo_y < 0 || box->halo_y > 4) return fail(SX_ERR_INVALID, "sx_box_sweep: halo_y outside [0, 4]");
+    const int wmax = 1 << 24;
+    if (box->w_center < 0 || box->w_center > wmax || box->w_other < 0 || box->w_other > wmax)
+        return fail(SX_ERR_INVALID, "sx_box_sweep: widths outside [0, 2^24]");
+    if (box->x_lo >= box->x_hi || (box->x_lo != INT32_MIN && box->x_lo > INT32_MAX - wmax) ||
+        box->x_hi < INT32_MIN + wmax)
+        return fail(SX_ERR_INVALID, "sx_box_sweep: bad column range");
+    if ((long long)box->y_base + box->out_rows > INT32_MAX - 4 || box->y_base < INT32_MIN + 4)
+        return fail(SX_ERR_INVALID, "sx_box_sweep: row range outside int32");
+    if (box->erode && (box->y_base != 0 || box->x_lo != 0 || box->x_hi > (1 << 30)))
+        return fail(SX_ERR_INVALID, "sx_box_sweep: erosion needs the domain [0, x_hi) x [0, out_rows), x_hi <= 2^30");
+    if (box->row_count > 0 && (!box->row_offsets || (!box->dense && !box->rows)))
+        return fail(SX_ERR_INVALID, "sx_box_sweep: null rows");
+    if (box->n > 0 && (!box->begin || !box->end)) return fail(SX_ERR_INVALID, "sx_box_sweep: null intervals");
+    if (box->out_rows == 0) return SX_OK;
+    const size_t need = sx_sweep_state_bytes(sx_sweep_tiles(box->out_rows));
+    if (!workspace || workspace_bytes < need)
+        return fail(SX_ERR_WORKSPACE, "sx_box_sweep: workspace needs %zu bytes, got %zu", need, workspace_bytes);
+    SxBoxArgs A;
+    A.begin = box->begin;
+    A.end = box->end;
+    A.off = box->row_offsets;
+    A.rows = box->rows;
+    A.row_count = box->row_count;
+    A.n = box->n;
+    A.dense = box->dense;
+    A.row0 = box->row0;
+    A.ybase = box->y_base;
+    A.nrows = box->out_rows;
+    A.xlo = box->x_lo;
+    A.xhi = box->x_hi;
+    A.w_center = box->w_center;
+    A.w_other = box->w_other;
+    A.out_begin = out_begin;
+    A.out_end = out_end;
+    A.out_off = out_offsets;
+    A.out_rows = out_row_ids;
+    A.capacity = capacity;
+    A.result = result;
+    cudaError_t err = sx_box_launch(A, box->erode ? 1 : 0, box->halo_y, workspace, workspace_bytes,
+                                    (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_box_sweep");
+    return SX_OK;
+}
+
 size_t sx_align_workspace_bytes(int32_t row_min, int32_t row_max)
 {
     long long nbits = (long long)row_max - row_min + 1;

@@ -68,6 +68,28 @@ struct SxAlignArgs {
     int* result;       // [0] rows_out count, [1] flags
 };
 
+// Box morphology over consecutive output rows (sx_box.cu)
+struct SxBoxArgs {
+    const int* begin;
+    const int* end;
+    const int* off;
+    const int* rows;  // read unless dense
+    int row_count;
+    long long n;
+    int dense;        // rows are row0, row0 + 1, ...
+    int row0;
+    int ybase, nrows;  // output rows ybase .. ybase + nrows - 1
+    int xlo, xhi;      // results are clipped to [xlo, xhi); erode: the domain is [0, xhi) x [0, nrows)
+    int w_center, w_other;
+    int* out_begin;
+    int* out_end;
+    int* out_off;
+    int* out_rows;  // null: every output row is kept
+    long long capacity;
+    int* result;    // intervals, flags, kept rows
+};
+cudaError_t sx_box_launch(const SxBoxArgs& A, int erode, int hy, void* workspace, size_t workspace_bytes,
+                          cudaStream_t stream);
 cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspace, size_t workspace_bytes,
                             cudaStream_t stream);
 cudaError_t sx_tile_max_launch(const int* const* offsets, const int* const* begins, const int* const* ends, int k,

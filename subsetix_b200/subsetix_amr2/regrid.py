@@ -24,6 +24,7 @@ from ..subsetix_cupy import (
 )
 from ..subsetix_cupy.expressions import _t
 from ..subsetix_cupy.interval_field import IntervalField
+from ..subsetix_cupy.morphology import _box_sweep, _dense_empty
 
 I32 = torch.int32
 
@@ -119,6 +120,13 @@ def enforce_two_level_grading_set(refine_set: IntervalSet, *, padding: int = 1, 
         return refine_set
     if mode not in {"von_neumann", "moore"}:
         raise ValueError("mode must be 'von_neumann' or 'moore'")
+    if int(width) > 0 and int(height) > 0 and int(refine_set.begin.shape[0]) > 0 and refine_set.row_count > 0:
+        # one launch: the rows' intervals, widened in every row (box) or in the middle one (cross), merged and clipped
+        out = _box_sweep(refine_set, padding, padding, padding if mode == "moore" else 0, y_base=0,
+                         out_rows=int(height), x_lo=0, x_hi=int(width))
+        if out is not None:
+            return out if int(out.begin.shape[0]) else _dense_empty(int(height), _t(out.row_offsets).device,
+                                                                    refine_set.begin)
     if mode == "moore":
         expanded = dilate_interval_set(refine_set, halo_x=padding, halo_y=padding)
     else:

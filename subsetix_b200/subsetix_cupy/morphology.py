@@ -4,13 +4,15 @@ Names, arguments, results and exceptions follow the reference module
 (``subsetix_cupy/morphology.py``).  The compute path is new:
 
 * Dilation does not build ``(2*halo_y + 1) * n`` candidate intervals and
-  sort them.  The occupied rows are shifted by every ``dy`` and aligned on
-  the device (``sx_align_rows``).  Then one union-mode row sweep
-  (``sx_bool_eval``, ``SX_MODE_UNION``) merges the widened intervals of up to
-  9 shifted copies per launch.  Larger ``halo_y`` chains sweeps of at most 9
-  copies each; box dilation composes exactly.
-* Clipping is one fused intersection with the domain rectangle on dense
-  rows.
+  sort them.  Up to ``halo_y = 4`` one launch (``sx_box_sweep``) merges the
+  widened intervals of the ``2*halo_y + 1`` source rows under every output
+  row; larger ``halo_y`` chains such launches, box dilation composes exactly.
+  Row lists too sparse for consecutive output rows are aligned on the device
+  (``sx_align_rows``) and swept by the union-mode row sweep (``sx_bool_eval``,
+  ``SX_MODE_UNION``) over at most 9 shifted copies.
+* Clipping, ghost zones and erosion use the same launch: rows of the domain,
+  columns clipped to it, and for erosion the widened gaps instead of the
+  intervals.
 * Inputs outside the sweeps' contract (empty, unsorted or overlapping
   intervals) are detected on the device.  They then take the reference's
   sort-and-merge construction, :func:`_build_interval_set_from_rows`, which
@@ -137,6 +139,59 @@ def _union_sweep(s: IntervalSet, shifts, widen: int, skip_empty: bool) -> Option
     return _wrap(s.begin, ob[:total].clone(), oe[:total].clone(), ooff, rows_out, dense)
 
 
+_BOX_MAX_HALO_Y = 4
+_BOX_MAX_WIDTH = 1 << 24
+_BOX_MAX_ROWS = (1 << 26) - 1
+
+
+def _box_sweep(s: IntervalSet, halo_y: int, w_center: int, w_other: int, *, y_base: int, out_rows: int, x_lo: int,
+               x_hi: int, erode: bool = False, compact: bool = False) -> Optional[IntervalSet]:
+    """One ``sx_box_sweep`` of ``s`` over rows ``y_base .. y_base + out_rows - 1``.
+
+    Returns None when the sizes are outside the launch's range or the set is
+    outside its contract; the general path then gives the result.  Without
+    ``compact`` the rows are ``arange(out_rows)``.
+    """
+    device = _t(s.row_offsets).device
+    n = int(s.begin.shape[0])
+    if (halo_y > _BOX_MAX_HALO_Y or max(w_center, w_other) > _BOX_MAX_WIDTH or not 0 < out_rows <= _BOX_MAX_ROWS
+            or (2 * halo_y + 1) * n + (2 * halo_y + 2) * out_rows >= 1 << 31 or (erode and x_hi > 1 << 30)
+            or y_base < -(1 << 31) + 8 or y_base + out_rows > (1 << 31) - 8):
+        return None
+    dense = _dense_key(s) is not None
+    ob, oe, off, ids, total, flags = _core.box_sweep(
+        _t(s.begin), _t(s.end), _t(s.row_offsets), _t(s.rows), device, dense=dense, y_base=y_base, out_rows=out_rows,
+        x_lo=x_lo, x_hi=x_hi, halo_y=halo_y, w_center=w_center, w_other=w_other, erode=erode, compact=compact)
+    if flags & _lib.FLAG_CONTRACT:
+        return None
+    if flags & (_lib.FLAG_CAPACITY | _lib.FLAG_TIMEOUT):
+        raise _lib.SubsetixError(f"box sweep failed (flags={flags})")
+    rows = ids if compact else torch.arange(out_rows, dtype=I32, device=device)
+    return _wrap(s.begin, ob[:total].clone(), oe[:total].clone(), off, rows, None if compact else out_rows)
+
+
+def _box_dilate(s: IntervalSet, halo_x: int, halo_y: int) -> Optional[IntervalSet]:
+    """Unbounded box dilation of a non-empty set by one launch; None where :func:`_union_sweep` has to run.
+
+    Output rows are consecutive from the first source row to the last, so a
+    row list with more than four candidates per source row is left to the
+    row alignment.
+    """
+    if halo_y > _BOX_MAX_HALO_Y or halo_x > _BOX_MAX_WIDTH:
+        return None
+    rows = _t(s.rows)
+    R = int(rows.numel())
+    if _dense_key(s) is not None:
+        first, last = 0, R - 1
+    else:
+        first, last = torch.cat([rows[0:1], rows[-1:]]).tolist()
+    span = last - first + 1 + 2 * halo_y
+    if span > 4 * R + 1024:
+        return None
+    return _box_sweep(s, halo_y, halo_x, halo_x, y_base=first - halo_y, out_rows=span, x_lo=-(1 << 31),
+                      x_hi=(1 << 31) - 1, compact=True)
+
+
 def translate_interval_set(interval_set: IntervalSet, dx: int = 0, dy: int = 0) -> IntervalSet:
     """Shift every interval by ``dx`` and every row by ``dy`` (``morphology.py:113-137``)."""
     if not isinstance(dx, Integral) or not isinstance(dy, Integral):
@@ -222,13 +277,16 @@ def _dilate_unbounded(s: IntervalSet, halo_x: int, halo_y: int) -> IntervalSet:
         out = _union_sweep(s, [0], halo_x, skip_empty=False)
         return out if out is not None else _dilate_reference_order(s, halo_x, 0)
     step = min(halo_y, (_MAX_SHIFTS - 1) // 2)
-    out = _union_sweep(s, list(range(-step, step + 1)), halo_x, skip_empty=True)
+    out = _box_dilate(s, halo_x, step)
+    if out is None:
+        out = _union_sweep(s, list(range(-step, step + 1)), halo_x, skip_empty=True)
     if out is None:
         return _dilate_reference_order(s, halo_x, halo_y)
     rest = halo_y - step
     while rest > 0:
         step = min(rest, (_MAX_SHIFTS - 1) // 2)
-        out = _union_sweep(out, list(range(-step, step + 1)), 0, skip_empty=True)
+        more = _box_dilate(out, 0, step)
+        out = more if more is not None else _union_sweep(out, list(range(-step, step + 1)), 0, skip_empty=True)
         rest -= step
     return out
 
@@ -267,9 +325,9 @@ def _dense_empty(height: int, device, kind) -> IntervalSet:
 def clip_interval_set(interval_set: IntervalSet, *, width: int, height: int) -> IntervalSet:
     """Intersection with [0, width) x [0, height) on dense rows ``arange(height)`` (``morphology.py:268-319``).
 
-    One fused intersection sweep over the domain's rows.  Inputs outside the
-    sweep's contract take the reference's order: the exact intersection
-    kernel, then the sort-and-merge construction.
+    One box sweep over the domain's rows, else one fused intersection sweep.
+    Inputs outside the sweeps' contract take the reference's order: the exact
+    intersection kernel, then the sort-and-merge construction.
     """
     if width <= 0:
         raise ValueError("width must be positive")
@@ -281,6 +339,9 @@ def clip_interval_set(interval_set: IntervalSet, *, width: int, height: int) -> 
     kind = s.begin
     if H == 0 or int(s.begin.shape[0]) == 0 or s.row_count == 0:
         return _dense_empty(H, device, kind)
+    out = _box_sweep(s, 0, 0, 0, y_base=0, out_rows=H, x_lo=0, x_hi=W)
+    if out is not None:
+        return out if int(out.begin.shape[0]) else _dense_empty(H, device, kind)
     dom_rows = torch.arange(H, dtype=I32, device=device)
     dom_off = torch.arange(H + 1, dtype=I32, device=device)
     dom_b = torch.zeros(H, dtype=I32, device=device)
@@ -310,8 +371,13 @@ def ghost_zones(interval_set: IntervalSet, halo_x: int = 1, halo_y: int = 1, *, 
     """clip(dilate(S)) minus clip(S) (``morphology.py:322-341``)."""
     if height is None:
         height = int(interval_set.row_offsets.shape[0]) - 1
-    dilated = dilate_interval_set(interval_set, halo_x=halo_x, halo_y=halo_y)
-    clipped = clip_interval_set(dilated, width=width, height=height)
+    clipped = None
+    if halo_x >= 0 and halo_y >= 0 and width > 0 and height > 0 and int(interval_set.begin.shape[0]) > 0:
+        clipped = _box_sweep(interval_set, int(halo_y), int(halo_x), int(halo_x), y_base=0, out_rows=int(height),
+                             x_lo=0, x_hi=int(width))
+    if clipped is None:
+        dilated = dilate_interval_set(interval_set, halo_x=halo_x, halo_y=halo_y)
+        clipped = clip_interval_set(dilated, width=width, height=height)
     base = clip_interval_set(interval_set, width=width, height=height)
     return evaluate(make_difference(make_input(clipped), make_input(base))).copy()
 
@@ -323,6 +389,11 @@ def erode_interval_set(interval_set: IntervalSet, halo_x: int = 1, halo_y: int =
         height = int(interval_set.row_offsets.shape[0]) - 1
     if width <= 0 or height < 0:
         raise ValueError("width must be positive and height must be non-negative")
+    if halo_x >= 0 and halo_y >= 0 and height > 0 and int(interval_set.begin.shape[0]) > 0:
+        out = _box_sweep(interval_set, int(halo_y), int(halo_x), int(halo_x), y_base=0, out_rows=int(height), x_lo=0,
+                         x_hi=int(width), erode=True)
+        if out is not None:
+            return out
     base = clip_interval_set(interval_set, width=width, height=height)
     universe = full_interval_set(width, height)
     complement = evaluate(make_difference(make_input(universe), make_input(base)))
