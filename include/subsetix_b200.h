@@ -625,6 +625,10 @@ int sx_upwind_full(int dtype, const void* values, void* out, int32_t width, int3
                    double b, double dt, double dx, double dy, void* stream);
 int sx_amr_sync_full(int dtype, void* coarse, void* fine, const int8_t* actions, int32_t width, int32_t height,
                      int32_t batch, int32_t ratio, void* stream);
+/* sx_amr_sync_full into new arrays (no overlap with the inputs); actions may
+ * be NULL (nothing refined). */
+int sx_amr_sync_copy(int dtype, const void* coarse, const void* fine, const int8_t* actions, void* coarse_out,
+                     void* fine_out, int32_t width, int32_t height, int32_t batch, int32_t ratio, void* stream);
 /* One fixed-geometry step for ratio 2 in one pass: sx_upwind_full on both
  * levels followed by sx_amr_sync_full, value for value (a coarse cell's
  * synchronisation reads only its own new value and its fine block's). */

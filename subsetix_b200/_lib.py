@@ -183,6 +183,8 @@ _SIGNATURES = {
                                       ctypes.c_double, c_vp]),
     "sx_amr_sync_full": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                         ctypes.c_int32, c_vp]),
+    "sx_amr_sync_copy": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32,
+                                        ctypes.c_int32, ctypes.c_int32, c_vp]),
     "sx_amr_step_full": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32,
                                         ctypes.c_int32, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                         ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double, c_vp]),

@@ -1059,6 +1059,23 @@ int sx_amr_sync_full(int dtype, void* coarse, void* fine, const int8_t* actions,
     return SX_OK;
 }
 
+int sx_amr_sync_copy(int dtype, const void* coarse, const void* fine, const int8_t* actions, void* coarse_out,
+                     void* fine_out, int32_t width, int32_t height, int32_t batch, int32_t ratio, void* stream)
+{
+    if (dtype != SX_F32 && dtype != SX_F64) return fail(SX_ERR_INVALID, "sx_amr_sync_copy: dtype %d", dtype);
+    int rc = full_grid_check("sx_amr_sync_copy", width, height, batch);
+    if (rc != SX_OK) return rc;
+    if (ratio < 1 || (long long)width * ratio > INT32_MAX || (long long)height * ratio > INT32_MAX)
+        return fail(SX_ERR_INVALID, "sx_amr_sync_copy: bad ratio");
+    if (!coarse || !fine || !coarse_out || !fine_out) return fail(SX_ERR_INVALID, "sx_amr_sync_copy: null argument");
+    if (coarse == coarse_out || fine == fine_out)
+        return fail(SX_ERR_INVALID, "sx_amr_sync_copy: outputs must not alias inputs");
+    cudaError_t err = sx_amr_sync_copy_launch(dtype == SX_F64, coarse, fine, (const signed char*)actions, coarse_out,
+                                              fine_out, width, height, batch, ratio, (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_amr_sync_copy");
+    return SX_OK;
+}
+
 int sx_amr_step_full(int dtype, const void* coarse_in, const void* fine_in, void* coarse_out, void* fine_out,
                      const int8_t* actions, int32_t width, int32_t height, int32_t batch, double a, double b,
                      double dt, double dx_coarse, double dy_coarse, double dx_fine, double dy_fine, void* stream)

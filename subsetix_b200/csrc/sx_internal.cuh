@@ -157,6 +157,9 @@ cudaError_t sx_upwind_full_launch(int dbl, const void* in, void* out, int W, int
                                   double dt, double dx, double dy, cudaStream_t stream);
 cudaError_t sx_amr_sync_full_launch(int dbl, void* coarse, void* fine, const signed char* actions, int W, int H,
                                     int batch, int ratio, cudaStream_t stream);
+cudaError_t sx_amr_sync_copy_launch(int dbl, const void* coarse, const void* fine, const signed char* actions,
+                                    void* coarse_out, void* fine_out, int W, int H, int batch, int ratio,
+                                    cudaStream_t stream);
 cudaError_t sx_amr_regrid_full_launch(int dbl, const void* coarse, unsigned char* tags, signed char* actions, int W,
                                       int H, int batch, float threshold, int padding, int mode, cudaStream_t stream);
 cudaError_t sx_amr_step_full_launch(int dbl, const void* cin, const void* fin, void* cout, void* fout,

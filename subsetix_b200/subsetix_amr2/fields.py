@@ -9,7 +9,7 @@ warp per subset interval).  Value runs for the action field come from
 
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field as _field
 from enum import IntEnum
 from typing import Dict, Optional
 
@@ -26,9 +26,10 @@ from ..subsetix_cupy.expressions import (
     make_input,
     make_intersection,
 )
-from ..subsetix_cupy.interval_field import IntervalField, create_interval_field
+from ..subsetix_cupy.interval_field import IntervalField, _is_packed, _packed_field, create_interval_field
 from ..subsetix_cupy.morphology import full_interval_set
 from ..subsetix_cupy.multilevel import prolong_field, restrict_field, prolong_set
+from ._dense import grid_values
 
 I32 = torch.int32
 
@@ -159,7 +160,10 @@ def scatter_interval_subset(field: IntervalField, subset_field: IntervalField) -
 def clone_interval_field(field: IntervalField) -> IntervalField:
     if not isinstance(field, IntervalField):
         raise TypeError("field must be an IntervalField")
-    return IntervalField(interval_set=field.interval_set, values=like(field.values, _t(field.values).clone()),
+    values = like(field.values, _t(field.values).clone())
+    if _is_packed(field):
+        return _packed_field(field.interval_set, values, field.interval_cell_offsets)
+    return IntervalField(interval_set=field.interval_set, values=values,
                          interval_cell_offsets=field.interval_cell_offsets)
 
 
@@ -196,6 +200,9 @@ class ActionField:
     _refine_set_cache: Optional[IntervalSet] = None
     _fine_set_cache: Optional[IntervalSet] = None
     _coarse_only_cache: Optional[IntervalSet] = None
+    # (refine set, its action bytes or None): bytes kept with the cached set they belong to, whatever
+    # happens to the field's values afterwards
+    _refine_bytes: Optional[tuple] = _field(default=None, repr=False, compare=False)
 
     @classmethod
     def from_interval_set(cls, interval_set: IntervalSet, *, width: int, height: int, ratio: int,
@@ -218,6 +225,7 @@ class ActionField:
             raise ValueError("interval_set must cover exactly width * height cells")
         action = cls(field=field, ratio=int(ratio), width=w, height=h)
         action._refine_set_cache = _empty_interval_like(interval_set)
+        action._refine_bytes = (action._refine_set_cache, None)
         return action
 
     @classmethod
@@ -231,6 +239,24 @@ class ActionField:
         self._refine_set_cache = _interval_field_value_intervals(self.field, int(Action.REFINE))
         self._fine_set_cache = None
         self._coarse_only_cache = None
+        self._keep_bytes()
+
+    def _keep_bytes(self) -> None:
+        """Copy the action bytes of the refine set just cached from (or written to) the values."""
+        vals = _t(self.field.values)
+        self._refine_bytes = ((self._refine_set_cache, vals.clone()) if vals.dtype == torch.int8 and _is_packed(self.field)
+                              else None)
+
+    def _bytes_of_refine_set(self):
+        """``(known, bytes)``: the REFINE bytes of the cached refine set on a whole grid (None: no cell refined)."""
+        s = self.field.interval_set
+        if getattr(s, "_full_width", None) != self.width or s.row_count != self.height:
+            return False, None
+        refine = self.refine_set()
+        kept = self._refine_bytes
+        if kept is None or kept[0] is not refine:
+            return False, None
+        return kept[1] is None or kept[1].numel() == self.width * self.height, kept[1]
 
     def set_from_interval_set(self, refine_set: IntervalSet) -> None:
         """Mark ``refine_set`` (which must lie in the domain) REFINE, everything else KEEP."""
@@ -243,6 +269,7 @@ class ActionField:
             self._refine_set_cache = _empty_interval_like(domain)
             self._fine_set_cache = None
             self._coarse_only_cache = None
+            self._refine_bytes = (self._refine_set_cache, None)
             return
         outside = evaluate(make_difference(make_input(refine_set), make_input(domain)))
         if int(outside.begin.shape[0]) != 0:
@@ -254,6 +281,7 @@ class ActionField:
         self._refine_set_cache = aligned
         self._fine_set_cache = None
         self._coarse_only_cache = None
+        self._keep_bytes()
 
     def refine_set(self) -> IntervalSet:
         if self._refine_set_cache is None:
@@ -278,6 +306,39 @@ class ActionField:
         return self.field.values
 
 
+def _synchronize_whole_grids(coarse: IntervalField, fine: IntervalField, actions: ActionField, ratio: int, copy: bool):
+    """The synchronisation of two whole-grid fields by one dense kernel; None when the fields are anything else.
+
+    Whole grids are known by their markers (``full_interval_set``, packed
+    offsets), without device work, and the refine region by the bytes kept
+    with the cached refine set, so the result is that of the interval
+    kernels: coarse cells in it take the mean of their block, the others are
+    injected into theirs.
+    """
+    W, H = int(actions.width), int(actions.height)
+    if ratio < 2 or H > 65535 or not (_is_packed(coarse) and _is_packed(fine)):
+        return None
+    c, f = grid_values(coarse, W, H), grid_values(fine, W * ratio, H * ratio)
+    if c is None or f is None or c.device != f.device or c.requires_grad or f.requires_grad:
+        return None
+    known, acts = actions._bytes_of_refine_set()
+    if not known or (acts is not None and acts.device != c.device):
+        return None
+    lib = _lib.load()
+    code = _lib.SX_F64 if c.dtype == torch.float64 else _lib.SX_F32
+    st = stream_handle(c.device)
+    if not copy:
+        acts = torch.zeros(W * H, dtype=torch.int8, device=c.device) if acts is None else acts
+        _lib.check(lib.sx_amr_sync_full(code, ptr(c), ptr(f), ptr(acts), W, H, 1, ratio, st), "sx_amr_sync_full")
+        return coarse, fine
+    c_out, f_out = torch.empty(W * H, dtype=c.dtype, device=c.device), torch.empty(f.numel(), dtype=c.dtype,
+                                                                                   device=c.device)
+    _lib.check(lib.sx_amr_sync_copy(code, ptr(c), ptr(f), ptr(acts), ptr(c_out), ptr(f_out), W, H, 1, ratio, st),
+               "sx_amr_sync_copy")
+    return (_packed_field(coarse.interval_set, like(coarse.values, c_out), coarse.interval_cell_offsets),
+            _packed_field(fine.interval_set, like(fine.values, f_out), fine.interval_cell_offsets))
+
+
 def synchronize_interval_fields(coarse: IntervalField, fine: IntervalField, actions: ActionField, *, ratio: int,
                                 reducer: str = "mean", fill_fine_outside: bool = True, copy: bool = True):
     """coarse[refine] <- restrict(fine)[refine]; fine[prolong(coarse_only)] <- prolong(coarse[coarse_only]).
@@ -297,6 +358,10 @@ def synchronize_interval_fields(coarse: IntervalField, fine: IntervalField, acti
     cd, fd = _t(coarse.values).dtype, _t(fine.values).dtype
     if not ((cd == torch.float32 and fd == torch.float32) or (cd == torch.float64 and fd == torch.float64)):
         raise TypeError("coarse and fine interval fields must use float32 values")
+    whole = _synchronize_whole_grids(coarse, fine, actions, int(ratio), copy) if reducer == "mean" and fill_fine_outside \
+        else None
+    if whole is not None:
+        return whole
     coarse_target = clone_interval_field(coarse) if copy else coarse
     fine_target = clone_interval_field(fine) if copy else fine
     dtype = np.float64 if cd == torch.float64 else np.float32

@@ -60,6 +60,22 @@ class IntervalField:
         return int(_t(off)[-1].item())
 
 
+def _packed_field(interval_set: IntervalSet, values, offsets) -> IntervalField:
+    """Field whose ``offsets`` are the prefix sum of the interval lengths, marked so (see :func:`_is_packed`)."""
+    field = IntervalField(interval_set=interval_set, values=values, interval_cell_offsets=offsets)
+    object.__setattr__(field, "_packed", getattr(offsets, "_version", None))
+    return field
+
+
+def _is_packed(field: IntervalField) -> bool:
+    """Whether the field was made by :func:`_packed_field` and its offsets have not been modified since.
+
+    The answer costs no device work; False only means not known.
+    """
+    version = getattr(field, "_packed", None)
+    return version is not None and version == getattr(field.interval_cell_offsets, "_version", None)
+
+
 def _fill_dtype(fill_value, dtype) -> torch.dtype:
     if dtype is not None:
         return torch_dtype(dtype)
@@ -84,7 +100,7 @@ def create_interval_field(interval_set: IntervalSet, fill_value: float = 0.0, *,
     else:
         off, total = _core.cell_offsets(bt, _t(interval_set.end), device)
     values = torch.full((total,), fill_value, dtype=_fill_dtype(fill_value, dtype), device=device)
-    return IntervalField(interval_set=interval_set, values=like(b, values), interval_cell_offsets=like(b, off))
+    return _packed_field(interval_set, like(b, values), like(b, off))
 
 
 def _locate_interval(interval_set: IntervalSet, row: int, x: int) -> Optional[int]:
