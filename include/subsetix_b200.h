@@ -195,17 +195,23 @@ int sx_scan_i32(const int32_t* in, int64_t n, int32_t* out, int32_t* result, voi
  * (subsetix_cupy/morphology.py:211-386, subsetix_amr2/regrid.py:404-442).
  * Output row y = y_base + i, i < out_rows, looks at the source rows y - halo_y
  * .. y + halo_y (halo_y <= 4):
- *   erode = 0  merged union of their intervals, widened by w_center (row y) or
+ *   SX_BOX_DILATE  merged union of their intervals, widened by w_center (row y) or
  *              w_other (the other rows), clipped to [x_lo, x_hi);
- *   erode = 1  the columns of [0, x_hi) that no gap of those rows, widened the
+ *   SX_BOX_ERODE  the columns of [0, x_hi) that no gap of those rows, widened the
  *              same way, covers (a gap: a stretch of [0, x_hi) outside the set);
- *              y_base = 0, rows outside [0, out_rows) constrain nothing.
+ *              y_base = 0, rows outside [0, out_rows) constrain nothing;
+ *   SX_BOX_RESTRICT  instead, merged union of [floor(b / ratio), ceil(e /
+ *              ratio)) over the rows ratio * y .. ratio * y + ratio - 1
+ *              (multilevel.py:272-362), ratio 2 to 4; widths and columns unused.
  * dense = 1: rows are row0, row0 + 1, ... (`rows` is not read); else `rows` is
  * strictly increasing.  out_row_ids (out_rows entries) keeps only rows with
  * intervals and compacts out_offsets (out_rows + 1 entries); NULL keeps every
  * row.  result[3] = {intervals, flags, kept rows}.  Rows whose begins or ends
  * fall, empty intervals, and a begin - w or end + w outside int32 raise
  * SX_FLAG_CONTRACT.  workspace: sx_bool_workspace_bytes(out_rows). */
+#define SX_BOX_DILATE 0
+#define SX_BOX_ERODE 1
+#define SX_BOX_RESTRICT 2
 typedef struct sx_box {
     const int32_t* begin;
     const int32_t* end;
@@ -214,7 +220,7 @@ typedef struct sx_box {
     int64_t n;
     int32_t row_count, dense, row0;
     int32_t y_base, out_rows, x_lo, x_hi;
-    int32_t halo_y, w_center, w_other, erode;
+    int32_t halo_y, w_center, w_other, mode, ratio;
 } sx_box;
 int sx_box_sweep(const sx_box* box, int32_t* out_begin, int32_t* out_end, int32_t* out_offsets, int32_t* out_row_ids,
                  int64_t capacity, int32_t* result, void* workspace, size_t workspace_bytes, void* stream);

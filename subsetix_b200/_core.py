@@ -240,7 +240,8 @@ def merge_rows(begin: torch.Tensor, end: torch.Tensor, offsets: torch.Tensor, de
 
 
 def box_sweep(begin, end, offsets, rows, device, *, dense: bool, y_base: int, out_rows: int, x_lo: int, x_hi: int,
-              halo_y: int, w_center: int, w_other: int, erode: bool = False, compact: bool = False):
+              halo_y: int = 0, w_center: int = 0, w_other: int = 0, mode: int = _lib.BOX_DILATE, ratio: int = 0,
+              compact: bool = False):
     """sx_box_sweep and its read-back: ``(begin, end, offsets, row ids or None, total, flags)``.
 
     begin and end are capacity buffers; with ``compact`` offsets and row ids
@@ -248,11 +249,11 @@ def box_sweep(begin, end, offsets, rows, device, *, dense: bool, y_base: int, ou
     """
     lib = _lib.load()
     n, out_rows = int(begin.numel()), int(out_rows)
-    views = 2 * int(halo_y) + 1
-    cap = views * n + (views + 1) * out_rows if erode else max(1, views * n)
+    views = 1 if mode == _lib.BOX_RESTRICT else 2 * int(halo_y) + 1  # output rows that one source row reaches
+    cap = views * n + (views + 1) * out_rows if mode == _lib.BOX_ERODE else max(1, views * n)
     box = _lib.SxBox(ptr(begin), ptr(end), ptr(offsets), None if dense else ptr(rows), n, int(offsets.numel()) - 1,
                      1 if dense else 0, 0, int(y_base), out_rows, int(x_lo), int(x_hi), int(halo_y), int(w_center),
-                     int(w_other), 1 if erode else 0)
+                     int(w_other), int(mode), int(ratio))
     ob, oe = empty_i32(cap, device), empty_i32(cap, device)
     off = empty_i32(out_rows + 1, device)
     ids = empty_i32(out_rows, device) if compact else None
@@ -329,26 +330,36 @@ def check_rows(begin: torch.Tensor, end: torch.Tensor, offsets: torch.Tensor, de
     return int(flags.item()) if sync else flags
 
 
-def cell_offsets(begin: torch.Tensor, end: torch.Tensor, device, sync: bool = True):
-    """int32 exclusive scan of interval lengths.  Returns ``(offsets, total)``."""
+def cell_offsets(begin: torch.Tensor, end: torch.Tensor, device, sync: bool = True,
+                 result: Optional[torch.Tensor] = None):
+    """int32 exclusive scan of interval lengths.  Returns ``(offsets, total)``, without ``sync`` ``(offsets, result)``."""
     lib = _lib.load()
     n = int(begin.numel())
     out = empty_i32(n + 1, device)
-    result = empty_i32(2, device)
+    if result is None:
+        result = empty_i32(2, device)
     wsp, wsn = workspace(device, lib.sx_scan_workspace_bytes(n))
     _lib.check(lib.sx_cell_offsets(ptr(begin), ptr(end), n, ptr(out), ptr(result), wsp, wsn, stream_handle(device)),
                "sx_cell_offsets")
     if not sync:
         return out, result
     total, flags = read_pair(result)
-    if flags & _lib.FLAG_TIMEOUT:
-        raise _lib.SubsetixError("sx_cell_offsets: look-back wait timed out")
+    check_scan(flags, "sx_cell_offsets")
     return out, total
 
 
+def check_scan(flags: int, what: str) -> None:
+    if flags & _lib.FLAG_TIMEOUT:
+        raise _lib.SubsetixError(f"{what}: look-back wait timed out")
+
+
 def prolong_set(rows: torch.Tensor, offsets: torch.Tensor, begin: torch.Tensor, end: torch.Tensor, ratio: int,
-                device):
-    """sx_prolong_set.  Returns ``(rows_out, offsets_out, begin, end, unsorted)`` sized to the output."""
+                device, cells: bool = False):
+    """sx_prolong_set.  Returns ``(rows_out, offsets_out, begin, end, unsorted)`` sized to the output.
+
+    With ``cells`` also ``(cell offsets, cell total)`` of the intervals as
+    they come, from the same read-back.
+    """
     lib = _lib.load()
     R = int(rows.numel())
     n = int(begin.numel())
@@ -356,16 +367,21 @@ def prolong_set(rows: torch.Tensor, offsets: torch.Tensor, begin: torch.Tensor, 
     off_out = empty_i32(R * ratio + 1, device)
     ob = empty_i32(n * ratio, device)
     oe = empty_i32(n * ratio, device)
-    result = empty_i32(2, device)
+    result = empty_i32(4, device)
     wsp, wsn = workspace(device, lib.sx_prolong_set_workspace_bytes(R))
     _lib.check(lib.sx_prolong_set(ptr(rows), ptr(offsets), ptr(begin), ptr(end), R, n, int(ratio), ptr(rows_out),
                                   ptr(off_out), ptr(ob), ptr(oe), ptr(result), wsp, wsn, stream_handle(device)),
                "sx_prolong_set")
-    occupied, flags = read_pair(result)
-    if flags & _lib.FLAG_TIMEOUT:
-        raise _lib.SubsetixError("sx_prolong_set: look-back wait timed out")
+    if cells:
+        cell_off, _ = cell_offsets(ob, oe, device, sync=False, result=result[2:])
+        occupied, flags, total, scan_flags = result.tolist()
+        check_scan(scan_flags, "sx_cell_offsets")
+    else:
+        occupied, flags = read_pair(result[:2])
+    check_scan(flags, "sx_prolong_set")
     m = occupied * ratio
-    return rows_out[:m], off_out[: m + 1], ob, oe, bool(flags & 1)
+    out = (rows_out[:m], off_out[: m + 1], ob, oe, bool(flags & 1))
+    return (*out, cell_off, total) if cells else out
 
 
 def _dtype_code(t: torch.Tensor) -> int:
@@ -385,16 +401,20 @@ def prolong_field(coarse_offsets, coarse_cell_offsets, n: int, fine_offsets, fin
                                     ptr(fine_values), stream_handle(device)), "sx_prolong_field")
 
 
-def coarse_fine_check(coarse, fine, ratio: int, device, sync: bool = True):
-    """Flags of sx_coarse_fine_check.  ``coarse``/``fine`` are ``(rows, offsets, begin, end)``."""
+def coarse_fine_check(coarse, fine, ratio: int, device, flags: Optional[torch.Tensor] = None):
+    """Flags of sx_coarse_fine_check.  ``coarse``/``fine`` are ``(rows, offsets, begin, end)``.
+
+    Given ``flags`` (one int on the device) they are left there unread.
+    """
     lib = _lib.load()
     cr, coff, cb, ce = coarse
     fr, foff, fb, fe = fine
-    flags = _flag_word(device)
+    own = flags is None
+    flags = _flag_word(device) if own else flags
     _lib.check(lib.sx_coarse_fine_check(ptr(cr), int(cr.numel()), ptr(coff), ptr(cb), ptr(ce), int(cb.numel()),
                                         ptr(fr), int(fr.numel()), ptr(foff), ptr(fb), ptr(fe), int(fb.numel()),
                                         int(ratio), ptr(flags), stream_handle(device)), "sx_coarse_fine_check")
-    return int(flags.item()) if sync else flags
+    return int(flags.item()) if own else flags
 
 
 def restrict_field(coarse_offsets, coarse_cell_offsets, coarse_n: int, fine_offsets, fine_cell_offsets, ratio: int,

@@ -24,6 +24,10 @@ SX_ERR_WORKSPACE = 4
 MODE_TABLE = 0
 MODE_UNION = 1
 
+BOX_DILATE = 0
+BOX_ERODE = 1
+BOX_RESTRICT = 2
+
 FLAG_CONTRACT = 1
 FLAG_LONG_TILE = 2
 FLAG_CAPACITY = 4
@@ -52,7 +56,7 @@ class SxRowList(ctypes.Structure):
 class SxBox(ctypes.Structure):
     _fields_ = [("begin", c_vp), ("end", c_vp), ("row_offsets", c_vp), ("rows", c_vp), ("n", ctypes.c_int64)] + [
         (name, ctypes.c_int32) for name in ("row_count", "dense", "row0", "y_base", "out_rows", "x_lo", "x_hi", "halo_y",
-                                            "w_center", "w_other", "erode")]
+                                            "w_center", "w_other", "mode", "ratio")]
 
 
 class SxFlatPlan(ctypes.Structure):

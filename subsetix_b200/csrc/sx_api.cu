@@ -212,7 +212,15 @@ int sx_box_sweep(const sx_box* box, int32_t* out_begin, int32_t* out_end, int32_
         return fail(SX_ERR_INVALID, "sx_box_sweep: bad column range");
     if ((long long)box->y_base + box->out_rows > INT32_MAX - 4 || box->y_base < INT32_MIN + 4)
         return fail(SX_ERR_INVALID, "sx_box_sweep: row range outside int32");
-    if (box->erode && (box->y_base != 0 || box->x_lo != 0 || box->x_hi > (1 << 30)))
+    if (box->mode != SX_BOX_DILATE && box->mode != SX_BOX_ERODE && box->mode != SX_BOX_RESTRICT)
+        return fail(SX_ERR_INVALID, "sx_box_sweep: mode %d", box->mode);
+    if (box->mode == SX_BOX_RESTRICT) {
+        if (box->ratio < 2 || box->ratio > 4) return fail(SX_ERR_INVALID, "sx_box_sweep: ratio outside [2, 4]");
+        if ((long long)box->y_base * box->ratio < INT32_MIN ||
+            ((long long)box->y_base + box->out_rows) * box->ratio > INT32_MAX)
+            return fail(SX_ERR_INVALID, "sx_box_sweep: source rows outside int32");
+    }
+    if (box->mode == SX_BOX_ERODE && (box->y_base != 0 || box->x_lo != 0 || box->x_hi > (1 << 30)))
         return fail(SX_ERR_INVALID, "sx_box_sweep: erosion needs the domain [0, x_hi) x [0, out_rows), x_hi <= 2^30");
     if (box->row_count > 0 && (!box->row_offsets || (!box->dense && !box->rows)))
         return fail(SX_ERR_INVALID, "sx_box_sweep: null rows");
@@ -242,8 +250,8 @@ int sx_box_sweep(const sx_box* box, int32_t* out_begin, int32_t* out_end, int32_
     A.out_rows = out_row_ids;
     A.capacity = capacity;
     A.result = result;
-    cudaError_t err = sx_box_launch(A, box->erode ? 1 : 0, box->halo_y, workspace, workspace_bytes,
-                                    (cudaStream_t)stream);
+    cudaError_t err = sx_box_launch(A, box->mode, box->mode == SX_BOX_RESTRICT ? box->ratio : box->halo_y, workspace,
+                                    workspace_bytes, (cudaStream_t)stream);
     if (err != cudaSuccess) return cuda_fail(err, "sx_box_sweep");
     return SX_OK;
 }

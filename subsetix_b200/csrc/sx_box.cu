@@ -12,6 +12,8 @@
 //            gap being a stretch of [0, xhi) outside the set; rows that the set
 //            lacks are one gap, rows outside the domain none
 //            (morphology.py:361-386).
+//   restrict the merged union of [floor(b / K), ceil(e / K)) over the K sub-rows
+//            K y .. K y + K - 1 (multilevel.py:272-362), K = 2, 3 or 4.
 // With out_rows only rows with runs are kept (their ids, compacted offsets), which
 // is the row list of an unbounded dilation.
 //
@@ -42,6 +44,19 @@ namespace {
 
 __host__ __device__ inline int slice_words(int cap) { return SXB_HDR_WORDS + 2 * ((cap + 11) & ~3); }
 
+enum { SXB_UNION = 0, SXB_ERODE = 1, SXB_RESTRICT = 2 };
+
+template <int K>
+__device__ __forceinline__ int floor_div(int a)
+{
+    const int q = a / K;
+    return a - q * K < 0 ? q - 1 : q;
+}
+
+// Source row of view l under output row y.
+template <int K, int MODE>
+__device__ __forceinline__ int source_row(int y, int l) { return MODE == SXB_RESTRICT ? K * y + l : y + l - K / 2; }
+
 // One view's elements: interval j of the row for dilate, gap j (before interval
 // j; the last one after the row's end) for erode.  B, E point at the row.
 struct Element {
@@ -49,25 +64,31 @@ struct Element {
     bool empty, bad;
 };
 
-template <bool ERODE>
-__device__ __forceinline__ int elements(int n, bool valid) { return ERODE ? (valid ? n + 1 : 0) : n; }
+template <int MODE>
+__device__ __forceinline__ int elements(int n, bool valid) { return MODE == SXB_ERODE ? (valid ? n + 1 : 0) : n; }
 
 // Transformed begin of element j: the sweep's key, never falling along a row.
 // Elements beyond the right edge share the key of the edge, so the element
 // before a piece is never one of them.
-template <bool ERODE>
+template <int K, int MODE>
 __device__ __forceinline__ int key(const SxBoxArgs& A, const int* B, const int* E, int n, int j, int w)
 {
-    if (ERODE) return (j == 0 ? 0 : min(max(E[j - 1], 0), A.xhi)) - w;
+    if (MODE == SXB_ERODE) return (j == 0 ? 0 : min(max(E[j - 1], 0), A.xhi)) - w;
+    if (MODE == SXB_RESTRICT) return floor_div<K>(B[j]);
     const int b = B[j];
     return b < A.xlo + w ? A.xlo : min(b - w, A.xhi);  // the launcher keeps xlo + w inside int32
 }
 
-template <bool ERODE>
+template <int K, int MODE>
 __device__ __forceinline__ Element element(const SxBoxArgs& A, const int* B, const int* E, int n, int j, int w)
 {
     Element r;
-    if (ERODE) {
+    if (MODE == SXB_RESTRICT) {
+        r.bad = E[j] <= B[j];
+        r.empty = false;
+        r.b = floor_div<K>(B[j]);
+        r.e = -floor_div<K>(-E[j]);
+    } else if (MODE == SXB_ERODE) {
         const int g0 = j == 0 ? 0 : min(max(E[j - 1], 0), A.xhi), g1 = j == n ? A.xhi : min(B[j], A.xhi);
         r.bad = j < n && E[j] <= B[j];
         r.empty = g1 <= g0;
@@ -84,7 +105,7 @@ __device__ __forceinline__ Element element(const SxBoxArgs& A, const int* B, con
 }
 
 // One piece of an output row; see sxu_sweep.  Returns the intervals it emits.
-template <int K, bool ERODE, bool WRITE>
+template <int K, int MODE, bool WRITE>
 __device__ __forceinline__ int sweep(const SxBoxArgs& A, const int* SB, const int* SE, const int (&lo)[K],
                                      const int (&n)[K], const int (&m)[K], const int (&p0)[K], int khi, long long rank,
                                      int (&pos)[K], int& ce, bool& open, bool& bad)
@@ -97,18 +118,18 @@ __device__ __forceinline__ int sweep(const SxBoxArgs& A, const int* SB, const in
         const int w = l == K / 2 ? A.w_center : A.w_other;
         const int *B = SB + lo[l], *E = SE + lo[l];
         pos[l] = p0[l];
-        h[l] = pos[l] < m[l] ? key<ERODE>(A, B, E, n[l], pos[l], w) : INT_MAX;
+        h[l] = pos[l] < m[l] ? key<K, MODE>(A, B, E, n[l], pos[l], w) : INT_MAX;
         el[l] = INT_MIN;
         // the running end: of the last element before the piece that is not empty
         for (int q = pos[l] - 1; q >= 0; --q) {
-            const Element x = element<ERODE>(A, B, E, n[l], q, w);
+            const Element x = element<K, MODE>(A, B, E, n[l], q, w);
             if (q == pos[l] - 1) el[l] = x.e;
             if (!x.empty) {
                 ce = max(ce, x.e);
                 open = true;
                 break;
             }
-            if (!ERODE || (q < n[l] && B[q] <= 0)) break;  // clipped away on the left, as is everything before it
+            if (MODE != SXB_ERODE || (q < n[l] && B[q] <= 0)) break;  // clipped away on the left, as is everything before it
         }
     }
     int out = 0;
@@ -124,7 +145,7 @@ __device__ __forceinline__ int sweep(const SxBoxArgs& A, const int* SB, const in
             if (h[l] == c && pos[l] < m[l]) {
                 const int w = l == K / 2 ? A.w_center : A.w_other;
                 const int *B = SB + lo[l], *E = SE + lo[l];
-                const Element x = element<ERODE>(A, B, E, n[l], pos[l], w);
+                const Element x = element<K, MODE>(A, B, E, n[l], pos[l], w);
                 if (x.bad || x.e < el[l]) bad = true;
                 el[l] = x.e;
                 if (!x.empty) {
@@ -132,14 +153,14 @@ __device__ __forceinline__ int sweep(const SxBoxArgs& A, const int* SB, const in
                     some = true;
                 }
                 const int q = ++pos[l];
-                h[l] = q < m[l] ? key<ERODE>(A, B, E, n[l], q, w) : INT_MAX;
+                h[l] = q < m[l] ? key<K, MODE>(A, B, E, n[l], q, w) : INT_MAX;
                 if (h[l] < c) bad = true;
             }
         }
         if (!some) continue;
         if (!open || c > ce) {
             const long long o = rank + out;
-            if (ERODE) {  // the stretch before this gap
+            if (MODE == SXB_ERODE) {  // the stretch before this gap
                 const int from = open ? ce : 0;
                 if (c > from) {
                     if (WRITE && o < A.capacity) {
@@ -210,7 +231,7 @@ __device__ __forceinline__ int lookback(const SxSweepState& st, int tile, int in
     return exclusive;
 }
 
-template <int K, bool ERODE>
+template <int K, int MODE>
 __global__ void __launch_bounds__(32 * SXB_WARPS) box_kernel(SxBoxArgs A, SxSweepState st, int tiles, int lg, int cap)
 {
     extern __shared__ __align__(16) int sxb_smem[];
@@ -237,7 +258,7 @@ __global__ void __launch_bounds__(32 * SXB_WARPS) box_kernel(SxBoxArgs A, SxSwee
     int at = 0;  // ordinal of the first source row at or after the current one
     if (!A.dense && act) {
         int a = 0, b = A.row_count;
-        const int v = y - K / 2;
+        const int v = source_row<K, MODE>(y, 0);
         while (a < b) {
             const int mid = (a + b) >> 1;
             if (A.rows[mid] < v) a = mid + 1; else b = mid;
@@ -246,7 +267,7 @@ __global__ void __launch_bounds__(32 * SXB_WARPS) box_kernel(SxBoxArgs A, SxSwee
     }
 #pragma unroll
     for (int l = 0; l < K; ++l) {
-        const int v = y + l - K / 2;
+        const int v = source_row<K, MODE>(y, l);
         int ord = -1;
         if (act) {
             if (A.dense) {
@@ -256,12 +277,12 @@ __global__ void __launch_bounds__(32 * SXB_WARPS) box_kernel(SxBoxArgs A, SxSwee
                 ord = at++;
             }
         }
-        const bool valid = act && (!ERODE || (v >= 0 && v < A.nrows));
+        const bool valid = act && (MODE != SXB_ERODE || (v >= 0 && v < A.nrows));
         const int a = ord >= 0 && valid ? A.off[ord] : 0, b = ord >= 0 && valid ? A.off[ord + 1] : 0;
         if (b < a) bad = true;  // row offsets must not run backwards
         lo[l] = a;
         n[l] = b > a ? b - a : 0;
-        m[l] = elements<ERODE>(n[l], valid);
+        m[l] = elements<MODE>(n[l], valid);
         if (n[l] > 0) {
             gs = min(gs, a);
             ge = max(ge, b);
@@ -313,26 +334,26 @@ __global__ void __launch_bounds__(32 * SXB_WARPS) box_kernel(SxBoxArgs A, SxSwee
             }
         if (big_m > 0) {
             const int *B = SB + big_lo, *E = SE + big_lo;
-            if (!last) khi = key<ERODE>(A, B, E, big_n, (int)(((long long)(piece + 1) * big_m) >> lg), big_w);
+            if (!last) khi = key<K, MODE>(A, B, E, big_n, (int)(((long long)(piece + 1) * big_m) >> lg), big_w);
             if (piece > 0) {
-                const int klo = key<ERODE>(A, B, E, big_n, (int)(((long long)piece * big_m) >> lg), big_w);
+                const int klo = key<K, MODE>(A, B, E, big_n, (int)(((long long)piece * big_m) >> lg), big_w);
 #pragma unroll
                 for (int l = 0; l < K; ++l) {
                     const int w = l == K / 2 ? A.w_center : A.w_other;
                     int a = 0, b = m[l];
                     while (a < b) {
                         const int mid = (a + b) >> 1;
-                        if (key<ERODE>(A, SB + lo[l], SE + lo[l], n[l], mid, w) < klo) a = mid + 1; else b = mid;
+                        if (key<K, MODE>(A, SB + lo[l], SE + lo[l], n[l], mid, w) < klo) a = mid + 1; else b = mid;
                     }
                     p0[l] = a;
                 }
             }
         }
     }
-    int count = sweep<K, ERODE, false>(A, SB, SE, lo, n, m, p0, khi, 0, pos, ce, open, bad);
+    int count = sweep<K, MODE, false>(A, SB, SE, lo, n, m, p0, khi, 0, pos, ce, open, bad);
     // the stretch after the last gap; a row of the domain without any gap is whole
     const int from = open ? ce : 0;
-    const bool tail = ERODE && last && act && from < A.xhi;
+    const bool tail = MODE == SXB_ERODE && last && act && from < A.xhi;
     if (tail) ++count;
 #pragma unroll
     for (int l = 0; l < K; ++l) {  // consecutive pieces of a row meet, and the last one ends with the row
@@ -359,8 +380,8 @@ __global__ void __launch_bounds__(32 * SXB_WARPS) box_kernel(SxBoxArgs A, SxSwee
     const int base = lookback(st, tile, total, __popc(km), flags, row_base);
     if (write) {
         const long long rank = (long long)base + incl - count;
-        const int swept = sweep<K, ERODE, true>(A, SB, SE, lo, n, m, p0, khi, rank, pos, ce, open, bad);
-        if (ERODE) {
+        const int swept = sweep<K, MODE, true>(A, SB, SE, lo, n, m, p0, khi, rank, pos, ce, open, bad);
+        if (MODE == SXB_ERODE) {
             if (tail && rank + swept < A.capacity) {
                 A.out_begin[rank + swept] = from;
                 A.out_end[rank + swept] = A.xhi;
@@ -397,25 +418,26 @@ int box_shape(const SxBoxArgs& A, size_t workspace_bytes)
     return lg;
 }
 
-template <int K, bool ERODE>
+template <int K, int MODE>
 cudaError_t box_go(const SxBoxArgs& A, const SxSweepState& st, int tiles, int lg, cudaStream_t stream)
 {
     // staged intervals per tile: 1.5 times the mean of the source rows under it
-    const long long src_rows = (32 >> lg) + K - 1;
+    const long long src_rows = MODE == SXB_RESTRICT ? (long long)(32 >> lg) * K : (32 >> lg) + K - 1;
     long long cap = (3 * (A.row_count > 0 ? A.n / A.row_count : 0) + 2) * src_rows / 2 + 32;
     if (cap > 6000) cap = 6000;
     const int bytes = SXB_WARPS * slice_words((int)cap) * (int)sizeof(int);
-    cudaError_t err = cudaFuncSetAttribute(box_kernel<K, ERODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t err = cudaFuncSetAttribute(box_kernel<K, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            SXB_WARPS * slice_words(6000) * (int)sizeof(int));
     if (err != cudaSuccess) return err;
     const int blocks = (tiles + SXB_WARPS - 1) / SXB_WARPS;
-    box_kernel<K, ERODE><<<blocks, 32 * SXB_WARPS, bytes, stream>>>(A, st, tiles, lg, (int)cap);
+    box_kernel<K, MODE><<<blocks, 32 * SXB_WARPS, bytes, stream>>>(A, st, tiles, lg, (int)cap);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t sx_box_launch(const SxBoxArgs& A, int erode, int hy, void* workspace, size_t workspace_bytes,
+// mode 0 and 1: arg is hy; mode 2: arg is the ratio.
+cudaError_t sx_box_launch(const SxBoxArgs& A, int mode, int arg, void* workspace, size_t workspace_bytes,
                           cudaStream_t stream)
 {
     if (A.nrows <= 0) return cudaSuccess;
@@ -426,22 +448,30 @@ cudaError_t sx_box_launch(const SxBoxArgs& A, int erode, int hy, void* workspace
     if (err != cudaSuccess) return err;
     const SxSweepState st = sx_sweep_state(workspace, tiles);
     const int t = (int)tiles;
-    if (erode) {
-        switch (hy) {
-            case 0: return box_go<1, true>(A, st, t, lg, stream);
-            case 1: return box_go<3, true>(A, st, t, lg, stream);
-            case 2: return box_go<5, true>(A, st, t, lg, stream);
-            case 3: return box_go<7, true>(A, st, t, lg, stream);
-            case 4: return box_go<9, true>(A, st, t, lg, stream);
+    if (mode == SXB_RESTRICT) {
+        switch (arg) {
+            case 2: return box_go<2, SXB_RESTRICT>(A, st, t, lg, stream);
+            case 3: return box_go<3, SXB_RESTRICT>(A, st, t, lg, stream);
+            case 4: return box_go<4, SXB_RESTRICT>(A, st, t, lg, stream);
             default: return cudaErrorInvalidValue;
         }
     }
-    switch (hy) {
-        case 0: return box_go<1, false>(A, st, t, lg, stream);
-        case 1: return box_go<3, false>(A, st, t, lg, stream);
-        case 2: return box_go<5, false>(A, st, t, lg, stream);
-        case 3: return box_go<7, false>(A, st, t, lg, stream);
-        case 4: return box_go<9, false>(A, st, t, lg, stream);
+    if (mode == SXB_ERODE) {
+        switch (arg) {
+            case 0: return box_go<1, SXB_ERODE>(A, st, t, lg, stream);
+            case 1: return box_go<3, SXB_ERODE>(A, st, t, lg, stream);
+            case 2: return box_go<5, SXB_ERODE>(A, st, t, lg, stream);
+            case 3: return box_go<7, SXB_ERODE>(A, st, t, lg, stream);
+            case 4: return box_go<9, SXB_ERODE>(A, st, t, lg, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    switch (arg) {
+        case 0: return box_go<1, SXB_UNION>(A, st, t, lg, stream);
+        case 1: return box_go<3, SXB_UNION>(A, st, t, lg, stream);
+        case 2: return box_go<5, SXB_UNION>(A, st, t, lg, stream);
+        case 3: return box_go<7, SXB_UNION>(A, st, t, lg, stream);
+        case 4: return box_go<9, SXB_UNION>(A, st, t, lg, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -122,42 +122,145 @@ __global__ void sx_prolong_set_intervals_kernel(const int* __restrict__ b, const
 }
 
 // ---------------------------------------------------------------------------
+// Field transfers between levels: blocks of coarse rows.
+//
+// A block takes one coarse row (several share a long row when rows are few) and
+// its threads take the row's cells one after another, whatever intervals they
+// lie in; the row's interval starts are staged in shared memory, FIELD_BATCH at a
+// time, and a thread finds its interval there.  Bound by bytes.  One warp per
+// interval, after a search for its row, left too little work per warp to keep
+// loads in flight: on a 4096^2 geometry (8 M coarse cells, float32) prolongation
+// took 133 us and restriction 116 us; 55 and 57 us here (69 and 100 us with one search
+// per cell instead of one per 128 cells of a warp), 26 us at the copy
+// rate.  For ratio 2 the two fine values of a sub-row move as one pair where they
+// start at an even value of an aligned array (always, when values are packed).
+// ---------------------------------------------------------------------------
+#define SX_FIELD_THREADS 256
+#define SX_FIELD_BATCH 512
+#define SX_FIELD_ITEMS 4
+
+template <typename T>
+struct SxPair;
+template <>
+struct SxPair<float> {
+    typedef float2 type;
+};
+template <>
+struct SxPair<double> {
+    typedef double2 type;
+};
+
+// Blocks per row, so that few rows still fill the chip.
+static int sx_field_split(int rows)
+{
+    int s = 1;
+    while (s < 64 && (long long)rows * s < 148 * 8) s <<= 1;
+    return s;
+}
+
+// What a thread knows of SX_FIELD_ITEMS cells of a coarse row, 32 apart (a warp
+// takes 128 consecutive cells): the cell, its interval within the batch and its
+// place in the interval (-1: past the row).
+struct SxFieldItems {
+    long long c[SX_FIELD_ITEMS];
+    int o[SX_FIELD_ITEMS], k[SX_FIELD_ITEMS];
+};
+
+// Calls f(items, first, s_c, s_f) for this block's share of the cells of row p.
+// s_c holds the batch's interval starts, first its first interval within the row
+// and s_f, for a fixed ratio, the starts of the fine intervals in the sub-rows
+// (stride SX_FIELD_BATCH + 1).  One search per 128 cells, then a walk.
+template <int RT, typename F>
+__device__ __forceinline__ void sx_field_cells(const int* __restrict__ off, const int* __restrict__ coff,
+                                               const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int p,
+                                               F f)
+{
+    __shared__ int s_c[SX_FIELD_BATCH + 1];
+    __shared__ int s_f[RT > 0 ? RT * (SX_FIELD_BATCH + 1) : 1];
+    const int i0 = off[p], i1 = off[p + 1];
+    for (int ib = i0; ib < i1; ib += SX_FIELD_BATCH) {
+        const int nb = min(SX_FIELD_BATCH, i1 - ib), first = ib - i0;
+        __syncthreads();
+        for (int j = threadIdx.x; j <= nb; j += SX_FIELD_THREADS) s_c[j] = coff[ib + j];
+#pragma unroll
+        for (int d = 0; d < RT; ++d) {
+            const int f0 = foff_rows[RT * p + d] + first;
+            for (int j = threadIdx.x; j <= nb; j += SX_FIELD_THREADS) s_f[d * (SX_FIELD_BATCH + 1) + j] = fcoff[f0 + j];
+        }
+        __syncthreads();
+        const long long end = s_c[nb], step = (long long)gridDim.y * SX_FIELD_THREADS * SX_FIELD_ITEMS;
+        for (long long w0 = s_c[0] + ((long long)blockIdx.y * SX_FIELD_THREADS + (threadIdx.x & ~31)) * SX_FIELD_ITEMS;
+             w0 < end; w0 += step) {
+            int lo = 0, hi = nb - 1;  // last interval starting at or before the warp's first cell
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (s_c[mid] <= w0) lo = mid; else hi = mid - 1;
+            }
+            SxFieldItems it;
+#pragma unroll
+            for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                it.c[q] = w0 + 32 * q + (threadIdx.x & 31);
+                while (lo + 1 < nb && s_c[lo + 1] <= it.c[q]) ++lo;
+                it.o[q] = lo;
+                it.k[q] = it.c[q] < end ? (int)(it.c[q] - s_c[lo]) : -1;
+            }
+            f(it, first, s_c, s_f);
+        }
+    }
+}
+
 // Field prolongation (kernels.py:384-455): piecewise-constant injection onto
 // the prolonged set.  Every coarse row must be occupied (the caller checks,
 // as the reference's alignment check does).  Coarse interval i (ordinal o
 // in row ordinal p) maps in sub-row d to the fine interval
 // f = fine_off[p*r + d] + o, and fine cell k of f takes coarse cell k / r.
-// One warp handles one coarse interval.  RT > 0 fixes the ratio at compile
-// time (2, the common one: k / r becomes a shift), RT = 0 takes r.
-// ---------------------------------------------------------------------------
+// RT > 0 fixes the ratio at compile time.
 template <typename T, int RT>
-__global__ void sx_prolong_field_kernel(const int* __restrict__ off, int rows, const int* __restrict__ coff, int n,
-                                        const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int rr,
-                                        const T* __restrict__ cv, T* __restrict__ fv)
+__global__ void __launch_bounds__(SX_FIELD_THREADS)
+    sx_prolong_field_kernel(const int* __restrict__ off, const int* __restrict__ coff, int n,
+                            const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int rr,
+                            const T* __restrict__ cv, T* __restrict__ fv, int pair)
 {
+    typedef typename SxPair<T>::type P2;
     const int r = RT > 0 ? RT : rr;
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
+    const int p = blockIdx.x;
     const long long ncells = coff[n];
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const int cb = coff[i];
-        if (coff[i + 1] - cb <= 0) continue;
-        const int p = sx_row_of(off, rows, i);
-        const int o = i - off[p];
+    sx_field_cells<RT>(off, coff, foff_rows, fcoff, p, [&](const SxFieldItems& it, int first, const int* s_c,
+                                                           const int* s_f) {
+        T v[SX_FIELD_ITEMS];
+#pragma unroll
+        for (int q = 0; q < SX_FIELD_ITEMS; ++q) v[q] = it.k[q] >= 0 ? cv[it.c[q]] : (T)0;
+#pragma unroll(RT > 0 ? RT : 1)
         for (int d = 0; d < r; ++d) {
-            const int f = foff_rows[p * r + d] + o;
-            const int fs = fcoff[f];
-            const int fw = fcoff[f + 1] - fs;
-            // Rows whose begins decrease are re-sorted on the fine level, so
-            // fine interval f may be wider than coarse interval i; the
-            // reference then reads past i, and past the array at its end.
-            // Here reads stay inside the array (0 beyond it).
-            for (int t = lane; t < fw; t += 32) {
-                const long long src = (long long)cb + t / r;
-                fv[fs + t] = src < ncells ? cv[src] : (T)0;
+            const int* fst = RT > 0 ? s_f + d * (SX_FIELD_BATCH + 1) : fcoff + foff_rows[p * r + d] + first;
+#pragma unroll
+            for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                if (it.k[q] < 0) continue;
+                const long long fs = fst[it.o[q]], fw = fst[it.o[q] + 1] - fs, t0 = (long long)it.k[q] * r;
+                if (RT == 2 && pair && !(fs & 1) && t0 + 2 <= fw) {
+                    P2 w;
+                    w.x = v[q];
+                    w.y = v[q];
+                    *(P2*)(fv + fs + t0) = w;
+                } else {
+#pragma unroll(RT > 0 ? RT : 1)
+                    for (int t = 0; t < r; ++t)
+                        if (t0 + t < fw) fv[fs + t0 + t] = v[q];
+                }
+                // Rows whose begins decrease are re-sorted on the fine level, so
+                // fine interval f may be wider than coarse interval i; the
+                // reference then reads past i, and past the array at its end.
+                // Here reads stay inside the array (0 beyond it).
+                const int cb = s_c[it.o[q]];
+                if (t0 + r < fw && it.c[q] + 1 == s_c[it.o[q] + 1]) {
+                    for (long long t = t0 + r; t < fw; ++t) {
+                        const long long src = cb + t / r;
+                        fv[fs + t] = src < ncells ? cv[src] : (T)0;
+                    }
+                }
             }
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -200,43 +303,74 @@ __global__ void sx_restrict_check_kernel(const int* __restrict__ crows, int crow
 
 // RT as in sx_prolong_field_kernel.
 template <typename T, int RT>
-__global__ void sx_restrict_field_kernel(const int* __restrict__ coff_rows, int crow_count, const int* __restrict__ ccoff,
-                                         int cn, const int* __restrict__ foff_rows, const int* __restrict__ fcoff,
-                                         int rr, int reducer, T norm, const T* __restrict__ fv, T* __restrict__ cv)
+__global__ void __launch_bounds__(SX_FIELD_THREADS)
+    sx_restrict_field_kernel(const int* __restrict__ coff_rows, const int* __restrict__ ccoff,
+                             const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int rr, int reducer,
+                             T norm, const T* __restrict__ fv, T* __restrict__ cv, int pair)
 {
+    typedef typename SxPair<T>::type P2;
     const int r = RT > 0 ? RT : rr;
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < cn; i += warps) {
-        const int p = sx_row_of(coff_rows, crow_count, i);
-        const int cb = ccoff[i];
-        const int w = ccoff[i + 1] - cb;
-        if (w <= 0) continue;
-        const int ordinal = i - coff_rows[p];
-        for (int k = lane; k < w; k += 32) {
-            T acc = (T)0, lo = (T)0, hi = (T)0;
-            bool have = false;
-            for (int dy = 0; dy < r; ++dy) {
-                const int f = foff_rows[p * r + dy] + ordinal;
-                const int fend = fcoff[f + 1];
-                const int start = fcoff[f] + k * r;
-                for (int dx = 0; dx < r; ++dx) {
-                    const int idx = start + dx;
-                    if (idx >= fend) break;
-                    const T v = fv[idx];
-                    if (reducer == 2) {
-                        if (!have || v < lo) lo = v;
-                    } else if (reducer == 3) {
-                        if (!have || v > hi) hi = v;
+    const int p = blockIdx.x;
+    sx_field_cells<RT>(coff_rows, ccoff, foff_rows, fcoff, p, [&](const SxFieldItems& it, int first, const int*,
+                                                                  const int* s_f) {
+        T acc[SX_FIELD_ITEMS], best[SX_FIELD_ITEMS];
+        bool have[SX_FIELD_ITEMS];
+#pragma unroll
+        for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+            acc[q] = best[q] = (T)0;
+            have[q] = false;
+        }
+        auto add = [&](int q, T v) {
+            if (reducer >= 2) {
+                if (!have[q] || (reducer == 2 ? v < best[q] : v > best[q])) best[q] = v;
+            } else {
+                acc[q] = sx_add(acc[q], v);
+            }
+            have[q] = true;
+        };
+        if (RT == 2) {
+            P2 v[2][SX_FIELD_ITEMS];
+            int got[2][SX_FIELD_ITEMS];  // values of the pair inside the fine interval
+#pragma unroll
+            for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+                for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                    const int* fst = s_f + dy * (SX_FIELD_BATCH + 1) + it.o[q];
+                    got[dy][q] = 0;
+                    if (it.k[q] < 0) continue;
+                    const long long start = fst[0] + 2ll * it.k[q], fend = fst[1];
+                    got[dy][q] = start + 2 <= fend ? 2 : start < fend ? 1 : 0;
+                    if (got[dy][q] == 2 && pair && !(start & 1)) {
+                        v[dy][q] = *(const P2*)(fv + start);
                     } else {
-                        acc = sx_add(acc, v);
+                        if (got[dy][q] > 0) v[dy][q].x = fv[start];
+                        if (got[dy][q] > 1) v[dy][q].y = fv[start + 1];
                     }
-                    have = true;
+                }
+#pragma unroll
+            for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+                for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                    if (got[dy][q] > 0) add(q, v[dy][q].x);
+                    if (got[dy][q] > 1) add(q, v[dy][q].y);
+                }
+        } else {
+            for (int dy = 0; dy < r; ++dy) {
+                const int* fst = RT > 0 ? s_f + dy * (SX_FIELD_BATCH + 1) : fcoff + foff_rows[p * r + dy] + first;
+#pragma unroll
+                for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                    if (it.k[q] < 0) continue;
+                    const long long start = fst[it.o[q]] + (long long)it.k[q] * r, fend = fst[it.o[q] + 1];
+#pragma unroll(RT > 0 ? RT : 1)
+                    for (int dx = 0; dx < r; ++dx)
+                        if (start + dx < fend) add(q, fv[start + dx]);
                 }
             }
-            cv[cb + k] = reducer == 0 ? sx_mul(acc, norm) : reducer == 1 ? acc : reducer == 2 ? lo : hi;
         }
-    }
+#pragma unroll
+        for (int q = 0; q < SX_FIELD_ITEMS; ++q)
+            if (it.k[q] >= 0) cv[it.c[q]] = reducer == 0 ? sx_mul(acc[q], norm) : reducer == 1 ? acc[q] : best[q];
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1479,25 +1613,30 @@ cudaError_t sx_prolong_set_launch(const int* rows_in, const int* off, const int*
     return cudaGetLastError();
 }
 
+template <typename T>
+static int sx_pairs_aligned(const void* p) { return ((uintptr_t)p & (2 * sizeof(T) - 1)) == 0; }
+
+template <typename T>
+static void sx_prolong_field_go(const int* off, int rows, const int* coff, int n, const int* foff_rows,
+                                const int* fcoff, int r, const T* cv, T* fv, cudaStream_t stream)
+{
+    const dim3 grid(rows, sx_field_split(rows));
+    const int pair = sx_pairs_aligned<T>(fv);
+    auto kernel = r == 2   ? sx_prolong_field_kernel<T, 2>
+                  : r == 3 ? sx_prolong_field_kernel<T, 3>
+                  : r == 4 ? sx_prolong_field_kernel<T, 4>
+                           : sx_prolong_field_kernel<T, 0>;
+    kernel<<<grid, SX_FIELD_THREADS, 0, stream>>>(off, coff, n, foff_rows, fcoff, r, cv, fv, pair);
+}
+
 cudaError_t sx_prolong_field_launch(const int* off, int rows, const int* coff, int n, const int* foff_rows,
                                     const int* fcoff, int r, const void* cv, void* fv, int dbl, cudaStream_t stream)
 {
-    const int grid = sx_grid((long long)n * 32, 256);
-    if (dbl) {
-        if (r == 2)
-            sx_prolong_field_kernel<double, 2><<<grid, 256, 0, stream>>>(off, rows, coff, n, foff_rows, fcoff, r,
-                                                                         (const double*)cv, (double*)fv);
-        else
-            sx_prolong_field_kernel<double, 0><<<grid, 256, 0, stream>>>(off, rows, coff, n, foff_rows, fcoff, r,
-                                                                         (const double*)cv, (double*)fv);
-    } else {
-        if (r == 2)
-            sx_prolong_field_kernel<float, 2><<<grid, 256, 0, stream>>>(off, rows, coff, n, foff_rows, fcoff, r,
-                                                                        (const float*)cv, (float*)fv);
-        else
-            sx_prolong_field_kernel<float, 0><<<grid, 256, 0, stream>>>(off, rows, coff, n, foff_rows, fcoff, r,
-                                                                        (const float*)cv, (float*)fv);
-    }
+    if (rows <= 0) return cudaSuccess;
+    if (dbl)
+        sx_prolong_field_go<double>(off, rows, coff, n, foff_rows, fcoff, r, (const double*)cv, (double*)fv, stream);
+    else
+        sx_prolong_field_go<float>(off, rows, coff, n, foff_rows, fcoff, r, (const float*)cv, (float*)fv, stream);
     return cudaGetLastError();
 }
 
@@ -1511,30 +1650,30 @@ cudaError_t sx_restrict_check_launch(const int* crows, int crow_count, const int
     return cudaGetLastError();
 }
 
+template <typename T>
+static void sx_restrict_field_go(const int* coff_rows, int rows, const int* ccoff, const int* foff_rows,
+                                 const int* fcoff, int r, int reducer, T norm, const T* fv, T* cv, cudaStream_t stream)
+{
+    const dim3 grid(rows, sx_field_split(rows));
+    const int pair = sx_pairs_aligned<T>(fv);
+    auto kernel = r == 2   ? sx_restrict_field_kernel<T, 2>
+                  : r == 3 ? sx_restrict_field_kernel<T, 3>
+                  : r == 4 ? sx_restrict_field_kernel<T, 4>
+                           : sx_restrict_field_kernel<T, 0>;
+    kernel<<<grid, SX_FIELD_THREADS, 0, stream>>>(coff_rows, ccoff, foff_rows, fcoff, r, reducer, norm, fv, cv, pair);
+}
+
 cudaError_t sx_restrict_field_launch(const int* coff_rows, int crow_count, const int* ccoff, int cn,
                                      const int* foff_rows, const int* fcoff, int r, int reducer, double norm,
                                      const void* fv, void* cv, int dbl, cudaStream_t stream)
 {
-    const int grid = sx_grid((long long)cn * 32, 256);
-    if (dbl) {
-        if (r == 2)
-            sx_restrict_field_kernel<double, 2><<<grid, 256, 0, stream>>>(coff_rows, crow_count, ccoff, cn, foff_rows,
-                                                                          fcoff, r, reducer, norm, (const double*)fv,
-                                                                          (double*)cv);
-        else
-            sx_restrict_field_kernel<double, 0><<<grid, 256, 0, stream>>>(coff_rows, crow_count, ccoff, cn, foff_rows,
-                                                                          fcoff, r, reducer, norm, (const double*)fv,
-                                                                          (double*)cv);
-    } else {
-        if (r == 2)
-            sx_restrict_field_kernel<float, 2><<<grid, 256, 0, stream>>>(coff_rows, crow_count, ccoff, cn, foff_rows,
-                                                                         fcoff, r, reducer, (float)norm,
-                                                                         (const float*)fv, (float*)cv);
-        else
-            sx_restrict_field_kernel<float, 0><<<grid, 256, 0, stream>>>(coff_rows, crow_count, ccoff, cn, foff_rows,
-                                                                         fcoff, r, reducer, (float)norm,
-                                                                         (const float*)fv, (float*)cv);
-    }
+    if (crow_count <= 0 || cn <= 0) return cudaSuccess;
+    if (dbl)
+        sx_restrict_field_go<double>(coff_rows, crow_count, ccoff, foff_rows, fcoff, r, reducer, norm,
+                                     (const double*)fv, (double*)cv, stream);
+    else
+        sx_restrict_field_go<float>(coff_rows, crow_count, ccoff, foff_rows, fcoff, r, reducer, (float)norm,
+                                    (const float*)fv, (float*)cv, stream);
     return cudaGetLastError();
 }
 

@@ -88,7 +88,7 @@ struct SxBoxArgs {
     long long capacity;
     int* result;    // intervals, flags, kept rows
 };
-cudaError_t sx_box_launch(const SxBoxArgs& A, int erode, int hy, void* workspace, size_t workspace_bytes,
+cudaError_t sx_box_launch(const SxBoxArgs& A, int mode, int arg, void* workspace, size_t workspace_bytes,
                           cudaStream_t stream);
 cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspace, size_t workspace_bytes,
                             cudaStream_t stream);

@@ -89,18 +89,32 @@ def create_interval_field(interval_set: IntervalSet, fill_value: float = 0.0, *,
     With ``dtype`` None the dtype is inferred from ``fill_value`` as NumPy
     does (a Python float gives float64).
     """
+    off, total, device = _offsets_of(interval_set)
+    values = torch.full((total,), fill_value, dtype=_fill_dtype(fill_value, dtype), device=device)
+    b = interval_set.begin
+    return _packed_field(interval_set, like(b, values), like(b, off))
+
+
+def _offsets_of(interval_set: IntervalSet):
+    """``(cell offsets, cells, device)`` of a set (one read-back unless it is empty)."""
     b = interval_set.begin
     if int(np.prod(b.shape)) != int(np.prod(interval_set.end.shape)):
         raise ValueError("IntervalSet begin/end size mismatch")
     bt = _t(b)
     device = _t(interval_set.row_offsets).device
     if bt.numel() == 0:
-        off = torch.zeros(1, dtype=I32, device=device)
-        total = 0
-    else:
-        off, total = _core.cell_offsets(bt, _t(interval_set.end), device)
-    values = torch.full((total,), fill_value, dtype=_fill_dtype(fill_value, dtype), device=device)
-    return _packed_field(interval_set, like(b, values), like(b, off))
+        return torch.zeros(1, dtype=I32, device=device), 0, device
+    off, total = _core.cell_offsets(bt, _t(interval_set.end), device)
+    return off, total, device
+
+
+def _unset_interval_field(interval_set: IntervalSet, dtype: torch.dtype, off: Optional[torch.Tensor] = None,
+                          total: int = 0) -> IntervalField:
+    """:func:`create_interval_field` without the fill, for callers that write every cell (offsets given or computed)."""
+    if off is None:
+        off, total, _ = _offsets_of(interval_set)
+    b = interval_set.begin
+    return _packed_field(interval_set, like(b, torch.empty(total, dtype=dtype, device=off.device)), like(b, off))
 
 
 def _locate_interval(interval_set: IntervalSet, row: int, x: int) -> Optional[int]:

@@ -145,7 +145,8 @@ _BOX_MAX_ROWS = (1 << 26) - 1
 
 
 def _box_sweep(s: IntervalSet, halo_y: int, w_center: int, w_other: int, *, y_base: int, out_rows: int, x_lo: int,
-               x_hi: int, erode: bool = False, compact: bool = False) -> Optional[IntervalSet]:
+               x_hi: int, mode: int = _lib.BOX_DILATE, ratio: int = 0, compact: bool = False
+               ) -> Optional[IntervalSet]:
     """One ``sx_box_sweep`` of ``s`` over rows ``y_base .. y_base + out_rows - 1``.
 
     Returns None when the sizes are outside the launch's range or the set is
@@ -155,19 +156,27 @@ def _box_sweep(s: IntervalSet, halo_y: int, w_center: int, w_other: int, *, y_ba
     device = _t(s.row_offsets).device
     n = int(s.begin.shape[0])
     if (halo_y > _BOX_MAX_HALO_Y or max(w_center, w_other) > _BOX_MAX_WIDTH or not 0 < out_rows <= _BOX_MAX_ROWS
-            or (2 * halo_y + 1) * n + (2 * halo_y + 2) * out_rows >= 1 << 31 or (erode and x_hi > 1 << 30)
+            or (2 * halo_y + 1) * n + (2 * halo_y + 2) * out_rows >= 1 << 31 or (mode == _lib.BOX_ERODE and x_hi > 1 << 30)
             or y_base < -(1 << 31) + 8 or y_base + out_rows > (1 << 31) - 8):
         return None
     dense = _dense_key(s) is not None
     ob, oe, off, ids, total, flags = _core.box_sweep(
         _t(s.begin), _t(s.end), _t(s.row_offsets), _t(s.rows), device, dense=dense, y_base=y_base, out_rows=out_rows,
-        x_lo=x_lo, x_hi=x_hi, halo_y=halo_y, w_center=w_center, w_other=w_other, erode=erode, compact=compact)
+        x_lo=x_lo, x_hi=x_hi, halo_y=halo_y, w_center=w_center, w_other=w_other, mode=mode, ratio=ratio, compact=compact)
     if flags & _lib.FLAG_CONTRACT:
         return None
     if flags & (_lib.FLAG_CAPACITY | _lib.FLAG_TIMEOUT):
         raise _lib.SubsetixError(f"box sweep failed (flags={flags})")
     rows = ids if compact else torch.arange(out_rows, dtype=I32, device=device)
     return _wrap(s.begin, ob[:total].clone(), oe[:total].clone(), off, rows, None if compact else out_rows)
+
+
+def _row_span(s: IntervalSet):
+    """First and last row id of a non-empty row list (one read-back unless the rows are known to be dense)."""
+    if _dense_key(s) is not None:
+        return 0, s.row_count - 1
+    rows = _t(s.rows)
+    return tuple(torch.cat([rows[0:1], rows[-1:]]).tolist())
 
 
 def _box_dilate(s: IntervalSet, halo_x: int, halo_y: int) -> Optional[IntervalSet]:
@@ -179,17 +188,25 @@ def _box_dilate(s: IntervalSet, halo_x: int, halo_y: int) -> Optional[IntervalSe
     """
     if halo_y > _BOX_MAX_HALO_Y or halo_x > _BOX_MAX_WIDTH:
         return None
-    rows = _t(s.rows)
-    R = int(rows.numel())
-    if _dense_key(s) is not None:
-        first, last = 0, R - 1
-    else:
-        first, last = torch.cat([rows[0:1], rows[-1:]]).tolist()
+    first, last = _row_span(s)
     span = last - first + 1 + 2 * halo_y
-    if span > 4 * R + 1024:
+    if span > 4 * s.row_count + 1024:
         return None
     return _box_sweep(s, halo_y, halo_x, halo_x, y_base=first - halo_y, out_rows=span, x_lo=-(1 << 31),
                       x_hi=(1 << 31) - 1, compact=True)
+
+
+def _box_restrict(s: IntervalSet, ratio: int) -> Optional[IntervalSet]:
+    """Restriction of a non-empty set by one launch (as :func:`_box_dilate`); ratios 2 to 4."""
+    if not 2 <= ratio <= 4:
+        return None
+    first, last = _row_span(s)
+    y_base, out_rows = first // ratio, last // ratio - first // ratio + 1
+    if (out_rows > 4 * s.row_count + 1024 or y_base * ratio < -(1 << 31)
+            or (y_base + out_rows) * ratio > (1 << 31) - 1):
+        return None
+    return _box_sweep(s, 0, 0, 0, y_base=y_base, out_rows=out_rows, x_lo=-(1 << 31), x_hi=(1 << 31) - 1,
+                      mode=_lib.BOX_RESTRICT, ratio=ratio, compact=True)
 
 
 def translate_interval_set(interval_set: IntervalSet, dx: int = 0, dy: int = 0) -> IntervalSet:
@@ -391,7 +408,7 @@ def erode_interval_set(interval_set: IntervalSet, halo_x: int = 1, halo_y: int =
         raise ValueError("width must be positive and height must be non-negative")
     if halo_x >= 0 and halo_y >= 0 and height > 0 and int(interval_set.begin.shape[0]) > 0:
         out = _box_sweep(interval_set, int(halo_y), int(halo_x), int(halo_x), y_base=0, out_rows=int(height), x_lo=0,
-                         x_hi=int(width), erode=True)
+                         x_hi=int(width), mode=_lib.BOX_ERODE)
         if out is not None:
             return out
     base = clip_interval_set(interval_set, width=width, height=height)

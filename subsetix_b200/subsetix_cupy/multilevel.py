@@ -5,11 +5,13 @@ of the reference.  The device work is new:
 
 * ``prolong_set`` writes ``[b*r, e*r)`` on rows ``row*r + d`` directly at
   their final positions (``sx_prolong_set``): no repeat, sort or unique.
-* ``restrict_set`` aligns each group of ``r`` fine rows onto its coarse row
-  (``sx_align_rows`` with ``div = r``), then merges the coarsened intervals
-  ``[floor(b/r), ceil(e/r))`` of the ``r`` sub-rows in one union-mode sweep.
-* ``prolong_field`` and ``restrict_field`` run one warp per coarse interval
-  and keep the reference's summation order (``sx_prolong_field``,
+* ``restrict_set`` merges the coarsened intervals ``[floor(b/r), ceil(e/r))``
+  of the ``r`` sub-rows under every coarse row in one launch for ratios 2 to 4
+  (``sx_box_sweep``); other ratios and sparse rows align each group of ``r``
+  fine rows onto its coarse row (``sx_align_rows`` with ``div = r``) and take
+  one union-mode sweep.
+* ``prolong_field`` and ``restrict_field`` run blocks of coarse rows and keep
+  the reference's summation order (``sx_prolong_field``,
   ``sx_restrict_field``).  Float64 fields are kept in float64 when
   ``dtype=np.float64`` is requested, an addition of this package.  The
   reference always returns float32.
@@ -28,8 +30,8 @@ import torch
 from .. import _core, _lib
 from .._runtime import like
 from .expressions import IntervalSet, _t, evaluate, make_difference, make_input
-from .interval_field import IntervalField, create_interval_field, torch_dtype
-from .morphology import _build_interval_set_from_rows, _empty_set, _wrap
+from .interval_field import IntervalField, _is_packed, _offsets_of, _unset_interval_field, create_interval_field, torch_dtype
+from .morphology import _box_restrict, _build_interval_set_from_rows, _empty_set, _wrap
 
 I32 = torch.int32
 _MAX_SUBROWS = 9  # leaves per union sweep
@@ -139,25 +141,31 @@ class MultiLevelField2D:
 # Sets
 # ---------------------------------------------------------------------------
 
-def _prolong_set_impl(interval_set: IntervalSet, ratio: int) -> IntervalSet:
-    """``[b*r, e*r)`` on rows ``row*r + 0..r-1`` of every occupied row (``multilevel.py:213-264``)."""
+def _prolong_set_impl(interval_set: IntervalSet, ratio: int, cells: bool = False):
+    """``[b*r, e*r)`` on rows ``row*r + 0..r-1`` of every occupied row (``multilevel.py:213-264``).
+
+    With ``cells`` returns ``(set, cell offsets, cells, rising)``; rising: no
+    row's begins fall, so fine interval ``o`` of a row is its coarse interval ``o``.
+    """
     if ratio < 1:
         raise ValueError("ratio must be >= 1")
     s = interval_set
-    if ratio == 1:
-        return s
     r = int(ratio)
     device = _t(s.row_offsets).device
     R = s.row_count
     n = int(s.begin.shape[0])
-    if R == 0 or n == 0:
-        if R > 0:
-            rows_out = (_t(s.rows)[:, None] * r + torch.arange(r, dtype=I32, device=device)[None, :]).reshape(-1)
+    if r == 1 or R == 0 or n == 0:
+        if r == 1:
+            out = s
         else:
-            rows_out = torch.zeros(0, dtype=I32, device=device)
-        return _empty_set(device, rows_out.to(I32), s.begin)
-    rows_out, off, ob, oe, unsorted = _core.prolong_set(_t(s.rows), _t(s.row_offsets), _t(s.begin), _t(s.end), r,
-                                                        device)
+            if R > 0:
+                rows_out = (_t(s.rows)[:, None] * r + torch.arange(r, dtype=I32, device=device)[None, :]).reshape(-1)
+            else:
+                rows_out = torch.zeros(0, dtype=I32, device=device)
+            out = _empty_set(device, rows_out.to(I32), s.begin)
+        return (out, *_offsets_of(out)[:2], False) if cells else out
+    rows_out, off, ob, oe, unsorted, *more = _core.prolong_set(_t(s.rows), _t(s.row_offsets), _t(s.begin), _t(s.end), r,
+                                                               device, cells=cells)
     if unsorted:
         # The reference sorts each output row by begin (a stable lexsort);
         # rows whose begins decrease need the same stable order here.
@@ -166,7 +174,10 @@ def _prolong_set_impl(interval_set: IntervalSet, ratio: int) -> IntervalSet:
         key = (per.to(torch.int64) << 32) | (ob.to(torch.int64) + (1 << 31))
         order = torch.sort(key, stable=True).indices
         ob, oe = ob[order], oe[order]
-    return _wrap(s.begin, ob, oe, off, rows_out)
+        if cells:
+            more = _core.cell_offsets(ob, oe, device)
+    out = _wrap(s.begin, ob, oe, off, rows_out)
+    return (out, *more, not unsorted) if cells else out
 
 
 def prolong_set(interval_set: IntervalSet, ratio: int) -> IntervalSet:
@@ -199,6 +210,9 @@ def restrict_set(interval_set: IntervalSet, ratio: int) -> IntervalSet:
         return _empty_set(device, None, s.begin)
     if int(s.begin.shape[0]) == 0:
         return _empty_set(device, torch.unique(torch.div(_t(s.rows), r, rounding_mode="floor")).to(I32), s.begin)
+    out = _box_restrict(s, r)
+    if out is not None:
+        return out
     if r > _MAX_SUBROWS:
         return _restrict_reference_order(s, r)
     rows, off = _t(s.rows), _t(s.row_offsets)
@@ -218,16 +232,17 @@ def restrict_set(interval_set: IntervalSet, ratio: int) -> IntervalSet:
     return _wrap(s.begin, ob[:total].clone(), oe[:total].clone(), ooff, rows_out)
 
 
-def _check_coarse_fine(coarse: IntervalSet, fine: IntervalSet, ratio: int, device, with_bounds: bool) -> None:
-    """The reference's alignment checks, in its order (``multilevel.py:169-210,433-451``)."""
-    cs = (_t(coarse.rows), _t(coarse.row_offsets), _t(coarse.begin), _t(coarse.end))
-    fs = (_t(fine.rows), _t(fine.row_offsets), _t(fine.begin), _t(fine.end))
-    flags = _core.coarse_fine_check(cs, fs, ratio, device)
+def _parts(s: IntervalSet) -> tuple:
+    return _t(s.rows), _t(s.row_offsets), _t(s.begin), _t(s.end)
+
+
+def _raise_misaligned(flags: int) -> None:
+    """The reference's alignment errors, in its order (``multilevel.py:169-210,433-451``)."""
     if flags & 1:
         raise ValueError("fine set row count does not match coarse x ratio")
     if flags & 2:
         raise ValueError("fine set rows do not align with refinement ratio")
-    if with_bounds and flags & 8:
+    if flags & 8:
         raise ValueError("fine field is not aligned with coarse geometry for restriction")
 
 
@@ -254,17 +269,21 @@ def prolong_field(field: IntervalField, ratio: int, *, dtype=None) -> IntervalFi
         raise ValueError("ratio must be >= 1")
     out_t = _value_dtype(dtype)
     coarse = field.interval_set
-    fine_set = _prolong_set_impl(coarse, ratio)
-    fine_field = create_interval_field(fine_set, fill_value=0.0, dtype=out_t)
+    fine_set, fine_off, total, rising = _prolong_set_impl(coarse, ratio, cells=True)
+    fine_field = _unset_interval_field(fine_set, out_t, fine_off, total)
     fv = _t(fine_field.values)
     cv = _t(field.values)
-    if fv.numel() == 0 or cv.numel() == 0:
+    if fv.numel() == 0:
+        return fine_field
+    if cv.numel() == 0:
+        fv.zero_()
         return fine_field
     if ratio == 1:
         fv.copy_(cv.to(out_t))
         return fine_field
     n = int(coarse.begin.shape[0])
     if n == 0:
+        fv.zero_()
         return fine_field
     device = fv.device
     # The reference's mapping check (multilevel.py:184-205) fails exactly
@@ -272,6 +291,8 @@ def prolong_field(field: IntervalField, ratio: int, *, dtype=None) -> IntervalFi
     # When the counts agree, the fine rows are coarse_row*r + d by construction.
     if int(fine_set.rows.shape[0]) != coarse.row_count * int(ratio):
         raise ValueError("fine set row count does not match coarse x ratio")
+    if not (rising and _is_packed(field)):
+        fv.zero_()  # fine intervals re-sorted within a row, or offsets of unknown origin: some cells may stay unwritten
     _core.prolong_field(_t(coarse.row_offsets), _t(field.interval_cell_offsets), n, _t(fine_set.row_offsets),
                         _t(fine_field.interval_cell_offsets), int(ratio), cv.to(out_t).contiguous(), fv, device)
     return fine_field
@@ -287,12 +308,25 @@ def restrict_field(field: IntervalField, ratio: int, *, reducer: str = "mean", d
     out_t = _value_dtype(dtype)
     fine_set = field.interval_set
     coarse_set = restrict_set(fine_set, ratio)
-    coarse_field = create_interval_field(coarse_set, fill_value=0.0, dtype=out_t)
+    r, n = int(ratio), int(coarse_set.begin.shape[0])
+    device = _t(coarse_set.row_offsets).device
+    check = 0
+    if n and r > 1:  # the cell total and the alignment check come back in one read
+        res = _core.empty_i32(3, device)
+        off, _ = _core.cell_offsets(_t(coarse_set.begin), _t(coarse_set.end), device, sync=False, result=res)
+        _core.coarse_fine_check(_parts(coarse_set), _parts(fine_set), r, device, flags=res[2:])
+        total, scan_flags, check = res.tolist()
+        _core.check_scan(scan_flags, "sx_cell_offsets")
+        coarse_field = _unset_interval_field(coarse_set, out_t, off, total)
+    else:
+        coarse_field = _unset_interval_field(coarse_set, out_t)
     fv = _t(field.values)
     cv = _t(coarse_field.values)
-    if fv.numel() == 0 or cv.numel() == 0:
+    if cv.numel() == 0:
         return coarse_field
-    r = int(ratio)
+    if fv.numel() == 0:
+        cv.zero_()
+        return coarse_field
     if r <= 0:
         raise ValueError("ratio must be >= 1")
     if r == 1:
@@ -301,11 +335,7 @@ def restrict_field(field: IntervalField, ratio: int, *, reducer: str = "mean", d
     code = _REDUCER_CODES.get(reducer)
     if code is None:
         raise ValueError(f"unsupported reducer '{reducer}'")
-    n = int(coarse_set.begin.shape[0])
-    if n == 0:
-        return coarse_field
-    device = cv.device
-    _check_coarse_fine(coarse_set, fine_set, r, device, with_bounds=True)
+    _raise_misaligned(check)
     _core.restrict_field(_t(coarse_set.row_offsets), _t(coarse_field.interval_cell_offsets), n,
                          _t(fine_set.row_offsets), _t(field.interval_cell_offsets), r, code,
                          fv.to(out_t).contiguous(), cv, device)
