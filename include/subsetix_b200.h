@@ -43,7 +43,7 @@ typedef enum sx_status {
 
 /* Device flag bits reported in result[1]. */
 #define SX_FLAG_CONTRACT 1u  /* input outside the fused path's contract: rerun the exact path */
-#define SX_FLAG_LONG_TILE 2u /* a row tile exceeded the shared-memory cap: rerun the exact path */
+#define SX_FLAG_LONG_TILE 2u /* rows too long or too wide for sx_bool_eval_even: rerun with sx_bool_eval */
 #define SX_FLAG_CAPACITY 4u  /* output capacity exceeded (outputs truncated) */
 #define SX_FLAG_TIMEOUT 8u   /* a bounded device wait gave up (results invalid) */
 
@@ -95,14 +95,15 @@ typedef struct sx_leaf {
  * merge-path tile kernel, 4 = segmented sweep in block tiles, 5 = segmented
  * sweep in warp tiles (table mode; the default), 6 = kernel 5 with 16-bit
  * keys (tiles of at most 8 rows; wider-spanning tiles take the row sweep),
- * 7 = row-lane sweep (a warp per 32-row tile, a lane per row, 16-bit
- * coordinates in shared memory; tiles spanning more than 65534 columns take
- * the row sweep over global memory);
+ * 7 = row-lane sweep (a warp per tile of 8, 16 or 32 rows, its lanes dealt out
+ * to the rows, 16-bit coordinates in shared memory; tiles above staging_cap
+ * are swept in groups of rows, groups spanning more than 65534 columns with
+ * 32-bit coordinates);
  * blocks_per_sm: residency cap of the global sweep; staging_cap: elements per
  * warp of the staged sweep, or boundaries per tile of kernels 3 to 7; warps:
  * warps per block of kernels 4 to 7 (in 5 to 7 each warp owns a tile);
  * tile_rows: rows per tile of kernels 4 to 6 (at most 32, at most 8 for 6;
- * kernel 7 takes 0 or 32).  Results never depend on the tuning.
+ * kernel 7 takes 0, 8, 16 or 32).  Results never depend on the tuning.
  * Two fields exist for tests of the failure path and are zero otherwise:
  * wait_limit caps the polls of every look-back wait of kernels 4 to 7 (0 =
  * the built-in limit of 2^22 polls); withhold_tile = t + 1 makes tile t of
@@ -130,6 +131,17 @@ int sx_bool_eval(const sx_leaf* leaves /* host array of k */, int k, int32_t row
                  int mode, int32_t* out_begin, int32_t* out_end, int32_t* out_offsets, int64_t capacity,
                  int32_t* result, void* workspace, size_t workspace_bytes, const sx_tuning* tuning /* host */,
                  void* stream);
+
+/* sx_bool_eval with SX_MODE_TABLE and kernel 7 (which tuning must name), for
+ * operands expected to have even rows: a row that does not fit staging_cap
+ * alone, or a group of rows spanning more than 65534 columns, ends the sweep
+ * with SX_FLAG_LONG_TILE in result[1] and undefined outputs instead of being
+ * swept slowly; the caller then runs sx_bool_eval.  It saves the pass that
+ * would have to look for such tiles first. */
+int sx_bool_eval_even(const sx_leaf* leaves /* host array of k */, int k, int32_t rows,
+                      const uint32_t* table /* host, 8 words */, int32_t* out_begin, int32_t* out_end,
+                      int32_t* out_offsets, int64_t capacity, int32_t* result, void* workspace,
+                      size_t workspace_bytes, const sx_tuning* tuning, void* stream);
 
 /* Largest number of leaf boundaries (2 x intervals, summed over the leaves)
  * in one tile of tile_rows_a aligned rows (out[0]) and of tile_rows_b aligned

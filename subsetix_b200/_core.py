@@ -29,6 +29,8 @@ OP_UNION, OP_INTERSECTION, OP_DIFFERENCE = 0, 1, 2
 TUNING: dict = {}
 TUNED: dict = {}
 
+_TILE_INTERVALS = 1600  # a mean tile of the automatic row-lane sweep (13 KB of shared memory)
+
 
 def workload_key(sizes: Sequence[int], rows: int) -> str:
     """Bucket of a set-algebra workload: leaf count, log2 rows, log2 mean boundaries per 32-row tile."""
@@ -81,23 +83,45 @@ def _default_keys(leaves, rows: int, tile_rows: int = 32) -> int:
 
 
 def auto_tuning(leaves, rows: int, device) -> dict:
-    """The automatic launch shape of a truth-table sweep (one launch and one read-back, two when rows are skewed).
+    """The launch shape of a truth-table sweep measured on its operands (one launch and one read-back, two when rows are skewed).
 
     Even rows (the largest 8-row tile within 3x the mean plus 256
-    boundaries): the row-lane sweep on 16-row tiles, two lanes per row, when
-    every such tile spans at most 65534 columns (16-bit coordinates), else
-    8-row warp tiles with 32-bit keys; buffers are sized for the largest tile,
-    so no tile leaves the staged sweep.  Skewed rows: 32-row block tiles
-    sized for their largest tile, which evens out the load.
+    boundaries): the row-lane sweep on 16-row tiles when every such tile
+    spans at most 65534 columns (16-bit coordinates), else 8-row warp tiles
+    with 32-bit keys; buffers are sized for the largest tile, so no tile
+    leaves the staged sweep (tiles that no buffer holds: 8 rows, for twice
+    the warps).  Skewed rows: 32-row block tiles sized for their
+    largest tile, which evens out the load.
     """
     need16, need8, span16 = tile_stats(leaves, rows, device, 16, 8)
     mean8 = 2 * sum(int(leaf[0].numel()) for leaf in leaves) / max(1, (rows + 7) // 8)
     if need8 <= 3 * mean8 + 256:
         if span16 <= 65534:
-            return {"kernel": 7, "staging_cap": min(need16, 25000), "tile_rows": 16, "warps": 2}
+            return {"kernel": 7, "staging_cap": min(need16, 25000), "tile_rows": 16 if need16 <= 25000 else 8,
+                    "warps": 2}
         return {"kernel": 5, "staging_cap": min(need8, 25000), "tile_rows": 8, "warps": 2}
     need32 = max_tile_boundaries(leaves, rows, device, tile_rows=32)
     return {"kernel": 4, "staging_cap": min(need32, 25000), "tile_rows": 32, "warps": 4}
+
+
+def even_tuning(leaves, rows: int) -> dict:
+    """The launch shape of ``sx_bool_eval_even``, from the operands' sizes alone.
+
+    The row-lane sweep on tiles of 16 rows, or 8 when rows are so long that a
+    mean tile would exceed ``_TILE_INTERVALS``.  Slices hold the mean tile and
+    a tenth more, or, for light tiles, where room costs no residency, two and
+    a half times the mean; the tiles above that are swept in groups of rows
+    by the same launch.  Measured: five shape leaves over 128 copies of 4096
+    rows (mean 16-row tile 1155 intervals, largest 1253) 421 us with 16 rows,
+    433 us with 8, 474 us with 32, 615 us when the slices fall short of the
+    largest tiles; 163 uneven small sets (mean 236, largest 954) 464 us with
+    2.5 times the mean, 500 us with 1.5 times.
+    """
+    total = sum(int(leaf[0].numel()) for leaf in leaves)
+    tr = 16 if 16 * total <= _TILE_INTERVALS * rows else 8
+    mean = tr * total // max(1, rows)
+    room = max(mean + mean // 10 + 48, min(5 * mean // 2, 600))
+    return {"kernel": 7, "staging_cap": min(2 * room, 25000), "tile_rows": tr, "warps": 2}
 
 
 def bool_eval(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]], rows: int, table: Sequence[int],
@@ -119,6 +143,17 @@ def bool_eval(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, i
             tr = int(tuning.get("tile_rows", 0)) or {5: 8, 6: 8, 7: 16}.get(tuning["kernel"], 32)
             tuning["staging_cap"] = min(max_tile_boundaries(leaves, rows, device, tile_rows=tr), 25000)
     elif mode == _lib.MODE_TABLE and not TUNING and rows > 0:
+        # Most operands have rows alike, and the sweep that assumes it needs no pass that
+        # measures them first (59 us and a read-back beside a 270 us sweep of 5 x 128 x 4096
+        # rows; 35 us of 160 at 256 rows).  It gives up early on others (rows too long, or
+        # too wide for 16-bit coordinates); those are measured and swept again, 70 to 110 us
+        # later than if they had been measured first.
+        ob, oe, ooff, result = bool_eval_async(leaves, rows, table, mode, device, out,
+                                               tuning=even_tuning(leaves, rows), even=True)
+        total, flags = read_pair(result)
+        if flags != _lib.FLAG_LONG_TILE:
+            return ob, oe, ooff, total, flags
+        out = (ob, oe)
         tuning = auto_tuning(leaves, rows, device)
     ob, oe, ooff, result = bool_eval_async(leaves, rows, table, mode, device, out, tuning=tuning)
     if result is None:
@@ -130,8 +165,8 @@ def bool_eval(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, i
 def bool_eval_async(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]], rows: int,
                     table: Sequence[int], mode: int, device, out: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
                     result: Optional[torch.Tensor] = None, offsets: Optional[torch.Tensor] = None,
-                    tuning: Optional[dict] = None, scratch: Optional[torch.Tensor] = None):
-    """Enqueue the row sweep without waiting.
+                    tuning: Optional[dict] = None, scratch: Optional[torch.Tensor] = None, even: bool = False):
+    """Enqueue the row sweep without waiting (``even``: ``sx_bool_eval_even``, a truth table with a kernel 7 tuning).
 
     Returns ``(begin, end, offsets, result)``; ``result`` is the device pair
     ``(total, flags)``, or None when there are no rows.  ``scratch`` (bytes,
@@ -177,8 +212,12 @@ def bool_eval_async(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Ten
     tun = _lib.SxTuning(int(t.get("kernel", 0)), int(t.get("blocks_per_sm", 0)), int(t.get("staging_cap", 0)),
                         int(t.get("warps", 0)), int(t.get("tile_rows", 0)), int(t.get("wait_limit", 0)),
                         int(t.get("withhold_tile", 0)))
-    rc = lib.sx_bool_eval(arr, k, int(rows), tab, int(mode), ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp, wsn,
-                          ctypes.byref(tun), stream_handle(device))
+    if even:
+        rc = lib.sx_bool_eval_even(arr, k, int(rows), tab, ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp, wsn,
+                                   ctypes.byref(tun), stream_handle(device))
+    else:
+        rc = lib.sx_bool_eval(arr, k, int(rows), tab, int(mode), ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp,
+                              wsn, ctypes.byref(tun), stream_handle(device))
     _lib.check(rc, "sx_bool_eval")
     return ob, oe, ooff, result
 

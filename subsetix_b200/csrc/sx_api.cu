@@ -56,9 +56,9 @@ size_t sx_bool_workspace_bytes(int32_t rows)
     return sx_sweep_state_bytes(r);  // the look-back state of 1-row tiles: every tuning fits
 }
 
-int sx_bool_eval(const sx_leaf* leaves, int k, int32_t rows, const uint32_t* table, int mode, int32_t* out_begin,
-                 int32_t* out_end, int32_t* out_offsets, int64_t capacity, int32_t* result, void* workspace,
-                 size_t workspace_bytes, const sx_tuning* tuning, void* stream)
+static int bool_eval(const sx_leaf* leaves, int k, int32_t rows, const uint32_t* table, int mode, int32_t* out_begin,
+                     int32_t* out_end, int32_t* out_offsets, int64_t capacity, int32_t* result, void* workspace,
+                     size_t workspace_bytes, const sx_tuning* tuning, int give_up, void* stream)
 {
     if (mode != SX_MODE_TABLE && mode != SX_MODE_UNION)
         return fail(SX_ERR_INVALID, "sx_bool_eval: unknown mode %d", mode);
@@ -90,6 +90,7 @@ int sx_bool_eval(const sx_leaf* leaves, int k, int32_t rows, const uint32_t* tab
     }
     A.k = k;
     A.rows = rows;
+    A.give_up = give_up;
     for (int i = 0; i < 8; ++i) A.table[i] = table ? table[i] : 0u;
     A.out_begin = out_begin;
     A.out_end = out_end;
@@ -124,6 +125,24 @@ int sx_bool_eval(const sx_leaf* leaves, int k, int32_t rows, const uint32_t* tab
     cudaError_t err = sx_sweep_launch(A, mode == SX_MODE_UNION, workspace, workspace_bytes, (cudaStream_t)stream);
     if (err != cudaSuccess) return cuda_fail(err, "sx_bool_eval");
     return SX_OK;
+}
+
+int sx_bool_eval(const sx_leaf* leaves, int k, int32_t rows, const uint32_t* table, int mode, int32_t* out_begin,
+                 int32_t* out_end, int32_t* out_offsets, int64_t capacity, int32_t* result, void* workspace,
+                 size_t workspace_bytes, const sx_tuning* tuning, void* stream)
+{
+    return bool_eval(leaves, k, rows, table, mode, out_begin, out_end, out_offsets, capacity, result, workspace,
+                     workspace_bytes, tuning, 0, stream);
+}
+
+int sx_bool_eval_even(const sx_leaf* leaves, int k, int32_t rows, const uint32_t* table, int32_t* out_begin,
+                      int32_t* out_end, int32_t* out_offsets, int64_t capacity, int32_t* result, void* workspace,
+                      size_t workspace_bytes, const sx_tuning* tuning, void* stream)
+{
+    if (!tuning || tuning->kernel != 7)
+        return fail(SX_ERR_INVALID, "sx_bool_eval_even: needs a tuning with kernel 7, the row-lane sweep");
+    return bool_eval(leaves, k, rows, table, SX_MODE_TABLE, out_begin, out_end, out_offsets, capacity, result,
+                     workspace, workspace_bytes, tuning, 1, stream);
 }
 
 int sx_tile_boundaries_max(const sx_leaf* leaves, int k, int32_t rows, int32_t tile_rows_a, int32_t tile_rows_b,

@@ -17,7 +17,7 @@
 
 // Bits of the device flag word that kernels raise.
 #define SXF_CONTRACT 1u   // input outside the fast path's contract: rerun the exact path
-#define SXF_LONG_TILE 2u  // reserved: a tile exceeded a capacity limit
+#define SXF_LONG_TILE 2u  // a row too long, or a tile too wide, for the staged sweep that was asked for
 #define SXF_CAPACITY 4u   // an output would have exceeded the caller's capacity
 #define SXF_TIMEOUT 8u    // a bounded wait gave up (look-back predecessor never published)
 

@@ -41,6 +41,7 @@ struct SxBoolArgs {
     int tune_warps;      // segmented sweeps: warps per block
     int tune_tile_rows;  // segmented sweeps: rows per tile (at most 32; 8 for kernel 6)
     unsigned wait_limit; // look-back polls before giving up (0: SX_LOOKBACK_SPIN_LIMIT); tests of the failure path
+    int give_up;         // row-lane sweep: report SXF_LONG_TILE instead of sweeping tiles that cannot be staged
     int withhold_tile;   // t + 1: tile t never publishes its look-back status (tests of the failure path)
 };
 

@@ -2055,11 +2055,15 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 }
 
 // ---------------------------------------------------------------------------
-// Row-lane sweep with 16-bit coordinates (sx_tuning kernel 7).
+// Row-lane sweep with 16-bit coordinates (sx_tuning kernel 7, the automatic
+// choice).
 //
-// A warp owns a tile of 32 aligned rows and lane r sweeps row r, so a step
-// needs no combined (row, x) keys, no piece search and no search for the
-// row offsets of the output.
+// A warp owns a tile of up to 32 aligned rows and its lanes are dealt out to the
+// rows: the same number each, or, once a row holds twice its share of the
+// intervals, one each and the others in proportion.  A row's lanes sweep it in
+// pieces, so a step needs no combined (row, x) keys and the output row offsets
+// come from a scan, and skewed rows even out inside the tile (with a fixed number
+// of lanes per row a warp waits for its longest row).
 //
 // Staging.  One bulk copy per leaf array (begins, ends) into the warp's
 // slice of shared memory, above a gap; then interval j of leaf l becomes the
@@ -2073,10 +2077,9 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // while the raw copies above are read: a pair is written at most 31 + 25 l
 // words above its own raw begin's distance from the slice start, below every
 // raw word not yet read.  xmin is the tile's smallest first begin and xmax
-// its largest last end; a tile with xmax - xmin > 65534 takes the
-// global-memory sweep, and a coordinate outside [xmin, xmin + 65534] in a
-// narrower tile breaks the contract (on canonical rows every coordinate lies
-// between its row's first begin and last end).
+// its largest last end; a coordinate outside [xmin, xmin + 65534] in a tile
+// with xmax - xmin <= 65534 breaks the contract (on canonical rows every
+// coordinate lies between its row's first begin and last end).
 //
 // Step: the smallest head c; each leaf whose head equals c toggles its state
 // bit and loads its next halfword (predicated, no divergence); f(state) from
@@ -2084,11 +2087,27 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // rise strictly, so one compare per step checks the contract (non-empty,
 // sorted, non-touching intervals).  Row r's output halfwords go to an area
 // as large as its input plus one word (the dead raw copies).  A scan of the
-// per-row counts gives the row offsets, the look-back the tile's base; the
+// per-piece counts gives the row offsets, the look-back the tile's base; the
 // lanes pack their output words over the dead pair lists and the warp writes
 // them out coalesced.  Every wait is bounded.
+//
+// A tile whose lists exceed the slice is swept in groups of rows that fit, twice
+// (count, then write).  Groups that span more than 65534 columns, and rows that do
+// not fit alone, are swept by the same lanes over the raw 32-bit arrays
+// (sxr_raw_piece), or, where the caller asked for it (sx_bool_eval_even), end the
+// sweep with SXF_LONG_TILE: a warp takes 2 to 10 times as long over them as the
+// segmented sweeps.  So no pass over the input is needed before the launch to size
+// the slices for the largest tile and to look for wide tiles; such a pass took 59 us
+// of kernel and a read-back beside the 270 us sweep of the five-leaf shape expression
+// over 128 copies of 4096 rows (466 us in all; 410 us without it, with the sweep at
+// 288 us).  The sweep is bound by the latency of a tile's stages: 18 warps per SM are
+// all that the slices leave room for.
+//
+// Registers: 80 for five leaves, which costs no residency beside the slices (at 48
+// the same sweep took 319 us), 64 for up to four (two leaves, 163 small sets: 91 us;
+// 94 us at 80).  The grouped sweep is out of line: inlined it took 121 registers and
+// 346 us.
 // ---------------------------------------------------------------------------
-#define SXR_TR 32
 #define SXR_SPAN 65534
 #define SXR_SENTINEL 0xFFFFu
 #define SXR_HDR_WORDS 4
@@ -2103,7 +2122,7 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // region's 2 (n + 8 k) words: k (tr + 1) + tr - 16 k.
 __host__ __device__ inline int sxr_gap_words(int k, int tr)
 {
-    const int lists = (k - 1) * (tr - 7) + tr;
+    const int lists = (tr > 7 ? (k - 1) * (tr - 7) : 0) + tr;
     const int outputs = k * (tr + 1) + tr - 16 * k;
     return ((lists > outputs ? lists : outputs) + 4 + 3) & ~3;
 }
@@ -2137,61 +2156,161 @@ __device__ __forceinline__ unsigned sxr_min_head(const unsigned* h)
     return c;
 }
 
-// A tile of 32 / LPR rows: lanes LPR r .. LPR r + LPR - 1 sweep row r in
-// pieces [p_i, p_{i+1}) of its keys, the pivots p_i being halfwords of the
-// row's longest leaf at positions i m / LPR (m its boundaries).  A piece
-// starts in every other leaf at the first key not below p_i (a binary search
-// within the row) with the parity of that position as the leaf's state bit,
-// and writes at most as many outputs as it reads inputs, so piece i's output
-// area starts where the inputs of the pieces before it end.  Consecutive
+// One piece of a row over raw begins and ends (global or staged): boundaries
+// p0[l] .. pe[l] - 1 of every leaf, boundary 2 i being the begin of the row's
+// interval i and 2 i + 1 its end.  Coordinates must rise strictly inside
+// [klo, khi).  Returns the changes of f; with WRITE change number r of the row
+// goes to the begins (r even) or ends (r odd) of run r / 2 from rank `first` on.
+template <int K, bool WRITE>
+__device__ int sxr_raw_piece(const SxBoolArgs& A, const int* const (&B)[K], const int* const (&E)[K],
+                             const int (&p0)[K], const int (&pe)[K], long long klo, long long khi, long long first,
+                             bool& bad)
+{
+    int pos[K], h[K];
+    unsigned state = 0u;
+    int rem = 0;
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        pos[l] = p0[l];
+        state |= (unsigned)(p0[l] & 1) << l;
+        if (pe[l] < p0[l]) bad = true;
+        else rem += pe[l] - p0[l];
+        h[l] = pos[l] < pe[l] ? (pos[l] & 1 ? E[l] : B[l])[pos[l] >> 1] : INT_MAX;
+    }
+    if (bad) return 0;
+    bool fprev = sx_table(A, state);
+    long long cprev = klo - 1;
+    int n = 0;
+    while (rem > 0) {
+        int c = INT_MAX;
+#pragma unroll
+        for (int l = 0; l < K; ++l) c = min(c, h[l]);
+        bad = bad || c <= cprev || c >= khi;
+        cprev = c;
+#pragma unroll
+        for (int l = 0; l < K; ++l) {
+            if (h[l] == c && pos[l] < pe[l]) {
+                state ^= 1u << l;
+                --rem;
+                const int q = ++pos[l];
+                h[l] = q < pe[l] ? (q & 1 ? E[l] : B[l])[q >> 1] : INT_MAX;
+            }
+        }
+        const bool f = sx_table(A, state);
+        if (f != fprev) {
+            if (WRITE) {
+                const long long r = first + n, o = r >> 1;
+                if (o < A.capacity) (r & 1 ? A.out_end : A.out_begin)[o] = c;
+            }
+            ++n;
+        }
+        fprev = f;
+    }
+    return n;
+}
+
+// First boundary of a row (cnt of them) whose coordinate is not below v.
+__device__ __forceinline__ int sxr_raw_lower(const int* B, const int* E, int cnt, long long v)
+{
+    int lo = 0, hi = cnt;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if ((mid & 1 ? E : B)[mid >> 1] < v) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// A row of m boundaries in its longest leaf and L lanes: piece i takes the keys
+// [p_i, p_{i+1}), the pivots p_i being halfwords of that leaf at positions
+// i m / L.  A piece starts in every other leaf at the first key not below p_i (a
+// binary search within the row) with the parity of that position as the leaf's
+// state bit, and writes at most as many outputs as it reads inputs, so piece i's
+// output area starts where the inputs of the pieces before it end.  Consecutive
 // pieces must meet: each piece's end positions are checked against the next
 // piece's start positions (with the per-piece rising keys, that checks the
 // contract across pieces).
-template <int K, int LPR>
-__global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepState st, int tiles, int cap_words)
-{
-    extern __shared__ __align__(16) unsigned char sxr_smem[];
-    constexpr int TR = SXR_TR / LPR;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, NW = blockDim.x >> 5;
-    if (blockIdx.x * NW + wid >= tiles) return;  // exactly `tiles` warps take tickets
-    unsigned* base_w = (unsigned*)(sxr_smem + (size_t)wid * sxr_slice_bytes(cap_words));
-    unsigned long long* bar = (unsigned long long*)base_w;
-    unsigned* const W = base_w + SXR_HDR_WORDS;  // pair lists, then the output areas
-    unsigned short* const h16 = (unsigned short*)W;
-    const int gap = sxr_gap_words(K, TR);
-    unsigned* const raw = W + gap;  // the bulk copies
-    const int row = lane / LPR, piece = lane % LPR;
-    const int first_lane = row * LPR;
+// What a group of rows leaves for its writing: this lane's piece, its changes of f
+// (khw, excl before it in the group), and where the staged ones lie.
+template <int K>
+struct SxrRaw {
+    int rp0[K], rpe[K];
+    long long rlo, rhi;
+    const int *RB[K], *RE[K];
+};
 
-    int tile = 0;
-    if (lane == 0) {
-        tile = (int)atomicAdd(&st.counters[0], 1u);
-        sxs_bar_init(bar);
-    }
-    tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
-    const int r0 = tile * TR;
-    const int nrows = min(TR, A.rows - r0);
-    const bool act = row < nrows;
-    // this lane's row in every leaf, relative to the tile's first interval
+template <int K>
+struct SxrGroup {
+    int row, khw, excl, total, src, xmin;  // src: halfword of the piece's staged changes
+    bool act, last, staged, broken, ok;
+    SxrRaw<K>* raw;
+};
+
+// One group: rows q0 .. q0 + gn - 1, at most `room` intervals (more, in a single
+// row, are not staged).  Without RAW a group that cannot be staged is only
+// reported (G.staged false).
+template <int K, bool RAW>
+__device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, int TR, int room, unsigned* W, unsigned* raw,
+                                          unsigned long long* bar, unsigned& use, unsigned& flags,
+                                          SxrGroup<K>& G)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned short* const h16 = (unsigned short*)W;
+    // lane r: row r of the group in every leaf, relative to the group's first interval
     int lo[K], hi[K], n[K], g0[K];
-    bool ok = true;
-    long long RBl = 0, PBl = 0;
+    int PBl = 0, mine = 0, all = 0;
+    bool ok = true;  // row offsets must rise
 #pragma unroll
     for (int l = 0; l < K; ++l) {
-        const int a = A.leaf[l].off[r0 + min(row, nrows)];
-        const int b = A.leaf[l].off[r0 + min(row + 1, nrows)];
-        g0[l] = __shfl_sync(0xFFFFFFFFu, a, 0);
-        n[l] = __shfl_sync(0xFFFFFFFFu, b, (nrows - 1) * LPR) - g0[l];
-        lo[l] = act ? a - g0[l] : n[l];
-        hi[l] = act ? b - g0[l] : n[l];
-        ok = ok && lo[l] >= 0 && lo[l] <= hi[l] && hi[l] <= n[l];
-        RBl += (long long)((n[l] + 11) & ~3);
-        PBl += (long long)n[l] + TR + 1;
+        lo[l] = A.leaf[l].off[q0 + min(lane, gn)];
+        hi[l] = A.leaf[l].off[q0 + min(lane + 1, gn)];
+        ok = ok && lo[l] >= 0 && lo[l] <= hi[l];
     }
-    ok = __all_sync(0xFFFFFFFFu, ok);  // row offsets must rise through the tile
-    const bool fits = ok && gap + 2 * RBl <= (long long)cap_words;
-    const int OA = (int)PBl;  // output areas start after the pair lists
-    unsigned flags = ok ? 0u : SXF_CONTRACT;
+    ok = __all_sync(0xFFFFFFFFu, ok);
+    if (!ok) flags |= SXF_CONTRACT;
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        g0[l] = __shfl_sync(0xFFFFFFFFu, lo[l], 0);
+        n[l] = ok ? __shfl_sync(0xFFFFFFFFu, hi[l], gn - 1) - g0[l] : 0;
+        lo[l] = ok ? lo[l] - g0[l] : 0;
+        hi[l] = ok ? hi[l] - g0[l] : 0;
+        mine += hi[l] - lo[l];
+        all += n[l];
+        PBl += n[l] + TR + 1;
+    }
+    G.ok = ok;
+    G.staged = false;
+    if (!RAW && ok && all > room) return;
+    const bool fits = ok && all <= room;
+    const int OA = PBl;  // output areas start after the pair lists
+    // The group's lanes dealt out to its rows, every row's leader lane in `leaders`:
+    // the same number each while no row holds twice its share (a row with half the
+    // lanes of its neighbours would hold the warp up for longer than that row),
+    // else one each and the others along the running sum of the rows' intervals.
+    int upper = min(lane + 1, gn) * (32 / gn);  // first lane of the next row
+    if (lane + 1 >= gn) upper = 32;
+    if ((long long)gn * __reduce_max_sync(0xFFFFFFFFu, mine) > 2ll * all) {
+        int part = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, part, o);
+            if (lane >= o) part += y;
+        }
+        upper = min(lane + 1 + (int)floorf((float)part * ((float)(32 - gn) / (float)all) + 0.5f), 32);
+    }
+    int from = __shfl_up_sync(0xFFFFFFFFu, upper, 1);
+    if (lane == 0) from = 0;
+    const int lanes = upper - from;
+    const unsigned leaders = __reduce_or_sync(0xFFFFFFFFu, lane < gn ? 1u << from : 0u);
+    const unsigned upto = leaders & (0xFFFFFFFFu >> (31 - lane));
+    const int row = __popc(upto) - 1, first_lane = 31 - __clz(upto), piece = lane - first_lane;
+    const int L = __shfl_sync(0xFFFFFFFFu, lanes, row);
+    const bool act = ok && piece < L;
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        const int a = __shfl_sync(0xFFFFFFFFu, lo[l], row), b = __shfl_sync(0xFFFFFFFFu, hi[l], row);
+        lo[l] = act ? a : n[l];
+        hi[l] = act ? b : n[l];
+    }
     // 1. bulk copies: lane q < K copies leaf q's begins, lane K + q its ends
     int rb[K], re[K];
 #pragma unroll
@@ -2232,10 +2351,13 @@ __global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepSt
             re[l] = __shfl_sync(0xFFFFFFFFu, first, K + l);
         }
         __syncwarp();
+        // an earlier group's reads and writes of the slice come before the copies
+        if (use) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (lane == 0) sxs_bar_expect(bar, (unsigned)bytes);
         __syncwarp();
         if (len > 0u) sxs_bulk_copy(raw + pos, (const void*)a0, len, bar);
-        copied = __all_sync(0xFFFFFFFFu, sxs_bar_wait(bar));
+        copied = __all_sync(0xFFFFFFFFu, sxs_bar_wait(bar, use & 1u));
+        ++use;
         if (!copied) flags |= SXF_TIMEOUT;
     }
     // 2. the tile's coordinate range: first begin and last end of every row
@@ -2334,9 +2456,12 @@ __global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepSt
             if (l == big) bigw = pb[l] + lo[l] + qr[l];
         const unsigned short* Lb = h16 + 2 * bigw;
         unsigned klo = 0u, khi = SXR_SENTINEL;
-        if (LPR > 1) {
-            klo = piece == 0 ? 0u : (m > 0 ? (unsigned)Lb[(piece * m) / LPR] : SXR_SENTINEL);
-            khi = piece == LPR - 1 ? SXR_SENTINEL : (m > 0 ? (unsigned)Lb[((piece + 1) * m) / LPR] : SXR_SENTINEL);
+        // piece * m / L in floats: neighbours round the same product alike
+        const float part = (float)m / (float)L;
+        const int split = (int)((float)piece * part), next = (int)((float)(piece + 1) * part);
+        if (L > 1) {
+            klo = piece == 0 ? 0u : (m > 0 ? (unsigned)Lb[split] : SXR_SENTINEL);
+            khi = piece == L - 1 ? SXR_SENTINEL : (m > 0 ? (unsigned)Lb[next] : SXR_SENTINEL);
         }
         unsigned state = 0u;
 #pragma unroll
@@ -2344,7 +2469,7 @@ __global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepSt
             const unsigned short* Ll = h16 + 2 * (pb[l] + lo[l] + qr[l]);
             const int cnt = 2 * (hi[l] - lo[l]);
             int pos = 0;
-            if (LPR > 1 && piece > 0) pos = l == big ? (piece * m) / LPR : sxs_lower_bound16(Ll, cnt, klo);
+            if (piece > 0) pos = l == big ? split : sxs_lower_bound16(Ll, cnt, klo);
             if (cnt == 0) pos = 0;
             sa[l] = pa[l] = sxs_saddr(Ll + pos);
             h[l] = pos < cnt ? (unsigned)Ll[pos] : SXR_SENTINEL;
@@ -2370,31 +2495,58 @@ __global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepSt
         }
         khw = (int)((oa - o0) >> 1);
     }
-    if (LPR > 1) {
-        // consecutive pieces of a row meet: this piece ends where the next one starts
+    // consecutive pieces of a row meet: this piece ends where the next one starts
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        const unsigned nxt = __shfl_down_sync(0xFFFFFFFFu, sa[l], 1);
+        if (staged && act && piece < L - 1 && pa[l] != nxt) bad = true;
+    }
+    G.row = row;
+    G.act = act;
+    G.last = act && piece == L - 1;
+    G.staged = staged;
+    G.xmin = xmin;
+    G.src = 2 * (OA + cap_excl) + prov;
+    // groups that cannot be staged: the same pieces over the raw arrays
+    if (RAW && ok && !staged && !A.give_up) {
+        SxrRaw<K>& X = *G.raw;
+        X.rlo = LLONG_MIN + 1;
+        X.rhi = LLONG_MAX;
+        int m = 0, big = 0;
 #pragma unroll
         for (int l = 0; l < K; ++l) {
-            const unsigned nxt = __shfl_down_sync(0xFFFFFFFFu, sa[l], 1);
-            if (staged && act && piece < LPR - 1 && pa[l] != nxt) bad = true;
+            X.RB[l] = (fits && copied ? (const int*)raw + rb[l] : A.leaf[l].begin + g0[l]) + lo[l];
+            X.RE[l] = (fits && copied ? (const int*)raw + re[l] : A.leaf[l].end + g0[l]) + lo[l];
+            X.rp0[l] = 0;
+            X.rpe[l] = 2 * (hi[l] - lo[l]);
+            if (X.rpe[l] > m) {
+                m = X.rpe[l];
+                big = l;
+            }
         }
+        if (act && m > 0) {
+            const int at = (int)((long long)piece * m / L), to = (int)((long long)(piece + 1) * m / L);
+#pragma unroll
+            for (int l = 0; l < K; ++l)
+                if (l == big) {
+                    if (piece > 0) X.rlo = (at & 1 ? X.RE[l] : X.RB[l])[at >> 1];
+                    if (piece < L - 1) X.rhi = (to & 1 ? X.RE[l] : X.RB[l])[to >> 1];
+                }
+#pragma unroll
+            for (int l = 0; l < K; ++l)
+                if (piece > 0) X.rp0[l] = sxr_raw_lower(X.RB[l], X.RE[l], X.rpe[l], X.rlo);
+        }
+#pragma unroll
+        for (int l = 0; l < K; ++l) {
+            const int nxt = __shfl_down_sync(0xFFFFFFFFu, X.rp0[l], 1);
+            if (act && piece < L - 1) X.rpe[l] = nxt;
+        }
+        khw = act ? sxr_raw_piece<K, false>(A, X.RB, X.RE, X.rp0, X.rpe, X.rlo, X.rhi, 0, bad) : 0;
     }
-    if (__any_sync(0xFFFFFFFFu, bad)) {
+    G.broken = __any_sync(0xFFFFFFFFu, bad);
+    if (G.broken) {
         flags |= SXF_CONTRACT;
         khw = 0;  // pieces may overlap on such input: the tile writes nothing
-    }
-    // fallback tile: one lane per row over global memory
-    int s_row[K], lim_row[K];
-    int nint = 0;
-    if (ok && !staged) {
-#pragma unroll
-        for (int l = 0; l < K; ++l) {
-            s_row[l] = g0[l] + lo[l];
-            lim_row[l] = 2 * (hi[l] - lo[l]);
-        }
-        bool fb_bad = false, fb_over = false;
-        if (act && piece == 0) nint = sx_sweep_table<K, false>(A, s_row, lim_row, nullptr, nullptr, 0, fb_bad, fb_over);
-        if (__any_sync(0xFFFFFFFFu, fb_bad)) flags |= SXF_CONTRACT;
-        khw = 2 * nint;
     }
     int incl = khw;
 #pragma unroll
@@ -2402,37 +2554,125 @@ __global__ void __launch_bounds__(256) sx_rlane16_kernel(SxBoolArgs A, SxSweepSt
         const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
         if (lane >= o) incl += y;
     }
-    const int excl = incl - khw;  // halfwords of the pieces before this one
-    const int total = __shfl_sync(0xFFFFFFFFu, incl, 31) >> 1;
-    // 6. look-back, then pack the output halfwords over the dead pair lists
-    const int base = sxs_lookback(A, st, tile, total, flags);
-    bool over = false;
-    if (staged) {
+    G.khw = khw;
+    G.excl = incl - khw;
+    G.total = __shfl_sync(0xFFFFFFFFu, incl, 31) >> 1;
+}
+
+// Writes a group's runs from rank `at` on, and its row offsets.
+template <int K, bool RAW>
+__device__ __forceinline__ void sxr_put(const SxBoolArgs& A, const SxrGroup<K>& G, unsigned* W, int q0, int at)
+{
+    const int lane = threadIdx.x & 31;
+    if (G.staged) {
+        unsigned short* const h16 = (unsigned short*)W;
         __syncwarp();  // every lane's sweep has read its pairs
-        if (act) {
-            const unsigned short* src = h16 + 2 * (OA + cap_excl) + prov;
-            for (int i = 0; i < khw; ++i) h16[excl + i] = src[i];
+        if (G.act) {
+            const unsigned short* src = h16 + G.src;
+            for (int i = 0; i < G.khw; ++i) h16[G.excl + i] = src[i];
         }
         __syncwarp();
-        const unsigned* pw = W;
-        for (int i = lane; i < total; i += 32) {
-            const unsigned kv = pw[i];
-            const long long o = (long long)base + i;
-            if (o < A.capacity) {
-                A.out_begin[o] = xmin + (int)(kv & 0xFFFFu);
-                A.out_end[o] = xmin + (int)(kv >> 16);
-            } else {
-                over = true;
+        for (int i = lane; i < G.total; i += 32) {
+            const unsigned kv = W[i];
+            const long long o = (long long)at + i;
+            if (o < A.capacity) {  // an output beyond the capacity shows in the reported total
+                A.out_begin[o] = G.xmin + (int)(kv & 0xFFFFu);
+                A.out_end[o] = G.xmin + (int)(kv >> 16);
             }
         }
-    } else if (ok && act && piece == 0 && nint > 0) {
-        bool fb_bad = false;
-        sx_sweep_table<K, true>(A, s_row, lim_row, A.out_begin, A.out_end, (long long)base + (excl >> 1), fb_bad, over);
+    } else if (RAW && !G.broken && G.act && G.khw > 0) {
+        const SxrRaw<K>& X = *G.raw;
+        bool bad = false;
+        sxr_raw_piece<K, true>(A, X.RB, X.RE, X.rp0, X.rpe, X.rlo, X.rhi, 2ll * at + G.excl, bad);
     }
-    if (act && piece == LPR - 1) A.out_off[r0 + row + 1] = base + (incl >> 1);
+    if (G.last) A.out_off[q0 + G.row + 1] = at + ((G.excl + G.khw) >> 1);
+}
+
+// A tile that does not fit its slice, or is too wide for 16 bits: groups of rows
+// that fit, swept once to count and, when the look-back has placed the tile, again
+// to write.  Rare, and kept out of line so that it costs the others no registers.
+template <int K>
+__device__ __noinline__ void sxr_slow_tile(const SxBoolArgs& A, const SxSweepState& st, int tile, int tiles, int r0,
+                                           int nrows, int TR, int room, unsigned* W, unsigned* raw,
+                                           unsigned long long* bar, unsigned use, unsigned flags)
+{
+    const int lane = threadIdx.x & 31;
+    // running sum of the rows' intervals (lane r: rows 0 .. r of the tile)
+    int sum = 0;
+#pragma unroll
+    for (int l = 0; l < K; ++l) sum += A.leaf[l].off[r0 + min(lane + 1, nrows)] - A.leaf[l].off[r0 + min(lane, nrows)];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+        if (lane >= o) sum += y;
+    }
+    SxrRaw<K> rawx;
+    SxrGroup<K> G;
+    G.raw = &rawx;
+    int base = 0, done = 0;  // the tile's base; intervals of the groups before
+    bool give_up = (flags & SXF_LONG_TILE) != 0u;  // another tile has given up
+    for (int phase = 0; phase < 2; ++phase) {
+        done = 0;
+        for (int gr = 0; gr < nrows && !give_up;) {
+            const int upto = __shfl_sync(0xFFFFFFFFu, sum, gr > 0 ? gr - 1 : 0);
+            const int before = gr > 0 ? upto : 0;
+            const unsigned in = __ballot_sync(0xFFFFFFFFu, lane >= gr && lane < nrows && sum - before <= room);
+            const int gn = max(1, __popc(in));  // a row that does not fit alone is swept from global memory
+            __syncwarp();
+            sxr_group<K, true>(A, r0 + gr, gn, TR, room, W, raw, bar, use, flags, G);
+            if (A.give_up && !G.staged) {
+                flags |= SXF_LONG_TILE;
+                if (lane == 0) atomicOr(&st.counters[2], SXF_LONG_TILE);
+                give_up = true;
+                done = 0;
+                break;
+            }
+            if (phase == 1) sxr_put<K, true>(A, G, W, r0 + gr, base + done);
+            done += G.total;
+            gr += gn;
+        }
+        if (phase == 0) base = sxs_lookback(A, st, tile, done, flags);
+    }
+    sxs_report(A, tile, tiles, base, done, flags);
+}
+
+template <int K>
+__global__ void __launch_bounds__(256, K <= 4 ? 4 : 3)
+    sx_rlane16_kernel(const __grid_constant__ SxBoolArgs A, const __grid_constant__ SxSweepState st, int tiles,
+                      int cap_words, int TR)
+{
+    extern __shared__ __align__(16) unsigned char sxr_smem[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, NW = blockDim.x >> 5;
+    if (blockIdx.x * NW + wid >= tiles) return;  // exactly `tiles` warps take tickets
+    unsigned* base_w = (unsigned*)(sxr_smem + (size_t)wid * sxr_slice_bytes(cap_words));
+    unsigned long long* bar = (unsigned long long*)base_w;
+    unsigned* const W = base_w + SXR_HDR_WORDS;  // pair lists, then the output areas
+    const int gap = sxr_gap_words(K, TR);
+    unsigned* const raw = W + gap;  // the bulk copies
+    int tile = 0;
+    unsigned flags = 0u, use = 0u;
+    if (lane == 0) {
+        tile = (int)atomicAdd(&st.counters[0], 1u);
+        if (A.give_up) flags = *(volatile unsigned*)&st.counters[2];
+        sxs_bar_init(bar);
+    }
+    tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
+    flags = __shfl_sync(0xFFFFFFFFu, flags, 0);
+    const int r0 = tile * TR;
+    const int nrows = min(TR, A.rows - r0);
     if (tile == 0 && lane == 0) A.out_off[0] = 0;
-    (void)over;  // an output beyond the capacity shows in the reported total
-    sxs_report(A, tile, tiles, base, total, flags);
+    const int room = (cap_words - gap) / 2 - 11 * K;  // intervals that fit whatever their alignment
+    SxrGroup<K> G;
+    G.staged = false;
+    G.ok = true;
+    if (flags == 0u) sxr_group<K, false>(A, r0, nrows, TR, room, W, raw, bar, use, flags, G);
+    if (!G.staged && G.ok) {
+        sxr_slow_tile<K>(A, st, tile, tiles, r0, nrows, TR, room, W, raw, bar, use, flags);
+        return;
+    }
+    const int base = sxs_lookback(A, st, tile, G.total, flags);
+    sxr_put<K, false>(A, G, W, r0, base);
+    sxs_report(A, tile, tiles, base, G.total, flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -2839,31 +3079,21 @@ static cudaError_t sx_wseg16_launch_k(const SxBoolArgs& A, const SxSweepState& s
     return cudaGetLastError();
 }
 
-template <int K, int LPR>
-static cudaError_t sx_rlane16_launch_kl(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
-                                        int warps, cudaStream_t stream)
+template <int K>
+static cudaError_t sx_rlane16_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
+                                       int warps, int tr, cudaStream_t stream)
 {
     static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int bytes = warps * (int)sxr_slice_bytes(cap_words);
     if (bytes > configured) {
         cudaError_t err =
-            cudaFuncSetAttribute(sx_rlane16_kernel<K, LPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            cudaFuncSetAttribute(sx_rlane16_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (err != cudaSuccess) return err;
         configured = bytes;
     }
     const int blocks = (tiles + warps - 1) / warps;
-    sx_rlane16_kernel<K, LPR><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words);
+    sx_rlane16_kernel<K><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words, tr);
     return cudaGetLastError();
-}
-
-// Lanes per row from the tile height: 32 rows one lane each, 16 rows two, 8 rows four.
-template <int K>
-static cudaError_t sx_rlane16_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
-                                       int warps, int tr, cudaStream_t stream)
-{
-    if (tr == 8) return sx_rlane16_launch_kl<K, 4>(A, st, tiles, cap_words, warps, stream);
-    if (tr == 16) return sx_rlane16_launch_kl<K, 2>(A, st, tiles, cap_words, warps, stream);
-    return sx_rlane16_launch_kl<K, 1>(A, st, tiles, cap_words, warps, stream);
 }
 
 // Union sweep shape: log2 of the lanes per row.  More lanes while whole rows
@@ -2962,7 +3192,7 @@ cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspac
     if (seg) {
         tr = A.tune_tile_rows > 0 ? A.tune_tile_rows : (A.tune_kernel == 4 ? 32 : 8);
         if (A.tune_kernel == 6 && tr > 8) tr = 8;  // 16-bit keys hold 3 row bits
-        if (A.tune_kernel == 7) tr = A.tune_tile_rows == 8 || A.tune_tile_rows == 32 ? A.tune_tile_rows : 16;
+        if (A.tune_kernel == 7) tr = A.tune_tile_rows > 0 ? A.tune_tile_rows : 16;
         if (sx_sweep_state_bytes(((long long)A.rows + tr - 1) / tr) > workspace_bytes) tr = 32;
     }
     const long long tiles = ((long long)A.rows + tr - 1) / tr;

@@ -32,7 +32,7 @@ __device__ __forceinline__ void sxs_bar_init(unsigned long long* bar)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// The single arrival of the barrier's phase 0, announcing `bytes` of copies.
+// The single arrival of a phase of the barrier, announcing `bytes` of copies.
 __device__ __forceinline__ void sxs_bar_expect(unsigned long long* bar, unsigned bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sxs_saddr(bar)), "r"(bytes)
@@ -49,19 +49,20 @@ __device__ __forceinline__ void sxs_bulk_copy(void* dst, const void* src, unsign
                  : "memory");
 }
 
-// Bounded wait for phase 0 of `bar`; false if it did not complete.  Each
+// Bounded wait for the phase of `bar` with the given parity (0, then 1, ...);
+// false if it did not complete.  Each
 // try_wait may suspend the thread for up to SXS_WAIT_HINT_NS (it resumes as
 // soon as the phase completes), so waiting warps take no issue slots; the
 // whole wait is bounded by SXS_WAIT_LIMIT tries.
-__device__ __forceinline__ bool sxs_bar_wait(unsigned long long* bar)
+__device__ __forceinline__ bool sxs_bar_wait(unsigned long long* bar, unsigned parity = 0u)
 {
     const unsigned a = sxs_saddr(bar);
     for (unsigned i = 0; i < SXS_WAIT_LIMIT; ++i) {
         unsigned done;
         asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0, %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %3, %2;\n selp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
-            : "r"(a), "n"(SXS_WAIT_HINT_NS)
+            : "r"(a), "n"(SXS_WAIT_HINT_NS), "r"(parity)
             : "memory");
         if (done) return true;
     }
