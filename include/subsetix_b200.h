@@ -653,6 +653,12 @@ int sx_amr_sync_copy(int dtype, const void* coarse, const void* fine, const int8
 int sx_amr_step_full(int dtype, const void* coarse_in, const void* fine_in, void* coarse_out, void* fine_out,
                      const int8_t* actions, int32_t width, int32_t height, int32_t batch, double a, double b,
                      double dt, double dx_coarse, double dy_coarse, double dx_fine, double dy_fine, void* stream);
+/* `steps` such steps (1 to SX_AMR_MAX_STEPS) in one pass over the arrays. */
+#define SX_AMR_MAX_STEPS 5
+int sx_amr_steps_full(int dtype, const void* coarse_in, const void* fine_in, void* coarse_out, void* fine_out,
+                      const int8_t* actions, int32_t width, int32_t height, int32_t batch, int32_t steps, double a,
+                      double b, double dt, double dx_coarse, double dy_coarse, double dx_fine, double dy_fine,
+                      void* stream);
 int sx_amr_regrid_full(int dtype, const void* coarse, uint8_t* tags, int8_t* actions, int32_t width, int32_t height,
                        int32_t batch, float threshold, int32_t padding, int mode, void* stream);
 

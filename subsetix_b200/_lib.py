@@ -32,6 +32,7 @@ FLAG_CONTRACT = 1
 FLAG_LONG_TILE = 2
 FLAG_CAPACITY = 4
 FLAG_TIMEOUT = 8
+AMR_MAX_STEPS = 5  # steps of one sx_amr_steps_full call
 
 c_i32p = ctypes.POINTER(ctypes.c_int32)
 c_vp = ctypes.c_void_p
@@ -195,6 +196,10 @@ _SIGNATURES = {
     "sx_amr_step_full": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32,
                                         ctypes.c_int32, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                         ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double, c_vp]),
+    "sx_amr_steps_full": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32,
+                                         ctypes.c_int32, ctypes.c_int32, ctypes.c_double, ctypes.c_double,
+                                         ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,
+                                         ctypes.c_double, c_vp]),
     "sx_amr_regrid_full": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, c_vp, ctypes.c_int32, ctypes.c_int32,
                                           ctypes.c_int32, ctypes.c_float, ctypes.c_int32, ctypes.c_int, c_vp]),
     "sx_mass_integral": (ctypes.c_int, [ctypes.c_int, c_vp, ctypes.c_int64, ctypes.c_double, c_vp, ctypes.c_int, c_vp,

@@ -188,6 +188,57 @@ __device__ __forceinline__ float sx_grad_norm(float gx, float gy)
 }
 
 // ---------------------------------------------------------------------------
+// Division by a divisor known beforehand: with z = RN(1 / d), q = RN(x z) and the
+// remainder r = x - q d, which one fma gives exactly, RN(q + r z) is the correctly
+// rounded x / d (P. Markstein, IBM J. Res. Dev. 34, 1990; N. Brisebarre, J.-M. Muller
+// and S. K. Raina, IEEE Trans. Computers 53, 2004) as long as nothing under- or
+// overflows: three operations instead of a general division.  For d within
+// 2^-60 .. 2^24 (SX_BY_CONST is only chosen then) that holds for x = 0 (-0 comes out
+// as +0) and for |x| >= 2^-100 (float32) or 2^-900 (float64); a quotient that
+// overflows comes out as NaN.  So callers test for smaller x and for results that
+// are not finite, and divide there.  (Float32: 2^64 x is large enough for every x, and
+// 2^-64 times the quotient is exact unless the result is subnormal: SX_BY_SCALED, for
+// fields with tails below 2^-76.  For those the three operations in float64 and one
+// rounding to float32 are exact: a quotient of 24-bit numbers is either a tie of two
+// neighbours, and a float64 number, or at least 2^-49 of itself away from it.)
+// ---------------------------------------------------------------------------
+#define SX_BY_DIVISION 0  // divide
+#define SX_BY_POW2 1      // multiply by the exact reciprocal of a power of two
+#define SX_BY_CONST 2     // the three operations above
+#define SX_BY_SCALED 3    // the same on 2^64 x (float32), for small x
+#define SX_BY_DOUBLE 4    // the same in float64 (float32), for subnormal quotients
+
+// Magnitudes below which a nonzero value counts as small, as high words shifted left
+// by one: differences of values that are zero or above it are zero or above
+// 2^-100 (float32) and 2^-900 (float64), where the remainder is exact.
+#define SX_SMALL_F32 ((unsigned)(127 - 76) << 24)
+#define SX_SMALL_F64 ((unsigned)(1023 - 840) << 21)
+
+// Order key of |x| in which zero comes last: min over several values < SX_SMALL says
+// that one of them is small and not zero.
+__device__ __forceinline__ unsigned sx_small_key(float x) { return 2u * __float_as_uint(x) - 1u; }
+__device__ __forceinline__ unsigned sx_small_key(double x)
+{
+    return (2u * (unsigned)__double2hiint(x) | (__double2loint(x) != 0 ? 1u : 0u)) - 1u;
+}
+template <typename T>
+inline bool sx_known_divisor(T d)
+{
+    return d >= (T)0x1p-60 && d <= (T)0x1p24;
+}
+// The key of a subnormal value, nonzero.
+template <typename T>
+__device__ __forceinline__ bool sx_is_subnormal(unsigned key)
+{
+    return key < (sizeof(T) == 4 ? 1u << 24 : 1u << 21) - 1u;
+}
+template <typename T>
+__device__ __forceinline__ bool sx_is_small(unsigned key)
+{
+    return key < (sizeof(T) == 4 ? SX_SMALL_F32 : SX_SMALL_F64);
+}
+
+// ---------------------------------------------------------------------------
 // Arithmetic helpers without contraction (float and double)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float sx_add(float a, float b) { return __fadd_rn(a, b); }

@@ -166,6 +166,11 @@ cudaError_t sx_amr_regrid_full_launch(int dbl, const void* coarse, unsigned char
 cudaError_t sx_amr_step_full_launch(int dbl, const void* cin, const void* fin, void* cout, void* fout,
                                     const signed char* actions, int W, int H, int batch, double a, double b, double dt,
                                     double dxc, double dyc, double dxf, double dyf, cudaStream_t stream);
+float sx_least_radicand(float thr);  // sx_grad_norm(gx, gy) >= thr is gx^2 + gy^2 >= this
+#define SX_AMR_MAX_STEPS 5  // also in the public header
+cudaError_t sx_amr_steps_full_launch(int dbl, const void* cin, const void* fin, void* cout, void* fout,
+                                     const signed char* actions, int W, int H, int batch, int steps, double a, double b,
+                                     double dt, double dxc, double dyc, double dxf, double dyf, cudaStream_t stream);
 int sx_upwind_adjoint_parts(long long cells);
 cudaError_t sx_upwind_adjoint_launch(const int* rows, const int* off, int row_count, const int* b, const int* e,
                                      const int* coff, int n, long long cells, const int* lookup, const void* w,

@@ -16,7 +16,7 @@
 // first is used.  Measured (B200, gradient tags on 4096^2): mask 29 us, count
 // 7.9 us, runs 3 us; one kernel with the counts and the look-back inside the mask
 // pass took 36 us (blocks wait at its barriers and in its tail), 49 us with the
-// square root that least_radicand removes.
+// square root that sx_least_radicand removes.
 
 #include <cmath>
 #include <cstring>
@@ -68,7 +68,7 @@ __device__ __forceinline__ Strip load_strip(const float* __restrict__ d, int x0,
 
 // The radicand of sx_grad_norm.  A correctly rounded square root never falls, so
 // sqrt(s) >= threshold is s >= the smallest radicand whose root reaches the
-// threshold (least_radicand, found on the host): same bits, no square root.
+// threshold (sx_least_radicand, found on the host): same bits, no square root.
 __device__ __forceinline__ float grad_square(float gx, float gy) { return __fmaf_rn(gx, gx, __fmul_rn(gy, gy)); }
 
 // Left and right neighbours of a strip's cells.
@@ -309,9 +309,20 @@ __global__ void __launch_bounds__(256) mask_runs_kernel(const unsigned* __restri
     if (lane == 0 && open) oe[first + count - 1] = W;
 }
 
+template <bool GRAD, bool VEC>
+void mask_go(const float* d, int W, int H, float thr, unsigned* mask, cudaStream_t stream)
+{
+    const int strips = (W + 127) / 128;
+    const long long tasks = (long long)strips * ((H + RLE_ROWS - 1) / RLE_ROWS);
+    mask_kernel<GRAD, VEC><<<(int)((tasks + RLE_THREADS / 32 - 1) / (RLE_THREADS / 32)), RLE_THREADS, 0, stream>>>(
+        d, W, H, thr, mask, (W + 31) / 32, strips, tasks);
+}
+
+}  // namespace
+
 // Smallest non-negative float whose correctly rounded square root is >= thr
 // (NaN for a NaN threshold: no cell passes, as in the comparison itself).
-float least_radicand(float thr)
+float sx_least_radicand(float thr)
 {
     if (!(thr > 0.0f)) return thr != thr ? thr : 0.0f;
     unsigned lo = 0u, hi = 0x7F800000u;  // sqrt(+inf) passes for every threshold
@@ -326,17 +337,6 @@ float least_radicand(float thr)
     return s;
 }
 
-template <bool GRAD, bool VEC>
-void mask_go(const float* d, int W, int H, float thr, unsigned* mask, cudaStream_t stream)
-{
-    const int strips = (W + 127) / 128;
-    const long long tasks = (long long)strips * ((H + RLE_ROWS - 1) / RLE_ROWS);
-    mask_kernel<GRAD, VEC><<<(int)((tasks + RLE_THREADS / 32 - 1) / (RLE_THREADS / 32)), RLE_THREADS, 0, stream>>>(
-        d, W, H, thr, mask, (W + 31) / 32, strips, tasks);
-}
-
-}  // namespace
-
 int sx_mask_tiles(int H) { return (H + 7) / 8; }
 
 cudaError_t sx_mask_launch(const float* d, int W, int H, float thr, int grad, unsigned* mask, int* offsets, int* result,
@@ -347,7 +347,7 @@ cudaError_t sx_mask_launch(const float* d, int W, int H, float thr, int grad, un
     if (err != cudaSuccess) return err;
     const bool vec = (W & 3) == 0 && ((uintptr_t)d & 15u) == 0;
     if (grad) {
-        thr = least_radicand(thr);
+        thr = sx_least_radicand(thr);
         if (vec) mask_go<true, true>(d, W, H, thr, mask, stream);
         else mask_go<true, false>(d, W, H, thr, mask, stream);
     } else {

@@ -11,14 +11,15 @@ with ``sx_upwind_full`` (both levels), ``sx_amr_sync_full`` (restriction
 into refined coarse cells and prolongation into the rest, in one pass) and
 ``sx_amr_regrid_full`` (gradient tag and grading into action bytes).  For
 ratio 2 the upwind of both levels and the synchronisation run as one kernel
-per step (``sx_amr_step_full``, ``fused=True``).  The results are bit-identical to ``AMR2Simulation`` on the same
+per step (``sx_amr_step_full``, ``fused=True``), and steps with no regrid
+between them as one kernel for up to five (``sx_amr_steps_full``).  The results are bit-identical to ``AMR2Simulation`` on the same
 initial field, in float32 and in float64.  The first synchronisation of a
 step always follows the previous step's last one with nothing in between,
 so it recomputes identical values and is skipped.
 
-Every step is a fixed sequence of launches on fixed buffers, so it is
-captured once per (regrid or not) x (buffer parity) into a CUDA graph and
-replayed with no host synchronisation.  The interval sets of the geometry
+A regrid period is a fixed sequence of launches on fixed buffers, so it is
+captured once per buffer parity into a CUDA graph and replayed with no host
+synchronisation; so is a single step, with a regrid or without.  The interval sets of the geometry
 (refine, fine, coarse-only) are rebuilt on request from the action bytes,
 which give the same sets as the reference's interval pipeline.
 
@@ -94,6 +95,7 @@ class FusedTwoLevelAMR:
         self.time = 0.0
         self._synced = False
         self._graphs = {}
+        self._flips = {}  # regrid period -> whether its graph ends in the other pair of buffers
         # set_initial_field: actions from the initial gradient, then fine = prolong(coarse)
         self._regrid()
         keep = torch.zeros_like(self.actions)
@@ -139,12 +141,31 @@ class FusedTwoLevelAMR:
                                     self.dx_fine, self.dy_fine, self._stream()), "sx_amr_step_full")
         self.cur = nxt
 
-    def _step_body(self, regrid: bool) -> None:
+    def _fused_steps(self, n: int) -> None:
+        """``n`` steps on fixed actions, in as few launches as they allow, of nearly equal step counts."""
+        lib = _lib.load()
+        a, b = self.velocity
+        launches = -(-n // _lib.AMR_MAX_STEPS)
+        for i in range(launches):
+            steps = n * (i + 1) // launches - n * i // launches
+            if steps == 1:
+                self._fused_advance_sync()
+                continue
+            nxt = 1 - self.cur
+            _check(lib.sx_amr_steps_full(self.code, ptr(self.coarse[self.cur]), ptr(self.fine[self.cur]),
+                                         ptr(self.coarse[nxt]), ptr(self.fine[nxt]), ptr(self.actions), self.width,
+                                         self.height, self.batch, steps, a, b, self.dt, self.dx_coarse, self.dy_coarse,
+                                         self.dx_fine, self.dy_fine, self._stream()), "sx_amr_steps_full")
+            self.cur = nxt
+
+    def _step_body(self, regrid: bool, n: int = 1) -> None:
+        """``n`` steps, after a regrid when asked."""
         if regrid:
             self._regrid()
         if self.fused:
-            self._fused_advance_sync()
-        else:
+            self._fused_steps(n)
+            return
+        for _ in range(n):
             self._advance()
             self._sync()
 
@@ -187,9 +208,9 @@ class FusedTwoLevelAMR:
             g = torch.cuda.CUDAGraph()
             with torch.cuda.stream(s):
                 with torch.cuda.graph(g, stream=s):
-                    for i in range(period):
-                        self._step_body(i == 0)
+                    self._step_body(True, period)
             torch.cuda.current_stream(self.device).wait_stream(s)
+            self._flips[period] = self.cur ^ parity
             self.cur = saved
             self._graphs[key] = g
         return g
@@ -198,9 +219,10 @@ class FusedTwoLevelAMR:
         """Advance ``steps`` steps.
 
         With ``graph``, every whole regrid period (the regrid and its
-        ``regrid_every`` steps) is one CUDA-graph replay, and the steps
-        outside whole periods are one replay each.  The launches, and so the
-        results, are the same as without graphs.
+        ``regrid_every`` steps) and every single step is one CUDA-graph
+        replay; steps outside whole periods are launched as they come when
+        one kernel takes several.  The launches, and so the results, are the
+        same as without graphs.
         """
         period = max(1, int(regrid_every))
         if not self._synced:
@@ -210,21 +232,20 @@ class FusedTwoLevelAMR:
         while left > 0:
             if graph and period > 1 and self.step_count % period == 0 and left >= period:
                 self._period_graph(period, self.cur).replay()
-                self.cur ^= period & 1
-                for _ in range(period):
-                    self.step_count += 1
-                    self.time += self.dt
-                left -= period
-                continue
-            regrid = self.step_count % period == 0
-            if graph:
-                self._graph(regrid, self.cur).replay()
-                self.cur = 1 - self.cur
+                self.cur ^= self._flips[period]
+                n = period
             else:
-                self._step_body(regrid)
-            self.step_count += 1
-            self.time += self.dt
-            left -= 1
+                regrid = self.step_count % period == 0
+                n = min(left, period - self.step_count % period) if self.fused else 1
+                if graph and n == 1:
+                    self._graph(regrid, self.cur).replay()
+                    self.cur = 1 - self.cur
+                else:
+                    self._step_body(regrid, n)
+            for _ in range(n):
+                self.step_count += 1
+                self.time += self.dt
+            left -= n
 
     def prepare_graphs(self, regrid_every: Optional[int] = None) -> None:
         """Capture the step graphs ahead of time (no work is done): the four
