@@ -190,22 +190,15 @@ def bool_eval_async(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Ten
         return ob, oe, ooff, None
     if result is None:
         result = empty_i32(2, device)
-    arr = (_lib.SxLeaf * k)()
-    for i, leaf in enumerate(leaves):
-        b, e, off, widen = leaf[:4]
-        scale = leaf[4] if len(leaf) > 4 else 0
-        ends = leaf[5] if len(leaf) > 5 else None
-        arr[i].begin = ptr(b)
-        arr[i].end = ptr(e)
-        arr[i].row_offsets = ptr(off)
-        arr[i].row_ends = ptr(ends)
-        arr[i].widen = int(widen)
-        arr[i].scale = int(scale)
+    arr = (_lib.SxLeaf * k)(*[_lib.SxLeaf(ptr(leaf[0]), ptr(leaf[1]), ptr(leaf[2]),
+                                          ptr(leaf[5]) if len(leaf) > 5 else None, int(leaf[3]),
+                                          int(leaf[4]) if len(leaf) > 4 else 0) for leaf in leaves])
     tab = (ctypes.c_uint32 * 8)(*[int(x) & 0xFFFFFFFF for x in (list(table) + [0] * 8)[:8]])
+    need = int(lib.sx_bool_workspace_bytes(int(rows)))
     if scratch is None:
-        wsp, wsn = workspace(device, lib.sx_bool_workspace_bytes(int(rows)))
+        wsp, wsn = workspace(device, need)
     else:
-        if int(scratch.numel()) < int(lib.sx_bool_workspace_bytes(int(rows))):
+        if int(scratch.numel()) < need:
             raise ValueError("scratch below sx_bool_workspace_bytes(rows)")
         wsp, wsn = scratch.data_ptr(), int(scratch.numel())
     t = TUNING if tuning is None else tuning
@@ -281,10 +274,10 @@ def merge_rows(begin: torch.Tensor, end: torch.Tensor, offsets: torch.Tensor, de
 def box_sweep(begin, end, offsets, rows, device, *, dense: bool, y_base: int, out_rows: int, x_lo: int, x_hi: int,
               halo_y: int = 0, w_center: int = 0, w_other: int = 0, mode: int = _lib.BOX_DILATE, ratio: int = 0,
               compact: bool = False):
-    """sx_box_sweep and its read-back: ``(begin, end, offsets, row ids or None, total, flags)``.
+    """sx_box_sweep and its read-back: ``(intervals, offsets, row ids or None, total, flags)``.
 
-    begin and end are capacity buffers; with ``compact`` offsets and row ids
-    are cut to the kept rows.
+    ``intervals`` holds the begins and the ends, two rows of the output's
+    capacity; with ``compact`` offsets and row ids are cut to the kept rows.
     """
     lib = _lib.load()
     n, out_rows = int(begin.numel()), int(out_rows)
@@ -293,17 +286,17 @@ def box_sweep(begin, end, offsets, rows, device, *, dense: bool, y_base: int, ou
     box = _lib.SxBox(ptr(begin), ptr(end), ptr(offsets), None if dense else ptr(rows), n, int(offsets.numel()) - 1,
                      1 if dense else 0, 0, int(y_base), out_rows, int(x_lo), int(x_hi), int(halo_y), int(w_center),
                      int(w_other), int(mode), int(ratio))
-    ob, oe = empty_i32(cap, device), empty_i32(cap, device)
+    out = torch.empty((2, (cap + 3) & ~3), dtype=I32, device=device)  # both rows 16-byte aligned
     off = empty_i32(out_rows + 1, device)
     ids = empty_i32(out_rows, device) if compact else None
     result = empty_i32(3, device)
     wsp, wsn = workspace(device, lib.sx_bool_workspace_bytes(out_rows))
-    _lib.check(lib.sx_box_sweep(ctypes.byref(box), ptr(ob), ptr(oe), ptr(off), ptr(ids), cap, ptr(result), wsp, wsn,
-                                stream_handle(device)), "sx_box_sweep")
+    _lib.check(lib.sx_box_sweep(ctypes.byref(box), ptr(out[0]), ptr(out[1]), ptr(off), ptr(ids), cap, ptr(result),
+                                wsp, wsn, stream_handle(device)), "sx_box_sweep")
     total, flags, kept = result.tolist()
     if compact:
         off, ids = off[:kept + 1], ids[:kept]
-    return ob, oe, off, ids, total, flags
+    return out, off, ids, total, flags
 
 
 def align_rows(lists: Sequence[tuple], row_min: int, row_max: int, device, want_offsets: Sequence[bool],

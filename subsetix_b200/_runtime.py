@@ -71,7 +71,13 @@ def like(kind_source, t: torch.Tensor):
     return t
 
 
+# The current stream's handle without a Stream object around it (0.3 against 4 us).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_handle(device: torch.device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return int(_raw_stream(device.index))
     return int(torch.cuda.current_stream(device).cuda_stream)
 
 
@@ -115,5 +121,5 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 def read_pair(result: torch.Tensor) -> Tuple[int, int]:
     """Synchronising read of a device ``result`` pair (count, flags)."""
-    host = result.cpu()
-    return int(host[0]), int(host[1])
+    first, second = result.tolist()
+    return first, second

@@ -346,27 +346,28 @@ def _count_leaves(node) -> int:
     return 1 if node[0] == "leaf" else _count_leaves(node[1]) + _count_leaves(node[2])
 
 
-def _eval_bool(node, state: int) -> bool:
+# Column of leaf i in a truth table of up to 8 leaves: bit s is bit i of s.
+_LEAF_COLUMNS = [sum(1 << s for s in range(256) if (s >> i) & 1) for i in range(_FUSED_MAX_LEAVES)]
+
+
+def _column(node) -> int:
+    """The node's value in every state at once, bit s for state s."""
     op = node[0]
     if op == "leaf":
-        return bool((state >> node[1]) & 1)
-    a = _eval_bool(node[1], state)
-    b = _eval_bool(node[2], state)
+        return _LEAF_COLUMNS[node[1]]
+    a, b = _column(node[1]), _column(node[2])
     if op == "union":
-        return a or b
+        return a | b
     if op == "intersection":
-        return a and b
+        return a & b
     if op == "difference":
-        return a and not b
-    return a != b
+        return a & ~b
+    return a ^ b
 
 
 def truth_table(node, k: int) -> List[int]:
-    words = [0] * 8
-    for state in range(1 << k):
-        if _eval_bool(node, state):
-            words[state >> 5] |= 1 << (state & 31)
-    return words
+    column = _column(node) & ((1 << (1 << k)) - 1)
+    return [(column >> (32 * w)) & 0xFFFFFFFF for w in range(8)]
 
 
 def _same_rows(sets: Sequence[IntervalSet]) -> bool:
@@ -381,6 +382,8 @@ def _same_rows(sets: Sequence[IntervalSet]) -> bool:
     others = [_t(s.rows) for s in sets[1:] if _t(s.rows).data_ptr() != r0.data_ptr() or n0 == 0]
     if not others or n0 == 0:
         return True
+    if len(others) == 1:
+        return torch.equal(r0, others[0])
     # one device comparison and one read-back for all the sets
     same = torch.stack([torch.eq(r0, o).all() for o in others])
     return bool(same.all())

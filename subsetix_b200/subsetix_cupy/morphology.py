@@ -160,7 +160,7 @@ def _box_sweep(s: IntervalSet, halo_y: int, w_center: int, w_other: int, *, y_ba
             or y_base < -(1 << 31) + 8 or y_base + out_rows > (1 << 31) - 8):
         return None
     dense = _dense_key(s) is not None
-    ob, oe, off, ids, total, flags = _core.box_sweep(
+    out, off, ids, total, flags = _core.box_sweep(
         _t(s.begin), _t(s.end), _t(s.row_offsets), _t(s.rows), device, dense=dense, y_base=y_base, out_rows=out_rows,
         x_lo=x_lo, x_hi=x_hi, halo_y=halo_y, w_center=w_center, w_other=w_other, mode=mode, ratio=ratio, compact=compact)
     if flags & _lib.FLAG_CONTRACT:
@@ -168,7 +168,8 @@ def _box_sweep(s: IntervalSet, halo_y: int, w_center: int, w_other: int, *, y_ba
     if flags & (_lib.FLAG_CAPACITY | _lib.FLAG_TIMEOUT):
         raise _lib.SubsetixError(f"box sweep failed (flags={flags})")
     rows = ids if compact else torch.arange(out_rows, dtype=I32, device=device)
-    return _wrap(s.begin, ob[:total].clone(), oe[:total].clone(), off, rows, None if compact else out_rows)
+    begin, end = out[:, :(total + 3) & ~3].contiguous()  # one copy of what is used
+    return _wrap(s.begin, begin[:total], end[:total], off, rows, None if compact else out_rows)
 
 
 def _row_span(s: IntervalSet):
