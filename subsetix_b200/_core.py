@@ -491,6 +491,30 @@ def row_lookup(rows, height: int, device, sync: bool = True):
     return lookup, (bool(flags.item()) if sync else flags)
 
 
+def stencil_geometry(rows, offsets, begin, end, height: int, device):
+    """What a stencil needs to know about a new set, with one read-back.
+
+    Returns ``(lookup, out_of_range, row flags, cell offsets, cells, (first
+    column, last column + 1))``; the last three hold for sorted, disjoint rows.
+    """
+    lib, s = _lib.load(), stream_handle(device)
+    n, rows_n = int(begin.numel()), int(rows.numel())
+    facts = empty_i32(6, device)
+    at = facts.data_ptr()
+    lookup, cell_off = empty_i32(height, device), empty_i32(n + 1, device)
+    _lib.check(lib.sx_row_lookup(ptr(rows), rows_n, int(height), ptr(lookup), at, s), "sx_row_lookup")
+    _lib.check(lib.sx_check_rows(ptr(begin), ptr(end), ptr(offsets), max(int(offsets.numel()) - 1, 0), n, at + 4, s),
+               "sx_check_rows")
+    wsp, wsn = workspace(device, lib.sx_scan_workspace_bytes(n))
+    _lib.check(lib.sx_cell_offsets(ptr(begin), ptr(end), n, ptr(cell_off), at + 8, wsp, wsn, s), "sx_cell_offsets")
+    # no cells: the plan's launch finds the columns only
+    _lib.check(lib.sx_upwind_flat_plan(None, None, 0, ptr(begin), ptr(end), None, n, 0, None, int(height), None, None,
+                                       None, None, at + 16, s), "sx_upwind_flat_plan")
+    bad, flags, cells, scan_flags, lo, hi = facts.tolist()
+    check_scan(scan_flags, "sx_cell_offsets")
+    return lookup, bool(bad), flags, cell_off, cells, (lo, hi)
+
+
 def upwind(rows, offsets, begin, end, cell_offs, cells: int, lookup, values, out, width: int, height: int, a, b, dt,
            dx, dy, direct: bool, device, row_ids=None):
     lib = _lib.load()
@@ -542,11 +566,15 @@ def upwind_chunked(offsets, begin, end, cell_offs, chunk_info, chunks: int, look
 
 
 class FlatPlan:
-    """Plan of sx_upwind_flat for sorted, disjoint rows and packed values, with the columns it spans (one read-back)."""
+    """Plan of sx_upwind_flat for sorted, disjoint rows and packed values, with the columns it spans.
+
+    ``columns`` is that span, where known; else it is read back.
+    """
 
     __slots__ = ("cells", "lo", "hi", "_keep", "_struct", "_ref")
 
-    def __init__(self, rows, offsets, begin, end, cell_offs, cells: int, lookup, height: int, device):
+    def __init__(self, rows, offsets, begin, end, cell_offs, cells: int, lookup, height: int, device,
+                 columns: Optional[Tuple[int, int]] = None):
         lib = _lib.load()
         n, cells = int(begin.numel()), int(cells)
         groups = (cells + 3) // 4
@@ -559,7 +587,7 @@ class FlatPlan:
                                            ptr(flags), ptr(side), ptr(span), stream_handle(device)),
                    "sx_upwind_flat_plan")
         self.cells = cells
-        self.lo, self.hi = span.tolist()
+        self.lo, self.hi = span.tolist() if columns is None else columns
         self._keep = (below, above, flags, side)
         self._struct = _lib.SxFlatPlan(ptr(below), ptr(above), ptr(flags), ptr(side), n, cells)
         self._ref = ctypes.byref(self._struct)

@@ -221,8 +221,29 @@ __device__ __forceinline__ unsigned sx_small_key(double x)
 {
     return (2u * (unsigned)__double2hiint(x) | (__double2loint(x) != 0 ? 1u : 0u)) - 1u;
 }
+// The same for the differences themselves (x above): 2^-100 and 2^-900, and the
+// magnitudes from which a quotient may overflow (d >= 2^-60): 2^60 and 2^900.
+#define SX_SMALL_DIFF_F32 ((unsigned)(127 - 100) << 24)
+#define SX_SMALL_DIFF_F64 ((unsigned)(1023 - 900) << 21)
+#define SX_LARGE_DIFF_F32 ((unsigned)(127 + 60) << 24)
+#define SX_LARGE_DIFF_F64 ((unsigned)(1023 + 900) << 21)
+__device__ __forceinline__ unsigned sx_large_key(float x) { return 2u * __float_as_uint(x); }
+__device__ __forceinline__ unsigned sx_large_key(double x) { return 2u * (unsigned)__double2hiint(x); }
+
+// x / d by the three operations, z = RN(1 / d).
+__device__ __forceinline__ float sx_by_const(float x, float d, float z)
+{
+    const float q = __fmul_rn(x, z);
+    return __fmaf_rn(__fmaf_rn(q, -d, x), z, q);
+}
+__device__ __forceinline__ double sx_by_const(double x, double d, double z)
+{
+    const double q = __dmul_rn(x, z);
+    return __fma_rn(__fma_rn(q, -d, x), z, q);
+}
+
 template <typename T>
-inline bool sx_known_divisor(T d)
+__host__ __device__ inline bool sx_known_divisor(T d)
 {
     return d >= (T)0x1p-60 && d <= (T)0x1p24;
 }

@@ -28,7 +28,7 @@
 // the domain (span_kernel checks it when the plan is built) no test is left:
 // a neighbour in the set is a neighbour in the domain.  Geometry with cells
 // outside the domain keeps the chunk kernel.  Measured (B200): one float64 step
-// on 2500^2 26.1 -> 15.1 us, the uneven batch 1337 -> 626 us (327 M cells; its
+// on 2500^2 26.1 -> 15.1 us (12.3 with over_group), the uneven batch 1337 -> 626 us (327 M cells; its
 // 9.5 bytes a cell take 475 us at the copy rate), the three-level composite's
 // 300 level steps 5.1 -> 2.8 ms and its 150 transposed ones, sums over blocks
 // included, 5.2 -> 3.2 ms.  Same values as sx_upwind, bit for bit; the adjoint's
@@ -276,24 +276,55 @@ __device__ __forceinline__ void side_group(const T* __restrict__ v, const T (&ce
     }
 }
 
-// Divides eight differences by the spacings, or multiplies them by the exact
-// reciprocals of power-of-two spacings: one branch for the group.
-template <typename T>
-__device__ __forceinline__ void over_group(T (&x)[4], T (&y)[4], T dx, T dy, int pow2)
+// Divides eight differences by the spacings: by their exact reciprocals
+// (SX_BY_POW2: dx and dy hold those), or by the three operations for a known divisor
+// (zx and zy: RN of the reciprocals) unless a difference is too small or too large
+// for those, or by division.  One branch for the group.  Spacings that are no powers of
+// two, before (division) and after: one float64 step on 2500^2 15.1 -> 12.3 us, float32
+// on 3000^2 12.6 -> 10.4, the 120 level steps and 60 transposed ones of a composite of
+// base 600 in float32 389 -> 257 and 470 -> 370 us.  Not in the banded step (CONST):
+// with a reciprocal to keep per axis and band its 626 us became 654.
+template <typename T, bool CONST>
+__device__ __forceinline__ void over_group(T (&x)[4], T (&y)[4], T dx, T dy, T zx, T zy, int way)
 {
-    if (pow2) {
+    if (way == SX_BY_POW2) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             x[k] = sx_mul(x[k], dx);
             y[k] = sx_mul(y[k], dy);
         }
-    } else {
+        return;
+    }
+    if (CONST && way == SX_BY_CONST) {
+        unsigned small = 0xFFFFFFFFu, large = 0u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            x[k] = sx_div(x[k], dx);
-            y[k] = sx_div(y[k], dy);
+            small = min(small, min(sx_small_key(x[k]), sx_small_key(y[k])));
+            large = max(large, max(sx_large_key(x[k]), sx_large_key(y[k])));
+        }
+        if (small >= (sizeof(T) == 4 ? SX_SMALL_DIFF_F32 : SX_SMALL_DIFF_F64) &&
+            large < (sizeof(T) == 4 ? SX_LARGE_DIFF_F32 : SX_LARGE_DIFF_F64)) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                x[k] = sx_by_const(x[k], dx, zx);
+                y[k] = sx_by_const(y[k], dy, zy);
+            }
+            return;
         }
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x[k] = sx_div(x[k], dx);
+        y[k] = sx_div(y[k], dy);
+    }
+}
+
+// How to divide by the spacings (dx and dy become their reciprocals for SX_BY_POW2).
+template <typename T>
+int spacing_way(T& dx, T& dy)
+{
+    if (sx_pow2_pair(dx, dy)) return SX_BY_POW2;
+    return sx_known_divisor(dx) && sx_known_divisor(dy) ? SX_BY_CONST : SX_BY_DIVISION;
 }
 
 // One step.  SGN holds the upwind sides the velocity selects (bit 0: a >= 0,
@@ -312,7 +343,8 @@ __global__ void __launch_bounds__(FLAT_THREADS,
                                                    : BAND_STEP_BLOCKS_F64)
     flat_step_kernel(const T* __restrict__ v, T* __restrict__ out, long long cells, const int* __restrict__ nbr,
                      const unsigned short* __restrict__ bits, const int4* __restrict__ side, T a, T bb, T dt, T dx,
-                     T dy, int pow2, const int* __restrict__ band_cell, const T* __restrict__ band_table, int nbands)
+                     T dy, T zx, T zy, int way, const int* __restrict__ band_cell, const T* __restrict__ band_table,
+                     int nbands)
 {
     constexpr bool LEFT = (SGN & 1) != 0, DOWN = (SGN & 2) != 0;
     const int lane = threadIdx.x & 31;
@@ -355,7 +387,7 @@ __global__ void __launch_bounds__(FLAT_THREADS,
             dx = __ldg(band_table + 4 * q);
             dy = __ldg(band_table + 4 * q + 1);
             dt = __ldg(band_table + 4 * q + 2);
-            pow2 = __ldg(band_table + 4 * q + 3) != (T)0;
+            way = __ldg(band_table + 4 * q + 3) != (T)0 ? SX_BY_POW2 : SX_BY_DIVISION;
         }
         T vn[4], vs[4], x[4], y[4], res[4];
         row_group<T>(v, base, DOWN ? m & 15u : (m >> 4) & 15u, (m >> (DOWN ? 12 : 13)) & 1u, side, vn);
@@ -376,7 +408,7 @@ __global__ void __launch_bounds__(FLAT_THREADS,
                                           __ldg(t + 2));
             }
         } else {
-            over_group<T>(x, y, dx, dy, pow2);
+            over_group<T, !BANDS>(x, y, dx, dy, zx, zy, way);
 #pragma unroll
             for (int k = 0; k < 4; ++k) res[k] = sx_upwind_update(cen[k], x[k], y[k], a, bb, dt);
         }
@@ -399,7 +431,7 @@ __global__ void __launch_bounds__(FLAT_THREADS)
     flat_adjoint_kernel(const T* __restrict__ w, const T* __restrict__ u, T* __restrict__ ubar, long long cells,
                         const int* __restrict__ dn, const int* __restrict__ up,
                         const unsigned short* __restrict__ bits, const int4* __restrict__ side_dn,
-                        const int4* __restrict__ side_up, T a, T bb, T dt, T dx, T dy, int pow2,
+                        const int4* __restrict__ side_up, T a, T bb, T dt, T dx, T dy, T zx, T zy, int way,
                         unsigned* __restrict__ counter, double* __restrict__ partial, double* __restrict__ grads,
                         int accumulate)
 {
@@ -441,8 +473,8 @@ __global__ void __launch_bounds__(FLAT_THREADS)
             dux[k] = LEFT ? sx_sub(uc[k], us[k]) : sx_sub(us[k], uc[k]);
             duy[k] = DOWN ? sx_sub(uc[k], ur[k]) : sx_sub(ur[k], uc[k]);
         }
-        over_group<T>(tx, ty, dx, dy, pow2);
-        over_group<T>(dux, duy, dx, dy, pow2);
+        over_group<T, true>(tx, ty, dx, dy, zx, zy, way);
+        over_group<T, true>(dux, duy, dx, dy, zx, zy, way);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             res[k] = sx_sub(wc[k], sx_mul(dt, sx_add(sx_mul(a, tx[k]), sx_mul(bb, ty[k]))));
@@ -501,79 +533,85 @@ __global__ void __launch_bounds__(FLAT_THREADS)
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 template <typename T, bool BANDS, bool VEC, int ROUNDS>
-void step_go(int sgn, int blocks, const T* v, T* out, const SxFlatPlan& P, T a, T bb, T dt, T dx, T dy, int pow2,
+void step_go(int sgn, int blocks, const T* v, T* out, const SxFlatPlan& P, T a, T bb, T dt, T dx, T dy, int way,
              const int* band_cell, const T* band_table, int nbands, cudaStream_t stream)
 {
+    const T zx = (T)1 / dx, zy = (T)1 / dy;
     switch (sgn) {
         case 0:
             flat_step_kernel<T, BANDS, VEC, 0, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
-                v, out, P.cells, P.up, P.bits, P.side_up, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands);
+                v, out, P.cells, P.up, P.bits, P.side_up, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
         case 1:
             flat_step_kernel<T, BANDS, VEC, 1, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
-                v, out, P.cells, P.up, P.bits, P.side_up, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands);
+                v, out, P.cells, P.up, P.bits, P.side_up, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
         case 2:
             flat_step_kernel<T, BANDS, VEC, 2, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
-                v, out, P.cells, P.dn, P.bits, P.side_dn, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands);
+                v, out, P.cells, P.dn, P.bits, P.side_dn, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
         default:
             flat_step_kernel<T, BANDS, VEC, 3, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
-                v, out, P.cells, P.dn, P.bits, P.side_dn, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands);
+                v, out, P.cells, P.dn, P.bits, P.side_dn, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
     }
 }
 
 template <typename T, bool BANDS, int ROUNDS>
-void step_rounds(const SxFlatPlan& P, const T* v, T* out, T a, T bb, T dt, T dx, T dy, int pow2, const int* band_cell,
+void step_rounds(const SxFlatPlan& P, const T* v, T* out, T a, T bb, T dt, T dx, T dy, int way, const int* band_cell,
                  const T* band_table, int nbands, cudaStream_t stream)
 {
     const long long per = (long long)FLAT_THREADS * 4 * ROUNDS;
     const int blocks = (int)((P.cells + per - 1) / per);
     const int sgn = (a >= (T)0 ? 1 : 0) | (bb >= (T)0 ? 2 : 0);
     if (aligned16(v) && aligned16(out))
-        step_go<T, BANDS, true, ROUNDS>(sgn, blocks, v, out, P, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands,
+        step_go<T, BANDS, true, ROUNDS>(sgn, blocks, v, out, P, a, bb, dt, dx, dy, way, band_cell, band_table, nbands,
                                         stream);
     else
-        step_go<T, BANDS, false, ROUNDS>(sgn, blocks, v, out, P, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands,
+        step_go<T, BANDS, false, ROUNDS>(sgn, blocks, v, out, P, a, bb, dt, dx, dy, way, band_cell, band_table, nbands,
                                          stream);
 }
 
 template <typename T, bool BANDS>
-void step_run(const SxFlatPlan& P, const T* v, T* out, T a, T bb, T dt, T dx, T dy, int pow2, const int* band_cell,
+void step_run(const SxFlatPlan& P, const T* v, T* out, T a, T bb, T dt, T dx, T dy, int way, const int* band_cell,
               const T* band_table, int nbands, cudaStream_t stream)
 {
     // Without bands one run per block is faster at every size (33 M cells, float32: 86 us against 98 to 108).
     if (BANDS && P.cells >= (long long)FLAT_THREADS * 4 * BAND_ROUNDS * 148 * BAND_BLOCKS)
-        step_rounds<T, BANDS, BANDS ? BAND_ROUNDS : 1>(P, v, out, a, bb, dt, dx, dy, pow2, band_cell, band_table,
+        step_rounds<T, BANDS, BANDS ? BAND_ROUNDS : 1>(P, v, out, a, bb, dt, dx, dy, way, band_cell, band_table,
                                                        nbands, stream);
     else
-        step_rounds<T, BANDS, 1>(P, v, out, a, bb, dt, dx, dy, pow2, band_cell, band_table, nbands, stream);
+        step_rounds<T, BANDS, 1>(P, v, out, a, bb, dt, dx, dy, way, band_cell, band_table, nbands, stream);
 }
 
 template <typename T, bool VEC>
-void adjoint_go(int blocks, const SxFlatPlan& P, const T* w, const T* u, T* ubar, T a, T bb, T dt, T dx, T dy, int pow2,
+void adjoint_go(int blocks, const SxFlatPlan& P, const T* w, const T* u, T* ubar, T a, T bb, T dt, T dx, T dy, int way,
                 unsigned* counter, double* partial, double* grads, int accumulate, cudaStream_t stream)
 {
+    const T zx = (T)1 / dx, zy = (T)1 / dy;
     switch ((a >= (T)0 ? 1 : 0) | (bb >= (T)0 ? 2 : 0)) {
         case 0:
             flat_adjoint_kernel<T, VEC, 0><<<blocks, FLAT_THREADS, 0, stream>>>(
-                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, pow2, counter,
+                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
+                counter,
                 partial, grads, accumulate);
             break;
         case 1:
             flat_adjoint_kernel<T, VEC, 1><<<blocks, FLAT_THREADS, 0, stream>>>(
-                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, pow2, counter,
+                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
+                counter,
                 partial, grads, accumulate);
             break;
         case 2:
             flat_adjoint_kernel<T, VEC, 2><<<blocks, FLAT_THREADS, 0, stream>>>(
-                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, pow2, counter,
+                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
+                counter,
                 partial, grads, accumulate);
             break;
         default:
             flat_adjoint_kernel<T, VEC, 3><<<blocks, FLAT_THREADS, 0, stream>>>(
-                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, pow2, counter,
+                w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
+                counter,
                 partial, grads, accumulate);
             break;
     }
@@ -583,15 +621,15 @@ template <typename T>
 void adjoint_run(const SxFlatPlan& P, const T* w, const T* u, T* ubar, T a, T bb, T dt, T dx, T dy, void* scratch,
                  double* grads, int accumulate, cudaStream_t stream)
 {
-    const int pow2 = sx_pow2_pair(dx, dy);
+    const int way = spacing_way(dx, dy);
     const int blocks = sx_flat_adjoint_parts(P.cells);
     unsigned* counter = (unsigned*)scratch;
     double* partial = (double*)scratch + 2;
     if (aligned16(w) && aligned16(u) && aligned16(ubar))
-        adjoint_go<T, true>(blocks, P, w, u, ubar, a, bb, dt, dx, dy, pow2, counter, partial, grads, accumulate,
+        adjoint_go<T, true>(blocks, P, w, u, ubar, a, bb, dt, dx, dy, way, counter, partial, grads, accumulate,
                             stream);
     else
-        adjoint_go<T, false>(blocks, P, w, u, ubar, a, bb, dt, dx, dy, pow2, counter, partial, grads, accumulate,
+        adjoint_go<T, false>(blocks, P, w, u, ubar, a, bb, dt, dx, dy, way, counter, partial, grads, accumulate,
                              stream);
 }
 
@@ -627,11 +665,11 @@ cudaError_t sx_flat_step_launch(const SxFlatPlan& P, int dbl, const void* v, voi
 {
     if (P.cells <= 0) return cudaSuccess;
     if (dbl) {
-        const int p = sx_pow2_pair(dx, dy);
+        const int p = spacing_way(dx, dy);
         step_run<double, false>(P, (const double*)v, (double*)out, a, bb, dt, dx, dy, p, nullptr, nullptr, 0, stream);
     } else {
         float fx = (float)dx, fy = (float)dy;
-        const int p = sx_pow2_pair(fx, fy);
+        const int p = spacing_way(fx, fy);
         step_run<float, false>(P, (const float*)v, (float*)out, (float)a, (float)bb, (float)dt, fx, fy, p, nullptr,
                                nullptr, 0, stream);
     }

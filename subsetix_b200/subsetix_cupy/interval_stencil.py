@@ -83,18 +83,17 @@ def _geometry(interval_set, height: int) -> _Geometry:
         return cache
     rows = _t(interval_set.rows)
     device = _t(interval_set.row_offsets).device
-    lookup, bad = _core.row_lookup(rows, height, device)
+    b, e, off = _t(interval_set.begin), _t(interval_set.end), _t(interval_set.row_offsets)
+    lookup, bad, flags, coff, cells, columns = _core.stencil_geometry(rows, off, b, e, height, device)
     if bad:
         # The reference's lookup scatter wraps rows outside [0, height)
         # (interval_stencil.py:183-191); they are rejected here.
         raise ValueError("interval_set rows exceed provided height")
-    flags = _core.check_rows(_t(interval_set.begin), _t(interval_set.end), _t(interval_set.row_offsets), device)
     direct = not (flags & (_lib.ROWS_UNSORTED_BEGIN | _lib.ROWS_OVERLAP | _lib.ROWS_EMPTY))
-    coff, cells, flat = None, 0, None
     if direct:
-        b, e, off = _t(interval_set.begin), _t(interval_set.end), _t(interval_set.row_offsets)
-        coff, cells = _core.cell_offsets(b, e, device)
-        flat = _core.FlatPlan(rows, off, b, e, coff, cells, lookup, height, device)
+        flat = _core.FlatPlan(rows, off, b, e, coff, cells, lookup, height, device, columns)
+    else:
+        coff, cells, flat = None, 0, None
     geo = _Geometry(height, lookup, direct, cells, coff, flat)
     try:
         object.__setattr__(interval_set, "_sx_stencil", geo)
