@@ -41,6 +41,7 @@ template <typename T>
 __global__ void index_copy_kernel(long long n, const int* __restrict__ dst_idx, const int* __restrict__ src_idx,
                                   const T* __restrict__ src, T* __restrict__ dst)
 {
+    sx_after_previous();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long s = src_idx ? src_idx[i] : i;
         const long long d = dst_idx ? dst_idx[i] : i;
@@ -81,6 +82,7 @@ __global__ void segment_add_kernel(long long nseg, const int* __restrict__ seg_o
                                    const int* __restrict__ dst_idx, T* __restrict__ src, T* __restrict__ dst,
                                    int zero_src)
 {
+    sx_after_previous();
     constexpr int BATCH = 4;
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < nseg;
          s += (long long)gridDim.x * blockDim.x) {
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, i
                                                              const int* __restrict__ plan, const T* __restrict__ in,
                                                              T* __restrict__ out)
 {
+    sx_after_previous();
     typedef typename Pair<T>::type P2;
     const int run = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (run >= runs) return;
@@ -166,6 +169,7 @@ __global__ void __launch_bounds__(256) run_block_mean_adj_kernel(int runs, int r
                                                                  const int* __restrict__ plan, T* __restrict__ out_bar,
                                                                  T* __restrict__ in_bar)
 {
+    sx_after_previous();
     typedef typename Pair<T>::type P2;
     const int run = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (run >= runs) return;
@@ -246,10 +250,10 @@ cudaError_t sx_index_copy_launch(int dtype, long long n, const int* dst_idx, con
 {
     if (n <= 0) return cudaSuccess;
     if (dtype == 1)
-        index_copy_kernel<double><<<grid_for(n), 256, 0, stream>>>(n, dst_idx, src_idx, (const double*)src,
+        sx_launch_early(index_copy_kernel<double>, dim3(grid_for(n)), dim3(256), 0, stream, n, dst_idx, src_idx, (const double*)src,
                                                                     (double*)dst);
     else
-        index_copy_kernel<float><<<grid_for(n), 256, 0, stream>>>(n, dst_idx, src_idx, (const float*)src, (float*)dst);
+        sx_launch_early(index_copy_kernel<float>, dim3(grid_for(n)), dim3(256), 0, stream, n, dst_idx, src_idx, (const float*)src, (float*)dst);
     return cudaGetLastError();
 }
 
@@ -284,10 +288,10 @@ cudaError_t sx_index_segment_add_launch(int dtype, long long nseg, const int* se
 {
     if (nseg <= 0) return cudaSuccess;
     if (dtype == 1)
-        segment_add_kernel<double><<<grid_for(nseg), 256, 0, stream>>>(nseg, seg_off, src_idx, dst_idx, (double*)src,
+        sx_launch_early(segment_add_kernel<double>, dim3(grid_for(nseg)), dim3(256), 0, stream, nseg, seg_off, src_idx, dst_idx, (double*)src,
                                                                         (double*)dst, zero_src);
     else
-        segment_add_kernel<float><<<grid_for(nseg), 256, 0, stream>>>(nseg, seg_off, src_idx, dst_idx, (float*)src,
+        sx_launch_early(segment_add_kernel<float>, dim3(grid_for(nseg)), dim3(256), 0, stream, nseg, seg_off, src_idx, dst_idx, (float*)src,
                                                                        (float*)dst, zero_src);
     return cudaGetLastError();
 }
@@ -302,17 +306,17 @@ void run_go(long long runs, int ratio, int stride, double norm, const int* plan,
     const bool pair = ratio == 2 && ((uintptr_t)fine & (2 * sizeof(T) - 1)) == 0;
     if (ADJ) {
         if (pair)
-            run_block_mean_adj_kernel<T, true><<<blocks, 256, 0, stream>>>((int)runs, ratio, stride, (T)norm, plan,
+            sx_launch_early(run_block_mean_adj_kernel<T, true>, dim3(blocks), dim3(256), 0, stream, (int)runs, ratio, stride, (T)norm, plan,
                                                                            coarse, fine);
         else
-            run_block_mean_adj_kernel<T, false><<<blocks, 256, 0, stream>>>((int)runs, ratio, stride, (T)norm, plan,
+            sx_launch_early(run_block_mean_adj_kernel<T, false>, dim3(blocks), dim3(256), 0, stream, (int)runs, ratio, stride, (T)norm, plan,
                                                                             coarse, fine);
     } else {
         if (pair)
-            run_block_mean_kernel<T, true><<<blocks, 256, 0, stream>>>((int)runs, ratio, stride, (T)norm, plan, fine,
+            sx_launch_early(run_block_mean_kernel<T, true>, dim3(blocks), dim3(256), 0, stream, (int)runs, ratio, stride, (T)norm, plan, fine,
                                                                        coarse);
         else
-            run_block_mean_kernel<T, false><<<blocks, 256, 0, stream>>>((int)runs, ratio, stride, (T)norm, plan, fine,
+            sx_launch_early(run_block_mean_kernel<T, false>, dim3(blocks), dim3(256), 0, stream, (int)runs, ratio, stride, (T)norm, plan, fine,
                                                                         coarse);
     }
 }

@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(FLAT_THREADS,
                      T dy, T zx, T zy, int way, const int* __restrict__ band_cell, const T* __restrict__ band_table,
                      int nbands)
 {
+    sx_after_previous();
     constexpr bool LEFT = (SGN & 1) != 0, DOWN = (SGN & 2) != 0;
     const int lane = threadIdx.x & 31;
     const long long groups = (cells + 3) >> 2;
@@ -435,6 +436,7 @@ __global__ void __launch_bounds__(FLAT_THREADS)
                         unsigned* __restrict__ counter, double* __restrict__ partial, double* __restrict__ grads,
                         int accumulate)
 {
+    sx_after_previous();
     constexpr bool LEFT = (SGN & 1) != 0, DOWN = (SGN & 2) != 0;
     __shared__ double s_a[FLAT_THREADS], s_b[FLAT_THREADS];
     __shared__ bool s_last;
@@ -539,19 +541,19 @@ void step_go(int sgn, int blocks, const T* v, T* out, const SxFlatPlan& P, T a, 
     const T zx = (T)1 / dx, zy = (T)1 / dy;
     switch (sgn) {
         case 0:
-            flat_step_kernel<T, BANDS, VEC, 0, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_step_kernel<T, BANDS, VEC, 0, ROUNDS>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 v, out, P.cells, P.up, P.bits, P.side_up, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
         case 1:
-            flat_step_kernel<T, BANDS, VEC, 1, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_step_kernel<T, BANDS, VEC, 1, ROUNDS>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 v, out, P.cells, P.up, P.bits, P.side_up, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
         case 2:
-            flat_step_kernel<T, BANDS, VEC, 2, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_step_kernel<T, BANDS, VEC, 2, ROUNDS>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 v, out, P.cells, P.dn, P.bits, P.side_dn, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
         default:
-            flat_step_kernel<T, BANDS, VEC, 3, ROUNDS><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_step_kernel<T, BANDS, VEC, 3, ROUNDS>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 v, out, P.cells, P.dn, P.bits, P.side_dn, a, bb, dt, dx, dy, zx, zy, way, band_cell, band_table, nbands);
             break;
     }
@@ -591,25 +593,25 @@ void adjoint_go(int blocks, const SxFlatPlan& P, const T* w, const T* u, T* ubar
     const T zx = (T)1 / dx, zy = (T)1 / dy;
     switch ((a >= (T)0 ? 1 : 0) | (bb >= (T)0 ? 2 : 0)) {
         case 0:
-            flat_adjoint_kernel<T, VEC, 0><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_adjoint_kernel<T, VEC, 0>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
                 counter,
                 partial, grads, accumulate);
             break;
         case 1:
-            flat_adjoint_kernel<T, VEC, 1><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_adjoint_kernel<T, VEC, 1>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
                 counter,
                 partial, grads, accumulate);
             break;
         case 2:
-            flat_adjoint_kernel<T, VEC, 2><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_adjoint_kernel<T, VEC, 2>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
                 counter,
                 partial, grads, accumulate);
             break;
         default:
-            flat_adjoint_kernel<T, VEC, 3><<<blocks, FLAT_THREADS, 0, stream>>>(
+            sx_launch_early(flat_adjoint_kernel<T, VEC, 3>, dim3(blocks), dim3(FLAT_THREADS), 0, stream,
                 w, u, ubar, P.cells, P.dn, P.up, P.bits, P.side_dn, P.side_up, a, bb, dt, dx, dy, zx, zy, way,
                 counter,
                 partial, grads, accumulate);

@@ -166,6 +166,31 @@ cudaError_t sx_amr_regrid_full_launch(int dbl, const void* coarse, unsigned char
 cudaError_t sx_amr_step_full_launch(int dbl, const void* cin, const void* fin, void* cout, void* fout,
                                     const signed char* actions, int W, int H, int batch, double a, double b, double dt,
                                     double dxc, double dyc, double dxf, double dyf, cudaStream_t stream);
+// Launch of a kernel that calls sx_after_previous() before it touches memory: its blocks
+// may take their places while the kernel before it in the stream still runs its last
+// ones, so a chain of short kernels does not wait for each launch.
+template <typename... P, typename... Q>
+cudaError_t sx_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Q... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+// Lets the next kernel of such a chain take places, then waits until all the memory
+// operations of the kernels before this one are done.
+__device__ __forceinline__ void sx_after_previous()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 float sx_least_radicand(float thr);  // sx_grad_norm(gx, gy) >= thr is gx^2 + gy^2 >= this
 #define SX_AMR_MAX_STEPS 5  // also in the public header
 cudaError_t sx_amr_steps_full_launch(int dbl, const void* cin, const void* fin, void* cout, void* fout,
