@@ -110,7 +110,7 @@ __global__ void segment_add_kernel(long long nseg, const int* __restrict__ seg_o
     }
 }
 
-// Runs of coarse cells, one warp each, two cells per lane.  Plan entry of a run:
+// Runs of coarse cells, two per warp, two cells of each per lane.  Plan entry of a run:
 // first coarse value, cells (at most 64), then the first child of each of
 // the r sub-rows; `stride` ints per entry (a multiple of 4).  Bound by the fine
 // values' bytes.  Per coarse cell the index tables took 4 (1 + r^2) bytes and a
@@ -118,7 +118,9 @@ __global__ void segment_add_kernel(long long nseg, const int* __restrict__ seg_o
 // values, in pairs where a sub-row of a run starts at an even value (PAIR: r = 2
 // and arrays aligned to a pair).  Measured (B200, 1.18 M coarse cells, float32):
 // mean 11.4 -> 7.0 us, transpose 30.8 -> 11.9 us (27.6 us while its stores stood
-// between its loads).
+// between its loads).  With every load of a run, then of two, before the first use, and
+// plan entries as one load each, a pass of the composite (190 means, 100 transposes)
+// went from 9.45 to 9.11 and 8.79 ms; four runs per warp 8.85.
 template <typename T>
 struct Pair;
 template <>
@@ -130,6 +132,8 @@ struct Pair<double> {
     typedef double2 type;
 };
 
+constexpr int RUNS_PER_WARP = 2;
+
 template <typename T, bool PAIR>
 __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, int stride, T norm,
                                                              const int* __restrict__ plan, const T* __restrict__ in,
@@ -137,31 +141,65 @@ __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, i
 {
     sx_after_previous();
     typedef typename Pair<T>::type P2;
-    const int run = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (run >= runs) return;
-    const int* p = plan + (long long)run * stride;
-    const int r = PAIR ? 2 : rr;
-    const int count = __ldg(p + 1);
-    const long long c0 = __ldg(p);
-    T acc[2] = {T(0), T(0)};
-    for (int dy = 0; dy < r; ++dy) {
-        const long long f0 = __ldg(p + 2 + dy);
+    const int first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RUNS_PER_WARP, lane = threadIdx.x & 31;
+    if constexpr (PAIR) {
+        int count[RUNS_PER_WARP];
+        long long c0[RUNS_PER_WARP], f[RUNS_PER_WARP][2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = lane + 32 * h;
-            if (k >= count) continue;
-            const T* src = in + f0 + (long long)k * r;
-            if (PAIR && (f0 & 1) == 0) {
-                const P2 v = *(const P2*)src;
-                acc[h] = cp_add(cp_add(acc[h], v.x), v.y);
-            } else {
-                for (int dx = 0; dx < r; ++dx) acc[h] = cp_add(acc[h], src[dx]);
+        for (int q = 0; q < RUNS_PER_WARP; ++q) {
+            const int4 p = first + q < runs ? __ldg((const int4*)(plan + (long long)(first + q) * stride)) : make_int4(0, 0, 0, 0);
+            c0[q] = p.x;
+            count[q] = p.y;
+            f[q][0] = p.z;
+            f[q][1] = p.w;
+        }
+        P2 v[RUNS_PER_WARP][2][2];
+#pragma unroll
+        for (int q = 0; q < RUNS_PER_WARP; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int dy = 0; dy < 2; ++dy) {
+                    const int k = lane + 32 * h;
+                    if (k >= count[q]) continue;
+                    const T* src = in + f[q][dy] + 2ll * k;
+                    if ((f[q][dy] & 1) == 0) {
+                        v[q][h][dy] = *(const P2*)src;
+                    } else {
+                        v[q][h][dy].x = src[0];
+                        v[q][h][dy].y = src[1];
+                    }
+                }
+#pragma unroll
+        for (int q = 0; q < RUNS_PER_WARP; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = lane + 32 * h;
+                if (k >= count[q]) continue;
+                const T a = cp_add(cp_add(T(0), v[q][h][0].x), v[q][h][0].y);
+                out[c0[q] + k] = cp_mul(cp_add(cp_add(a, v[q][h][1].x), v[q][h][1].y), norm);
             }
+    } else {
+        for (int run = first; run < min(runs, first + RUNS_PER_WARP); ++run) {
+            const int* p = plan + (long long)run * stride;
+            const int count = __ldg(p + 1);
+            const long long c0 = __ldg(p);
+            T acc[2] = {T(0), T(0)};
+            for (int dy = 0; dy < rr; ++dy) {
+                const long long f0 = __ldg(p + 2 + dy);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = lane + 32 * h;
+                    if (k >= count) continue;
+                    const T* src = in + f0 + (long long)k * rr;
+                    for (int dx = 0; dx < rr; ++dx) acc[h] = cp_add(acc[h], src[dx]);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (lane + 32 * h < count) out[c0 + lane + 32 * h] = cp_mul(acc[h], norm);
         }
     }
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-        if (lane + 32 * h < count) out[c0 + lane + 32 * h] = cp_mul(acc[h], norm);
 }
 
 template <typename T, bool PAIR>
@@ -171,66 +209,81 @@ __global__ void __launch_bounds__(256) run_block_mean_adj_kernel(int runs, int r
 {
     sx_after_previous();
     typedef typename Pair<T>::type P2;
-    const int run = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (run >= runs) return;
-    const int* p = plan + (long long)run * stride;
-    const int count = __ldg(p + 1);
-    const long long c0 = __ldg(p);
-    T w[2] = {T(0), T(0)};
+    const int first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RUNS_PER_WARP, lane = threadIdx.x & 31;
     if constexpr (PAIR) {
         // every load before the first store, so a warp waits for one round trip
-        const long long f[2] = {__ldg(p + 2), __ldg(p + 3)};
-        P2 v[2][2];
+        int count[RUNS_PER_WARP];
+        long long c0[RUNS_PER_WARP], f[RUNS_PER_WARP][2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = lane + 32 * h;
-            if (k >= count) continue;
-            w[h] = out_bar[c0 + k];
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy) {
-                const T* src = in_bar + f[dy] + 2ll * k;
-                if ((f[dy] & 1) == 0) {
-                    v[h][dy] = *(const P2*)src;
-                } else {
-                    v[h][dy].x = src[0];
-                    v[h][dy].y = src[1];
-                }
-            }
+        for (int q = 0; q < RUNS_PER_WARP; ++q) {
+            const int4 p = first + q < runs ? __ldg((const int4*)(plan + (long long)(first + q) * stride)) : make_int4(0, 0, 0, 0);
+            c0[q] = p.x;
+            count[q] = p.y;
+            f[q][0] = p.z;
+            f[q][1] = p.w;
         }
+        T w[RUNS_PER_WARP][2];
+        P2 v[RUNS_PER_WARP][2][2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = lane + 32 * h;
-            if (k >= count) continue;
-            const T a = cp_mul(w[h], norm);
-            out_bar[c0 + k] = T(0);
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy) {
-                T* dst = in_bar + f[dy] + 2ll * k;
-                v[h][dy].x = cp_add(v[h][dy].x, a);
-                v[h][dy].y = cp_add(v[h][dy].y, a);
-                if ((f[dy] & 1) == 0) {
-                    *(P2*)dst = v[h][dy];
-                } else {
-                    dst[0] = v[h][dy].x;
-                    dst[1] = v[h][dy].y;
-                }
-            }
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = lane + 32 * h;
-            w[h] = k < count ? cp_mul(out_bar[c0 + k], norm) : T(0);
-            if (k < count) out_bar[c0 + k] = T(0);
-        }
-        for (int dy = 0; dy < rr; ++dy) {
-            const long long f0 = __ldg(p + 2 + dy);
+        for (int q = 0; q < RUNS_PER_WARP; ++q)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int k = lane + 32 * h;
-                if (k >= count) continue;
-                T* dst = in_bar + f0 + (long long)k * rr;
-                for (int dx = 0; dx < rr; ++dx) dst[dx] = cp_add(dst[dx], w[h]);
+                if (k >= count[q]) continue;
+                w[q][h] = out_bar[c0[q] + k];
+#pragma unroll
+                for (int dy = 0; dy < 2; ++dy) {
+                    const T* src = in_bar + f[q][dy] + 2ll * k;
+                    if ((f[q][dy] & 1) == 0) {
+                        v[q][h][dy] = *(const P2*)src;
+                    } else {
+                        v[q][h][dy].x = src[0];
+                        v[q][h][dy].y = src[1];
+                    }
+                }
+            }
+#pragma unroll
+        for (int q = 0; q < RUNS_PER_WARP; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = lane + 32 * h;
+                if (k >= count[q]) continue;
+                const T a = cp_mul(w[q][h], norm);
+                out_bar[c0[q] + k] = T(0);
+#pragma unroll
+                for (int dy = 0; dy < 2; ++dy) {
+                    T* dst = in_bar + f[q][dy] + 2ll * k;
+                    v[q][h][dy].x = cp_add(v[q][h][dy].x, a);
+                    v[q][h][dy].y = cp_add(v[q][h][dy].y, a);
+                    if ((f[q][dy] & 1) == 0) {
+                        *(P2*)dst = v[q][h][dy];
+                    } else {
+                        dst[0] = v[q][h][dy].x;
+                        dst[1] = v[q][h][dy].y;
+                    }
+                }
+            }
+    } else {
+        for (int run = first; run < min(runs, first + RUNS_PER_WARP); ++run) {
+            const int* p = plan + (long long)run * stride;
+            const int count = __ldg(p + 1);
+            const long long c0 = __ldg(p);
+            T w[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = lane + 32 * h;
+                w[h] = k < count ? cp_mul(out_bar[c0 + k], norm) : T(0);
+                if (k < count) out_bar[c0 + k] = T(0);
+            }
+            for (int dy = 0; dy < rr; ++dy) {
+                const long long f0 = __ldg(p + 2 + dy);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = lane + 32 * h;
+                    if (k >= count) continue;
+                    T* dst = in_bar + f0 + (long long)k * rr;
+                    for (int dx = 0; dx < rr; ++dx) dst[dx] = cp_add(dst[dx], w[h]);
+                }
             }
         }
     }
@@ -302,8 +355,9 @@ template <typename T, bool ADJ>
 void run_go(long long runs, int ratio, int stride, double norm, const int* plan, T* coarse, T* fine,
             cudaStream_t stream)
 {
-    const int blocks = (int)((runs + 7) / 8);
-    const bool pair = ratio == 2 && ((uintptr_t)fine & (2 * sizeof(T) - 1)) == 0;
+    const int blocks = (int)((runs + 8 * RUNS_PER_WARP - 1) / (8 * RUNS_PER_WARP));
+    const bool pair = ratio == 2 && stride % 4 == 0 && ((uintptr_t)plan & 15u) == 0 &&
+                      ((uintptr_t)fine & (2 * sizeof(T) - 1)) == 0;
     if (ADJ) {
         if (pair)
             sx_launch_early(run_block_mean_adj_kernel<T, true>, dim3(blocks), dim3(256), 0, stream, (int)runs, ratio, stride, (T)norm, plan,

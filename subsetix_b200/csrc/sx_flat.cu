@@ -55,6 +55,13 @@ constexpr int BAND_BLOCKS = 4;
 constexpr int STEP_BLOCKS = 6;
 constexpr int BAND_STEP_BLOCKS_F32 = 5;
 constexpr int BAND_STEP_BLOCKS_F64 = 4;
+// Blocks per SM of the adjoint, all resident at once: every block ends with a reduction
+// and its share of the last block's sum, so more blocks cost more than they hide (the
+// three-level composite, 50 steps with gradients: 9.67 ms with 4 per SM, 9.94 with 8,
+// 10.5 with 16; 9.45 with the next group's plan loaded early).  Float64 takes 80
+// registers, three blocks.
+constexpr int ADJOINT_BLOCKS = 4;
+constexpr int ADJOINT_BLOCKS_F64 = 3;
 
 // Smallest begin and largest end over all intervals into span[0], span[1]
 // (which start at INT_MAX, INT_MIN).
@@ -428,7 +435,7 @@ __global__ void __launch_bounds__(FLAT_THREADS,
 // order and scales by -dt, so no second launch is needed.  scratch: a counter
 // (zero before the first call, left zero), then two doubles per block.
 template <typename T, bool VEC, int SGN>
-__global__ void __launch_bounds__(FLAT_THREADS)
+__global__ void __launch_bounds__(FLAT_THREADS, sizeof(T) == 4 ? ADJOINT_BLOCKS : ADJOINT_BLOCKS_F64)
     flat_adjoint_kernel(const T* __restrict__ w, const T* __restrict__ u, T* __restrict__ ubar, long long cells,
                         const int* __restrict__ dn, const int* __restrict__ up,
                         const unsigned short* __restrict__ bits, const int4* __restrict__ side_dn,
@@ -443,23 +450,34 @@ __global__ void __launch_bounds__(FLAT_THREADS)
     const int lane = threadIdx.x & 31;
     const long long groups = (cells + 3) >> 2;
     double ga = 0.0, gb = 0.0;
+    unsigned mn = 0u;  // the next group's plan: with it at hand, a round waits for memory once
+    int bdn = 0, bun = 0;
+    const long long first = (long long)blockIdx.x * FLAT_THREADS + threadIdx.x;
+    if (first < groups) {
+        mn = __ldg(bits + first);
+        bdn = __ldg(dn + first);
+        bun = __ldg(up + first);
+    }
     // whole warps stay in the loop together (the shuffles need every lane)
-    for (long long gw = (long long)blockIdx.x * FLAT_THREADS + (threadIdx.x & ~31); gw < groups;
-         gw += (long long)gridDim.x * FLAT_THREADS) {
+    for (long long gw = first - lane; gw < groups; gw += (long long)gridDim.x * FLAT_THREADS) {
         const long long g = gw + lane;
         const bool act = g < groups;
         const long long c0 = 4 * g;
         T wc[4], uc[4], wr[4], ur[4], ws[4], us[4], res[4];
-        unsigned m = 0u;
-        int bd = 0, bu = 0;
+        const unsigned m = mn;
+        const int bd = bdn, bu = bun;
 #pragma unroll
         for (int k = 0; k < 4; ++k) wc[k] = uc[k] = (T)0;
         if (act) {
-            m = __ldg(bits + g);
-            bd = __ldg(dn + g);
-            bu = __ldg(up + g);
             load_group<T, VEC>(w, c0, cells, wc);
             load_group<T, VEC>(u, c0, cells, uc);
+        }
+        mn = 0u;
+        const long long gn = g + (long long)gridDim.x * FLAT_THREADS;
+        if (gn < groups) {
+            mn = __ldg(bits + gn);
+            bdn = __ldg(dn + gn);
+            bun = __ldg(up + gn);
         }
         const unsigned md = m & 15u, mu = (m >> 4) & 15u;
         const bool id = (m >> 12) & 1u, iu = (m >> 13) & 1u;
@@ -624,7 +642,8 @@ void adjoint_run(const SxFlatPlan& P, const T* w, const T* u, T* ubar, T a, T bb
                  double* grads, int accumulate, cudaStream_t stream)
 {
     const int way = spacing_way(dx, dy);
-    const int blocks = sx_flat_adjoint_parts(P.cells);
+    int blocks = sx_flat_adjoint_parts(P.cells);
+    if (sizeof(T) == 8 && blocks > 148 * ADJOINT_BLOCKS_F64) blocks = 148 * ADJOINT_BLOCKS_F64;
     unsigned* counter = (unsigned*)scratch;
     double* partial = (double*)scratch + 2;
     if (aligned16(w) && aligned16(u) && aligned16(ubar))
@@ -643,7 +662,7 @@ int sx_flat_adjoint_parts(long long cells)
 {
     long long g = (cells + 4 * FLAT_THREADS - 1) / (4 * FLAT_THREADS);
     if (g < 1) g = 1;
-    if (g > 148 * 8) g = 148 * 8;
+    if (g > 148 * ADJOINT_BLOCKS) g = 148 * ADJOINT_BLOCKS;
     return (int)g;
 }
 
