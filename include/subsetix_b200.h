@@ -538,6 +538,13 @@ int sx_threshold_mask(const float* values, int32_t width, int32_t height, float 
                       int32_t* offsets, int32_t* result, void* workspace, size_t workspace_bytes, void* stream);
 int sx_mask_runs(const uint32_t* mask, int32_t width, int32_t height, const int32_t* offsets, int32_t* out_begin,
                  int32_t* out_end, void* stream);
+/* The value that ceil(fraction * m) (at least one) of the m values above
+ * epsilon reach (regrid.py:353-380).  result[0]: its bits, result[1]: m (0:
+ * nothing above epsilon, no value).  workspace:
+ * sx_select_top_workspace_bytes(). */
+size_t sx_select_top_workspace_bytes(void);
+int sx_select_top(const float* values, int64_t n, float epsilon, double fraction, int32_t* result, void* workspace,
+                  size_t workspace_bytes, void* stream);
 /* Gradient magnitude of a full grid, same formula (regrid.py:172-274, K14). */
 int sx_gradient_magnitude(const float* values, int32_t width, int32_t height, float* out, void* stream);
 int sx_gradient_threshold_rle(const float* values, int32_t width, int32_t height, float threshold, int32_t* counts,

@@ -10,6 +10,7 @@ returns sized arrays, so it synchronises at the same points
 from __future__ import annotations
 
 import ctypes
+import struct
 from typing import List, Optional, Sequence, Tuple
 
 import torch
@@ -632,6 +633,17 @@ def threshold_rle(values, width: int, height: int, threshold: float, gradient: b
     if total:
         _lib.check(lib.sx_mask_runs(ptr(mask), width, height, ptr(off), ptr(ob), ptr(oe), s), "sx_mask_runs")
     return ob, oe, off
+
+
+def select_top(values: torch.Tensor, epsilon: float, fraction: float, device) -> Tuple[float, int]:
+    """``(value, m)``: the value that ``ceil(fraction * m)`` of the ``m`` float32 values above ``epsilon`` reach."""
+    lib = _lib.load()
+    result = empty_i32(2, device)
+    scratch = torch.empty(int(lib.sx_select_top_workspace_bytes()), dtype=torch.uint8, device=device)
+    _lib.check(lib.sx_select_top(ptr(values), int(values.numel()), float(epsilon), float(fraction), ptr(result),
+                                 ptr(scratch), int(scratch.numel()), stream_handle(device)), "sx_select_top")
+    bits, above = result.tolist()
+    return struct.unpack("<f", struct.pack("<i", bits))[0], above
 
 
 def mass_integral(values, scale: float, device, out: Optional[torch.Tensor] = None, parts: int = 592):

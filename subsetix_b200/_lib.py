@@ -161,6 +161,9 @@ _SIGNATURES = {
     "sx_threshold_mask": (ctypes.c_int, [c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_float, ctypes.c_int, c_vp,
                                          c_vp, c_vp, c_vp, ctypes.c_size_t, c_vp]),
     "sx_mask_runs": (ctypes.c_int, [c_vp, ctypes.c_int32, ctypes.c_int32, c_vp, c_vp, c_vp, c_vp]),
+    "sx_select_top_workspace_bytes": (ctypes.c_size_t, []),
+    "sx_select_top": (ctypes.c_int, [c_vp, ctypes.c_int64, ctypes.c_float, ctypes.c_double, c_vp, c_vp, ctypes.c_size_t,
+                                     c_vp]),
     "sx_gradient_magnitude": (ctypes.c_int, [c_vp, ctypes.c_int32, ctypes.c_int32, c_vp, c_vp]),
     "sx_gradient_threshold_rle": (ctypes.c_int, [c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_float, c_vp, c_vp,
                                                  c_vp, c_vp, c_vp]),

@@ -896,6 +896,22 @@ int sx_mask_runs(const uint32_t* mask, int32_t width, int32_t height, const int3
     return SX_OK;
 }
 
+size_t sx_select_top_workspace_bytes(void) { return sx_select_bytes(); }
+
+int sx_select_top(const float* values, int64_t n, float epsilon, double fraction, int32_t* result, void* workspace,
+                  size_t workspace_bytes, void* stream)
+{
+    if (n < 0 || n > INT32_MAX) return fail(SX_ERR_INVALID, "sx_select_top: count out of range");
+    if (!(fraction >= 0.0 && fraction <= 1.0)) return fail(SX_ERR_INVALID, "sx_select_top: fraction outside [0, 1]");
+    if (!result || (n > 0 && !values)) return fail(SX_ERR_INVALID, "sx_select_top: null argument");
+    if (!workspace || workspace_bytes < sx_select_bytes() || ((uintptr_t)workspace & 3u) != 0)
+        return fail(SX_ERR_WORKSPACE, "sx_select_top: workspace needs %zu bytes, got %zu", sx_select_bytes(),
+                    workspace_bytes);
+    cudaError_t err = sx_select_launch(values, n, epsilon, fraction, workspace, result, (cudaStream_t)stream);
+    if (err != cudaSuccess) return cuda_fail(err, "sx_select_top");
+    return SX_OK;
+}
+
 int sx_gradient_magnitude(const float* values, int32_t width, int32_t height, float* out, void* stream)
 {
     if (width <= 0 || height <= 0) return fail(SX_ERR_INVALID, "sx_gradient_magnitude: width and height must be positive");

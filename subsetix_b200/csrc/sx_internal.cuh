@@ -191,6 +191,9 @@ __device__ __forceinline__ void sx_after_previous()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+size_t sx_select_bytes();
+cudaError_t sx_select_launch(const float* values, long long n, float eps, double fraction, void* workspace, int* result,
+                             cudaStream_t stream);
 float sx_least_radicand(float thr);  // sx_grad_norm(gx, gy) >= thr is gx^2 + gy^2 >= this
 #define SX_AMR_MAX_STEPS 5  // also in the public header
 cudaError_t sx_amr_steps_full_launch(int dbl, const void* cin, const void* fin, void* cout, void* fout,

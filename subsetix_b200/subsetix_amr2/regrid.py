@@ -89,14 +89,10 @@ def gradient_tag_set(field: IntervalField, *, width: int, height: int, frac_high
     frac_high = float(max(0.0, min(1.0, frac_high)))
     if frac_high <= 0.0:
         return _empty_interval_set(height)
-    values = _t(field.values).to(torch.float32)
-    positive = values[values > float(np.float32(epsilon))]
-    if positive.numel() == 0:
+    values = _t(field.values).to(torch.float32).contiguous()
+    threshold, above = _core.select_top(values, float(np.float32(epsilon)), frac_high, values.device)
+    if above == 0:
         return _empty_interval_set(height)
-    count = int(np.ceil(positive.numel() * frac_high))
-    count = max(1, min(int(positive.numel()), count))
-    idx = int(positive.numel()) - count
-    threshold = float(torch.kthvalue(positive, idx + 1).values.item())
     return intervals_above_threshold_interval_field(field, width=width, height=height,
                                                     threshold=max(threshold, float(epsilon)))
 
