@@ -30,6 +30,7 @@ OP_UNION, OP_INTERSECTION, OP_DIFFERENCE = 0, 1, 2
 TUNING: dict = {}
 TUNED: dict = {}
 
+_SM_SHARED = 228 * 1024  # shared memory of an SM; a block takes 1 KB beside its own
 _TILE_INTERVALS = 1600  # a mean tile of the automatic row-lane sweep (13 KB of shared memory)
 
 
@@ -109,19 +110,24 @@ def even_tuning(leaves, rows: int) -> dict:
     """The launch shape of ``sx_bool_eval_even``, from the operands' sizes alone.
 
     The row-lane sweep on tiles of 16 rows, or 8 when rows are so long that a
-    mean tile would exceed ``_TILE_INTERVALS``.  Slices hold the mean tile and
-    a tenth more, or, for light tiles, where room costs no residency, two and
-    a half times the mean; the tiles above that are swept in groups of rows
-    by the same launch.  Measured: five shape leaves over 128 copies of 4096
-    rows (mean 16-row tile 1155 intervals, largest 1253) 421 us with 16 rows,
-    433 us with 8, 474 us with 32, 615 us when the slices fall short of the
-    largest tiles; 163 uneven small sets (mean 236, largest 954) 464 us with
-    2.5 times the mean, 500 us with 1.5 times.
+    mean tile would exceed ``_TILE_INTERVALS``.  The sweep waits for latencies,
+    so its speed goes with the resident blocks: as many as slices for the
+    mean tile and a twentieth more allow (at most what the registers leave
+    room for), each with all the shared memory that this count gives it.  The
+    tiles above that are swept in groups of rows by the same launch.
+    Measured: five shape leaves over 128 copies of 4096 rows (mean 16-row tile
+    1155 intervals, largest 1253) 421 us with 16 rows, 433 us with 8, 474 us
+    with 32, 615 us when the slices fall short of the largest tiles; the sweep
+    alone 274 us at 10 blocks per SM, 289 us at 9.
     """
-    total = sum(int(leaf[0].numel()) for leaf in leaves)
+    k, total = len(leaves), sum(int(leaf[0].numel()) for leaf in leaves)
     tr = 16 if 16 * total <= _TILE_INTERVALS * rows else 8
     mean = tr * total // max(1, rows)
-    room = max(mean + mean // 10 + 48, min(5 * mean // 2, 600))
+    gap = max((k - 1) * (tr - 7) + tr, k * (tr + 1) + tr - 16 * k) + 4
+    fixed = 22 * k + 16 + gap  # words of a warp's slice beside two per interval
+    per_block = 2 * 4 * (2 * (mean + mean // 20 + 32) + fixed) + 1024
+    blocks = max(1, min(_SM_SHARED // per_block, 16 if k <= 4 else 12))
+    room = ((min(_SM_SHARED // blocks, 200 * 1024) - 1024) // 8 - fixed) // 2
     return {"kernel": 7, "staging_cap": min(2 * room, 25000), "tile_rows": tr, "warps": 2}
 
 

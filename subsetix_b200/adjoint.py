@@ -458,20 +458,31 @@ class _Segment:
                 for dst, src in zip(into, result):
                     dst.copy_(src)
 
+        def forward():
+            cur, _ = _run_composite(h, list(self.state), a, b, dt, n - 1, keep=False)
+            settle(h.step(cur, a, b, dt, out=self.state if n > 1 else None)[0], self.state)
+
+        def inputs():
+            cur, self.inputs = _run_composite(h, list(self.state), a, b, dt, n - 1, keep=True)
+            h._fill_ghosts(cur)
+            self.inputs.append(cur)
+
+        def backward():
+            w = list(self.w)
+            for j in reversed(range(n)):
+                w = h.step_adjoint(w, self.inputs[j], a, b, dt, self.grad, out=self.w if j == 0 and n > 1 else None)
+            settle(w, self.w)
+
+        # Captured one after another without torch.cuda.graph's emptying of the allocator's
+        # cache before each, which a new hierarchy would pay for.  They share their memory:
+        # one replays at a time, and the inputs that outlive their graph are held here.
         with torch.cuda.stream(side):
-            with torch.cuda.graph(self.fwd, stream=side):
-                cur, _ = _run_composite(h, list(self.state), a, b, dt, n - 1, keep=False)
-                settle(h.step(cur, a, b, dt, out=self.state if n > 1 else None)[0], self.state)
-            with torch.cuda.graph(self.keep, stream=side):
-                cur, self.inputs = _run_composite(h, list(self.state), a, b, dt, n - 1, keep=True)
-                h._fill_ghosts(cur)
-                self.inputs.append(cur)
-            with torch.cuda.graph(self.bwd, stream=side):
-                w = list(self.w)
-                for j in reversed(range(n)):
-                    w = h.step_adjoint(w, self.inputs[j], a, b, dt, self.grad,
-                                       out=self.w if j == 0 and n > 1 else None)
-                settle(w, self.w)
+            for graph, work in ((self.fwd, forward), (self.keep, inputs), (self.bwd, backward)):
+                graph.capture_begin(**({} if graph is self.fwd else {"pool": self.fwd.pool()}))
+                try:
+                    work()
+                finally:
+                    graph.capture_end()
         torch.cuda.current_stream(dev).wait_stream(side)
 
     def forward(self, states: Sequence[torch.Tensor]) -> List[torch.Tensor]:
