@@ -1,7 +1,7 @@
 """Launch autotuner for the row-sweep set algebra (sx_bool_eval).
 
 The candidates are the kernel kinds of ``sx_tuning``: the row-lane sweep
-(16-row tiles with two lanes per row, 32-row tiles with one), the warp-tile
+(16-row and 32-row tiles, its lanes dealt out to the rows), the warp-tile
 segmented sweep (8-row tiles, 32-bit and 16-bit keys) with several warps
 per block, the block-tile
 segmented sweep (32-row tiles) with two block sizes, the merge-path tile

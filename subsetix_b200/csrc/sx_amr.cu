@@ -16,6 +16,8 @@
 //                      into its fine block (kernels.py:384-418).  Refine and
 //                      coarse-only cells partition the grid, so one pass per
 //                      coarse cell does both halves;
+//   sx_amr_step_full   upwind on both levels and the synchronisation in one kernel
+//                      (ratio 2), sx_amr_steps_full up to five such steps;
 //   sx_amr_tag_full    the gradient tag of regrid.py:172-223,336-350: the
 //                      field is read as float32, the gradient has central
 //                      differences inside and one-sided ones at the edges,

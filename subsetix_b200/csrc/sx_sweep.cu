@@ -2099,9 +2099,9 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // segmented sweeps.  So no pass over the input is needed before the launch to size
 // the slices for the largest tile and to look for wide tiles; such a pass took 59 us
 // of kernel and a read-back beside the 270 us sweep of the five-leaf shape expression
-// over 128 copies of 4096 rows (466 us in all; 410 us without it, with the sweep at
-// 288 us).  The sweep is bound by the latency of a tile's stages: 18 warps per SM are
-// all that the slices leave room for.
+// over 128 copies of 4096 rows (466 us in all; 364 us without it, with the sweep at
+// 275 to 288 us).  The sweep is bound by the latency of a tile's stages: 20 warps per
+// SM are all that the slices leave room for.
 //
 // Registers: 80 for five leaves, which costs no residency beside the slices (at 48
 // the same sweep took 319 us), 64 for up to four (two leaves, 163 small sets: 91 us;
