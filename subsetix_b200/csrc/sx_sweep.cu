@@ -947,9 +947,10 @@ __global__ void __launch_bounds__(SXM_THREADS) sx_merge_kernel(SxBoolArgs A, SxS
 }
 
 // ---------------------------------------------------------------------------
-// Segmented sweep in block tiles (sx_tuning kernel 4; the automatic choice
-// for skewed rows).  The warp-tile forms below (kernels 5 and 6) share its
-// algorithm and are the automatic choice for even rows.
+// Segmented sweep in block tiles (sx_tuning kernel 4; the automatic choice for
+// skewed rows that the row-lane sweep gives up on).  The warp-tile forms below
+// (kernels 5 and 6) share its algorithm; 5 is the choice for even rows whose
+// tiles are too wide for 16 bits.
 //
 // A block owns one tile of 32 aligned rows, as in the merge-path kernel.
 // Thread 0 copies every leaf's begin and end ranges of the tile into shared
