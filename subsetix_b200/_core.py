@@ -153,7 +153,7 @@ def bool_eval(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, i
         # Most operands have rows alike, and the sweep that assumes it needs no pass that
         # measures them first (59 us and a read-back beside a 270 us sweep of 5 x 128 x 4096
         # rows; 35 us of 160 at 256 rows).  It gives up early on others (rows too long, or
-        # too wide for 16-bit coordinates); those are measured and swept again, 70 to 110 us
+        # too wide for 16-bit coordinates); those are measured and swept again, 45 to 110 us
         # later than if they had been measured first.
         ob, oe, ooff, result = bool_eval_async(leaves, rows, table, mode, device, out,
                                                tuning=even_tuning(leaves, rows), even=True)

@@ -2111,6 +2111,11 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // ---------------------------------------------------------------------------
 #define SXR_SPAN 65534
 #define SXR_SENTINEL 0xFFFFu
+// Intervals up to which a wide group is swept in place rather than given up.  Rows of
+// four intervals, two leaves (128 per tile): 84 us on 4096 rows and 139 on 100,000,
+// against 122 and 146 when the set was measured first; five leaves (320 per tile) 125 and
+// 311 against 125 and 166, so those give up.
+#define SXR_LIGHT 200
 #define SXR_HDR_WORDS 4
 
 // Words below the raw copies into which the padded pair lists grow, for k
@@ -2242,7 +2247,7 @@ struct SxrRaw {
 template <int K>
 struct SxrGroup {
     int row, khw, excl, total, src, xmin;  // src: halfword of the piece's staged changes
-    bool act, last, staged, broken, ok;
+    bool act, last, staged, broken, ok, light;
     SxrRaw<K>* raw;
 };
 
@@ -2279,6 +2284,7 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
         PBl += n[l] + TR + 1;
     }
     G.ok = ok;
+    G.light = all <= SXR_LIGHT;
     G.staged = false;
     if (!RAW && ok && all > room) return;
     const bool fits = ok && all <= room;
@@ -2509,7 +2515,7 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
     G.xmin = xmin;
     G.src = 2 * (OA + cap_excl) + prov;
     // groups that cannot be staged: the same pieces over the raw arrays
-    if (RAW && ok && !staged && !A.give_up) {
+    if (RAW && ok && !staged && (!A.give_up || G.light)) {
         SxrRaw<K>& X = *G.raw;
         X.rlo = LLONG_MIN + 1;
         X.rhi = LLONG_MAX;
@@ -2621,7 +2627,7 @@ __device__ __noinline__ void sxr_slow_tile(const SxBoolArgs& A, const SxSweepSta
             const int gn = max(1, __popc(in));  // a row that does not fit alone is swept from global memory
             __syncwarp();
             sxr_group<K, true>(A, r0 + gr, gn, TR, room, W, raw, bar, use, flags, G);
-            if (A.give_up && !G.staged) {
+            if (A.give_up && !G.staged && !G.light) {
                 flags |= SXF_LONG_TILE;
                 if (lane == 0) atomicOr(&st.counters[2], SXF_LONG_TILE);
                 give_up = true;

@@ -69,14 +69,16 @@ def test_skewed_rows_against_the_oracle(cuda_device, x_scale):
         np.testing.assert_array_equal(got[2], want.row_offsets)
 
 
-@pytest.mark.parametrize("heavy,x_scale,long_tile", [(0, 1, False), (40, 1, False), (3000, 1, True), (0, 9000, True),
-                                                     (40, 9000, True)])
-def test_the_even_sweep_gives_up_on_long_rows_and_wide_tiles(cuda_device, heavy, x_scale, long_tile):
+@pytest.mark.parametrize("heavy,x_scale,cap,long_tile", [
+    (0, 1, 600, False), (40, 1, 600, False), (3000, 1, 600, True),  # rows that no slice holds
+    (0, 9000, 600, False),  # wide, at most 192 intervals per tile: swept in place
+    (40, 9000, 600, True), (150, 9000, 2400, True)])  # wide, about 270 and 770
+def test_the_even_sweep_gives_up_on_long_rows_and_wide_tiles(cuda_device, heavy, x_scale, cap, long_tile):
     rng = np.random.default_rng(13)
     rows = 3000
     leaves = [tuple(torch.as_tensor(a, device=cuda_device) for a in _skewed(rng, rows, heavy, x_scale)) + (0,)
               for _ in range(2)]
-    tuning = dict(_core.even_tuning(leaves, rows), staging_cap=600)
+    tuning = dict(_core.even_tuning(leaves, rows), staging_cap=cap, tile_rows=16)
     _, _, _, result = _core.bool_eval_async(leaves, rows, [0b0110] + [0] * 7, _lib.MODE_TABLE, cuda_device,
                                             tuning=tuning, even=True)
     assert int(result[1]) == (_lib.FLAG_LONG_TILE if long_tile else 0)
