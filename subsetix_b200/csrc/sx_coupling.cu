@@ -38,8 +38,8 @@ __device__ __forceinline__ float cp_mul(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double cp_mul(double a, double b) { return __dmul_rn(a, b); }
 
 template <typename T>
-__global__ void index_copy_kernel(long long n, const int* __restrict__ dst_idx, const int* __restrict__ src_idx,
-                                  const T* __restrict__ src, T* __restrict__ dst)
+__global__ void index_copy_kernel(long long n, const int* dst_idx, const int* src_idx,
+                                  const T* src, T* __restrict__ dst)
 {
     sx_after_previous();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -78,8 +78,8 @@ __global__ void block_mean_adj_kernel(long long n, int group, T norm, const int*
 // memory round trips instead of two per source (ghost rings of about 10,000
 // cells: 11.6 -> 5.4 us per launch); the sum keeps the segment order.
 template <typename T>
-__global__ void segment_add_kernel(long long nseg, const int* __restrict__ seg_off, const int* __restrict__ src_idx,
-                                   const int* __restrict__ dst_idx, T* __restrict__ src, T* __restrict__ dst,
+__global__ void segment_add_kernel(long long nseg, const int* seg_off, const int* src_idx,
+                                   const int* dst_idx, T* __restrict__ src, T* __restrict__ dst,
                                    int zero_src)
 {
     sx_after_previous();
@@ -136,7 +136,7 @@ constexpr int RUNS_PER_WARP = 2;
 
 template <typename T, bool PAIR>
 __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, int stride, T norm,
-                                                             const int* __restrict__ plan, const T* __restrict__ in,
+                                                             const int* plan, const T* in,
                                                              T* __restrict__ out)
 {
     sx_after_previous();
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, i
         long long c0[RUNS_PER_WARP], f[RUNS_PER_WARP][2];
 #pragma unroll
         for (int q = 0; q < RUNS_PER_WARP; ++q) {
-            const int4 p = first + q < runs ? __ldg((const int4*)(plan + (long long)(first + q) * stride)) : make_int4(0, 0, 0, 0);
+            const int4 p = first + q < runs ? *(const int4*)(plan + (long long)(first + q) * stride) : make_int4(0, 0, 0, 0);
             c0[q] = p.x;
             count[q] = p.y;
             f[q][0] = p.z;
@@ -182,11 +182,11 @@ __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, i
     } else {
         for (int run = first; run < min(runs, first + RUNS_PER_WARP); ++run) {
             const int* p = plan + (long long)run * stride;
-            const int count = __ldg(p + 1);
-            const long long c0 = __ldg(p);
+            const int count = p[1];
+            const long long c0 = p[0];
             T acc[2] = {T(0), T(0)};
             for (int dy = 0; dy < rr; ++dy) {
-                const long long f0 = __ldg(p + 2 + dy);
+                const long long f0 = p[2 + dy];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int k = lane + 32 * h;
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) run_block_mean_kernel(int runs, int rr, i
 
 template <typename T, bool PAIR>
 __global__ void __launch_bounds__(256) run_block_mean_adj_kernel(int runs, int rr, int stride, T norm,
-                                                                 const int* __restrict__ plan, T* __restrict__ out_bar,
+                                                                 const int* plan, T* __restrict__ out_bar,
                                                                  T* __restrict__ in_bar)
 {
     sx_after_previous();
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) run_block_mean_adj_kernel(int runs, int r
         long long c0[RUNS_PER_WARP], f[RUNS_PER_WARP][2];
 #pragma unroll
         for (int q = 0; q < RUNS_PER_WARP; ++q) {
-            const int4 p = first + q < runs ? __ldg((const int4*)(plan + (long long)(first + q) * stride)) : make_int4(0, 0, 0, 0);
+            const int4 p = first + q < runs ? *(const int4*)(plan + (long long)(first + q) * stride) : make_int4(0, 0, 0, 0);
             c0[q] = p.x;
             count[q] = p.y;
             f[q][0] = p.z;
@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(256) run_block_mean_adj_kernel(int runs, int r
     } else {
         for (int run = first; run < min(runs, first + RUNS_PER_WARP); ++run) {
             const int* p = plan + (long long)run * stride;
-            const int count = __ldg(p + 1);
-            const long long c0 = __ldg(p);
+            const int count = p[1];
+            const long long c0 = p[0];
             T w[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) run_block_mean_adj_kernel(int runs, int r
                 if (k < count) out_bar[c0 + k] = T(0);
             }
             for (int dy = 0; dy < rr; ++dy) {
-                const long long f0 = __ldg(p + 2 + dy);
+                const long long f0 = p[2 + dy];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int k = lane + 32 * h;

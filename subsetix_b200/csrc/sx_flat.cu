@@ -91,7 +91,7 @@ __global__ void span_init_kernel(int* span)
 }
 
 // Last index in [lo, hi] whose entry is not above v (a[lo] <= v holds).
-__device__ __forceinline__ int last_not_above(const int* __restrict__ a, int lo, int hi, int v)
+__device__ __forceinline__ int last_not_above(const int* a, int lo, int hi, int v)
 {
     while (lo < hi) {
         const int mid = lo + ((hi - lo + 1) >> 1);
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(FLAT_THREADS)
 // Four consecutive values from c0: one vector load (two for float64) with VEC,
 // which needs a 16-byte aligned array and a whole group.
 template <typename T, bool VEC>
-__device__ __forceinline__ void load_group(const T* __restrict__ v, long long c0, long long cells, T (&r)[4])
+__device__ __forceinline__ void load_group(const T* v, long long c0, long long cells, T (&r)[4])
 {
     if (VEC && c0 + 4 <= cells) {
         if (sizeof(T) == 4) {
@@ -244,8 +244,8 @@ __device__ __forceinline__ void store_group(T* __restrict__ v, long long c0, lon
 // The neighbours of a group in one row: presence flags nm, the group's plan
 // entry base, and the side array when the group is irregular.
 template <typename T>
-__device__ __forceinline__ void row_group(const T* __restrict__ v, int base, unsigned nm, bool irregular,
-                                          const int4* __restrict__ side, T (&r)[4])
+__device__ __forceinline__ void row_group(const T* v, int base, unsigned nm, bool irregular,
+                                          const int4* side, T (&r)[4])
 {
     int idx[4];
     idx[0] = base;
@@ -253,30 +253,30 @@ __device__ __forceinline__ void row_group(const T* __restrict__ v, int base, uns
     idx[2] = idx[1] + (int)((nm >> 1) & 1u);
     idx[3] = idx[2] + (int)((nm >> 2) & 1u);
     if (irregular) {
-        const int4 s = __ldg(side + base);
+        const int4 s = side[base];
         idx[0] = s.x; idx[1] = s.y; idx[2] = s.z; idx[3] = s.w;
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) r[k] = (nm >> k) & 1u ? __ldg(v + idx[k]) : (T)0;
+    for (int k = 0; k < 4; ++k) r[k] = (nm >> k) & 1u ? v[idx[k]] : (T)0;
 }
 
 // The neighbours on one side within the value array: LEFT those at c - 1, else
 // those at c + 1; 0 where the cell has none.  Lanes hold consecutive groups.
 template <typename T, bool LEFT>
-__device__ __forceinline__ void side_group(const T* __restrict__ v, const T (&cen)[4], unsigned m, long long c0,
+__device__ __forceinline__ void side_group(const T* v, const T (&cen)[4], unsigned m, long long c0,
                                            int lane, T (&r)[4])
 {
     const unsigned hm = (m >> 8) & 15u;
     if (LEFT) {
         T prev = __shfl_up_sync(0xFFFFFFFFu, cen[3], 1);
-        if (lane == 0 && (hm & 1u)) prev = __ldg(v + c0 - 1);
+        if (lane == 0 && (hm & 1u)) prev = v[c0 - 1];
         r[0] = hm & 1u ? prev : (T)0;
 #pragma unroll
         for (int k = 1; k < 4; ++k) r[k] = (hm >> k) & 1u ? cen[k - 1] : (T)0;
     } else {
         T next = __shfl_down_sync(0xFFFFFFFFu, cen[0], 1);
         const bool has = (m >> 14) & 1u;
-        if (lane == 31 && has) next = __ldg(v + c0 + 4);
+        if (lane == 31 && has) next = v[c0 + 4];
         r[3] = has ? next : (T)0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) r[k] = (hm >> (k + 1)) & 1u ? cen[k + 1] : (T)0;
@@ -348,9 +348,9 @@ __global__ void __launch_bounds__(FLAT_THREADS,
                                   ROUNDS == 1      ? STEP_BLOCKS
                                   : sizeof(T) == 4 ? BAND_STEP_BLOCKS_F32
                                                    : BAND_STEP_BLOCKS_F64)
-    flat_step_kernel(const T* __restrict__ v, T* __restrict__ out, long long cells, const int* __restrict__ nbr,
-                     const unsigned short* __restrict__ bits, const int4* __restrict__ side, T a, T bb, T dt, T dx,
-                     T dy, T zx, T zy, int way, const int* __restrict__ band_cell, const T* __restrict__ band_table,
+    flat_step_kernel(const T* v, T* __restrict__ out, long long cells, const int* nbr,
+                     const unsigned short* bits, const int4* side, T a, T bb, T dt, T dx,
+                     T dy, T zx, T zy, int way, const int* band_cell, const T* band_table,
                      int nbands)
 {
     sx_after_previous();
@@ -370,8 +370,8 @@ __global__ void __launch_bounds__(FLAT_THREADS,
 #pragma unroll
     for (int k = 0; k < 4; ++k) cen[k] = (T)0;
     if (g < groups) {
-        m = __ldg(bits + g);
-        base = __ldg(nbr + g);
+        m = bits[g];
+        base = nbr[g];
         load_group<T, VEC>(v, 4 * g, cells, cen);
     }
 #pragma unroll 1
@@ -385,17 +385,17 @@ __global__ void __launch_bounds__(FLAT_THREADS,
 #pragma unroll
         for (int k = 0; k < 4; ++k) nxt[k] = (T)0;
         if (ROUNDS > 1 && round + 1 < ROUNDS && g < groups) {
-            mn = __ldg(bits + g);
-            bn = __ldg(nbr + g);
+            mn = bits[g];
+            bn = nbr[g];
             load_group<T, VEC>(v, 4 * g, cells, nxt);
         }
         if (BANDS && c0 >= band_end) {
-            while (q + 1 < nbands && c0 >= __ldg(band_cell + q + 1)) ++q;
-            band_end = q + 1 < nbands ? __ldg(band_cell + q + 1) : cells;
-            dx = __ldg(band_table + 4 * q);
-            dy = __ldg(band_table + 4 * q + 1);
-            dt = __ldg(band_table + 4 * q + 2);
-            way = __ldg(band_table + 4 * q + 3) != (T)0 ? SX_BY_POW2 : SX_BY_DIVISION;
+            while (q + 1 < nbands && c0 >= band_cell[q + 1]) ++q;
+            band_end = q + 1 < nbands ? band_cell[q + 1] : cells;
+            dx = band_table[4 * q];
+            dy = band_table[4 * q + 1];
+            dt = band_table[4 * q + 2];
+            way = band_table[4 * q + 3] != (T)0 ? SX_BY_POW2 : SX_BY_DIVISION;
         }
         T vn[4], vs[4], x[4], y[4], res[4];
         row_group<T>(v, base, DOWN ? m & 15u : (m >> 4) & 15u, (m >> (DOWN ? 12 : 13)) & 1u, side, vn);
@@ -409,11 +409,11 @@ __global__ void __launch_bounds__(FLAT_THREADS,
             int qk = q;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                while (qk + 1 < nbands && c0 + k >= __ldg(band_cell + qk + 1)) ++qk;
+                while (qk + 1 < nbands && c0 + k >= band_cell[qk + 1]) ++qk;
                 const T* t = band_table + 4 * qk;
-                const int p = __ldg(t + 3) != (T)0;
-                res[k] = sx_upwind_update(cen[k], sx_over(x[k], __ldg(t), p), sx_over(y[k], __ldg(t + 1), p), a, bb,
-                                          __ldg(t + 2));
+                const int p = t[3] != (T)0;
+                res[k] = sx_upwind_update(cen[k], sx_over(x[k], t[0], p), sx_over(y[k], t[1], p), a, bb,
+                                          t[2]);
             }
         } else {
             over_group<T, !BANDS>(x, y, dx, dy, zx, zy, way);
@@ -436,10 +436,10 @@ __global__ void __launch_bounds__(FLAT_THREADS,
 // (zero before the first call, left zero), then two doubles per block.
 template <typename T, bool VEC, int SGN>
 __global__ void __launch_bounds__(FLAT_THREADS, sizeof(T) == 4 ? ADJOINT_BLOCKS : ADJOINT_BLOCKS_F64)
-    flat_adjoint_kernel(const T* __restrict__ w, const T* __restrict__ u, T* __restrict__ ubar, long long cells,
-                        const int* __restrict__ dn, const int* __restrict__ up,
-                        const unsigned short* __restrict__ bits, const int4* __restrict__ side_dn,
-                        const int4* __restrict__ side_up, T a, T bb, T dt, T dx, T dy, T zx, T zy, int way,
+    flat_adjoint_kernel(const T* w, const T* u, T* __restrict__ ubar, long long cells,
+                        const int* dn, const int* up,
+                        const unsigned short* bits, const int4* side_dn,
+                        const int4* side_up, T a, T bb, T dt, T dx, T dy, T zx, T zy, int way,
                         unsigned* __restrict__ counter, double* __restrict__ partial, double* __restrict__ grads,
                         int accumulate)
 {
@@ -454,9 +454,9 @@ __global__ void __launch_bounds__(FLAT_THREADS, sizeof(T) == 4 ? ADJOINT_BLOCKS 
     int bdn = 0, bun = 0;
     const long long first = (long long)blockIdx.x * FLAT_THREADS + threadIdx.x;
     if (first < groups) {
-        mn = __ldg(bits + first);
-        bdn = __ldg(dn + first);
-        bun = __ldg(up + first);
+        mn = bits[first];
+        bdn = dn[first];
+        bun = up[first];
     }
     // whole warps stay in the loop together (the shuffles need every lane)
     for (long long gw = first - lane; gw < groups; gw += (long long)gridDim.x * FLAT_THREADS) {
@@ -475,9 +475,9 @@ __global__ void __launch_bounds__(FLAT_THREADS, sizeof(T) == 4 ? ADJOINT_BLOCKS 
         mn = 0u;
         const long long gn = g + (long long)gridDim.x * FLAT_THREADS;
         if (gn < groups) {
-            mn = __ldg(bits + gn);
-            bdn = __ldg(dn + gn);
-            bun = __ldg(up + gn);
+            mn = bits[gn];
+            bdn = dn[gn];
+            bun = up[gn];
         }
         const unsigned md = m & 15u, mu = (m >> 4) & 15u;
         const bool id = (m >> 12) & 1u, iu = (m >> 13) & 1u;

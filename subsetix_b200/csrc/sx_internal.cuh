@@ -168,7 +168,10 @@ cudaError_t sx_amr_step_full_launch(int dbl, const void* cin, const void* fin, v
                                     double dxc, double dyc, double dxf, double dyf, cudaStream_t stream);
 // Launch of a kernel that calls sx_after_previous() before it touches memory: its blocks
 // may take their places while the kernel before it in the stream still runs its last
-// ones, so a chain of short kernels does not wait for each launch.
+// ones, so a chain of short kernels does not wait for each launch.  Such a kernel is alive
+// while its inputs are written, so it reads global memory by ordinary loads only: neither
+// __ldg nor const __restrict__ parameters, which let the compiler use the read-only path
+// (for data that nobody writes during the whole kernel) and move loads above the wait.
 template <typename... P, typename... Q>
 cudaError_t sx_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Q... args)
 {
@@ -185,7 +188,7 @@ cudaError_t sx_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t 
     return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
 }
 // Lets the next kernel of such a chain take places, then waits until all the memory
-// operations of the kernels before this one are done.
+// operations of the kernels before this one are done and visible to ordinary loads.
 __device__ __forceinline__ void sx_after_previous()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
