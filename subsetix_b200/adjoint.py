@@ -72,9 +72,6 @@ class Level:
         nbytes = max(int(lib.sx_upwind_adjoint_scratch_bytes(self.cells)),
                      int(lib.sx_upwind_adjoint_chunked_scratch_bytes((1 << 31) - 1)))
         self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        # the flat adjoint's block counter must start at zero (every launch leaves it so)
-        self.flat_scratch = torch.zeros(int(lib.sx_upwind_flat_adjoint_scratch_bytes(self.cells)), dtype=torch.uint8,
-                                        device=device)
 
     def _chunk_plan(self) -> None:
         if not self._chunked and self.direct:
@@ -118,13 +115,29 @@ class Level:
                          self.width, self.height, a, b, dt, self.dx, self.dy, self.direct, self.device)
         return out
 
+    def adjoint_scratch(self) -> Optional[torch.Tensor]:
+        """Scratch of :meth:`adjoint` for calls that follow one another on one stream (None: it needs none).
+
+        Its block counter starts at zero and every launch leaves it so, but
+        launches that overlap would mix their counts: each pass and each
+        captured segment has its own.
+        """
+        if self.flat is None:
+            return None
+        return torch.zeros(int(_lib.load().sx_upwind_flat_adjoint_scratch_bytes(self.cells)), dtype=torch.uint8,
+                           device=self.device)
+
     def adjoint(self, w: torch.Tensor, u: torch.Tensor, a: float, b: float, dt: float, grad_ab: torch.Tensor,
-                out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """dL/du for one step (into ``out``), and dL/d(a, b) added into ``grad_ab`` (float64 device pair)."""
+                out: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """dL/du for one step (into ``out``), and dL/d(a, b) added into ``grad_ab`` (float64 device pair).
+
+        ``scratch`` is this stream's (:meth:`adjoint_scratch`), made for the call if not given.
+        """
         lib = _lib.load()
         ubar = torch.empty_like(w) if out is None else out
         if self.flat is not None:
-            self.flat.adjoint(w, u, ubar, a, b, dt, self.dx, self.dy, grad_ab, self.flat_scratch, self.device)
+            scratch = self.adjoint_scratch() if scratch is None else scratch
+            self.flat.adjoint(w, u, ubar, a, b, dt, self.dx, self.dy, grad_ab, scratch, self.device)
             return ubar
         g = torch.empty(2, dtype=torch.float64, device=self.device)
         code = _lib.SX_F64 if w.dtype == torch.float64 else _lib.SX_F32
@@ -188,13 +201,14 @@ class _Advect(torch.autograd.Function):
         a, b = ctx.ab
         w = [g.contiguous() if g is not None else torch.zeros_like(c) for g, c in zip(grad_out, ctx.checkpoints[0])]
         grad_ab = torch.zeros(2, dtype=torch.float64, device=levels[0].device)
+        scratch = [lvl.adjoint_scratch() for lvl in levels]
         seg_starts = list(range(0, steps, every))
         for si in reversed(range(len(seg_starts))):
             n = min(every, steps - seg_starts[si])
             trail = _run(levels, ctx.checkpoints[si], a, b, dt, n, keep=True)  # recompute the segment
             for j in reversed(range(n)):
                 for k, lvl in enumerate(levels):
-                    w[k] = lvl.adjoint(w[k], trail[k][j], a, b, dt, grad_ab)
+                    w[k] = lvl.adjoint(w[k], trail[k][j], a, b, dt, grad_ab, scratch=scratch[k])
         ctx.checkpoints = None
         grad_v = grad_ab.to(device=ctx.vel_device, dtype=ctx.vel_dtype)
         return (grad_v, None, None, None, None, *w)
@@ -370,11 +384,17 @@ class Hierarchy:
         self._restrict(new)
         return new, u
 
+    def adjoint_scratch(self) -> List[Optional[torch.Tensor]]:
+        """Every level's :meth:`Level.adjoint_scratch`."""
+        return [lvl.adjoint_scratch() for lvl in self.levels]
+
     def step_adjoint(self, w: List[torch.Tensor], inputs: List[torch.Tensor], a: float, b: float, dt: float,
-                     grad_ab: torch.Tensor, out: Optional[List[torch.Tensor]] = None) -> List[torch.Tensor]:
+                     grad_ab: torch.Tensor, out: Optional[List[torch.Tensor]] = None,
+                     scratch: Optional[List[Optional[torch.Tensor]]] = None) -> List[torch.Tensor]:
         """Transpose of :meth:`step` applied to ``w`` (modified); ``inputs`` are that step's upwind inputs.
 
-        The result is in ``out`` if given (tensors other than ``w``).
+        The result is in ``out`` if given (tensors other than ``w``);
+        ``scratch`` is this stream's (:meth:`adjoint_scratch`).
         """
         lib = _lib.load()
         r = self.ratio
@@ -383,7 +403,8 @@ class Hierarchy:
             _lib.check(lib.sx_run_block_mean_adj(_code(w[k]), runs, r, stride, 1.0 / (r * r), ptr(plan), ptr(w[k - 1]),
                                                  ptr(w[k]), stream_handle(w[k].device)), "sx_run_block_mean_adj")
         outs = [None] * len(w) if out is None else out
-        w = [lvl.adjoint(x, u, a, b, dt, grad_ab, y) for lvl, x, u, y in zip(self.levels, w, inputs, outs)]
+        scratch = [None] * len(w) if scratch is None else scratch
+        w = [lvl.adjoint(x, u, a, b, dt, grad_ab, y, z) for lvl, x, u, y, z in zip(self.levels, w, inputs, outs, scratch)]
         for k in range(len(self.levels) - 1, 0, -1):
             _, _, seg_off, src, dst = self.ghost[k]
             _lib.check(lib.sx_index_segment_add(_code(w[k]), int(dst.numel()), ptr(seg_off), ptr(src), ptr(dst),
@@ -449,6 +470,7 @@ class _Segment:
         self.state = [torch.zeros(lvl.cells, dtype=dtype, device=dev) for lvl in h.levels]
         self.w = [torch.zeros(lvl.cells, dtype=dtype, device=dev) for lvl in h.levels]
         self.grad = torch.zeros(2, dtype=torch.float64, device=dev)
+        self.scratch = h.adjoint_scratch()
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         self.fwd, self.keep, self.bwd = (torch.cuda.CUDAGraph() for _ in range(3))
@@ -470,7 +492,8 @@ class _Segment:
         def backward():
             w = list(self.w)
             for j in reversed(range(n)):
-                w = h.step_adjoint(w, self.inputs[j], a, b, dt, self.grad, out=self.w if j == 0 and n > 1 else None)
+                w = h.step_adjoint(w, self.inputs[j], a, b, dt, self.grad, out=self.w if j == 0 and n > 1 else None,
+                                   scratch=self.scratch)
             settle(w, self.w)
 
         # Captured one after another without torch.cuda.graph's emptying of the allocator's
@@ -549,6 +572,7 @@ class _AdvectComposite(torch.autograd.Function):
         zeros = [torch.zeros(n, dtype=c.dtype, device=c.device) for n, c in zip(h.inner_cells, ctx.checkpoints[0])]
         w = h.extend([g if g is not None else z for g, z in zip(grad_out, zeros)])
         grad_ab = torch.zeros(2, dtype=torch.float64, device=h.levels[0].device)
+        scratch = None if ctx.graphs else h.adjoint_scratch()
         starts = list(range(0, steps, every))
         for si in reversed(range(len(starts))):
             n = min(every, steps - starts[si])
@@ -558,7 +582,7 @@ class _AdvectComposite(torch.autograd.Function):
             else:
                 _, inputs = _run_composite(h, [x.clone() for x in ctx.checkpoints[si]], a, b, dt, n, keep=True)
                 for j in reversed(range(n)):
-                    w = h.step_adjoint(w, inputs[j], a, b, dt, grad_ab)
+                    w = h.step_adjoint(w, inputs[j], a, b, dt, grad_ab, scratch=scratch)
         ctx.checkpoints = None
         grads = h.interior(w)
         # a copy: the sum may be a segment's own buffer
