@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(256) span_kernel(const int* __restrict__ b, co
                                                    int* __restrict__ span)
 {
     int lo = INT_MAX, hi = INT_MIN;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (long long i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         lo = min(lo, b[i]);
         hi = max(hi, e[i]);
     }
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(FLAT_THREADS)
                      unsigned short* __restrict__ bits, int4* __restrict__ side_dn, int4* __restrict__ side_up)
 {
     __shared__ int s_i[2], s_p[2];
-    const int groups = (cells + 3) >> 2;
+    const int groups = (int)(((long long)cells + 3) >> 2);  // cells may be 2^31 - 1
     const int g0 = blockIdx.x * FLAT_THREADS;
     if (threadIdx.x == 0 || threadIdx.x == 32) {
         const int side = threadIdx.x >> 5;

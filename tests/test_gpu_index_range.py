@@ -1,0 +1,20 @@
+"""Index arithmetic at the top of the int32 range: the largest flat plan, the most rows of a mask, the longest tiles."""
+
+import pytest
+import torch
+
+from subsetix_b200 import _core
+
+pytestmark = pytest.mark.gpu
+
+
+def test_flat_plan_of_the_most_cells(cuda_device):
+    n = 2 ** 31 - 1  # 2^29 groups, the last with three cells
+    b, e, off, rows = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0], [n], [0, 1], [0]))
+    coff, lookup = torch.tensor([0, n], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    plan = _core.FlatPlan(rows, off, b, e, coff, n, lookup, 1, cuda_device)
+    assert (plan.lo, plan.hi) == (0, n) and plan.covers(n)
+    flags = plan._keep[2]
+    left, right = 0xF00, 1 << 14  # every cell has a left neighbour, every group's last cell a right one
+    assert flags[0] == (left & ~0x100) | right and flags[-1] == (left & ~0x800)
+    assert bool((flags[1:-1] == left | right).all())
