@@ -276,8 +276,9 @@ __global__ void __launch_bounds__(256) mask_runs_kernel(const unsigned* __restri
                                                         int words_per_row, const int* __restrict__ offsets,
                                                         int* __restrict__ ob, int* __restrict__ oe)
 {
-    const int y = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (y >= H) return;
+    const unsigned y = blockIdx.x * 8u + (threadIdx.x >> 5);  // not from the thread number: 2^27 rows take 2^32 threads
+    const int lane = threadIdx.x & 31;
+    if (y >= (unsigned)H) return;
     const int first = offsets[y], count = offsets[y + 1] - first;
     if (count == 0) return;
     const unsigned* row = mask + (long long)y * words_per_row;
@@ -313,7 +314,7 @@ template <bool GRAD, bool VEC>
 void mask_go(const float* d, int W, int H, float thr, unsigned* mask, cudaStream_t stream)
 {
     const int strips = (W + 127) / 128;
-    const long long tasks = (long long)strips * ((H + RLE_ROWS - 1) / RLE_ROWS);
+    const long long tasks = (long long)strips * (((long long)H + RLE_ROWS - 1) / RLE_ROWS);
     mask_kernel<GRAD, VEC><<<(int)((tasks + RLE_THREADS / 32 - 1) / (RLE_THREADS / 32)), RLE_THREADS, 0, stream>>>(
         d, W, H, thr, mask, (W + 31) / 32, strips, tasks);
 }
@@ -337,7 +338,7 @@ float sx_least_radicand(float thr)
     return s;
 }
 
-int sx_mask_tiles(int H) { return (H + 7) / 8; }
+int sx_mask_tiles(int H) { return (int)(((long long)H + 7) / 8); }
 
 cudaError_t sx_mask_launch(const float* d, int W, int H, float thr, int grad, unsigned* mask, int* offsets, int* result,
                            const SxScanState& st, cudaStream_t stream)
@@ -362,7 +363,7 @@ cudaError_t sx_gradient_launch(const float* d, int W, int H, float* out, cudaStr
 {
     if (W <= 0 || H <= 0) return cudaSuccess;
     const int strips = (W + 127) / 128;
-    const long long tasks = (long long)strips * ((H + RLE_ROWS - 1) / RLE_ROWS);
+    const long long tasks = (long long)strips * (((long long)H + RLE_ROWS - 1) / RLE_ROWS);
     const int blocks = (int)((tasks + RLE_THREADS / 32 - 1) / (RLE_THREADS / 32));
     if ((W & 3) == 0 && ((uintptr_t)d & 15u) == 0 && ((uintptr_t)out & 15u) == 0)
         gradient_kernel<true><<<blocks, RLE_THREADS, 0, stream>>>(d, W, H, out, strips, tasks);
@@ -374,6 +375,6 @@ cudaError_t sx_gradient_launch(const float* d, int W, int H, float* out, cudaStr
 cudaError_t sx_mask_runs_launch(const unsigned* mask, int W, int H, const int* offsets, int* ob, int* oe,
                                 cudaStream_t stream)
 {
-    mask_runs_kernel<<<(H + 7) / 8, 256, 0, stream>>>(mask, W, H, (W + 31) / 32, offsets, ob, oe);
+    mask_runs_kernel<<<sx_mask_tiles(H), 256, 0, stream>>>(mask, W, H, (W + 31) / 32, offsets, ob, oe);
     return cudaGetLastError();
 }

@@ -18,3 +18,12 @@ def test_flat_plan_of_the_most_cells(cuda_device):
     left, right = 0xF00, 1 << 14  # every cell has a left neighbour, every group's last cell a right one
     assert flags[0] == (left & ~0x100) | right and flags[-1] == (left & ~0x800)
     assert bool((flags[1:-1] == left | right).all())
+
+
+def test_mask_of_the_most_rows(cuda_device):
+    h = 2 ** 27 + 37  # 2^32 threads and more, one warp per row
+    values = (torch.arange(h, device="cuda", dtype=torch.int32) % 3 == 1).to(torch.float32)
+    b, e, off = _core.threshold_rle(values, 1, h, 0.5, False, cuda_device)
+    counts = values.to(torch.int32)
+    assert torch.equal(off[1:] - off[:-1], counts)
+    assert int(b.numel()) == int(off[-1]) and bool((b == 0).all()) and bool((e == 1).all())
