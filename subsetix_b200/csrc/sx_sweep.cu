@@ -2116,6 +2116,9 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // against 122 and 146 when the set was measured first; five leaves (320 per tile) 125 and
 // 311 against 125 and 166, so those give up.
 #define SXR_LIGHT 200
+// Intervals of one leaf that a row counts for, far above every slice: the sums over 8
+// leaves and 32 rows stay inside int32.
+#define SXR_ROW_MAX (1 << 22)
 #define SXR_HDR_WORDS 4
 
 // Words below the raw copies into which the padded pair lists grow, for k
@@ -2279,8 +2282,8 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
         n[l] = ok ? __shfl_sync(0xFFFFFFFFu, hi[l], gn - 1) - g0[l] : 0;
         lo[l] = ok ? lo[l] - g0[l] : 0;
         hi[l] = ok ? hi[l] - g0[l] : 0;
-        mine += hi[l] - lo[l];
-        all += n[l];
+        mine += min(hi[l] - lo[l], SXR_ROW_MAX);
+        all += min(n[l], 32 * SXR_ROW_MAX);
         PBl += n[l] + TR + 1;
     }
     G.ok = ok;
@@ -2607,7 +2610,8 @@ __device__ __noinline__ void sxr_slow_tile(const SxBoolArgs& A, const SxSweepSta
     // running sum of the rows' intervals (lane r: rows 0 .. r of the tile)
     int sum = 0;
 #pragma unroll
-    for (int l = 0; l < K; ++l) sum += A.leaf[l].off[r0 + min(lane + 1, nrows)] - A.leaf[l].off[r0 + min(lane, nrows)];
+    for (int l = 0; l < K; ++l)
+        sum += min(A.leaf[l].off[r0 + min(lane + 1, nrows)] - A.leaf[l].off[r0 + min(lane, nrows)], SXR_ROW_MAX);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xFFFFFFFFu, sum, o);

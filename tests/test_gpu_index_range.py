@@ -1,9 +1,12 @@
 """Index arithmetic at the top of the int32 range: the largest flat plan, the most rows of a mask, the longest tiles."""
 
+import ctypes
+
 import pytest
 import torch
 
-from subsetix_b200 import _core
+from subsetix_b200 import _core, _lib
+from subsetix_b200._runtime import ptr, stream_handle
 
 pytestmark = pytest.mark.gpu
 
@@ -27,3 +30,21 @@ def test_mask_of_the_most_rows(cuda_device):
     counts = values.to(torch.int32)
     assert torch.equal(off[1:] - off[:-1], counts)
     assert int(b.numel()) == int(off[-1]) and bool((b == 0).all()) and bool((e == 1).all())
+
+
+def test_even_sweep_gives_up_on_tiles_of_2_31_intervals(cuda_device):
+    n, rows = 2 ** 28, 8
+    j = torch.arange(n // rows, dtype=torch.int32, device="cuda").repeat(rows)
+    b, e = 2 * j, 2 * j + 1
+    del j
+    off = torch.arange(rows + 1, dtype=torch.int32, device="cuda") * (n // rows)
+    table, lib = (ctypes.c_uint32 * 8)(*[0] * 7, 1 << 31), _lib.load()
+    leaves = (_lib.SxLeaf * 8)(*[_lib.SxLeaf(ptr(b), ptr(e), ptr(off), None, 0, 0)] * 8)
+    tuning = _lib.SxTuning(*(_core.even_tuning([(b,)] * 8, rows).get(key, 0) for key, _ in _lib.SxTuning._fields_))
+    out, result = (torch.empty(32, dtype=torch.int32, device="cuda") for _ in range(2))
+    out_off = torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+    ws = torch.empty(int(lib.sx_bool_workspace_bytes(rows)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.sx_bool_eval_even(leaves, 8, rows, table, ptr(out), ptr(out[16:]), ptr(out_off), 16, ptr(result),
+                                     ptr(ws), int(ws.numel()), ctypes.byref(tuning), stream_handle(cuda_device)),
+               "sx_bool_eval_even")
+    assert result.tolist()[1] == _lib.FLAG_LONG_TILE
