@@ -60,20 +60,29 @@ class IntervalField:
         return int(_t(off)[-1].item())
 
 
+def _version(array):
+    """Modification count of a tensor; None for what counts none (inference tensors, other arrays)."""
+    try:
+        return array._version
+    except (AttributeError, RuntimeError):
+        return None
+
+
 def _packed_field(interval_set: IntervalSet, values, offsets) -> IntervalField:
     """Field whose ``offsets`` are the prefix sum of the interval lengths, marked so (see :func:`_is_packed`)."""
     field = IntervalField(interval_set=interval_set, values=values, interval_cell_offsets=offsets)
-    object.__setattr__(field, "_packed", getattr(offsets, "_version", None))
+    object.__setattr__(field, "_packed", _version(offsets))
     return field
 
 
 def _is_packed(field: IntervalField) -> bool:
     """Whether the field was made by :func:`_packed_field` and its offsets have not been modified since.
 
-    The answer costs no device work; False only means not known.
+    The answer costs no device work; False only means not known, as it is
+    for offsets made under ``torch.inference_mode()``.
     """
     version = getattr(field, "_packed", None)
-    return version is not None and version == getattr(field.interval_cell_offsets, "_version", None)
+    return version is not None and version == _version(field.interval_cell_offsets)
 
 
 def _fill_dtype(fill_value, dtype) -> torch.dtype:
