@@ -26,6 +26,7 @@ There is no counterpart in the reference, which has no derivatives.
 
 from __future__ import annotations
 
+import gc
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
@@ -471,6 +472,22 @@ class _Segment:
         self.w = [torch.zeros(lvl.cells, dtype=dtype, device=dev) for lvl in h.levels]
         self.grad = torch.zeros(2, dtype=torch.float64, device=dev)
         self.scratch = h.adjoint_scratch()
+        for last in (False, True):
+            try:
+                self._capture(h, n, a, b, dt)
+                break
+            except torch.OutOfMemoryError:
+                if last:
+                    raise
+            # A capture allocates from a pool of its own, and memory that the allocator keeps
+            # cached elsewhere is not released for it meanwhile: release it and capture again.
+            self.fwd = self.keep = self.bwd = self.inputs = None
+            torch.cuda.synchronize(dev)
+            gc.collect()
+            torch.cuda.empty_cache()
+
+    def _capture(self, h: "Hierarchy", n: int, a: float, b: float, dt: float) -> None:
+        dev = h.levels[0].device
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         self.fwd, self.keep, self.bwd = (torch.cuda.CUDAGraph() for _ in range(3))
@@ -504,8 +521,13 @@ class _Segment:
                 graph.capture_begin(**({} if graph is self.fwd else {"pool": self.fwd.pool()}))
                 try:
                     work()
-                finally:
-                    graph.capture_end()
+                except BaseException:
+                    try:
+                        graph.capture_end()
+                    except RuntimeError:
+                        pass  # the capture is over either way, and the first error is the one to report
+                    raise
+                graph.capture_end()
         torch.cuda.current_stream(dev).wait_stream(side)
 
     def forward(self, states: Sequence[torch.Tensor]) -> List[torch.Tensor]:
