@@ -45,6 +45,7 @@
 
 #include <climits>
 
+#include "sx_smem_limit.h"
 #include "sx_tile.cuh"
 
 #define SX_SWEEP_WARPS 8
@@ -2984,13 +2985,8 @@ static cudaError_t sx_sweep_launch_k(const SxBoolArgs& A, const SxSweepState& st
         pad = 233472 / A.tune_blocks_per_sm - 1024 - 256;
         if (pad > 232448) pad = 232448;
         if (pad < 0) pad = 0;
-        static int configured = 0;
-        if (pad > configured) {
-            cudaError_t err = cudaFuncSetAttribute(sx_sweep_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   pad);
-            if (err != cudaSuccess) return err;
-            configured = pad;
-        }
+        static SxSmemLimit limit;
+        if (cudaError_t err = limit.raise((const void*)sx_sweep_kernel<K>, pad); err != cudaSuccess) return err;
     }
     const int blocks = (tiles + SX_SWEEP_WARPS - 1) / SX_SWEEP_WARPS;
     sx_sweep_kernel<K><<<blocks, 32 * SX_SWEEP_WARPS, pad, stream>>>(A, st, tiles);
@@ -3001,13 +2997,9 @@ template <int K>
 static cudaError_t sx_sweep_smem_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int ecap,
                                           cudaStream_t stream)
 {
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int smem = SX_SMEM_WARPS * sx_smem_warp_ints(ecap) * (int)sizeof(int);
-    if (smem > configured) {
-        cudaError_t err = cudaFuncSetAttribute(sx_sweep_smem_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (err != cudaSuccess) return err;
-        configured = smem;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_sweep_smem_kernel<K>, smem); err != cudaSuccess) return err;
     const int blocks = (tiles + SX_SMEM_WARPS - 1) / SX_SMEM_WARPS;
     sx_sweep_smem_kernel<K><<<blocks, 32 * SX_SMEM_WARPS, smem, stream>>>(A, st, tiles, ecap);
     return cudaGetLastError();
@@ -3031,13 +3023,8 @@ template <int K>
 static cudaError_t sx_merge_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_bytes,
                                      cudaStream_t stream)
 {
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
-    if (cap_bytes > configured) {
-        cudaError_t err =
-            cudaFuncSetAttribute(sx_merge_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap_bytes);
-        if (err != cudaSuccess) return err;
-        configured = cap_bytes;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_merge_kernel<K>, cap_bytes); err != cudaSuccess) return err;
     sx_merge_kernel<K><<<tiles, SXM_THREADS, cap_bytes, stream>>>(A, st, tiles, cap_bytes);
     return cudaGetLastError();
 }
@@ -3046,13 +3033,9 @@ template <int K>
 static cudaError_t sx_seg_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_keys, int threads,
                                    int tr, cudaStream_t stream)
 {
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int bytes = 4 * cap_keys;
-    if (bytes > configured) {
-        cudaError_t err = cudaFuncSetAttribute(sx_seg_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (err != cudaSuccess) return err;
-        configured = bytes;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_seg_kernel<K>, bytes); err != cudaSuccess) return err;
     sx_seg_kernel<K><<<tiles, threads, bytes, stream>>>(A, st, tiles, cap_keys, tr);
     return cudaGetLastError();
 }
@@ -3061,13 +3044,9 @@ template <int K>
 static cudaError_t sx_wseg_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words, int warps,
                                     int tr, cudaStream_t stream)
 {
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int bytes = warps * (int)sxw_slice_bytes(K, tr, cap_words);
-    if (bytes > configured) {
-        cudaError_t err = cudaFuncSetAttribute(sx_wseg_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (err != cudaSuccess) return err;
-        configured = bytes;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_wseg_kernel<K>, bytes); err != cudaSuccess) return err;
     const int blocks = (tiles + warps - 1) / warps;
     sx_wseg_kernel<K><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words, tr);
     return cudaGetLastError();
@@ -3077,14 +3056,9 @@ template <int K>
 static cudaError_t sx_wseg16_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
                                       int warps, int tr, cudaStream_t stream)
 {
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int bytes = warps * (int)sxw_slice_bytes(K, tr, cap_words);
-    if (bytes > configured) {
-        cudaError_t err =
-            cudaFuncSetAttribute(sx_wseg16_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (err != cudaSuccess) return err;
-        configured = bytes;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_wseg16_kernel<K>, bytes); err != cudaSuccess) return err;
     const int blocks = (tiles + warps - 1) / warps;
     sx_wseg16_kernel<K><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words, tr);
     return cudaGetLastError();
@@ -3094,14 +3068,9 @@ template <int K>
 static cudaError_t sx_rlane16_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
                                        int warps, int tr, cudaStream_t stream)
 {
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int bytes = warps * (int)sxr_slice_bytes(cap_words);
-    if (bytes > configured) {
-        cudaError_t err =
-            cudaFuncSetAttribute(sx_rlane16_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (err != cudaSuccess) return err;
-        configured = bytes;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_rlane16_kernel<K>, bytes); err != cudaSuccess) return err;
     const int blocks = (tiles + warps - 1) / warps;
     sx_rlane16_kernel<K><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words, tr);
     return cudaGetLastError();
@@ -3136,13 +3105,9 @@ static cudaError_t sx_union_launch_k(const SxBoolArgs& A, const SxSweepState& st
     const long long src_rows = A.leaf[0].scale > 1 ? tr * K : tr + K - 1;
     long long cap = (3 * (A.capacity / K + 1) / A.rows + 1) * src_rows / 2 + 32;
     if (cap > 6000) cap = 6000;
-    static int configured = 0;  // largest dynamic shared memory set for this instantiation
     const int bytes = SXU_WARPS * sxu_slice_words((int)cap) * (int)sizeof(int);
-    if (bytes > configured) {
-        cudaError_t err = cudaFuncSetAttribute(sx_union_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (err != cudaSuccess) return err;
-        configured = bytes;
-    }
+    static SxSmemLimit limit;
+    if (cudaError_t err = limit.raise((const void*)sx_union_kernel<K>, bytes); err != cudaSuccess) return err;
     const int blocks = (tiles + SXU_WARPS - 1) / SXU_WARPS;
     sx_union_kernel<K><<<blocks, 32 * SXU_WARPS, bytes, stream>>>(A, st, tiles, lg, (int)cap, shared);
     return cudaGetLastError();
