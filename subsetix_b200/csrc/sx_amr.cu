@@ -391,7 +391,7 @@ __device__ __forceinline__ SxaPf sxp_div_double(SxaPf a, float d, double z)
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const double t = (double)x[k], q = __dmul_rn(t, z);
-        x[k] = (float)__fma_rn(__fma_rn(q, -(double)d, t), z, q);
+        x[k] = (float)__fma_rn(-__fma_rn(q, (double)d, -t), z, q);
     }
     return sxp_make(x);
 }
@@ -535,18 +535,24 @@ struct SxaStep {
     SxaSpan<T> xc, yc, xf, yf;
 };
 
+// Whether sxa_over gives the negated quotient: for the three operations on pairs, which
+// have no negated operands, that is what keeps the sign of a zero (see sx_by_const)
+// without a fourth one.
+template <int DIV>
+constexpr bool sxa_negated = DIV == SX_BY_CONST || DIV == SX_BY_SCALED;
+
 // t over the spacing; key takes the smallest key of the scaled quotients.
 template <typename T, int DIV>
 __device__ __forceinline__ SxaP<T> sxa_over(SxaP<T> t, const SxaSpan<T>& w, unsigned& key)
 {
     if constexpr (DIV == SX_BY_POW2) return sxp_mul(t, sxp_all(w.z));
     if constexpr (DIV == SX_BY_CONST) {
-        const SxaP<T> z = sxp_all(w.z), q = sxp_mul(t, z);
-        return sxp_fma(sxp_fma(q, sxp_all(-w.d), t), z, q);
+        const SxaP<T> nz = sxp_all(-w.z), nq = sxp_mul(t, nz);
+        return sxp_fma(sxp_fma(nq, sxp_all(w.d), t), nz, nq);
     }
     if constexpr (DIV == SX_BY_SCALED) {
-        const SxaP<T> u = sxp_mul(t, sxp_all((T)0x1p64)), z = sxp_all(w.z), q = sxp_mul(u, z);
-        const SxaP<T> v = sxp_mul(sxp_fma(sxp_fma(q, sxp_all(-w.d), u), z, q), sxp_all((T)0x1p-64));
+        const SxaP<T> u = sxp_mul(t, sxp_all((T)0x1p64)), nz = sxp_all(-w.z), nq = sxp_mul(u, nz);
+        const SxaP<T> v = sxp_mul(sxp_fma(sxp_fma(nq, sxp_all(w.d), u), nz, nq), sxp_all((T)0x1p-64));
         key = min(key, sxp_small_key(v));
         return v;
     }
@@ -564,7 +570,8 @@ __device__ __forceinline__ void sxa_step_row(const SxaRow<T>& Q, SxaP<T> vc, Sxa
 {
     typedef SxaP<T> P;
     constexpr bool LEFT = (SGN & 1) != 0, DOWN = (SGN & 2) != 0;
-    const P a = sxp_all(S.a), b = sxp_all(S.b), ndt = sxp_all(sizeof(T) == 4 ? -S.dt : S.dt);
+    const P a = sxp_all(sxa_negated<DIV> ? -S.a : S.a), b = sxp_all(sxa_negated<DIV> ? -S.b : S.b);
+    const P ndt = sxp_all(sizeof(T) == 4 ? -S.dt : S.dt);
     auto update = [&](P c, P h, P v, const SxaSpan<T>& wx, const SxaSpan<T>& wy) {
         const P tx = LEFT ? sxp_sub(c, h) : sxp_sub(h, c), ty = DOWN ? sxp_sub(c, v) : sxp_sub(v, c);
         return sxp_update(c, sxa_over<T, DIV>(tx, wx, key), sxa_over<T, DIV>(ty, wy, key), a, b, ndt);

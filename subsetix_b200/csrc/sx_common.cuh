@@ -189,12 +189,13 @@ __device__ __forceinline__ float sx_grad_norm(float gx, float gy)
 
 // ---------------------------------------------------------------------------
 // Division by a divisor known beforehand: with z = RN(1 / d), q = RN(x z) and the
-// remainder r = x - q d, which one fma gives exactly, RN(q + r z) is the correctly
+// remainder r = q d - x, which one fma gives exactly, RN(q - r z) is the correctly
 // rounded x / d (P. Markstein, IBM J. Res. Dev. 34, 1990; N. Brisebarre, J.-M. Muller
 // and S. K. Raina, IEEE Trans. Computers 53, 2004) as long as nothing under- or
 // overflows: three operations instead of a general division.  For d within
-// 2^-60 .. 2^24 (SX_BY_CONST is only chosen then) that holds for x = 0 (-0 comes out
-// as +0) and for |x| >= 2^-100 (float32) or 2^-900 (float64); a quotient that
+// 2^-60 .. 2^24 (SX_BY_CONST is only chosen then) that holds for x = 0 (either sign: r
+// is +0 then, so -r z is -0 and leaves q as it is; x - q d would turn -0 into +0)
+// and for |x| >= 2^-100 (float32) or 2^-900 (float64); a quotient that
 // overflows comes out as NaN.  So callers test for smaller x and for results that
 // are not finite, and divide there.  (Float32: 2^64 x is large enough for every x, and
 // 2^-64 times the quotient is exact unless the result is subnormal: SX_BY_SCALED, for
@@ -234,12 +235,12 @@ __device__ __forceinline__ unsigned sx_large_key(double x) { return 2u * (unsign
 __device__ __forceinline__ float sx_by_const(float x, float d, float z)
 {
     const float q = __fmul_rn(x, z);
-    return __fmaf_rn(__fmaf_rn(q, -d, x), z, q);
+    return __fmaf_rn(-__fmaf_rn(q, d, -x), z, q);
 }
 __device__ __forceinline__ double sx_by_const(double x, double d, double z)
 {
     const double q = __dmul_rn(x, z);
-    return __fma_rn(__fma_rn(q, -d, x), z, q);
+    return __fma_rn(-__fma_rn(q, d, -x), z, q);
 }
 
 template <typename T>
