@@ -137,7 +137,10 @@ int sx_bool_eval(const sx_leaf* leaves /* host array of k */, int k, int32_t row
  * alone, or a group of rows spanning more than 65534 columns, ends the sweep
  * with SX_FLAG_LONG_TILE in result[1] and undefined outputs instead of being
  * swept slowly; the caller then runs sx_bool_eval.  It saves the pass that
- * would have to look for such tiles first. */
+ * would have to look for such tiles first.  After SX_FLAG_LONG_TILE words 32,
+ * 33 and 34 of the workspace hold the intervals (of all leaves) of the largest
+ * 8 rows of a tile, those of the largest aligned 32 rows around a tile that
+ * gave up, and 1 (3: one was too wide).  result may point at word 40. */
 int sx_bool_eval_even(const sx_leaf* leaves /* host array of k */, int k, int32_t rows,
                       const uint32_t* table /* host, 8 words */, int32_t* out_begin, int32_t* out_end,
                       int32_t* out_offsets, int64_t capacity, int32_t* result, void* workspace,

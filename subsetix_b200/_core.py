@@ -16,7 +16,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 
 from . import _lib
-from ._runtime import ptr, read_pair, stream_handle, workspace
+from ._runtime import ptr, read_pair, stream_handle, workspace, workspace_words
 
 I32 = torch.int32
 
@@ -106,7 +106,7 @@ def auto_tuning(leaves, rows: int, device) -> dict:
     return {"kernel": 4, "staging_cap": min(need32, 25000), "tile_rows": 32, "warps": 4}
 
 
-def even_tuning(leaves, rows: int) -> dict:
+def even_tuning(leaves, rows: int, total: Optional[int] = None) -> dict:
     """The launch shape of ``sx_bool_eval_even``, from the operands' sizes alone.
 
     The row-lane sweep on tiles of 16 rows, or 8 when rows are so long that a
@@ -120,7 +120,8 @@ def even_tuning(leaves, rows: int) -> dict:
     with 32, 615 us when the slices fall short of the largest tiles; the sweep
     alone 274 us at 10 blocks per SM, 289 us at 9.
     """
-    k, total = len(leaves), sum(int(leaf[0].numel()) for leaf in leaves)
+    k = len(leaves)
+    total = sum(int(leaf[0].numel()) for leaf in leaves) if total is None else total
     tr = 16 if 16 * total <= _TILE_INTERVALS * rows else 8
     mean = tr * total // max(1, rows)
     gap = max((k - 1) * (tr - 7) + tr, k * (tr + 1) + tr - 16 * k) + 4
@@ -153,20 +154,77 @@ def bool_eval(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, i
         # Most operands have rows alike, and the sweep that assumes it needs no pass that
         # measures them first (59 us and a read-back beside a 270 us sweep of 5 x 128 x 4096
         # rows; 35 us of 160 at 256 rows).  It gives up early on others (rows too long, or
-        # too wide for 16-bit coordinates); those are measured and swept again, 45 to 110 us
-        # later than if they had been measured first.
-        ob, oe, ooff, result = bool_eval_async(leaves, rows, table, mode, device, out,
-                                               tuning=even_tuning(leaves, rows), even=True)
-        total, flags = read_pair(result)
-        if flags != _lib.FLAG_LONG_TILE:
-            return ob, oe, ooff, total, flags
-        out = (ob, oe)
-        tuning = auto_tuning(leaves, rows, device)
+        # too wide for 16-bit coordinates), and what it has counted by then shapes the launch
+        # for those.
+        return _eval_even(leaves, rows, table, device, out)
     ob, oe, ooff, result = bool_eval_async(leaves, rows, table, mode, device, out, tuning=tuning)
     if result is None:
         return ob, oe, ooff, 0, 0
     total, flags = read_pair(result)
     return ob, oe, ooff, total, flags
+
+
+def _eval_even(leaves, rows: int, table, device, out):
+    """:func:`bool_eval` of a truth table without a launch shape: the sweep for even rows, then another if it gives up."""
+    lib = _lib.load()
+    args, cap, (ob, oe, ooff) = _sweep_args(leaves, rows, table, device, out, None)
+    wsp, wsn, words = workspace_words(device, int(lib.sx_bool_workspace_bytes(int(rows))))
+    stream = stream_handle(device)
+    tuning = even_tuning(leaves, rows, cap)
+    outs = (ob.data_ptr(), oe.data_ptr(), ooff.data_ptr(), cap, wsp + 160, wsp, wsn)
+    _lib.check(lib.sx_bool_eval_even(*args, *outs, ctypes.byref(_tuning_struct(tuning)), stream), "sx_bool_eval_even")
+    most8, most32, why, *_, total, flags = words.tolist()
+    if flags == _lib.FLAG_LONG_TILE:
+        tuning = _uneven_tuning(leaves, rows, device, tuning, most8, most32, why == 3)
+        _lib.check(lib.sx_bool_eval(*args, _lib.MODE_TABLE, *outs, ctypes.byref(_tuning_struct(tuning)), stream),
+                   "sx_bool_eval")
+        total, flags = words.tolist()[8:]
+    return ob, oe, ooff, total, flags
+
+
+def _uneven_tuning(leaves, rows: int, device, even: dict, most8: int, most32: int, wide: bool) -> dict:
+    """The launch shape after ``sx_bool_eval_even`` (tuned ``even``) has given up, by what it has counted.
+
+    The choice is that of :func:`auto_tuning`: kernel 5 for even rows too
+    wide for 16 bits, its buffers for the largest 8 rows; kernel 4 for
+    skewed ones, its buffers for the largest 32 rows, those around a tile
+    that gave up or two tiles that fitted.  Even, narrow rows that no slice
+    holds are long; measuring them costs little beside their sweep.
+    """
+    mean8 = 2 * sum(int(leaf[0].numel()) for leaf in leaves) / max(1, (rows + 7) // 8)
+    if 2 * most8 > 3 * mean8 + 256:
+        return {"kernel": 4, "staging_cap": min(max(2 * most32, 2 * even["staging_cap"]), 25000), "tile_rows": 32,
+                "warps": 4}
+    if wide:
+        return {"kernel": 5, "staging_cap": min(2 * most8, 25000), "tile_rows": 8, "warps": 2}
+    return auto_tuning(leaves, rows, device)
+
+
+_TUNING_FIELDS = [name for name, _ in _lib.SxTuning._fields_]
+_TABLE_WORDS = ctypes.c_uint32 * 8
+
+
+def _tuning_struct(t: dict) -> "_lib.SxTuning":
+    return _lib.SxTuning(*[int(t.get(name, 0)) for name in _TUNING_FIELDS])
+
+
+def _sweep_args(leaves, rows: int, table, device, out, offsets):
+    """``((leaves, k, rows, table), capacity, (begin, end, offsets))`` of a sweep, for the C calls."""
+    k = len(leaves)
+    cap = max(1, sum([int(leaf[0].numel()) for leaf in leaves]))
+    if out is None:
+        ob = empty_i32(cap, device)
+        oe = empty_i32(cap, device)
+    else:
+        ob, oe = out
+        if ob.numel() < cap or oe.numel() < cap:
+            raise ValueError("output buffers below the required capacity")
+    ooff = empty_i32(rows + 1, device) if offsets is None else offsets
+    arr = (_lib.SxLeaf * k)(*[_lib.SxLeaf(ptr(leaf[0]), ptr(leaf[1]), ptr(leaf[2]),
+                                          ptr(leaf[5]) if len(leaf) > 5 else None, int(leaf[3]),
+                                          int(leaf[4]) if len(leaf) > 4 else 0) for leaf in leaves])
+    tab = _TABLE_WORDS(*[int(x) & 0xFFFFFFFF for x in (list(table) + [0] * 8)[:8]])
+    return (arr, k, int(rows), tab), cap, (ob, oe, ooff)
 
 
 def bool_eval_async(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]], rows: int,
@@ -181,26 +239,12 @@ def bool_eval_async(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Ten
     workspace, for launches captured in a graph.
     """
     lib = _lib.load()
-    k = len(leaves)
-    sizes = [int(leaf[0].numel()) for leaf in leaves]
-    cap = max(1, sum(sizes))
-    if out is None:
-        ob = empty_i32(cap, device)
-        oe = empty_i32(cap, device)
-    else:
-        ob, oe = out
-        if ob.numel() < cap or oe.numel() < cap:
-            raise ValueError("output buffers below the required capacity")
-    ooff = empty_i32(rows + 1, device) if offsets is None else offsets
+    args, cap, (ob, oe, ooff) = _sweep_args(leaves, rows, table, device, out, offsets)
     if rows == 0:
         ooff.zero_()
         return ob, oe, ooff, None
     if result is None:
         result = empty_i32(2, device)
-    arr = (_lib.SxLeaf * k)(*[_lib.SxLeaf(ptr(leaf[0]), ptr(leaf[1]), ptr(leaf[2]),
-                                          ptr(leaf[5]) if len(leaf) > 5 else None, int(leaf[3]),
-                                          int(leaf[4]) if len(leaf) > 4 else 0) for leaf in leaves])
-    tab = (ctypes.c_uint32 * 8)(*[int(x) & 0xFFFFFFFF for x in (list(table) + [0] * 8)[:8]])
     need = int(lib.sx_bool_workspace_bytes(int(rows)))
     if scratch is None:
         wsp, wsn = workspace(device, need)
@@ -208,16 +252,13 @@ def bool_eval_async(leaves: Sequence[Tuple[torch.Tensor, torch.Tensor, torch.Ten
         if int(scratch.numel()) < need:
             raise ValueError("scratch below sx_bool_workspace_bytes(rows)")
         wsp, wsn = scratch.data_ptr(), int(scratch.numel())
-    t = TUNING if tuning is None else tuning
-    tun = _lib.SxTuning(int(t.get("kernel", 0)), int(t.get("blocks_per_sm", 0)), int(t.get("staging_cap", 0)),
-                        int(t.get("warps", 0)), int(t.get("tile_rows", 0)), int(t.get("wait_limit", 0)),
-                        int(t.get("withhold_tile", 0)))
+    tun = _tuning_struct(TUNING if tuning is None else tuning)
     if even:
-        rc = lib.sx_bool_eval_even(arr, k, int(rows), tab, ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp, wsn,
-                                   ctypes.byref(tun), stream_handle(device))
+        rc = lib.sx_bool_eval_even(*args, ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp, wsn, ctypes.byref(tun),
+                                   stream_handle(device))
     else:
-        rc = lib.sx_bool_eval(arr, k, int(rows), tab, int(mode), ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp,
-                              wsn, ctypes.byref(tun), stream_handle(device))
+        rc = lib.sx_bool_eval(*args, int(mode), ptr(ob), ptr(oe), ptr(ooff), cap, ptr(result), wsp, wsn,
+                              ctypes.byref(tun), stream_handle(device))
     _lib.check(rc, "sx_bool_eval")
     return ob, oe, ooff, result
 

@@ -82,14 +82,26 @@ def stream_handle(device: torch.device) -> int:
 
 
 class _Workspace:
-    __slots__ = ("buf",)
+    __slots__ = ("buf", "words")
 
     def __init__(self):
         self.buf = None
+        self.words = None
 
 
 def workspace(device: torch.device, nbytes: int) -> Tuple[int, int]:
     """Pointer and size of the scratch buffer for the current stream (grown to ``nbytes``)."""
+    buf = _workspace(device, nbytes).buf
+    return buf.data_ptr(), buf.numel()
+
+
+def workspace_words(device: torch.device, nbytes: int) -> Tuple[int, int, torch.Tensor]:
+    """:func:`workspace` and its words 32 to 41: what sweeps leave there, and a place for their result at word 40."""
+    ws = _workspace(device, nbytes)
+    return ws.buf.data_ptr(), ws.buf.numel(), ws.words
+
+
+def _workspace(device: torch.device, nbytes: int) -> _Workspace:
     pools: Dict[Tuple[int, int], _Workspace] = getattr(_state, "pools", None)
     if pools is None:
         pools = {}
@@ -105,7 +117,8 @@ def workspace(device: torch.device, nbytes: int) -> Tuple[int, int]:
         # The old buffer may still be in use by queued kernels; the caching
         # allocator keeps its memory alive until the stream passes this point.
         ws.buf = torch.zeros(size, dtype=torch.uint8, device=device)
-    return ws.buf.data_ptr(), ws.buf.numel()
+        ws.words = ws.buf[128:168].view(torch.int32)
+    return ws
 
 
 def reset_workspaces() -> None:

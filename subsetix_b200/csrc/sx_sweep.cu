@@ -2121,6 +2121,7 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // leaves and 32 rows stay inside int32.
 #define SXR_ROW_MAX (1 << 22)
 #define SXR_HDR_WORDS 4
+#define SXR_STATS 32  // words of the look-back state's head: what a sweep that gave up found out
 
 // Words below the raw copies into which the padded pair lists grow, for k
 // leaves and tiles of tr rows.  Leaf l's list starts at most l (tr - 7) words
@@ -2251,17 +2252,19 @@ struct SxrRaw {
 template <int K>
 struct SxrGroup {
     int row, khw, excl, total, src, xmin;  // src: halfword of the piece's staged changes
-    bool act, last, staged, broken, ok, light;
+    bool act, last, staged, broken, ok, light, wide;  // wide: fits the slice, but not 16 bits
     SxrRaw<K>* raw;
 };
 
 // One group: rows q0 .. q0 + gn - 1, at most `room` intervals (more, in a single
-// row, are not staged).  Without RAW a group that cannot be staged is only
-// reported (G.staged false).
+// row, are not staged).  Without RAW the group is a whole tile: one that cannot be
+// staged is only reported (G.staged false), and with A.give_up its largest 8 rows
+// are noted in stats if they exceed `seen`, an earlier value of it.  With RAW it is swept over the raw arrays, unless A.give_up
+// wants to know of it (insist: it is written now).
 template <int K, bool RAW>
 __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, int TR, int room, unsigned* W, unsigned* raw,
                                           unsigned long long* bar, unsigned& use, unsigned& flags,
-                                          SxrGroup<K>& G)
+                                          SxrGroup<K>& G, unsigned* stats, unsigned seen, bool insist)
 {
     const int lane = threadIdx.x & 31;
     unsigned short* const h16 = (unsigned short*)W;
@@ -2289,7 +2292,12 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
     }
     G.ok = ok;
     G.light = all <= SXR_LIGHT;
-    G.staged = false;
+    G.staged = G.wide = false;
+    if (!RAW && A.give_up && ok) {
+        const int low = __reduce_add_sync(0xFFFFFFFFu, lane < 8 ? mine : 0);
+        const unsigned most = (unsigned)max(low, all - low);
+        if (lane == 0 && most > seen) atomicMax(stats, most);
+    }
     if (!RAW && ok && all > room) return;
     const bool fits = ok && all <= room;
     const int OA = PBl;  // output areas start after the pair lists
@@ -2389,6 +2397,7 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
         }
     }
     const bool staged = fits && copied && (xmin > xmax || (long long)xmax - (long long)xmin <= SXR_SPAN);
+    G.wide = fits && copied && !staged;
     bool bad = false;
     // 3. padded pair lists, leaf by leaf; qr[l] is this row's rank among the leaf's non-empty rows
     int qr[K], pb[K];
@@ -2519,7 +2528,7 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
     G.xmin = xmin;
     G.src = 2 * (OA + cap_excl) + prov;
     // groups that cannot be staged: the same pieces over the raw arrays
-    if (RAW && ok && !staged && (!A.give_up || G.light)) {
+    if (RAW && ok && !staged && (!A.give_up || G.light || insist)) {
         SxrRaw<K>& X = *G.raw;
         X.rlo = LLONG_MIN + 1;
         X.rhi = LLONG_MAX;
@@ -2599,6 +2608,38 @@ __device__ __forceinline__ void sxr_put(const SxBoolArgs& A, const SxrGroup<K>& 
     if (G.last) A.out_off[q0 + G.row + 1] = at + ((G.excl + G.khw) >> 1);
 }
 
+// A tile that ends the sweep (A.give_up).  What the caller needs for another launch is
+// left in stats: the intervals of the largest 8 rows (noted by the other tiles too)
+// and of the largest aligned 32 rows around such a tile, and 1, or 3 for a tile that
+// was too wide; tiles that would change nothing there only read it (every tile's
+// atomics on those words took 69 us on 100,000 rows, 36 us so).  It publishes a prefix at once, since all that follows it is void: the tiles
+// after it find SXF_LONG_TILE there and wait for nobody before it.
+template <int K>
+__device__ __noinline__ void sxr_give_up(const SxBoolArgs& A, const SxSweepState& st, int tile, int tiles, int TR,
+                                         bool wide)
+{
+    const int lane = threadIdx.x & 31, r = ((tile * TR) & ~31) + lane;
+    unsigned* const stats = st.counters + SXR_STATS;
+    int c = 0;
+    if (r < A.rows) {
+#pragma unroll
+        for (int l = 0; l < K; ++l) c += max(0, min(A.leaf[l].off[r + 1] - A.leaf[l].off[r], SXR_ROW_MAX));
+    }
+    int c8 = c;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) c8 += __shfl_xor_sync(0xFFFFFFFFu, c8, o);
+    const unsigned most8 = __reduce_max_sync(0xFFFFFFFFu, (unsigned)c8), all = __reduce_add_sync(0xFFFFFFFFu, (unsigned)c);
+    if (lane == 0) {
+        const volatile unsigned* const now = stats;
+        const unsigned n0 = now[0], n1 = now[1], n2 = now[2], why = wide ? 3u : 1u;
+        if (most8 > n0) atomicMax(stats, most8);
+        if (all > n1) atomicMax(stats + 1, all);
+        if (why & ~n2) atomicOr(stats + 2, why);
+        atomicExch(&st.tile_status[tile], ((unsigned long long)SXF_LONG_TILE << 34) | (SX_KIND_PREFIX << 32));
+    }
+    sxs_report(A, tile, tiles, 0, 0, SXF_LONG_TILE);
+}
+
 // A tile that does not fit its slice, or is too wide for 16 bits: groups of rows
 // that fit, swept once to count and, when the look-back has placed the tile, again
 // to write.  Rare, and kept out of line so that it costs the others no registers.
@@ -2622,22 +2663,18 @@ __device__ __noinline__ void sxr_slow_tile(const SxBoolArgs& A, const SxSweepSta
     SxrGroup<K> G;
     G.raw = &rawx;
     int base = 0, done = 0;  // the tile's base; intervals of the groups before
-    bool give_up = (flags & SXF_LONG_TILE) != 0u;  // another tile has given up
     for (int phase = 0; phase < 2; ++phase) {
         done = 0;
-        for (int gr = 0; gr < nrows && !give_up;) {
+        for (int gr = 0; gr < nrows;) {
             const int upto = __shfl_sync(0xFFFFFFFFu, sum, gr > 0 ? gr - 1 : 0);
             const int before = gr > 0 ? upto : 0;
             const unsigned in = __ballot_sync(0xFFFFFFFFu, lane >= gr && lane < nrows && sum - before <= room);
             const int gn = max(1, __popc(in));  // a row that does not fit alone is swept from global memory
             __syncwarp();
-            sxr_group<K, true>(A, r0 + gr, gn, TR, room, W, raw, bar, use, flags, G);
-            if (A.give_up && !G.staged && !G.light) {
-                flags |= SXF_LONG_TILE;
-                if (lane == 0) atomicOr(&st.counters[2], SXF_LONG_TILE);
-                give_up = true;
-                done = 0;
-                break;
+            sxr_group<K, true>(A, r0 + gr, gn, TR, room, W, raw, bar, use, flags, G, nullptr, 0u, phase == 1);
+            if (A.give_up && phase == 0 && !G.staged && !G.light) {
+                sxr_give_up<K>(A, st, tile, tiles, TR, G.wide);
+                return;
             }
             if (phase == 1) sxr_put<K, true>(A, G, W, r0 + gr, base + done);
             done += G.total;
@@ -2662,22 +2699,31 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : 3)
     const int gap = sxr_gap_words(K, TR);
     unsigned* const raw = W + gap;  // the bulk copies
     int tile = 0;
-    unsigned flags = 0u, use = 0u;
+    unsigned flags = 0u, use = 0u, seen = 0u, given_up = 0u;  // given_up: by another tile
     if (lane == 0) {
         tile = (int)atomicAdd(&st.counters[0], 1u);
-        if (A.give_up) flags = *(volatile unsigned*)&st.counters[2];
+        if (A.give_up) {
+            const volatile unsigned* const now = st.counters + SXR_STATS;
+            seen = now[0];
+            given_up = now[2];
+        }
         sxs_bar_init(bar);
     }
     tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
-    flags = __shfl_sync(0xFFFFFFFFu, flags, 0);
+    given_up = __shfl_sync(0xFFFFFFFFu, given_up, 0);
     const int r0 = tile * TR;
     const int nrows = min(TR, A.rows - r0);
     if (tile == 0 && lane == 0) A.out_off[0] = 0;
     const int room = (cap_words - gap) / 2 - 11 * K;  // intervals that fit whatever their alignment
     SxrGroup<K> G;
-    G.staged = false;
+    G.staged = G.wide = G.light = false;
     G.ok = true;
-    if (flags == 0u) sxr_group<K, false>(A, r0, nrows, TR, room, W, raw, bar, use, flags, G);
+    if (!given_up)
+        sxr_group<K, false>(A, r0, nrows, TR, room, W, raw, bar, use, flags, G, st.counters + SXR_STATS, seen, false);
+    if (A.give_up && (given_up || (G.wide && !G.light))) {
+        sxr_give_up<K>(A, st, tile, tiles, TR, G.wide);
+        return;
+    }
     if (!G.staged && G.ok) {
         sxr_slow_tile<K>(A, st, tile, tiles, r0, nrows, TR, room, W, raw, bar, use, flags);
         return;
