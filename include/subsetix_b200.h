@@ -96,7 +96,8 @@ typedef struct sx_leaf {
  * sweep in warp tiles (table mode; the default), 6 = kernel 5 with 16-bit
  * keys (tiles of at most 8 rows; wider-spanning tiles take the row sweep),
  * 7 = row-lane sweep (a warp per tile of 8, 16 or 32 rows, its lanes dealt out
- * to the rows, 16-bit coordinates in shared memory; tiles above staging_cap
+ * to the rows, 4, 2 or 1 each when staging_cap is at most a quarter above the
+ * mean tile, 16-bit coordinates in shared memory; tiles above staging_cap
  * are swept in groups of rows, groups spanning more than 65534 columns with
  * 32-bit coordinates);
  * blocks_per_sm: residency cap of the global sweep; staging_cap: elements per

@@ -1587,8 +1587,6 @@ cudaError_t sx_gather_i32_launch(const int* idx, int count, const int* src, int*
     return cudaGetLastError();
 }
 
-// Gradient magnitude of a full width x height grid into a float32 array
-// (regrid.py:172-274); the same per-cell formula as the fused RLE.
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------

@@ -464,12 +464,6 @@ __global__ void __launch_bounds__(32 * SX_SMEM_WARPS) sx_sweep_smem_kernel(SxBoo
 }
 
 // ---------------------------------------------------------------------------
-// Host side
-// ---------------------------------------------------------------------------
-
-
-
-// ---------------------------------------------------------------------------
 // Merge-path form of the table sweep (a tuning option, sx_tuning kernel 3).
 //
 // A block of SXM_THREADS threads owns one tile of 32 aligned rows.  Every
@@ -2061,11 +2055,11 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // choice).
 //
 // A warp owns a tile of up to 32 aligned rows and its lanes are dealt out to the
-// rows: the same number each, or, once a row holds twice its share of the
-// intervals, one each and the others in proportion.  A row's lanes sweep it in
-// pieces, so a step needs no combined (row, x) keys and the output row offsets
-// come from a scan, and skewed rows even out inside the tile (with a fixed number
-// of lanes per row a warp waits for its longest row).
+// rows: the same number each, or, once a row holds twice its share of the intervals,
+// one each and the others in proportion (LPR > 0, for even rows: always the same).  A
+// row's lanes sweep it in pieces, so a step needs no combined (row, x) keys and the
+// output row offsets come from a scan, and skewed rows even out inside the tile (with
+// a fixed number of lanes per row a warp waits for its longest row).
 //
 // Staging.  One bulk copy per leaf array (begins, ends) into the warp's
 // slice of shared memory, above a gap; then interval j of leaf l becomes the
@@ -2101,8 +2095,8 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 // segmented sweeps.  So no pass over the input is needed before the launch to size
 // the slices for the largest tile and to look for wide tiles; such a pass took 59 us
 // of kernel and a read-back beside the 270 us sweep of the five-leaf shape expression
-// over 128 copies of 4096 rows (466 us in all; 364 us without it, with the sweep at
-// 275 to 288 us).  The sweep is bound by the latency of a tile's stages: 20 warps per
+// over 128 copies of 4096 rows (466 us in all; 358 us without it, with the sweep at
+// 275 us).  The sweep is bound by the latency of a tile's stages: 20 warps per
 // SM are all that the slices leave room for.
 //
 // Registers: 80 for five leaves, which costs no residency beside the slices (at 48
@@ -2113,9 +2107,9 @@ __global__ void __launch_bounds__(256, K <= 5 ? 5 : 4) sx_wseg16_kernel(SxBoolAr
 #define SXR_SPAN 65534
 #define SXR_SENTINEL 0xFFFFu
 // Intervals up to which a wide group is swept in place rather than given up.  Rows of
-// four intervals, two leaves (128 per tile): 84 us on 4096 rows and 139 on 100,000,
-// against 122 and 146 when the set was measured first; five leaves (320 per tile) 125 and
-// 311 against 125 and 166, so those give up.
+// four intervals, two leaves (128 per tile): 79 us on 4096 rows and 130 on 100,000,
+// against 121 and 146 when the set was measured first; five leaves (320 per tile) 125 and
+// 311 in place, 102 and 168 given up, 119 and 166 measured first.
 #define SXR_LIGHT 200
 // Intervals of one leaf that a row counts for, far above every slice: the sums over 8
 // leaves and 32 rows stay inside int32.
@@ -2231,7 +2225,7 @@ __device__ __forceinline__ int sxr_raw_lower(const int* B, const int* E, int cnt
     return lo;
 }
 
-// A row of m boundaries in its longest leaf and L lanes: piece i takes the keys
+// Pieces.  A row of m boundaries in its longest leaf and L lanes: piece i takes the keys
 // [p_i, p_{i+1}), the pivots p_i being halfwords of that leaf at positions
 // i m / L.  A piece starts in every other leaf at the first key not below p_i (a
 // binary search within the row) with the parity of that position as the leaf's
@@ -2240,8 +2234,8 @@ __device__ __forceinline__ int sxr_raw_lower(const int* B, const int* E, int cnt
 // pieces must meet: each piece's end positions are checked against the next
 // piece's start positions (with the per-piece rising keys, that checks the
 // contract across pieces).
-// What a group of rows leaves for its writing: this lane's piece, its changes of f
-// (khw, excl before it in the group), and where the staged ones lie.
+
+// A piece of a group that is swept over the raw arrays.
 template <int K>
 struct SxrRaw {
     int rp0[K], rpe[K];
@@ -2249,6 +2243,8 @@ struct SxrRaw {
     const int *RB[K], *RE[K];
 };
 
+// What a group of rows leaves for its writing: this lane's piece, its changes of f
+// (khw, excl before it in the group), and where the staged ones lie.
 template <int K>
 struct SxrGroup {
     int row, khw, excl, total, src, xmin;  // src: halfword of the piece's staged changes
@@ -2256,55 +2252,13 @@ struct SxrGroup {
     SxrRaw<K>* raw;
 };
 
-// One group: rows q0 .. q0 + gn - 1, at most `room` intervals (more, in a single
-// row, are not staged).  Without RAW the group is a whole tile: one that cannot be
-// staged is only reported (G.staged false), and with A.give_up its largest 8 rows
-// are noted in stats if they exceed `seen`, an earlier value of it.  With RAW it is swept over the raw arrays, unless A.give_up
-// wants to know of it (insist: it is written now).
-template <int K, bool RAW>
-__device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, int TR, int room, unsigned* W, unsigned* raw,
-                                          unsigned long long* bar, unsigned& use, unsigned& flags,
-                                          SxrGroup<K>& G, unsigned* stats, unsigned seen, bool insist)
+// A group's lanes dealt out to its gn rows; lane r knows row r's intervals (mine, `all`
+// in the group).  The same number each while no row holds twice its share (a row with
+// half the lanes of its neighbours would hold the warp up for longer than that row),
+// else one each and the others along the running sum of the rows' intervals.
+__device__ __forceinline__ void sxr_deal(int mine, int all, int gn, int& row, int& first_lane, int& L)
 {
     const int lane = threadIdx.x & 31;
-    unsigned short* const h16 = (unsigned short*)W;
-    // lane r: row r of the group in every leaf, relative to the group's first interval
-    int lo[K], hi[K], n[K], g0[K];
-    int PBl = 0, mine = 0, all = 0;
-    bool ok = true;  // row offsets must rise
-#pragma unroll
-    for (int l = 0; l < K; ++l) {
-        lo[l] = A.leaf[l].off[q0 + min(lane, gn)];
-        hi[l] = A.leaf[l].off[q0 + min(lane + 1, gn)];
-        ok = ok && lo[l] >= 0 && lo[l] <= hi[l];
-    }
-    ok = __all_sync(0xFFFFFFFFu, ok);
-    if (!ok) flags |= SXF_CONTRACT;
-#pragma unroll
-    for (int l = 0; l < K; ++l) {
-        g0[l] = __shfl_sync(0xFFFFFFFFu, lo[l], 0);
-        n[l] = ok ? __shfl_sync(0xFFFFFFFFu, hi[l], gn - 1) - g0[l] : 0;
-        lo[l] = ok ? lo[l] - g0[l] : 0;
-        hi[l] = ok ? hi[l] - g0[l] : 0;
-        mine += min(hi[l] - lo[l], SXR_ROW_MAX);
-        all += min(n[l], 32 * SXR_ROW_MAX);
-        PBl += n[l] + TR + 1;
-    }
-    G.ok = ok;
-    G.light = all <= SXR_LIGHT;
-    G.staged = G.wide = false;
-    if (!RAW && A.give_up && ok) {
-        const int low = __reduce_add_sync(0xFFFFFFFFu, lane < 8 ? mine : 0);
-        const unsigned most = (unsigned)max(low, all - low);
-        if (lane == 0 && most > seen) atomicMax(stats, most);
-    }
-    if (!RAW && ok && all > room) return;
-    const bool fits = ok && all <= room;
-    const int OA = PBl;  // output areas start after the pair lists
-    // The group's lanes dealt out to its rows, every row's leader lane in `leaders`:
-    // the same number each while no row holds twice its share (a row with half the
-    // lanes of its neighbours would hold the warp up for longer than that row),
-    // else one each and the others along the running sum of the rows' intervals.
     int upper = min(lane + 1, gn) * (32 / gn);  // first lane of the next row
     if (lane + 1 >= gn) upper = 32;
     if ((long long)gn * __reduce_max_sync(0xFFFFFFFFu, mine) > 2ll * all) {
@@ -2318,15 +2272,71 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
     }
     int from = __shfl_up_sync(0xFFFFFFFFu, upper, 1);
     if (lane == 0) from = 0;
-    const int lanes = upper - from;
-    const unsigned leaders = __reduce_or_sync(0xFFFFFFFFu, lane < gn ? 1u << from : 0u);
+    const unsigned leaders = __reduce_or_sync(0xFFFFFFFFu, lane < gn ? 1u << from : 0u);  // every row's first lane
     const unsigned upto = leaders & (0xFFFFFFFFu >> (31 - lane));
-    const int row = __popc(upto) - 1, first_lane = 31 - __clz(upto), piece = lane - first_lane;
-    const int L = __shfl_sync(0xFFFFFFFFu, lanes, row);
+    row = __popc(upto) - 1;
+    first_lane = 31 - __clz(upto);
+    L = __shfl_sync(0xFFFFFFFFu, upper - from, row);
+}
+
+// One group: rows q0 .. q0 + gn - 1, at most `room` intervals (more, in a single
+// row, are not staged).  Without RAW the group is a whole tile: one that cannot be
+// staged is only reported (G.staged false), and with A.give_up its largest 8 rows
+// are noted in stats if they exceed `seen`, an earlier value of it.  With RAW it is swept over the raw arrays, unless A.give_up
+// wants to know of it (insist: it is written now).  LPR > 0: every row has that many
+// lanes (a whole tile of 32 / LPR rows, the last one with fewer of them).
+template <int K, bool RAW, int LPR>
+__device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, int TR, int room, unsigned* W, unsigned* raw,
+                                          unsigned long long* bar, unsigned& use, unsigned& flags,
+                                          SxrGroup<K>& G, unsigned* stats, unsigned seen, bool insist)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned short* const h16 = (unsigned short*)W;
+    // lane r: row r of the group (LPR > 0: this lane's row) in every leaf, relative to the
+    // group's first interval
+    int lo[K], hi[K], n[K], g0[K];
+    int PBl = 0, mine = 0, all = 0;
+    bool ok = true;  // row offsets must rise
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        const int r = LPR > 0 ? lane / (LPR > 0 ? LPR : 1) : lane;
+        lo[l] = A.leaf[l].off[q0 + min(r, gn)];
+        hi[l] = A.leaf[l].off[q0 + min(r + 1, gn)];
+        ok = ok && lo[l] >= 0 && lo[l] <= hi[l];
+    }
+    if constexpr (LPR == 0) ok = __all_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+    for (int l = 0; l < K; ++l) {
+        g0[l] = __shfl_sync(0xFFFFFFFFu, lo[l], 0);
+        n[l] = __shfl_sync(0xFFFFFFFFu, hi[l], LPR > 0 ? (gn - 1) * LPR : gn - 1) - g0[l];
+        lo[l] -= g0[l];
+        hi[l] -= g0[l];
+        if (LPR == 0 && !ok) n[l] = lo[l] = hi[l] = 0;
+        mine += min(hi[l] - lo[l], SXR_ROW_MAX);
+        all += min(n[l], 32 * SXR_ROW_MAX);
+        PBl += n[l] + TR + 1;
+    }
+    if constexpr (LPR > 0) ok = __all_sync(0xFFFFFFFFu, ok);  // nothing before this waits for the vote
+    if (!ok) flags |= SXF_CONTRACT;
+    G.ok = ok;
+    G.light = all <= SXR_LIGHT;
+    G.staged = G.wide = false;
+    if (!RAW && LPR == 0 && A.give_up && ok) {
+        const int low = __reduce_add_sync(0xFFFFFFFFu, lane < 8 ? mine : 0);
+        const unsigned most = (unsigned)max(low, all - low);
+        if (lane == 0 && most > seen) atomicMax(stats, most);
+    }
+    if (!RAW && LPR == 0 && ok && all > room) return;
+    const bool fits = ok && all <= room;
+    const int OA = PBl;  // output areas start after the pair lists
+    int row = lane / (LPR > 0 ? LPR : 1), first_lane = row * LPR, L = row < gn ? LPR : 0;
+    if constexpr (LPR == 0) sxr_deal(mine, all, gn, row, first_lane, L);
+    const int piece = lane - first_lane;
     const bool act = ok && piece < L;
 #pragma unroll
     for (int l = 0; l < K; ++l) {
-        const int a = __shfl_sync(0xFFFFFFFFu, lo[l], row), b = __shfl_sync(0xFFFFFFFFu, hi[l], row);
+        const int a = LPR > 0 ? lo[l] : __shfl_sync(0xFFFFFFFFu, lo[l], row);
+        const int b = LPR > 0 ? hi[l] : __shfl_sync(0xFFFFFFFFu, hi[l], row);
         lo[l] = act ? a : n[l];
         hi[l] = act ? b : n[l];
     }
@@ -2478,10 +2488,12 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
         unsigned klo = 0u, khi = SXR_SENTINEL;
         // piece * m / L in floats: neighbours round the same product alike
         const float part = (float)m / (float)L;
-        const int split = (int)((float)piece * part), next = (int)((float)(piece + 1) * part);
-        if (L > 1) {
+        const int split = LPR > 0 ? piece * m / (LPR > 0 ? LPR : 1) : (int)((float)piece * part);
+        const int next = LPR > 0 ? (piece + 1) * m / (LPR > 0 ? LPR : 1) : (int)((float)(piece + 1) * part);
+        const bool cut = LPR > 0 ? LPR > 1 : L > 1;
+        if (cut) {
             klo = piece == 0 ? 0u : (m > 0 ? (unsigned)Lb[split] : SXR_SENTINEL);
-            khi = piece == L - 1 ? SXR_SENTINEL : (m > 0 ? (unsigned)Lb[next] : SXR_SENTINEL);
+            khi = piece == (LPR > 0 ? LPR : L) - 1 ? SXR_SENTINEL : (m > 0 ? (unsigned)Lb[next] : SXR_SENTINEL);
         }
         unsigned state = 0u;
 #pragma unroll
@@ -2489,7 +2501,7 @@ __device__ __forceinline__ void sxr_group(const SxBoolArgs& A, int q0, int gn, i
             const unsigned short* Ll = h16 + 2 * (pb[l] + lo[l] + qr[l]);
             const int cnt = 2 * (hi[l] - lo[l]);
             int pos = 0;
-            if (piece > 0) pos = l == big ? split : sxs_lower_bound16(Ll, cnt, klo);
+            if (cut && piece > 0) pos = l == big ? split : sxs_lower_bound16(Ll, cnt, klo);
             if (cnt == 0) pos = 0;
             sa[l] = pa[l] = sxs_saddr(Ll + pos);
             h[l] = pos < cnt ? (unsigned)Ll[pos] : SXR_SENTINEL;
@@ -2671,7 +2683,7 @@ __device__ __noinline__ void sxr_slow_tile(const SxBoolArgs& A, const SxSweepSta
             const unsigned in = __ballot_sync(0xFFFFFFFFu, lane >= gr && lane < nrows && sum - before <= room);
             const int gn = max(1, __popc(in));  // a row that does not fit alone is swept from global memory
             __syncwarp();
-            sxr_group<K, true>(A, r0 + gr, gn, TR, room, W, raw, bar, use, flags, G, nullptr, 0u, phase == 1);
+            sxr_group<K, true, 0>(A, r0 + gr, gn, TR, room, W, raw, bar, use, flags, G, nullptr, 0u, phase == 1);
             if (A.give_up && phase == 0 && !G.staged && !G.light) {
                 sxr_give_up<K>(A, st, tile, tiles, TR, G.wide);
                 return;
@@ -2685,11 +2697,12 @@ __device__ __noinline__ void sxr_slow_tile(const SxBoolArgs& A, const SxSweepSta
     sxs_report(A, tile, tiles, base, done, flags);
 }
 
-template <int K>
+template <int K, int LPR>
 __global__ void __launch_bounds__(256, K <= 4 ? 4 : 3)
     sx_rlane16_kernel(const __grid_constant__ SxBoolArgs A, const __grid_constant__ SxSweepState st, int tiles,
-                      int cap_words, int TR)
+                      int cap_words, int tile_rows)
 {
+    const int TR = LPR > 0 ? 32 / (LPR > 0 ? LPR : 1) : tile_rows;
     extern __shared__ __align__(16) unsigned char sxr_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, NW = blockDim.x >> 5;
     if (blockIdx.x * NW + wid >= tiles) return;  // exactly `tiles` warps take tickets
@@ -2702,7 +2715,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : 3)
     unsigned flags = 0u, use = 0u, seen = 0u, given_up = 0u;  // given_up: by another tile
     if (lane == 0) {
         tile = (int)atomicAdd(&st.counters[0], 1u);
-        if (A.give_up) {
+        if (LPR == 0) {
             const volatile unsigned* const now = st.counters + SXR_STATS;
             seen = now[0];
             given_up = now[2];
@@ -2710,7 +2723,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : 3)
         sxs_bar_init(bar);
     }
     tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
-    given_up = __shfl_sync(0xFFFFFFFFu, given_up, 0);
+    if (LPR == 0) given_up = __shfl_sync(0xFFFFFFFFu, given_up, 0);
     const int r0 = tile * TR;
     const int nrows = min(TR, A.rows - r0);
     if (tile == 0 && lane == 0) A.out_off[0] = 0;
@@ -2718,19 +2731,20 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : 3)
     SxrGroup<K> G;
     G.staged = G.wide = G.light = false;
     G.ok = true;
-    if (!given_up)
-        sxr_group<K, false>(A, r0, nrows, TR, room, W, raw, bar, use, flags, G, st.counters + SXR_STATS, seen, false);
-    if (A.give_up && (given_up || (G.wide && !G.light))) {
+    if (LPR > 0 || !given_up)
+        sxr_group<K, false, LPR>(A, r0, nrows, TR, room, W, raw, bar, use, flags, G, st.counters + SXR_STATS, seen, false);
+    if (LPR == 0 && A.give_up && (given_up || (G.wide && !G.light))) {
         sxr_give_up<K>(A, st, tile, tiles, TR, G.wide);
         return;
     }
-    if (!G.staged && G.ok) {
-        sxr_slow_tile<K>(A, st, tile, tiles, r0, nrows, TR, room, W, raw, bar, use, flags);
+    if (G.staged || !G.ok) {
+        const int base = sxs_lookback(A, st, tile, G.total, flags);
+        sxr_put<K, false>(A, G, W, r0, base);
+        sxs_report(A, tile, tiles, base, G.total, flags);
         return;
     }
-    const int base = sxs_lookback(A, st, tile, G.total, flags);
-    sxr_put<K, false>(A, G, W, r0, base);
-    sxs_report(A, tile, tiles, base, G.total, flags);
+    // the call last: in front of the look-back it cost the common path 3 us of 262
+    sxr_slow_tile<K>(A, st, tile, tiles, r0, nrows, TR, room, W, raw, bar, use, flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -3110,16 +3124,32 @@ static cudaError_t sx_wseg16_launch_k(const SxBoolArgs& A, const SxSweepState& s
     return cudaGetLastError();
 }
 
+template <int K, int LPR>
+static cudaError_t sx_rlane16_launch_kl(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
+                                        int warps, int tr, cudaStream_t stream)
+{
+    static SxSmemLimit limit;
+    const int bytes = warps * (int)sxr_slice_bytes(cap_words);
+    if (cudaError_t err = limit.raise((const void*)sx_rlane16_kernel<K, LPR>, bytes); err != cudaSuccess) return err;
+    const int blocks = (tiles + warps - 1) / warps;
+    sx_rlane16_kernel<K, LPR><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words, tr);
+    return cudaGetLastError();
+}
+
+// Lanes per row fixed at compile time (even) or dealt out tile by tile.  Fixed, the shapes
+// expression over 128 copies of 4096 rows takes 262 us, dealt out 268; two sweeps' worth
+// of 256 uneven sets 130 us a sweep, dealt out 75.  sx_bool_eval_even does not know
+// its rows and deals; a tuning that gives the largest tile (staging_cap) shows them to be
+// even when that tile holds at most a quarter more than the mean one (shapes: 1.08, the
+// uneven sets: 3.9).
 template <int K>
 static cudaError_t sx_rlane16_launch_k(const SxBoolArgs& A, const SxSweepState& st, int tiles, int cap_words,
-                                       int warps, int tr, cudaStream_t stream)
+                                       int warps, int tr, bool even, cudaStream_t stream)
 {
-    const int bytes = warps * (int)sxr_slice_bytes(cap_words);
-    static SxSmemLimit limit;
-    if (cudaError_t err = limit.raise((const void*)sx_rlane16_kernel<K>, bytes); err != cudaSuccess) return err;
-    const int blocks = (tiles + warps - 1) / warps;
-    sx_rlane16_kernel<K><<<blocks, 32 * warps, bytes, stream>>>(A, st, tiles, cap_words, tr);
-    return cudaGetLastError();
+    if (!even) return sx_rlane16_launch_kl<K, 0>(A, st, tiles, cap_words, warps, tr, stream);
+    if (tr == 8) return sx_rlane16_launch_kl<K, 4>(A, st, tiles, cap_words, warps, tr, stream);
+    if (tr == 16) return sx_rlane16_launch_kl<K, 2>(A, st, tiles, cap_words, warps, tr, stream);
+    return sx_rlane16_launch_kl<K, 1>(A, st, tiles, cap_words, warps, tr, stream);
 }
 
 // Union sweep shape: log2 of the lanes per row.  More lanes while whole rows
@@ -3256,15 +3286,16 @@ cudaError_t sx_sweep_launch(const SxBoolArgs& A, bool union_mode, void* workspac
         const long long limit = (200 * 1024) / warps / 4 - SXR_HDR_WORDS;
         if (words > limit) words = limit;
         const int cw = (int)words;
+        const bool even = !A.give_up && A.tune_staging_cap > 0 && 4ll * A.tune_staging_cap <= 5 * avg;
         switch (A.k) {
-            case 1: return sx_rlane16_launch_k<1>(A, st, t, cw, warps, tr, stream);
-            case 2: return sx_rlane16_launch_k<2>(A, st, t, cw, warps, tr, stream);
-            case 3: return sx_rlane16_launch_k<3>(A, st, t, cw, warps, tr, stream);
-            case 4: return sx_rlane16_launch_k<4>(A, st, t, cw, warps, tr, stream);
-            case 5: return sx_rlane16_launch_k<5>(A, st, t, cw, warps, tr, stream);
-            case 6: return sx_rlane16_launch_k<6>(A, st, t, cw, warps, tr, stream);
-            case 7: return sx_rlane16_launch_k<7>(A, st, t, cw, warps, tr, stream);
-            case 8: return sx_rlane16_launch_k<8>(A, st, t, cw, warps, tr, stream);
+            case 1: return sx_rlane16_launch_k<1>(A, st, t, cw, warps, tr, even, stream);
+            case 2: return sx_rlane16_launch_k<2>(A, st, t, cw, warps, tr, even, stream);
+            case 3: return sx_rlane16_launch_k<3>(A, st, t, cw, warps, tr, even, stream);
+            case 4: return sx_rlane16_launch_k<4>(A, st, t, cw, warps, tr, even, stream);
+            case 5: return sx_rlane16_launch_k<5>(A, st, t, cw, warps, tr, even, stream);
+            case 6: return sx_rlane16_launch_k<6>(A, st, t, cw, warps, tr, even, stream);
+            case 7: return sx_rlane16_launch_k<7>(A, st, t, cw, warps, tr, even, stream);
+            case 8: return sx_rlane16_launch_k<8>(A, st, t, cw, warps, tr, even, stream);
             default: return cudaErrorInvalidValue;
         }
     }
