@@ -124,20 +124,46 @@ __global__ void sx_prolong_set_intervals_kernel(const int* __restrict__ b, const
 // ---------------------------------------------------------------------------
 // Field transfers between levels: blocks of coarse rows.
 //
-// A block takes one coarse row (several share a long row when rows are few) and
-// its threads take the row's cells one after another, whatever intervals they
-// lie in; the row's interval starts are staged in shared memory, FIELD_BATCH at a
-// time, and a thread finds its interval there.  Bound by bytes.  One warp per
-// interval, after a search for its row, left too little work per warp to keep
-// loads in flight: on a 4096^2 geometry (8 M coarse cells, float32) prolongation
-// took 133 us and restriction 116 us; 55 and 57 us here (69 and 100 us with one search
-// per cell instead of one per 128 cells of a warp), 26 us at the copy
-// rate.  For ratio 2 the two fine values of a sub-row move as one pair where they
-// start at an even value of an aligned array (always, when values are packed).
+// A block takes a coarse row, or a group of consecutive short ones where rows are many
+// (sx_field_grid), or a share of the cells of a long one where they are few, and its
+// threads take the cells one after another, whatever intervals they lie in: the interval
+// starts are staged in shared memory with their fine intervals' starts and ends,
+// SX_FIELD_BATCH at a time, and a warp finds its cells' intervals there, with one search
+// per 128 cells and a walk.  A share of more intervals than a batch finds its first and
+// last one by a warp's search (32 probes a round).  Bound by bytes.  One warp per interval,
+// after a search for its row, left too little work per warp to keep loads in flight; one
+// block per row whatever its length left most of a block idle on short rows and read long
+// ones whole in every block.  Kernels, measured (B200, float32, ratio 2, prolongation and
+// restriction; rows x intervals per row x cells per interval):
+//                                  warp per interval    block per row     here
+//   shapes on 4096^2 (10 M cells)   124 us  115 us      56 us   55 us     51 us   53 us
+//   1,000,000 x 1 x 4               541     568         2611    3890      56      62
+//   100,000 x 2 x 8                 76      78          187     273       29      33
+//   1 x 200,000 x 5                 29      31          1903    1627      15      15
+//   16 x 3 x 100,000                3054    2553        31      27        27      27
+// For ratio 2 the two fine values of a sub-row move as one pair where they start at an
+// even value of an aligned array (always, when values are packed).
 // ---------------------------------------------------------------------------
 #define SX_FIELD_THREADS 256
 #define SX_FIELD_BATCH 512
 #define SX_FIELD_ITEMS 4
+#define SX_FIELD_ROW_BLOCKS 8  // sub-rows shared out to that many blocks at any ratio
+// Resident blocks per SM asked of the compiler, by type and ratio (float32 on 10 M cells in
+// 19,490 intervals, 5, 6 and 8: prolongation by 2 59.5, 55.4, 51.3 us, by 3 (2.5 M cells)
+// 28.8, 38, 41; restriction by 2 59.4, 53.5, 67.4, by 3 40, 41, 36 with 7).
+template <typename T, int RT>
+constexpr int sx_prolong_blocks = sizeof(T) == 8 || RT == 0 ? 6 : RT == 2 ? 8 : 5;
+template <typename T, int RT>
+constexpr int sx_restrict_blocks = sizeof(T) == 8 ? (RT == 2 || RT == 0 ? 4 : 6) : RT == 2 ? 6 : 7;
+
+// x: groups of rows, about 40 a SM at most, so that uneven ones even out; y: shares of a
+// group's cells where the groups alone would not fill the chip.
+static dim3 sx_field_grid(int rows)
+{
+    const int fill = 148 * 8, most = 5 * fill;
+    const int per = (rows - 1) / most + 1, groups = (rows - 1) / per + 1;
+    return dim3(groups, groups >= fill ? 1 : (fill - 1) / groups + 1);
+}
 
 template <typename T>
 struct SxPair;
@@ -150,63 +176,139 @@ struct SxPair<double> {
     typedef double2 type;
 };
 
-// Blocks per row, so that few rows still fill the chip.
-static int sx_field_split(int rows)
+// Last i < n with a[i] <= v, for rising a with a[0] <= v; a whole warp probes 32 places at once.
+__device__ __forceinline__ int sx_warp_last(const int* __restrict__ a, int n, long long v)
 {
-    int s = 1;
-    while (s < 64 && (long long)rows * s < 148 * 8) s <<= 1;
-    return s;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = n;
+    while (len > 1) {
+        const int step = (len - 1) / 32 + 1;
+        const long long ahead = (long long)lane * step;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, ahead < len && a[lo + ahead] <= v);
+        const int k = m ? 31 - __clz(m) : 0;
+        lo += k * step;
+        len = min(step, len - k * step);
+    }
+    return lo;
 }
 
-// What a thread knows of SX_FIELD_ITEMS cells of a coarse row, 32 apart (a warp
-// takes 128 consecutive cells): the cell, its interval within the batch and its
-// place in the interval (-1: past the row).
+// What a thread knows of SX_FIELD_ITEMS coarse cells, 32 apart (a warp takes 128
+// consecutive cells): the cell, its interval within the batch and its place in the
+// interval (-1: past the stretch).
 struct SxFieldItems {
-    long long c[SX_FIELD_ITEMS];
+    unsigned c[SX_FIELD_ITEMS];
     int o[SX_FIELD_ITEMS], k[SX_FIELD_ITEMS];
 };
 
-// Calls f(items, first, s_c, s_f) for this block's share of the cells of row p.
-// s_c holds the batch's interval starts, first its first interval within the row
-// and s_f, for a fixed ratio, the starts of the fine intervals in the sub-rows
-// (stride SX_FIELD_BATCH + 1).  One search per 128 cells, then a walk.
-template <int RT, typename F>
-__device__ __forceinline__ void sx_field_cells(const int* __restrict__ off, const int* __restrict__ coff,
-                                               const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int p,
-                                               F f)
+// A batch of intervals: starts (one more than intervals) and their fine intervals' starts
+// and ends by sub-row; RT = 0: those of one sub-row, and the intervals' rows and places.
+template <int RT>
+struct SxFieldBatch {
+    int c[SX_FIELD_BATCH + 1];
+    int2 f[RT > 0 ? RT : 1][SX_FIELD_BATCH];
+    int2 at[RT > 0 ? 1 : SX_FIELD_BATCH];
+};
+
+// The fine interval of sub-row d under the interval `at` of the coarse set.
+__device__ __forceinline__ int2 sx_fine_interval(int2 at, int d, const int* __restrict__ foff_rows,
+                                                 const int* __restrict__ fcoff, int r)
 {
-    __shared__ int s_c[SX_FIELD_BATCH + 1];
-    __shared__ int s_f[RT > 0 ? RT * (SX_FIELD_BATCH + 1) : 1];
-    const int i0 = off[p], i1 = off[p + 1];
-    for (int ib = i0; ib < i1; ib += SX_FIELD_BATCH) {
-        const int nb = min(SX_FIELD_BATCH, i1 - ib), first = ib - i0;
-        __syncthreads();
-        for (int j = threadIdx.x; j <= nb; j += SX_FIELD_THREADS) s_c[j] = coff[ib + j];
-#pragma unroll
-        for (int d = 0; d < RT; ++d) {
-            const int f0 = foff_rows[RT * p + d] + first;
-            for (int j = threadIdx.x; j <= nb; j += SX_FIELD_THREADS) s_f[d * (SX_FIELD_BATCH + 1) + j] = fcoff[f0 + j];
+    const int f = foff_rows[at.x * r + d] + at.y;
+    return make_int2(fcoff[f], fcoff[f + 1]);
+}
+
+// Calls f(w0, hi, nb, B, d) for this block's share of the cells, by warps of 128 cells from
+// w0 on (below hi), lying in the nb intervals of batch B.  BY_ROW: sub-row by sub-row, every
+// gridDim.z-th, with the fine intervals of sub-row d in B.f[0]; ends(begin, end, fine) is
+// then called for each interval that ends in the share.
+template <int RT, bool BY_ROW, typename F, typename E>
+__device__ __forceinline__ void sx_field_cells(const int* __restrict__ off, int rows, const int* __restrict__ coff,
+                                               const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int r,
+                                               F f, E ends)
+{
+    __shared__ SxFieldBatch<RT> B;
+    __shared__ int s_i[2];
+    constexpr int ROUND = SX_FIELD_THREADS * SX_FIELD_ITEMS;
+    const int per = (int)(((long long)rows + gridDim.x - 1) / gridDim.x);
+    const long long group = (long long)blockIdx.x * per;
+    if (group >= rows) return;
+    const int p0 = (int)group, p1 = (int)min((long long)rows, group + per) - 1;
+    int i0 = off[p0], i1 = off[p1 + 1] - 1;
+    if (i0 > i1) return;
+    long long c0 = coff[i0], c1 = coff[i1 + 1];
+    const int wid = threadIdx.x >> 5;
+    if (gridDim.y > 1) {
+        const long long share = ((c1 - c0 + gridDim.y - 1) / gridDim.y + ROUND - 1) / ROUND * ROUND;
+        const long long from = c0 + blockIdx.y * share, to = min(c1, from + share);
+        if (from >= to) return;
+        if (i1 - i0 >= SX_FIELD_BATCH) {  // more than a batch: only the share's intervals
+            if (wid < 2) {
+                const int i = i0 + sx_warp_last(coff + i0, i1 - i0 + 1, wid == 0 ? from : to - 1);
+                if ((threadIdx.x & 31) == 0) s_i[wid] = i;
+            }
+            __syncthreads();
+            i0 = s_i[0];
+            i1 = s_i[1];
         }
+        c0 = from;
+        c1 = to;
+    }
+    for (int ib = i0; ib <= i1; ib += SX_FIELD_BATCH) {
+        const int nb = min(SX_FIELD_BATCH, i1 - ib + 1);
         __syncthreads();
-        const long long end = s_c[nb], step = (long long)gridDim.y * SX_FIELD_THREADS * SX_FIELD_ITEMS;
-        for (long long w0 = s_c[0] + ((long long)blockIdx.y * SX_FIELD_THREADS + (threadIdx.x & ~31)) * SX_FIELD_ITEMS;
-             w0 < end; w0 += step) {
-            int lo = 0, hi = nb - 1;  // last interval starting at or before the warp's first cell
+        for (int j = threadIdx.x; j <= nb; j += SX_FIELD_THREADS) B.c[j] = coff[ib + j];
+        for (int j = threadIdx.x; j < nb; j += SX_FIELD_THREADS) {
+            int lo = p0, hi = p1;  // the interval's row
             while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (s_c[mid] <= w0) lo = mid; else hi = mid - 1;
+                const int mid = lo + ((hi - lo + 1) >> 1);
+                if (off[mid] <= ib + j) lo = mid; else hi = mid - 1;
             }
-            SxFieldItems it;
+            const int2 at = make_int2(lo, ib + j - off[lo]);
+            if (RT == 0) B.at[RT > 0 ? 0 : j] = at;
 #pragma unroll
-            for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
-                it.c[q] = w0 + 32 * q + (threadIdx.x & 31);
-                while (lo + 1 < nb && s_c[lo + 1] <= it.c[q]) ++lo;
-                it.o[q] = lo;
-                it.k[q] = it.c[q] < end ? (int)(it.c[q] - s_c[lo]) : -1;
+            for (int d = 0; d < RT; ++d) B.f[d][j] = sx_fine_interval(at, d, foff_rows, fcoff, RT);
+        }
+        for (int d = BY_ROW ? blockIdx.z : 0; d < (BY_ROW ? r : 1); d += gridDim.z) {
+            __syncthreads();
+            if (BY_ROW) {
+                for (int j = threadIdx.x; j < nb; j += SX_FIELD_THREADS) {
+                    const int2 fine = sx_fine_interval(B.at[RT > 0 ? 0 : j], d, foff_rows, fcoff, r);
+                    B.f[0][j] = fine;
+                    if (B.c[j + 1] > c0 && B.c[j + 1] <= c1) ends(B.c[j], B.c[j + 1], fine);
+                }
+                __syncthreads();
             }
-            f(it, first, s_c, s_f);
+            const long long lo = max(c0, (long long)B.c[0]), hi = min(c1, (long long)B.c[nb]);
+            for (long long w0 = lo + wid * 32 * SX_FIELD_ITEMS; w0 < hi; w0 += ROUND) f(w0, hi, nb, B, d);
         }
     }
+}
+
+// Last interval of the batch that starts at or before c.
+template <int RT>
+__device__ __forceinline__ int sx_batch_last(const SxFieldBatch<RT>& B, int nb, long long c)
+{
+    int lo = 0, hi = nb - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (B.c[mid] <= c) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+template <int RT>
+__device__ __forceinline__ SxFieldItems sx_field_items(const SxFieldBatch<RT>& B, int nb, long long w0, long long hi)
+{
+    SxFieldItems it;
+    int lo = sx_batch_last(B, nb, w0);
+#pragma unroll
+    for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+        it.c[q] = (unsigned)w0 + 32 * q + (threadIdx.x & 31);
+        while (lo + 1 < nb && (unsigned)B.c[lo + 1] <= it.c[q]) ++lo;
+        it.o[q] = lo;
+        it.k[q] = it.c[q] < (unsigned)hi ? (int)it.c[q] - B.c[lo] : -1;
+    }
+    return it;
 }
 
 // Field prolongation (kernels.py:384-455): piecewise-constant injection onto
@@ -214,53 +316,87 @@ __device__ __forceinline__ void sx_field_cells(const int* __restrict__ off, cons
 // as the reference's alignment check does).  Coarse interval i (ordinal o
 // in row ordinal p) maps in sub-row d to the fine interval
 // f = fine_off[p*r + d] + o, and fine cell k of f takes coarse cell k / r.
-// RT > 0 fixes the ratio at compile time.
+// RT > 0 fixes the ratio at compile time; with RT = 0 a warp's lanes take consecutive
+// fine cells of a sub-row, so that its stores stay together at any ratio (by 5, 4096 rows
+// of 30 intervals of 60 cells: 283 us, 470 with a coarse cell per lane).
 template <typename T, int RT>
-__global__ void __launch_bounds__(SX_FIELD_THREADS)
-    sx_prolong_field_kernel(const int* __restrict__ off, const int* __restrict__ coff, int n,
+__global__ void __launch_bounds__(SX_FIELD_THREADS, sx_prolong_blocks<T, RT>)
+    sx_prolong_field_kernel(const int* __restrict__ off, int rows, const int* __restrict__ coff, int n,
                             const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int rr,
                             const T* __restrict__ cv, T* __restrict__ fv, int pair)
 {
     typedef typename SxPair<T>::type P2;
     const int r = RT > 0 ? RT : rr;
-    const int p = blockIdx.x;
     const long long ncells = coff[n];
-    sx_field_cells<RT>(off, coff, foff_rows, fcoff, p, [&](const SxFieldItems& it, int first, const int* s_c,
-                                                           const int* s_f) {
-        T v[SX_FIELD_ITEMS];
+    __shared__ T s_cell[RT > 0 ? 1 : SX_FIELD_THREADS / 32][RT > 0 ? 1 : 32 * SX_FIELD_ITEMS];  // RT = 0: a warp's cells
+    // Rows whose begins decrease are re-sorted on the fine level, so fine
+    // interval f may be wider than coarse interval i; the reference then reads
+    // past i, and past the array at its end.  Here reads stay inside the array
+    // (0 beyond it).
+    auto beyond = [&](int begin, int end, int2 fine) {
+        for (long long t = (long long)(end - begin) * r; end > begin && t < fine.y - fine.x; ++t) {
+            const long long src = begin + t / r;
+            fv[fine.x + t] = src < ncells ? cv[src] : (T)0;
+        }
+    };
+    sx_field_cells<RT, RT == 0>(off, rows, coff, foff_rows, fcoff, r, [&](long long w0, long long hi, int nb,
+                                                                             const SxFieldBatch<RT>& B, int sub) {
+        if constexpr (RT == 0) {
+            const int lane = threadIdx.x & 31, cells = (int)min((long long)32 * SX_FIELD_ITEMS, hi - w0);
+            const int first = sx_batch_last(B, nb, w0), c32 = 32 / r, dx32 = 32 - c32 * r;
+            T* const cell = s_cell[threadIdx.x >> 5];
+            __syncwarp();  // the values of the warp's stretch before are read
 #pragma unroll
-        for (int q = 0; q < SX_FIELD_ITEMS; ++q) v[q] = it.k[q] >= 0 ? cv[it.c[q]] : (T)0;
-#pragma unroll(RT > 0 ? RT : 1)
-        for (int d = 0; d < r; ++d) {
-            const int* fst = RT > 0 ? s_f + d * (SX_FIELD_BATCH + 1) : fcoff + foff_rows[p * r + d] + first;
-#pragma unroll
-            for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
-                if (it.k[q] < 0) continue;
-                const long long fs = fst[it.o[q]], fw = fst[it.o[q] + 1] - fs, t0 = (long long)it.k[q] * r;
-                if (RT == 2 && pair && !(fs & 1) && t0 + 2 <= fw) {
-                    P2 w;
-                    w.x = v[q];
-                    w.y = v[q];
-                    *(P2*)(fv + fs + t0) = w;
-                } else {
-#pragma unroll(RT > 0 ? RT : 1)
-                    for (int t = 0; t < r; ++t)
-                        if (t0 + t < fw) fv[fs + t0 + t] = v[q];
+            for (int q = 0; q < SX_FIELD_ITEMS; ++q)
+                if (lane + 32 * q < cells) cell[lane + 32 * q] = cv[w0 + lane + 32 * q];
+            __syncwarp();
+            // column dx under cell w0 + c, in interval o, which ends before cell w0 + next; value
+            // at, of an interval whose values end before stop (unsigned: both stay below 2^32)
+            int o = first - 1, c = lane / r, dx = lane - c * r, next = 0;
+            unsigned at = 0u, stop = 0u;
+            while (c < cells) {
+                if (c >= next) {
+                    do ++o; while (o + 1 < nb && B.c[o + 1] <= (int)w0 + c);
+                    next = B.c[o + 1] - (int)w0;
+                    at = B.f[0][o].x + ((unsigned)((int)w0 - B.c[o]) + c) * r + dx;
+                    stop = B.f[0][o].y;
                 }
-                // Rows whose begins decrease are re-sorted on the fine level, so
-                // fine interval f may be wider than coarse interval i; the
-                // reference then reads past i, and past the array at its end.
-                // Here reads stay inside the array (0 beyond it).
-                const int cb = s_c[it.o[q]];
-                if (t0 + r < fw && it.c[q] + 1 == s_c[it.o[q] + 1]) {
-                    for (long long t = t0 + r; t < fw; ++t) {
-                        const long long src = cb + t / r;
-                        fv[fs + t] = src < ncells ? cv[src] : (T)0;
+                if (at < stop) fv[at] = cell[c];
+                at += 32u;
+                c += c32;
+                dx += dx32;
+                if (dx >= r) {
+                    dx -= r;
+                    ++c;
+                }
+            }
+        } else {
+            const SxFieldItems it = sx_field_items(B, nb, w0, hi);
+            T v[SX_FIELD_ITEMS];
+#pragma unroll
+            for (int q = 0; q < SX_FIELD_ITEMS; ++q) v[q] = it.k[q] >= 0 ? cv[it.c[q]] : (T)0;
+#pragma unroll
+            for (int d = 0; d < RT; ++d) {
+#pragma unroll
+                for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                    if (it.k[q] < 0) continue;
+                    const int2 fine = B.f[d][it.o[q]];
+                    const unsigned at = fine.x + (unsigned)it.k[q] * RT, stop = fine.y;  // both below 2^32
+                    if (RT == 2 && pair && !(at & 1u) && at + 2 <= stop) {
+                        P2 w;
+                        w.x = v[q];
+                        w.y = v[q];
+                        *(P2*)(fv + at) = w;
+                    } else {
+#pragma unroll
+                        for (int t = 0; t < RT; ++t)
+                            if (at + t < stop) fv[at + t] = v[q];
                     }
+                    if (at + RT < stop && it.c[q] + 1 == (unsigned)B.c[it.o[q] + 1]) beyond(B.c[it.o[q]], B.c[it.o[q] + 1], fine);
                 }
             }
         }
-    });
+    }, beyond);
 }
 
 // ---------------------------------------------------------------------------
@@ -303,16 +439,16 @@ __global__ void sx_restrict_check_kernel(const int* __restrict__ crows, int crow
 
 // RT as in sx_prolong_field_kernel.
 template <typename T, int RT>
-__global__ void __launch_bounds__(SX_FIELD_THREADS)
-    sx_restrict_field_kernel(const int* __restrict__ coff_rows, const int* __restrict__ ccoff,
+__global__ void __launch_bounds__(SX_FIELD_THREADS, sx_restrict_blocks<T, RT>)
+    sx_restrict_field_kernel(const int* __restrict__ coff_rows, int rows, const int* __restrict__ ccoff,
                              const int* __restrict__ foff_rows, const int* __restrict__ fcoff, int rr, int reducer,
                              T norm, const T* __restrict__ fv, T* __restrict__ cv, int pair)
 {
     typedef typename SxPair<T>::type P2;
     const int r = RT > 0 ? RT : rr;
-    const int p = blockIdx.x;
-    sx_field_cells<RT>(coff_rows, ccoff, foff_rows, fcoff, p, [&](const SxFieldItems& it, int first, const int*,
-                                                                  const int* s_f) {
+    sx_field_cells<RT, false>(coff_rows, rows, ccoff, foff_rows, fcoff, r, [&](long long w0, long long hi, int nb,
+                                                                                   const SxFieldBatch<RT>& B, int) {
+        const SxFieldItems it = sx_field_items(B, nb, w0, hi);
         T acc[SX_FIELD_ITEMS], best[SX_FIELD_ITEMS];
         bool have[SX_FIELD_ITEMS];
 #pragma unroll
@@ -335,10 +471,10 @@ __global__ void __launch_bounds__(SX_FIELD_THREADS)
             for (int dy = 0; dy < 2; ++dy)
 #pragma unroll
                 for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
-                    const int* fst = s_f + dy * (SX_FIELD_BATCH + 1) + it.o[q];
                     got[dy][q] = 0;
                     if (it.k[q] < 0) continue;
-                    const long long start = fst[0] + 2ll * it.k[q], fend = fst[1];
+                    const int2 fine = B.f[RT > 0 ? dy % RT : 0][it.o[q]];
+                    const long long start = fine.x + 2ll * it.k[q], fend = fine.y;
                     got[dy][q] = start + 2 <= fend ? 2 : start < fend ? 1 : 0;
                     if (got[dy][q] == 2 && pair && !(start & 1)) {
                         v[dy][q] = *(const P2*)(fv + start);
@@ -354,14 +490,27 @@ __global__ void __launch_bounds__(SX_FIELD_THREADS)
                     if (got[dy][q] > 0) add(q, v[dy][q].x);
                     if (got[dy][q] > 1) add(q, v[dy][q].y);
                 }
-        } else {
-            for (int dy = 0; dy < r; ++dy) {
-                const int* fst = RT > 0 ? s_f + dy * (SX_FIELD_BATCH + 1) : fcoff + foff_rows[p * r + dy] + first;
+        } else if (RT > 0) {
+#pragma unroll
+            for (int dy = 0; dy < RT; ++dy)
 #pragma unroll
                 for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
                     if (it.k[q] < 0) continue;
-                    const long long start = fst[it.o[q]] + (long long)it.k[q] * r, fend = fst[it.o[q] + 1];
-#pragma unroll(RT > 0 ? RT : 1)
+                    const int2 fine = B.f[RT > 0 ? dy : 0][it.o[q]];
+                    const long long start = fine.x + (long long)it.k[q] * r, fend = fine.y;
+#pragma unroll
+                    for (int dx = 0; dx < RT; ++dx)
+                        if (start + dx < fend) add(q, fv[start + dx]);
+                }
+        } else {
+            // cell after cell: the lines of a warp's blocks stay in L1 until they are summed
+#pragma unroll
+            for (int q = 0; q < SX_FIELD_ITEMS; ++q) {
+                if (it.k[q] < 0) continue;
+                for (int dy = 0; dy < r; ++dy) {
+                    const int2 fine = sx_fine_interval(B.at[RT > 0 ? 0 : it.o[q]], dy, foff_rows, fcoff, r);
+                    const long long start = fine.x + (long long)it.k[q] * r, fend = fine.y;
+#pragma unroll 4
                     for (int dx = 0; dx < r; ++dx)
                         if (start + dx < fend) add(q, fv[start + dx]);
                 }
@@ -370,7 +519,7 @@ __global__ void __launch_bounds__(SX_FIELD_THREADS)
 #pragma unroll
         for (int q = 0; q < SX_FIELD_ITEMS; ++q)
             if (it.k[q] >= 0) cv[it.c[q]] = reducer == 0 ? sx_mul(acc[q], norm) : reducer == 1 ? acc[q] : best[q];
-    });
+    }, [](int, int, int2) {});
 }
 
 // ---------------------------------------------------------------------------
@@ -1618,13 +1767,15 @@ template <typename T>
 static void sx_prolong_field_go(const int* off, int rows, const int* coff, int n, const int* foff_rows,
                                 const int* fcoff, int r, const T* cv, T* fv, cudaStream_t stream)
 {
-    const dim3 grid(rows, sx_field_split(rows));
+    const int subs = r >= 2 && r <= 4 ? 1 : r < SX_FIELD_ROW_BLOCKS ? r : SX_FIELD_ROW_BLOCKS;
+    dim3 grid = sx_field_grid(rows);
+    grid.z = subs;
     const int pair = sx_pairs_aligned<T>(fv);
     auto kernel = r == 2   ? sx_prolong_field_kernel<T, 2>
                   : r == 3 ? sx_prolong_field_kernel<T, 3>
                   : r == 4 ? sx_prolong_field_kernel<T, 4>
                            : sx_prolong_field_kernel<T, 0>;
-    kernel<<<grid, SX_FIELD_THREADS, 0, stream>>>(off, coff, n, foff_rows, fcoff, r, cv, fv, pair);
+    kernel<<<grid, SX_FIELD_THREADS, 0, stream>>>(off, rows, coff, n, foff_rows, fcoff, r, cv, fv, pair);
 }
 
 cudaError_t sx_prolong_field_launch(const int* off, int rows, const int* coff, int n, const int* foff_rows,
@@ -1652,13 +1803,13 @@ template <typename T>
 static void sx_restrict_field_go(const int* coff_rows, int rows, const int* ccoff, const int* foff_rows,
                                  const int* fcoff, int r, int reducer, T norm, const T* fv, T* cv, cudaStream_t stream)
 {
-    const dim3 grid(rows, sx_field_split(rows));
+    const dim3 grid = sx_field_grid(rows);
     const int pair = sx_pairs_aligned<T>(fv);
     auto kernel = r == 2   ? sx_restrict_field_kernel<T, 2>
                   : r == 3 ? sx_restrict_field_kernel<T, 3>
                   : r == 4 ? sx_restrict_field_kernel<T, 4>
                            : sx_restrict_field_kernel<T, 0>;
-    kernel<<<grid, SX_FIELD_THREADS, 0, stream>>>(coff_rows, ccoff, foff_rows, fcoff, r, reducer, norm, fv, cv, pair);
+    kernel<<<grid, SX_FIELD_THREADS, 0, stream>>>(coff_rows, rows, ccoff, foff_rows, fcoff, r, reducer, norm, fv, cv, pair);
 }
 
 cudaError_t sx_restrict_field_launch(const int* coff_rows, int crow_count, const int* ccoff, int cn,
