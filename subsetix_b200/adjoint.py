@@ -15,11 +15,11 @@ states per level instead of ``steps``.
 takes its coarse parents' values (injection), every level is advanced on its
 cells plus that ring, and after the step the coarse cells under a finer level
 take the mean of their children (restriction, finest level first).  Each
-coupling is a gather over an index table or a block mean over runs of cells,
-built once for the fixed geometry (``sx_index_copy``, ``sx_run_block_mean``);
-the backward pass applies their transposes (``sx_index_segment_add``,
-``sx_run_block_mean_adj``) around the adjoint upwind kernel, in reverse
-order.
+coupling is a gather over an index table or a block mean over runs of cells
+(over a table of cells where runs are short), built once for the fixed geometry
+(``sx_index_copy``, ``sx_run_block_mean``, ``sx_index_block_mean``); the backward
+pass applies their transposes (``sx_index_segment_add``, ``sx_run_block_mean_adj``,
+``sx_index_block_mean_adj``) around the adjoint upwind kernel, in reverse order.
 
 There is no counterpart in the reference, which has no derivatives.
 """
@@ -35,6 +35,13 @@ import torch
 from . import _core, _lib
 from ._runtime import ptr, stream_handle
 from .subsetix_cupy.expressions import IntervalSet, _t
+
+# Block means go by runs of cells from this mean length on, else cell by cell: 1.18 M coarse
+# cells in runs of 8, float32, 12.4 us by runs and 8.3 by cells (transposes 18.8 and 14.5), in
+# runs of 16 7.1 and 8.3 (10.2 and 12.4), in runs of 2 44 and 8.3 (75 and 16.5).  Few runs are
+# quick at any length (20,000 of one cell 3.1 us, by cells 4.2).
+_RUN_CELLS = 12
+_FEW_RUNS = 30000
 
 _ROWS_UNSAFE = _lib.ROWS_UNSORTED_BEGIN | _lib.ROWS_OVERLAP | _lib.ROWS_EMPTY
 
@@ -340,7 +347,11 @@ class Hierarchy:
             child = _positions(s, s_off, chy, chx)
             if bool((cpos < 0).any()) or bool((child < 0).any()):
                 raise ValueError(f"level {k}: a coarse cell under it does not have all its children in it")
-            self.cover.append(self._cover_runs(covered, prev, lvl, r))
+            runs = self._cover_runs(covered, prev, lvl, r)
+            if runs[0] > _FEW_RUNS and int(cpos.numel()) < _RUN_CELLS * runs[0]:
+                runs = None
+            cells = (cpos.contiguous(), inner[child.to(torch.int64)].contiguous()) if runs is None else None
+            self.cover.append((runs, cells))
 
     @staticmethod
     def _cover_runs(covered: IntervalSet, prev: Level, lvl: Level, r: int) -> tuple:
@@ -372,9 +383,14 @@ class Hierarchy:
         lib = _lib.load()
         r = self.ratio
         for k in range(len(self.levels) - 1, 0, -1):
-            runs, stride, plan = self.cover[k]
-            _lib.check(lib.sx_run_block_mean(_code(u[k]), runs, r, stride, 1.0 / (r * r), ptr(plan), ptr(u[k]),
-                                             ptr(u[k - 1]), stream_handle(u[k].device)), "sx_run_block_mean")
+            runs, cells = self.cover[k]
+            code, st = _code(u[k]), stream_handle(u[k].device)
+            if runs is not None:
+                _lib.check(lib.sx_run_block_mean(code, runs[0], r, runs[1], 1.0 / (r * r), ptr(runs[2]), ptr(u[k]),
+                                                 ptr(u[k - 1]), st), "sx_run_block_mean")
+            else:
+                _lib.check(lib.sx_index_block_mean(code, int(cells[0].numel()), r * r, 1.0 / (r * r), ptr(cells[0]),
+                                                   ptr(cells[1]), ptr(u[k]), ptr(u[k - 1]), st), "sx_index_block_mean")
 
     def step(self, u: List[torch.Tensor], a: float, b: float, dt: float, out: Optional[List[torch.Tensor]] = None
              ) -> Tuple[List[torch.Tensor], List[torch.Tensor]]:
@@ -400,9 +416,15 @@ class Hierarchy:
         lib = _lib.load()
         r = self.ratio
         for k in range(1, len(self.levels)):
-            runs, stride, plan = self.cover[k]
-            _lib.check(lib.sx_run_block_mean_adj(_code(w[k]), runs, r, stride, 1.0 / (r * r), ptr(plan), ptr(w[k - 1]),
-                                                 ptr(w[k]), stream_handle(w[k].device)), "sx_run_block_mean_adj")
+            runs, cells = self.cover[k]
+            code, st = _code(w[k]), stream_handle(w[k].device)
+            if runs is not None:
+                _lib.check(lib.sx_run_block_mean_adj(code, runs[0], r, runs[1], 1.0 / (r * r), ptr(runs[2]),
+                                                     ptr(w[k - 1]), ptr(w[k]), st), "sx_run_block_mean_adj")
+            else:
+                _lib.check(lib.sx_index_block_mean_adj(code, int(cells[0].numel()), r * r, 1.0 / (r * r),
+                                                       ptr(cells[0]), ptr(cells[1]), ptr(w[k - 1]), ptr(w[k]), st),
+                           "sx_index_block_mean_adj")
         outs = [None] * len(w) if out is None else out
         scratch = [None] * len(w) if scratch is None else scratch
         w = [lvl.adjoint(x, u, a, b, dt, grad_ab, y, z) for lvl, x, u, y, z in zip(self.levels, w, inputs, outs, scratch)]
