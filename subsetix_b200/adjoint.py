@@ -63,18 +63,19 @@ class Level:
         self.off = _t(s.row_offsets)
         self.begin = _t(s.begin)
         self.end = _t(s.end)
-        self.cell_off, self.cells = _core.cell_offsets(self.begin, self.end, device)
-        self.lookup, bad = _core.row_lookup(self.rows, self.height, device)
+        self.lookup, bad, flags, self.cell_off, self.cells, columns = _core.stencil_geometry(
+            self.rows, self.off, self.begin, self.end, self.height, device)
         if bad:
             raise ValueError("interval_set rows exceed provided height")
-        self.direct = not (_core.check_rows(self.begin, self.end, self.off, device) & _ROWS_UNSAFE)
+        self.direct = not flags & _ROWS_UNSAFE
         self.device = device
         self._chunk_off, self._chunks, self._table = None, 0, None
         self._chunked = False
-        self.flat = (_core.FlatPlan(self.rows, self.off, self.begin, self.end, self.cell_off, self.cells, self.lookup,
-                                    self.height, device) if self.direct else None)
-        if self.flat is not None and not self.flat.covers(self.width):
-            self.flat = None  # cells outside the domain: the chunk plan's kernels test every column
+        self.flat = None
+        if self.direct and self.cells > 0 and columns[0] >= 0 and columns[1] <= self.width:
+            self.flat = _core.FlatPlan(self.rows, self.off, self.begin, self.end, self.cell_off, self.cells, self.lookup,
+                                       self.height, device, columns)
+        elif self.direct:  # cells outside the domain: the chunk plan's kernels test every column
             self._chunk_plan()  # built here, so that steps can be captured
         lib = _lib.load()
         nbytes = max(int(lib.sx_upwind_adjoint_scratch_bytes(self.cells)),
