@@ -13,7 +13,7 @@
 // both passes on 4096^2, where one read of the field takes 10 us at the copy
 // rate.  The mask is 1/32 of the field and stays in L2.  A warp takes 128 columns
 // of RLE_ROWS rows, four cells per lane by 16-byte loads, all loaded before the
-// first is used.  Measured (B200, gradient tags on 4096^2): mask 29 us, count
+// first is used.  Measured (B200, gradient tags on 4096^2): mask 27 us, count
 // 7.9 us, runs 3 us; one kernel with the counts and the look-back inside the mask
 // pass took 36 us (blocks wait at its barriers and in its tail), 49 us with the
 // square root that sx_least_radicand removes.
@@ -28,6 +28,7 @@ namespace {
 constexpr int RLE_THREADS = 256;
 // Rows per warp: 2, 4 and 8 took 29, 26.6 and 30 us on 4096^2 (gradient tags).
 constexpr int RLE_ROWS = 4;
+constexpr int NARROW = 48;  // columns below which the gradient takes a cell per thread
 
 // Cells of one row in a warp's 128-column strip: lane's cells are x0 + 4 lane ..
 // + 3 with VEC (rows 16-byte aligned, width a multiple of 4), else x0 + lane +
@@ -226,6 +227,23 @@ __global__ void __launch_bounds__(RLE_THREADS)
     }
 }
 
+// The same for narrow grids, a cell per thread: strips leave most lanes of a warp
+// without a cell (200,000 rows, strips and this kernel: 3 columns 62 and 6.3 us, 16
+// columns 55 and 17, 32 columns 55 and 25; strips take 55 us for 64 columns too).
+__global__ void __launch_bounds__(RLE_THREADS)
+    narrow_gradient_kernel(const float* __restrict__ d, int W, int H, float* __restrict__ out)
+{
+    const long long cells = (long long)W * H, step = (long long)gridDim.x * RLE_THREADS;
+    for (long long i = (long long)blockIdx.x * RLE_THREADS + threadIdx.x; i < cells; i += step) {
+        const int y = (int)(i / W), x = (int)(i - (long long)y * W);
+        const float left = x > 0 ? d[i - 1] : 0.0f, right = x + 1 < W ? d[i + 1] : 0.0f;
+        const float up = y > 0 ? d[i - W] : 0.0f, down = y + 1 < H ? d[i + W] : 0.0f;
+        float gx, gy;
+        cell_gradient<false>(d[i], left, right, up, down, x, y, W, H, gx, gy);
+        out[i] = sx_grad_norm(gx, gy);
+    }
+}
+
 // Exclusive scan of the rows' run counts: a warp counts the run starts of a row,
 // a block of eight rows takes its place by a look-back.
 __global__ void __launch_bounds__(RLE_THREADS) mask_count_kernel(const unsigned* __restrict__ mask, int H,
@@ -362,6 +380,11 @@ cudaError_t sx_mask_launch(const float* d, int W, int H, float thr, int grad, un
 cudaError_t sx_gradient_launch(const float* d, int W, int H, float* out, cudaStream_t stream)
 {
     if (W <= 0 || H <= 0) return cudaSuccess;
+    if (W < NARROW) {
+        const long long need = ((long long)W * H + RLE_THREADS - 1) / RLE_THREADS;
+        narrow_gradient_kernel<<<(int)(need < 148 * 32 ? need : 148 * 32), RLE_THREADS, 0, stream>>>(d, W, H, out);
+        return cudaGetLastError();
+    }
     const int strips = (W + 127) / 128;
     const long long tasks = (long long)strips * (((long long)H + RLE_ROWS - 1) / RLE_ROWS);
     const int blocks = (int)((tasks + RLE_THREADS / 32 - 1) / (RLE_THREADS / 32));

@@ -26,10 +26,17 @@ def test_flat_plan_of_the_most_cells(cuda_device):
 def test_mask_of_the_most_rows(cuda_device):
     h = 2 ** 27 + 37  # 2^32 threads and more, one warp per row
     values = (torch.arange(h, device="cuda", dtype=torch.int32) % 3 == 1).to(torch.float32)
-    b, e, off = _core.threshold_rle(values, 1, h, 0.5, False, cuda_device)
+    lib, st = _lib.load(), stream_handle(cuda_device)
+    mask, off = (torch.empty(h + i, dtype=torch.int32, device="cuda") for i in (0, 1))
+    result = torch.empty(2, dtype=torch.int32, device="cuda")
+    ws = torch.empty(int(lib.sx_threshold_mask_workspace_bytes(h)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.sx_threshold_mask(ptr(values), 1, h, 0.5, 0, ptr(mask), ptr(off), ptr(result), ptr(ws),
+                                     int(ws.numel()), st), "sx_threshold_mask")
     counts = values.to(torch.int32)
     assert torch.equal(off[1:] - off[:-1], counts)
-    assert int(b.numel()) == int(off[-1]) and bool((b == 0).all()) and bool((e == 1).all())
+    b, e = (torch.full((int(off[-1]),), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    _lib.check(lib.sx_mask_runs(ptr(mask), 1, h, ptr(off), ptr(b), ptr(e), st), "sx_mask_runs")
+    assert result.tolist() == [int(off[-1]), 0] and bool((b == 0).all()) and bool((e == 1).all())
 
 
 def test_even_sweep_gives_up_on_tiles_of_2_31_intervals(cuda_device):
