@@ -348,29 +348,32 @@ class Hierarchy:
             child = _positions(s, s_off, chy, chx)
             if bool((cpos < 0).any()) or bool((child < 0).any()):
                 raise ValueError(f"level {k}: a coarse cell under it does not have all its children in it")
-            runs = self._cover_runs(covered, prev, lvl, r)
-            if runs[0] > _FEW_RUNS and int(cpos.numel()) < _RUN_CELLS * runs[0]:
-                runs = None
+            runs = None
+            if prev.direct:  # else neighbouring cells need not be neighbouring values
+                runs = self._cover_runs(covered, c_off, cpos, child, inner, r)
+                if runs[0] > _FEW_RUNS and int(cpos.numel()) < _RUN_CELLS * runs[0]:
+                    runs = None
             cells = (cpos.contiguous(), inner[child.to(torch.int64)].contiguous()) if runs is None else None
             self.cover.append((runs, cells))
 
     @staticmethod
-    def _cover_runs(covered: IntervalSet, prev: Level, lvl: Level, r: int) -> tuple:
-        """Plan of sx_run_block_mean: ``(runs, ints per run, plan)``, runs of up to 64 cells of one covered interval."""
-        b, e = _t(covered.begin).to(torch.int64), _t(covered.end).to(torch.int64)
-        y = _t(covered.interval_rows()).to(torch.int64)
-        per = (e - b + 63) // 64
-        which = torch.repeat_interleave(torch.arange(b.numel(), device=b.device), per)
-        nth = torch.arange(which.numel(), device=b.device) - (torch.cumsum(per, 0) - per)[which]
-        x, row = b[which] + 64 * nth, y[which]
-        stride = (2 + r + 3) // 4 * 4
-        plan = torch.zeros((which.numel(), stride), dtype=torch.int32, device=b.device)
-        plan[:, 0] = _positions(prev.interval_set, prev.cell_off, row.to(torch.int32), x.to(torch.int32))
-        plan[:, 1] = torch.clamp(e[which] - x, max=64)
-        for dy in range(r):
-            plan[:, 2 + dy] = _positions(lvl.interval_set, lvl.cell_off, (row * r + dy).to(torch.int32),
-                                         (x * r).to(torch.int32))
-        return int(plan.shape[0]), stride, plan
+    def _cover_runs(covered: IntervalSet, c_off, cpos, child, inner, r: int) -> tuple:
+        """Plan of sx_run_block_mean: ``(runs, ints per run, plan)``, runs of up to 64 cells of one covered interval.
+
+        ``cpos`` and ``child`` are the covered cells' values and their
+        children's in the finer set (``inner``: in the finer level).
+        """
+        size = (c_off[1:] - c_off[:-1]).to(torch.int64)
+        per = (size + 63) // 64
+        which = torch.repeat_interleave(torch.arange(size.numel(), device=size.device), per)
+        nth = torch.arange(which.numel(), device=size.device) - (torch.cumsum(per, 0) - per)[which]
+        cell = c_off[:-1].to(torch.int64)[which] + 64 * nth
+        plan = torch.zeros((which.numel(), (2 + r + 3) // 4 * 4), dtype=torch.int32, device=size.device)
+        plan[:, 0] = cpos[cell]
+        plan[:, 1] = torch.clamp(size[which] - 64 * nth, max=64)
+        rows = torch.arange(r, device=size.device) * r  # a sub-row's first child among a cell's
+        plan[:, 2:2 + r] = inner[child[cell[:, None] * (r * r) + rows].to(torch.int64)]
+        return int(plan.shape[0]), int(plan.shape[1]), plan
 
     # -- the coupled step and its transpose ------------------------------------------------------------------------
     def _fill_ghosts(self, u: List[torch.Tensor]) -> None:

@@ -1,4 +1,4 @@
-"""Composite levels whose covered cells lie in short runs: block means by runs and by cells give the same passes."""
+"""Composite levels whose covered cells lie in short runs, or not in runs at all: block means by runs and by cells agree."""
 
 import numpy as np
 import pytest
@@ -6,6 +6,7 @@ import torch
 
 from subsetix_b200 import adjoint
 from subsetix_b200.subsetix_cupy import full_interval_set
+from subsetix_b200.subsetix_cupy.expressions import IntervalSet
 from tests.gpu_util import dev_set
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +40,21 @@ def test_both_forms_agree(cuda_device, monkeypatch, size, apart):
     assert (H.cover[1][0] is None) == (size < 12)
     for x, y in zip(_run(by_runs), _run(H)):
         assert torch.equal(x, y)
+
+
+def test_overlapping_rows_of_the_coarse_level(cuda_device):
+    """A coarse row as [0, 14) and [10, 24): cells side by side whose values lie apart."""
+    n = 24
+    b = np.tile(np.array([0, 10], np.int32), n)
+    coarse = IntervalSet(*(torch.as_tensor(np.asarray(a, np.int32), device="cuda") for a in
+                           (b, b + 14, 2 * np.arange(n + 1), np.arange(n))))
+    H = adjoint.Hierarchy([coarse, dev_set(_patches(n, 15, 40))], n, n)  # one patch, cells 2 to 16
+    u = H.extend([torch.rand(28 * n, dtype=torch.float64, device="cuda"),
+                  torch.rand(30 * 30, dtype=torch.float64, device="cuda")])
+    want, inner = u[0].clone(), H.interior(u)[1]
+    y, x = (t.reshape(-1).to(torch.int32) for t in torch.meshgrid(*2 * [torch.arange(2, 17, device="cuda")], indexing="ij"))
+    at = adjoint._positions(coarse, H.levels[0].cell_off, y, x).long()
+    block = inner.view(15, 2, 15, 2)
+    want[at] = ((block[:, 0, :, 0] + block[:, 0, :, 1] + block[:, 1, :, 0] + block[:, 1, :, 1]) * 0.25).reshape(-1)
+    H._restrict(u)
+    assert torch.equal(u[0], want)
