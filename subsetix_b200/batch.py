@@ -129,15 +129,14 @@ class SetBatch:
             s = self.combined
             dev = _t(s.row_offsets).device
             b, e, off, rows = _t(s.begin), _t(s.end), _t(s.row_offsets), _t(s.rows)
-            cell_off, cells = _core.cell_offsets(b, e, dev)
             H = self.total_rows
-            lookup, bad = _core.row_lookup(rows, H, dev)
+            lookup, bad, flags, cell_off, cells, columns = _core.stencil_geometry(rows, off, b, e, H, dev)
             if bad:
                 raise ValueError("batch rows outside the band layout")
-            direct = not (_core.check_rows(b, e, off, dev) & _ROWS_UNSAFE)
+            direct = not flags & _ROWS_UNSAFE
             flat, band_cell = None, None
             if direct and self.bases:
-                flat = _core.FlatPlan(rows, off, b, e, cell_off, cells, lookup, H, dev)
+                flat = _core.FlatPlan(rows, off, b, e, cell_off, cells, lookup, H, dev, columns)
                 # first value of the rows from each band's base on, and of the rows after its last one
                 edges = torch.tensor(self.bases + [x + h for x, h in zip(self.bases, self.heights)], dtype=I32,
                                      device=dev)
