@@ -177,12 +177,14 @@ def traffic_per_launch(copies: int, kernel: str):
     """DRAM bytes of one fused launch from the committed ncu summary of that kernel, scaled by the copy count.
 
     Returns ``(bytes, source)``; the summary records the copy count of its
-    capture and the bytes per copy (traffic grows with the copies).
+    capture and the bytes per copy (traffic grows with the copies).  A summary
+    whose title names another instance of the kernel does not count.
     """
     path = os.path.join(REPO, "profiles", kernel.split("<")[0] + "_shapes4096.md")
     per_copy = captured = None
     try:
-        for line in open(path):
+        lines = open(path).read().splitlines()
+        for line in lines if lines and kernel in lines[0] else []:
             if line.startswith("traffic_bytes_per_copy:"):
                 per_copy = float(line.split(":")[1])
             elif line.startswith("traffic_capture_copies:"):

@@ -533,7 +533,8 @@ int sx_upwind_flat_adjoint(int dtype, const sx_flat_plan* plan, const void* grad
  * (exclusive scan of counts), out_begin/out_end written. */
 int sx_threshold_rle(const float* values, int32_t width, int32_t height, float threshold, int gradient, int32_t* counts,
                      const int32_t* offsets, int32_t* out_begin, int32_t* out_end, void* stream);
-/* The same in one pass over the values: sx_threshold_mask writes one bit per
+/* The same in one pass over the values, for all but tall, narrow grids, where
+ * sx_threshold_rle is the faster way: sx_threshold_mask writes one bit per
  * cell, mask[height][ceil(width / 32)], offsets[height + 1] (exclusive scan of
  * the rows' run counts) and result = {runs, flags}; sx_mask_runs then stores
  * the runs.  workspace: sx_threshold_mask_workspace_bytes(height). */
@@ -605,7 +606,8 @@ int sx_cell_quads(int dtype, const int32_t* row_offsets, const int32_t* rows, in
  *                            = 0; in_idx entries must be distinct;
  *   sx_run_block_mean{,_adj} the same on runs of consecutive coarse cells (the
  *                            children of consecutive cells are consecutive in
- *                            each of the `ratio` sub-rows).  plan: `stride`
+ *                            each of the `ratio` sub-rows); the tables are
+ *                            the faster way for runs of under 12 cells.  plan: `stride`
  *                            ints per run (a multiple of 4, >= 2 + ratio):
  *                            first coarse value, cells (1 to 64), first child
  *                            of each sub-row;

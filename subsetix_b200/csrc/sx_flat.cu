@@ -28,7 +28,7 @@
 // the domain (span_kernel checks it when the plan is built) no test is left:
 // a neighbour in the set is a neighbour in the domain.  Geometry with cells
 // outside the domain keeps the chunk kernel.  Measured (B200): one float64 step
-// on 2500^2 26.1 -> 15.1 us (12.3 with over_group), the uneven batch 1337 -> 626 us (327 M cells; its
+// on 2500^2 26.1 -> 15.1 us (12.3 with over_group), the uneven batch 1337 -> 644 us (327 M cells; its
 // 9.5 bytes a cell take 475 us at the copy rate), the three-level composite's
 // 300 level steps 5.1 -> 2.8 ms and its 150 transposed ones, sums over blocks
 // included, 5.2 -> 3.2 ms.  Same values as sx_upwind, bit for bit; the adjoint's
