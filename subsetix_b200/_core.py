@@ -188,13 +188,13 @@ def _uneven_tuning(leaves, rows: int, device, even: dict, most8: int, most32: in
     The choice is that of :func:`auto_tuning`: kernel 5 for even rows too
     wide for 16 bits, its buffers for the largest 8 rows; kernel 4 for
     skewed ones, its buffers for the largest 32 rows, those around a tile
-    that gave up or two tiles that fitted.  Even, narrow rows that no slice
+    that gave up or tiles that fitted.  Even, narrow rows that no slice
     holds are long; measuring them costs little beside their sweep.
     """
     mean8 = 2 * sum(int(leaf[0].numel()) for leaf in leaves) / max(1, (rows + 7) // 8)
     if 2 * most8 > 3 * mean8 + 256:
-        return {"kernel": 4, "staging_cap": min(max(2 * most32, 2 * even["staging_cap"]), 25000), "tile_rows": 32,
-                "warps": 4}
+        fitted = 32 // even["tile_rows"] * even["staging_cap"]
+        return {"kernel": 4, "staging_cap": min(max(2 * most32, fitted), 25000), "tile_rows": 32, "warps": 4}
     if wide:
         return {"kernel": 5, "staging_cap": min(2 * most8, 25000), "tile_rows": 8, "warps": 2}
     return auto_tuning(leaves, rows, device)
